@@ -16,6 +16,7 @@ from __future__ import annotations
 
 import inspect
 import uuid
+import weakref
 from typing import Callable, Dict, Tuple
 
 import torch as th
@@ -47,11 +48,19 @@ class jit:
         self._compiled: Dict[Tuple, tuple] = {}     # signature -> (forward, backward, fw_meta, bw_meta)
         self._metas: Dict[Tuple, tuple] = {}        # signature -> (fw_meta, bw_meta)
         self.forward_func = self.backward_func = None
-        self.apply = self._register_ops()
+        self.apply = self._op_apply = self._register_ops()
+        self._host_op = None                        # native host path, made on the first eager call on a CUDA device
 
     # ------------------------------------------------------------------ public
     def __call__(self, *args):
-        return self.apply(*args)
+        # under torch.compile (and with .apply replaced) the custom op; else the native path, which declines whatever
+        # it does not serve: other devices, fake tensors, functorch, dispatch modes, subclasses
+        if th.compiler.is_compiling() or self.apply is not self._op_apply or not args or not args[0].is_cuda:
+            return self.apply(*args)
+        if self._host_op is None:
+            self._host_op = self._make_host_op()
+        out = self._host_op.call(args)
+        return self.apply(*args) if out is None else out
 
     def naive(self, *args, dtype=th.float32):
         """Plain PyTorch loop over time; defines what the compiled op computes
@@ -83,6 +92,44 @@ class jit:
         fwd, bwd, fw_meta, bw_meta = self._compiled[key]
         self.forward_func, self.backward_func, self.fw_meta, self.bw_meta = fwd, bwd, fw_meta, bw_meta
         return self._compiled[key]
+
+    def _make_host_op(self):
+        from . import runtime
+        me = weakref.ref(self)          # the native object must not keep this one alive
+        return runtime.host().HostOp(self.ninputs + self.nstates, lambda args: me()._host_spec(args))
+
+    def _host_spec(self, args):
+        """The native path's record of this call's specialisation, or None where the custom op has to serve (a
+        debugging mode is on).  Its Python closures run until the kernels they compile can be handed over."""
+        from . import runtime
+        from .twopass import device_status
+        nin, nst, nout = self.ninputs, self.nstates, self.noutputs
+        inputs, state = split_list(args, [nin, nst])
+        fwd, bwd = self._specialise(inputs, state)[:2]
+        if not hasattr(fwd, "host_program"):        # padded or empty problems are served by their closures alone
+            return None
+        aligned, reach = fwd.host_checks()
+
+        def run(which, fn):
+            def call(spec, *a):
+                res = fn(*a)
+                prog = None if spec.has(which) else fwd.host_program(which)
+                if prog is not None:
+                    spec.set(which, prog)
+                return res
+            return call
+
+        bw_op = self._bw_op
+
+        def backward(up, args_, saved):
+            if th.is_grad_enabled():                # create_graph=True
+                return bw_op(*up, *args_, *saved)
+            dx, ds0 = bwd(up[:nout], up[nout:], args_[:nin], saved[:nst], saved[nst:])
+            return (*dx, *ds0)
+
+        return runtime.host().Spec(nin, nst, nout, args[0].device.index, device_status(args[0].device).word.data_ptr(),
+                                   aligned, reach, run("forward", lambda a: fwd(a[:nin], a[nin:])),
+                                   run("infer", lambda a: fwd.infer(a[:nin], a[nin:])), run("backward", backward))
 
     def _dry_metas(self, inputs, state):
         key = _signature(tuple(inputs) + tuple(state))

@@ -1165,12 +1165,13 @@ def _stage_inputs(kb: KernelBuilder, p: Problem, used: Sequence[bool], allow_mn:
 def emit_forward(p: Problem, g: StepGraph, aux_names: List[str], n_out: int, tile: Tile,
                  dstage: int, dck: int, use_tma: bool, min_blocks: int, prelude: str,
                  kname: str = "frnn_fw", final_ckpt: bool = False, step_unroll: int = 2, pack2: bool = False,
-                 col_major: bool = False, max_acc: int = 2) -> KernelSource:
+                 col_major: bool = False, max_acc: int = 2, infer: bool = False) -> KernelSource:
     """Forward scan.  ``g`` computes [*outputs, *new_states, *aux] from
     [*inputs, *states].  Kernel parameters, in order: used inputs, initial
     states, outputs, final states, checkpoints, aux, error word.  With
     ``final_ckpt`` one more fp32 checkpoint (the final state) is stored at
-    index ceil(T/dck)."""
+    index ceil(T/dck).  With ``infer`` there is no backward pass to come: no
+    checkpoints, no aux, and no such parameters."""
     kb = KernelBuilder(p, tile, dstage, use_tma)
     w, t = kb.w, tile
     ns = len(p.states)
@@ -1187,9 +1188,10 @@ def emit_forward(p: Problem, g: StepGraph, aux_names: List[str], n_out: int, til
         kb.add_param(f"out{j}", "void", False, p.B * p.T * p.H * p.M * ELT[p.out_dt[j]])
     for k in range(ns):
         kb.add_param(f"sT_{k}", "void", False, _spec_bytes(p.states[k]))
-    for k in range(ns):
-        kb.add_param(f"ck{k}", "float", False, ck_bytes)
-    kb.add_param("aux", "float", False, len(aux_names) * p.B * p.H * p.T * p.M * 4)
+    if not infer:
+        for k in range(ns):
+            kb.add_param(f"ck{k}", "float", False, ck_bytes)
+        kb.add_param("aux", "float", False, len(aux_names) * p.B * p.H * p.T * p.M * 4)
     kb.add_param("err", "int", False, 4)
 
     const_inputs = _stage_inputs(kb, p, used, allow_mn=True)
@@ -1262,14 +1264,15 @@ def emit_forward(p: Problem, g: StepGraph, aux_names: List[str], n_out: int, til
         w.open(f"if (warp == 0 && c + 1 < {nchunk})")
         w(f"fw_issue(sp, &full[0], t0 + {dstage}, min({dstage}, {p.T} - t0 - {dstage}), lane, b, h, m0{tma_call});")
         w.close()
-    sub_len = math.gcd(dstage, dck)
+    sub_len = dstage if infer else math.gcd(dstage, dck)
     w("#pragma unroll 1")
     w.open(f"for (int tl0 = 0; tl0 < nv; tl0 += {sub_len})")
-    w.open(f"if ((t0 + tl0) % {dck} == 0)")
-    for k in range(ns):
-        base = _elem_off(ckspec, [(0, "b"), (1, "h"), (2, f"(t0 + tl0) / {dck}")])
-        kb.emit_tile_global(vname(p.st_names[k]), ckspec, f"ck{k}", base, 3, 4, load=False)
-    w.close()
+    if not infer:
+        w.open(f"if ((t0 + tl0) % {dck} == 0)")
+        for k in range(ns):
+            base = _elem_off(ckspec, [(0, "b"), (1, "h"), (2, f"(t0 + tl0) / {dck}")])
+            kb.emit_tile_global(vname(p.st_names[k]), ckspec, f"ck{k}", base, 3, 4, load=False)
+        w.close()
     w(f"const int tl1 = min(tl0 + {sub_len}, nv);")
     w(f"#pragma unroll {step_unroll}")
     w.open("for (int tl = tl0; tl < tl1; tl++)")
@@ -1324,7 +1327,7 @@ def emit_forward(p: Problem, g: StepGraph, aux_names: List[str], n_out: int, til
     for k in range(ns):
         kb.emit_tile_global(vname(p.st_names[k]), p.states[k], f"sT_{k}",
                             _elem_off(p.states[k], [(0, "b"), (1, "h")]), 2, 3, load=False)
-        if final_ckpt:
+        if final_ckpt and not infer:
             base = _elem_off(ckspec, [(0, "b"), (1, "h"), (2, str(nck))])
             kb.emit_tile_global(vname(p.st_names[k]), ckspec, f"ck{k}", base, 3, 4, load=False)
     w.close()

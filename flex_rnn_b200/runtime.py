@@ -69,6 +69,29 @@ def lib() -> ctypes.CDLL:
     return _lib
 
 
+_host = None
+
+
+def host():
+    """The native host path of a call (csrc/frnn_host.cpp), bound to the C-ABI library (built first if absent)."""
+    global _host
+    if _host is not None:
+        return _host
+    L = lib()
+    with _lock:
+        if _host is None:
+            import importlib.util
+            from . import build as _build
+            if not os.path.exists(_build.HOST_LIB):
+                _build.build_host()
+            spec = importlib.util.spec_from_file_location("_frnn_host", _build.HOST_LIB)
+            m = importlib.util.module_from_spec(spec)
+            spec.loader.exec_module(m)
+            m.bind(*[ctypes.cast(f, ctypes.c_void_p).value for f in (L.frnn_launch, L.frnn_tensor_map_encode, L.frnn_last_error)])
+            _host = m
+    return _host
+
+
 def _check(rc: int, what: str):
     if rc != 0:
         raise FrnnError(f"{what} failed (code {rc}): {lib().frnn_last_error().decode(errors='replace')}")

@@ -531,10 +531,12 @@ def make_plan(step: Callable, inputs: Sequence[th.Tensor], state: Sequence[th.Te
 
 
 def generate_forward(plan: Plan, tile: Optional[lower.Tile] = None, pack: Optional[bool] = None,
-                     stage: Optional[int] = None, unroll: Optional[int] = None) -> lower.KernelSource:
+                     stage: Optional[int] = None, unroll: Optional[int] = None, infer: bool = False) -> lower.KernelSource:
     """Emit the forward kernel.  The optional arguments replace the plan's
     choices: the tile, packed arithmetic on or off, timesteps staged per chunk
-    and the unroll factor of the step loop."""
+    and the unroll factor of the step loop.  ``infer``: the kernel of a call
+    without gradients, which saves nothing for a backward pass (a decode step
+    of a 128x128 fp32 state moves half the bytes)."""
     p, tu = plan.problem, plan.tuning
     pack2 = bool(tu.pack2 & 2) if pack is None else bool(pack)
     tile = tile or plan.fw_tile
@@ -548,10 +550,11 @@ def generate_forward(plan: Plan, tile: Optional[lower.Tile] = None, pack: Option
         while unroll > 1 and unroll * step_bytes > 40 * 1024:
             unroll //= 2
     while True:
-        fw = emit_forward(p, plan.g_fw, plan.aux, plan.n_out, tile, stage, plan.D, tu.use_tma,
+        g_fw, aux = (plan.g_fw, plan.aux) if not infer else (plan.g_fw.pruned(plan.g_fw.outputs[:plan.n_out + plan.n_st]), [])
+        fw = emit_forward(p, g_fw, aux, plan.n_out, tile, stage, plan.D, tu.use_tma,
                           tu.fw_min_blocks, prelude(), final_ckpt=plan.reverse is not None or plan.post_split,
                           step_unroll=unroll or tu.fw_unroll, pack2=pack2, col_major=bool(tu.col_major),
-                          max_acc=tu.fw_acc)
+                          max_acc=tu.fw_acc, infer=infer)
         ncta = fw.grid[0] * fw.grid[1] * fw.grid[2]
         # CTAs an SM will hold at once: as many as there are per SM, but no more than the register file admits
         # (the state tiles plus about 96 registers of vectors and addresses per thread, unless the launch bounds
@@ -891,6 +894,7 @@ def build_twopass(step, inputs, state, dryrun=False, tuning: Optional[Tuning] = 
     st_align = [x.data_ptr() % 16 == 0 for x in state]
     fw_used = plan.g_fw.used_inputs()
     bw_used = [a or b for a, b in zip(plan.g_re.used_inputs(), plan.g_bw.used_inputs())]
+    infer_used = plan.g_fw.pruned(plan.g_fw.outputs[:nout + nst]).used_inputs()[:nin]
     emulated = _launcher is not None
     emu_words: Dict[str, th.Tensor] = {}
 
@@ -948,7 +952,7 @@ def build_twopass(step, inputs, state, dryrun=False, tuning: Optional[Tuning] = 
     no_tune = (_launcher is not None or not plan.tuning.autotune
                or p.B * p.T * p.H * p.M * p.N < plan.tuning.autotune_min_work)
     tuned = {"fw": no_tune or forced_fw, "launch_fw": launch_fw, "fw_src": fw_src, "bw": no_tune or forced_bw,
-             "launch_bw": launch_bw, "bw_src": bw_src,
+             "launch_bw": launch_bw, "bw_src": bw_src, "infer": no_tune or forced_fw,
              "fw_choice": max(0, tu0.fw_variant), "bw_choice": max(0, tu0.bw_variant), "fw_log": [], "bw_log": []}
 
     def timed(launcher, ptrs, device, reps=5):
@@ -992,38 +996,59 @@ def build_twopass(step, inputs, state, dryrun=False, tuning: Optional[Tuning] = 
             tuned["bw_choice"], tuned["bw_log"] = best[3], log
             forward.sources = (tuned["fw_src"], best[2])       # type: ignore[attr-defined]
 
-    def autotune_forward(ptrs, device):
+    def autotune_forward(ptrs, device, infer=False):
         """Time the alternative forward kernels once on the real arguments (the
         forward kernel only writes its outputs) and keep the fastest."""
-        tuned["fw"] = True
+        first = infer_kernel() if infer else (fw_src, launch_fw)
         best, log = None, []
         for k, kw in enumerate(forward_variants(plan)):
             try:
-                ks = fw_src if k == 0 else generate_forward(plan, **kw)
-                launcher = launch_fw if k == 0 else make(ks)
+                ks = first[0] if k == 0 else generate_forward(plan, infer=infer, **kw)
+                launcher = first[1] if k == 0 else make(ks)
                 ms = timed(launcher, ptrs, device)
             except (lower.LoweringError, RuntimeError):
                 continue
             log.append((k, ks.info["tile"], bool(ks.info["packed"]), round(ms, 4)))
             if best is None or ms < best[0]:
                 best = (ms, launcher, ks, k)
+        if infer:
+            tuned["infer"] = True
+            if best is not None:
+                tuned["launch_infer"], tuned["infer_src"] = best[1], best[2]
+            return
+        tuned["fw"] = True
         if best is not None:
             tuned["launch_fw"], tuned["fw_src"] = best[1], best[2]
             tuned["fw_choice"], tuned["fw_log"] = best[3], log
             forward.sources = (best[2], tuned["bw_src"])       # type: ignore[attr-defined]
 
-    def forward(inputs_, state0):
+    def infer_kernel():
+        """(source, launcher) of the planned kernel for calls without gradients, made on first use."""
+        if "launch_infer" not in tuned:
+            kw = forward_variants(plan)[tu0.fw_variant] if tu0.fw_variant > 0 else {}
+            tuned["infer_src"] = generate_forward(plan, infer=True, **kw)
+            tuned["launch_infer"] = make(tuned["infer_src"])
+        return tuned["infer_src"], tuned["launch_infer"]
+
+    def check_args(inputs_, state0):
         verify_meta(inputs_, in_meta, "input Tensor metadata doesn't match compilation\n")
         verify_meta(state0, st_meta, "initial state Tensor metadata doesn't match compilation\n")
         check_align(inputs_, in_align, "input")
         check_align(state0, st_align, "initial state")
+
+    cont = lambda *shape: (shape, lower._contig(shape))
+
+    def alloc_results(state0, device):
+        outs = tuple(alloc(f"output #{j + 1}", *cont(p.B, p.T, p.H, p.M), o[2], device)
+                     for j, o in enumerate(fw_meta[:nout]))
+        return outs, tuple(alloc_like(f"final state #{k + 1}", s, device) for k, s in enumerate(state0))
+
+    def forward(inputs_, state0):
+        check_args(inputs_, state0)
         device = inputs_[0].device
         with _device_ctx(device):
             check_before(device)
-            cont = lambda *shape: (shape, lower._contig(shape))
-            outs = tuple(alloc(f"output #{j + 1}", *cont(p.B, p.T, p.H, p.M), o[2], device)
-                         for j, o in enumerate(fw_meta[:nout]))
-            stT = tuple(alloc_like(f"final state #{k + 1}", s, device) for k, s in enumerate(state0))
+            outs, stT = alloc_results(state0, device)
             store = tuple(alloc(f"checkpoints of state #{k + 1}", *cont(p.B, p.H, plan.nck, p.M, p.N), th.float32, device)
                           for k, _ in enumerate(state0))
             aux = alloc("saved row sums", *cont(len(plan.aux), p.B, p.H, p.T, p.M), th.float32, device)
@@ -1037,6 +1062,24 @@ def build_twopass(step, inputs, state, dryrun=False, tuning: Optional[Tuning] = 
             check_status(device, "forward")
             check_guard(device)
         return (*outs, *stT, *store, aux)
+
+    def infer(inputs_, state0):
+        """The forward pass of a call without gradients: outputs and final states, nothing saved."""
+        check_args(inputs_, state0)
+        device = inputs_[0].device
+        with _device_ctx(device):
+            check_before(device)
+            outs, stT = alloc_results(state0, device)
+            infer_kernel()
+            ptrs = [x.data_ptr() for x, u in zip(inputs_, infer_used) if u]
+            ptrs += [s.data_ptr() for s in state0] + [o.data_ptr() for o in outs] + [s.data_ptr() for s in stT]
+            ptrs.append(err_word(device).data_ptr())
+            if not tuned["infer"]:
+                autotune_forward(ptrs, device, infer=True)
+            tuned["launch_infer"](ptrs, device)
+            check_status(device, "forward")
+            check_guard(device)
+        return (*outs, *stT)
 
     def backward(doutput, dstateT, inputs_, state_store, aux_):
         doutput = tuple(d.contiguous() for d in doutput)
@@ -1080,7 +1123,55 @@ def build_twopass(step, inputs, state, dryrun=False, tuning: Optional[Tuning] = 
         th.cuda.synchronize(idx)
         return int(_status[idx].word.item())
 
+    def host_program(which: str) -> Optional[dict]:
+        """What the native host path needs to launch ``which`` ("forward", "infer" or "backward") without Python: the
+        buffers to allocate and the kernel's parameters as numbers of buffers (the call's tensors, then the allocated
+        ones, then the error word; backward: inputs, upstream gradients, saved tensors).  None before the first call
+        of that kind has compiled (and, for large problems, timed) the kernel, and for the debugging modes."""
+        if emulated or strict or guard is not None or not tuned[{"forward": "fw", "infer": "infer", "backward": "bw"}[which]]:
+            return None
+        launcher = tuned.get({"forward": "launch_fw", "infer": "launch_infer", "backward": "launch_bw"}[which])
+        idx = dev.index if dev.index is not None else th.cuda.current_device()
+        if not isinstance(launcher, _CudaLauncher) or idx not in launcher.mods:
+            return None
+        st = list(range(nin, nin + nst))
+        zeroed, cast_from = [], []
+        if which == "backward":
+            given = nin + nout + nst + nst + 1
+            metas = list(bw_meta)
+            where = list(range(given, given + nin + nst))          # gradients of inputs, of initial states
+            for i, go in enumerate(plan.grads):
+                if go.atomic:                                       # accumulated in fp32, then converted
+                    where[i] = given + len(metas)
+                    zeroed.append(len(metas))
+                    cast_from += [-1] * (i + 1 - len(cast_from))
+                    cast_from[i] = len(metas)
+                    metas.append((bw_meta[i][0], lower._contig(bw_meta[i][0]), th.float32))
+            params = [i for i in range(nin) if bw_used[i]] + list(range(nin, given)) + where[nin:] + where[:nin]
+            returned = nin + nst
+        else:
+            given = nin + nst
+            metas = list(fw_meta if which == "forward" else fw_meta[:nout + nst])
+            used = fw_used[:nin] if which == "forward" else infer_used
+            params = [i for i in range(nin) if used[i]] + st + list(range(given, given + len(metas)))
+            returned = len(metas)
+        params.append(given + len(metas))
+        ks = launcher.ks
+        assert len(params) + len(ks.tmaps) == len(ks.params)
+        kernel = {"module": launcher.mods[idx]._h.value, "grid": list(ks.grid), "block": ks.block, "smem": ks.smem_bytes,
+                  "params": params, "maps": ks.tmaps}
+        return {"kernels": [kernel], "zeroed": zeroed, "cast_from": cast_from, "returned": returned,
+                "alloc": [(tuple(s), tuple(t), d) for s, t, d in metas]}
+
+    def host_checks():
+        """(16-byte aligned at compilation, bytes from the first to the end of the last element) of every argument."""
+        reach = [lower._spec_bytes(s) for s in list(p.inputs) + list(p.states)]
+        return [bool(a) for a in in_align + st_align], reach
+
     forward.plan = plan                     # type: ignore[attr-defined]
+    forward.infer = infer                   # type: ignore[attr-defined]
+    forward.host_program = host_program     # type: ignore[attr-defined]
+    forward.host_checks = host_checks       # type: ignore[attr-defined]
     forward.sources = (fw_src, bw_src)      # type: ignore[attr-defined]
     forward.launchers = (launch_fw, launch_bw)   # type: ignore[attr-defined]
     forward.kernel_status = kernel_status   # type: ignore[attr-defined]

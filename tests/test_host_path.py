@@ -1,0 +1,85 @@
+"""The native host path of an eager call (csrc/frnn_host.cpp) and the kernels of calls without gradients: same
+results as the custom op, whatever the call looks like."""
+import pytest
+import torch
+
+import flex_rnn_b200
+from flex_rnn_b200 import examples as X
+from flex_rnn_b200 import workloads as W
+from flex_rnn_b200.twopass import Tuning, build_twopass
+
+
+@pytest.mark.parametrize("op", ["delta_rule", "mamba2", "gla"])
+@pytest.mark.parametrize("T", [1, 7, 19])
+def test_emulated_forward_without_gradients(op, T):
+    """The kernel that saves nothing gives the outputs and final states of the one that does."""
+    from emu.emu import EmuLauncher
+    if op in W.STEPS:
+        *ins, s0 = W.synthetic(op, 1, T, 2, 16, 16, torch.float32)[0]
+        ins, sts, step = ins, [s0], W.STEPS[op]
+    else:
+        (ins, sts), step = X.zoo_case(op, 1, T, 2, 16, 16), X.ZOO[op]
+    tu = Tuning(fw_r=2, fw_c=4, fw_mb=16, fw_stage=min(4, T), bw_r=2, bw_c=4, seg=min(2, T), nslots=2 if T > 3 else 1)
+    fwd, _, _, _ = build_twopass(step, tuple(ins), tuple(sts), tuning=tu, _launcher=EmuLauncher)
+    full, short = fwd(tuple(ins), tuple(sts)), fwd.infer(tuple(ins), tuple(sts))
+    assert len(short) == 2 and all(torch.equal(a, b) for a, b in zip(short, full))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("op,B,T,M,N,dt", [("delta_rule", 2, 33, 64, 64, torch.float32), ("mamba2", 2, 17, 32, 64, torch.bfloat16),
+                                           ("gated_delta_rule", 3, 1, 64, 128, torch.bfloat16), ("rwkv7", 1, 40, 24, 40, torch.float16)])
+def test_native_path_equals_custom_op(op, B, T, M, N, dt):
+    xs, dy, dS = W.synthetic(op, B, T, 2, M, N, dt, device="cuda")
+    f = flex_rnn_b200.jit(W.STEPS[op])
+    leaves = [x.detach().requires_grad_() for x in xs]
+
+    def both(call):
+        y, S = call(*leaves)
+        return [y, S, *torch.autograd.grad((y, S), leaves, (dy, dS))]
+    want = both(f.apply)
+    for _ in range(3):              # the first call of a kind runs through the Python closures, later ones do not
+        for a, b in zip(both(f), want):
+            assert a.shape == b.shape and a.dtype == b.dtype and a.stride() == b.stride()
+            assert torch.equal(a, b) or float((a.float() - b.float()).norm()) <= 1e-5 * float(b.float().norm())   # atomics
+    for _ in range(3):
+        with torch.no_grad():
+            assert all(torch.equal(a, b) for a, b in zip(f(*xs), want))
+    # an output left out of the loss, an input that needs no gradient, and a change of layout
+    y, S = f(leaves[0].detach(), *leaves[1:])
+    (g,) = torch.autograd.grad(y, [leaves[1]], dy.transpose(0, 1).contiguous().transpose(0, 1))
+    y2, S2 = f.apply(*leaves)
+    (g2,) = torch.autograd.grad(y2, [leaves[1]], dy)
+    assert torch.equal(g, g2)
+    strided = [torch.stack([x, x], -1)[..., 0].detach().requires_grad_() for x in xs]
+    assert all(torch.equal(a, b) for a, b in zip(f(*strided), f.apply(*strided)))
+
+
+@pytest.mark.gpu
+def test_native_path_graph_semantics():
+    """Second use of a freed graph raises, create_graph gives the custom op's graph, other streams and a changed
+    input are honoured."""
+    xs, dy, dS = W.synthetic("delta_rule", 1, 20, 2, 64, 64, torch.float32, device="cuda")
+    f = flex_rnn_b200.jit(W.delta_rule)
+    leaves = [x.detach().requires_grad_() for x in xs]
+    y, S = f(*leaves)
+    first = torch.autograd.grad(y, leaves, dy, retain_graph=True)
+    again = torch.autograd.grad(y, leaves, dy)
+    assert all(torch.equal(a, b) for a, b in zip(first, again))
+    with pytest.raises(RuntimeError, match="second time"):
+        torch.autograd.grad(y, leaves, dy)
+    y, S = f(*leaves)
+    g = torch.autograd.grad(y, leaves, dy, create_graph=True)
+    assert torch.equal(g[0], first[0])
+    with pytest.raises(RuntimeError, match="autograd"):
+        torch.autograd.grad(g[0].sum(), leaves)
+    y, S = f(*leaves)
+    with torch.no_grad():
+        leaves[0].add_(1.0)
+    with pytest.raises(RuntimeError, match="modified by an inplace operation"):
+        torch.autograd.grad(y, leaves, dy)
+    st = torch.cuda.Stream()
+    st.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(st), torch.no_grad():
+        y2, _ = f(*leaves)
+    torch.cuda.current_stream().wait_stream(st)
+    assert torch.equal(y2, f.apply(*leaves)[0])
