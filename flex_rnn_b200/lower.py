@@ -645,6 +645,11 @@ class Problem:
     st_names: List[str]
     out_dt: List[int]                    # dtype code of each output
     naux: int
+    res_states: List[TensorSpec] = field(default_factory=list)   # final states and gradients of initial states: ``empty_like``
+                                                                 # layouts, which a state with gaps does not share
+
+    def __post_init__(self):
+        self.res_states = self.res_states or self.states
 
     def in_cls(self, i: int) -> Shape:
         s = self.inputs[i].shape
@@ -1187,7 +1192,7 @@ def emit_forward(p: Problem, g: StepGraph, aux_names: List[str], n_out: int, til
     for j in range(n_out):
         kb.add_param(f"out{j}", "void", False, p.B * p.T * p.H * p.M * ELT[p.out_dt[j]])
     for k in range(ns):
-        kb.add_param(f"sT_{k}", "void", False, _spec_bytes(p.states[k]))
+        kb.add_param(f"sT_{k}", "void", False, _spec_bytes(p.res_states[k]))
     if not infer:
         for k in range(ns):
             kb.add_param(f"ck{k}", "float", False, ck_bytes)
@@ -1325,8 +1330,8 @@ def emit_forward(p: Problem, g: StepGraph, aux_names: List[str], n_out: int, til
         w("}")
     w.close()  # chunk loop
     for k in range(ns):
-        kb.emit_tile_global(vname(p.st_names[k]), p.states[k], f"sT_{k}",
-                            _elem_off(p.states[k], [(0, "b"), (1, "h")]), 2, 3, load=False)
+        kb.emit_tile_global(vname(p.st_names[k]), p.res_states[k], f"sT_{k}",
+                            _elem_off(p.res_states[k], [(0, "b"), (1, "h")]), 2, 3, load=False)
         if final_ckpt and not infer:
             base = _elem_off(ckspec, [(0, "b"), (1, "h"), (2, str(nck))])
             kb.emit_tile_global(vname(p.st_names[k]), ckspec, f"ck{k}", base, 3, 4, load=False)
@@ -1504,7 +1509,7 @@ def emit_backward(p: Problem, g_re: StepGraph, g_bw: StepGraph, aux_names: List[
         kb.add_param(f"ck{k}", "float", True, p.B * p.H * nck_store * p.M * p.N * 4)
     kb.add_param("aux", "float", True, p.naux * p.B * p.H * p.T * p.M * 4)
     for k in range(ns):
-        kb.add_param(f"ds0_{k}", "void", False, _spec_bytes(p.states[k]))
+        kb.add_param(f"ds0_{k}", "void", False, _spec_bytes(p.res_states[k]))
     for go in grads:
         kb.add_param(f"dx{go.index}", "void", False, _spec_bytes(go.spec))
     kb.add_param("err", "int", False, 4)
@@ -2257,8 +2262,8 @@ def emit_backward(p: Problem, g_re: StepGraph, g_bw: StepGraph, aux_names: List[
     w.close()   # chunk loop
 
     for k in range(ns):
-        kb.emit_tile_global(vname(dnext_names[k]), p.states[k], f"ds0_{k}",
-                            _elem_off(p.states[k], [(0, "b"), (1, "h")]), 2, 3, load=False)
+        kb.emit_tile_global(vname(dnext_names[k]), p.res_states[k], f"ds0_{k}",
+                            _elem_off(p.res_states[k], [(0, "b"), (1, "h")]), 2, 3, load=False)
     for go in grads:
         if go.over_t and go.cls == M1:
             idx0 = _elem_off(go.spec, [(0, "b"), (2, "h")])

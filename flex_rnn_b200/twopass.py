@@ -396,7 +396,8 @@ def make_plan(step: Callable, inputs: Sequence[th.Tensor], state: Sequence[th.Te
             reverse = lower.Reverse(g_x, signs, max(1, tu.rev_resync))
     dy_names, dnext_names = list(dy_names), list(dnext_names)
     prob = Problem(B, T, H, M, N, [_spec(x) for x in inputs], list(in_names), [_spec(s) for s in state],
-                   list(st_names), [_DT[d] for d in out_dtypes], len(aux))
+                   list(st_names), [_DT[d] for d in out_dtypes], len(aux),
+                   [_spec(th.empty_like(s, device="meta")) for s in state])
     dx_meta = tuple(th.empty_like(x, device="meta") for x in inputs)
 
     def make_grads(rows_split: bool) -> List[GradOut]:
