@@ -1,0 +1,2205 @@
+"""Chunked form of step functions whose state update is a decay plus rank-1 terms.
+
+Many step functions - Delta Rule, Gated Delta Rule, RWKV-7, Mamba-2, gated linear attention, retention - have the form
+
+    sigma_d = S . alpha_d                    (row sums, d = 1..nd)
+    S'      = S * w + sum_r p_r (x) kappa_r  (decay over columns, or one per head, or none; r = 1..nr)
+    p_r, y  = row functions of (sigma, inputs)
+
+with vectors alpha, kappa, w over the columns that depend on the inputs only.  ``normal_form`` finds it in a traced
+step graph (``StepGraph``), whatever way the step function was written, or says that there is none.
+
+C such steps in a row need the state only at their start:
+
+    sigma_d,j = S_0 . (alpha_d,j * W_j-1) + sum_{i<j,r} p_r,i Gram_dr,ji,   Gram_dr,ji = alpha_d,j . (kappa_r,i * W_j-1/W_i)
+    S_C       = S_0 * W_C + sum_{i,r} p_r,i (x) (kappa_r,i * W_C/W_i),      W_j = w_1 * ... * w_j
+
+so that per chunk the state takes part in two matrix products of C columns instead of C times in two vector products,
+which is work for the tensor cores (``emit_scan``).  The ratios W_j/W_i are products of the decays between, never
+quotients: a decay of zero is nothing special.  The adjoint recurrence has the same form, with alpha and kappa
+exchanged and time reversed, so one emitter makes the forward scan and the scan of the state gradient; the gradients of
+the vectors then follow chunk by chunk, in parallel, from the states and state gradients at the chunk boundaries
+(``emit_vector_grads``).
+
+All products are fp32-accurate: an fp32 operand x enters the tf32 tensor cores as x (they read its leading 11 bits) and
+as what that leaves out, rounded to 11 more; every pair of terms is multiplied, fp32 accumulators; the state itself is
+accumulated by fp32 additions outside the tensor cores.
+"""
+from __future__ import annotations
+
+import math
+from dataclasses import dataclass, field
+from typing import Callable, Dict, List, Optional, Sequence, Tuple
+
+import torch as th
+
+from . import lower
+from .graph import MN, M1, N1, S11, Arg, Node, Shape, StepGraph
+from .lower import DT_F32, ELT, KernelBuilder, KernelSource, Problem, TensorSpec, W, _contig, _elem_off, _spec_bytes, op_expr
+
+
+# ---------------------------------------------------------------------------
+# normal form
+# ---------------------------------------------------------------------------
+
+class _NotNormal(Exception):
+    pass
+
+
+@dataclass
+class Normal:
+    """A step function in the form above.  ``hoist``: nodes that depend on the inputs only; ``row``: nodes of the row
+    functions, over the values ``sig<d>`` (row sums of the state), ``dg<k>`` (column sums of the vectors ``diags[k]``)
+    and hoisted values."""
+    inputs: List[str]
+    shape: Dict[str, Shape]
+    hoist: List[Node]
+    row: List[Node]
+    alphas: List[str]
+    kappas: List[str]
+    ps: List[str]                 # row values p_r (row or hoisted names)
+    ys: List[str]
+    decay: Optional[str]          # None: no decay; a column vector, or one value per head
+    diags: List[str]              # vectors z_k whose column sums dg<k> the row functions read
+    diag_at: List[Tuple[int, int]]    # dg<k> is the inner product of kappa_r and of alpha_d before its decay: (d, r)
+
+
+@dataclass
+class _Tile:
+    coef: Optional[Arg]                    # factor of S: None = S does not occur, 1.0 or a name (N1 or S11)
+    terms: List[Tuple[Arg, Arg]]           # (row value, column vector)
+
+
+def normal_form(g: StepGraph, in_names: Sequence[str], st_name: str, n_out: int) -> Optional[Normal]:
+    """``g`` computes [*outputs, new state, ...] from inputs and one state; None if it is not of the chunked form."""
+    try:
+        return _normal_form(g, list(in_names), st_name, n_out)
+    except _NotNormal:
+        return None
+
+
+def _normal_form(g: StepGraph, in_names: List[str], st_name: str, n_out: int) -> Normal:
+    shape = {k: v for k, v in g.shape.items()}
+    hoist: List[Node] = []
+    row: List[Node] = []
+    val: Dict[str, object] = {}            # graph value -> Arg (free) | ("row", name) | _Tile
+    known: Dict[tuple, str] = {}
+    alphas: List[str] = []
+    diags: List[str] = []
+    rowset = set()
+
+    def no():
+        raise _NotNormal()
+
+    def cls(a: Arg) -> Shape:
+        return shape[a] if isinstance(a, str) else S11
+
+    def is_row(a: Arg) -> bool:
+        return isinstance(a, str) and a in rowset
+
+    def mk(op: str, args: Sequence[Arg]) -> Arg:
+        """A node of the hoisted or of the row graph, whichever its operands belong to."""
+        args = list(args)
+        if op == "mul":
+            if 1.0 in args:
+                args.remove(1.0)
+                return args[0]
+            if 0.0 in args:
+                return 0.0
+        if op in ("add", "sub") and args[1] == 0.0:
+            return args[0]
+        if op == "add" and args[0] == 0.0:
+            return args[1]
+        if op == "sub" and args[0] == 0.0:
+            op, args = "neg", [args[1]]
+        if op == "neg" and not isinstance(args[0], str):
+            return -args[0]
+        s = (max(cls(a)[0] for a in args), max(cls(a)[1] for a in args))
+        rowy = any(is_row(a) for a in args)
+        if s == MN or (rowy and s[1]):
+            no()
+        if op in ("mul", "add"):
+            args.sort(key=lambda a: (shape.get(a) == N1, str(a)) if isinstance(a, str) else (False, str(a)))
+        key = (op, *args)
+        if key not in known:
+            nm = f"c{len(known)}"
+            known[key] = nm
+            shape[nm] = s
+            (row if rowy else hoist).append(Node(nm, op, args, s))
+            if rowy:
+                rowset.add(nm)
+        return known[key]
+
+    def factors(k: Arg) -> Tuple[Arg, Arg]:
+        """A column vector as (scalar, vector): the scalar goes to the row side, so that the vectors that meet the
+        state stay plain inputs where they can (16-bit inputs need no second tf32 term)."""
+        n = next((n for n in hoist if n.name == k), None)
+        if n is not None and n.op == "mul":
+            s1, s2 = cls(n.args[0]), cls(n.args[1])
+            if s2 == N1 and s1 == S11:
+                f, v = factors(n.args[1])
+                return mk("mul", [n.args[0], f]), v
+            if s1 == N1 and s2 == N1:
+                (f1, v1), (f2, v2) = factors(n.args[0]), factors(n.args[1])
+                return mk("mul", [f1, f2]), mk("mul", [v1, v2])
+        if n is not None and n.op == "neg" and cls(n.args[0]) == N1:
+            f, v = factors(n.args[0])
+            return mk("mul", [-1.0, f]), v
+        return 1.0, k
+
+    def tile_of(v) -> _Tile:
+        return v if isinstance(v, _Tile) else no()
+
+    def scale(t: _Tile, x: Arg, op: str = "mul") -> _Tile:
+        if not is_row(x) and cls(x)[0] == 0:
+            f = (lambda a: mk("mul", [a, x])) if op == "mul" else (lambda a: mk("div", [a, x]))
+            coef = None if t.coef is None else f(t.coef)
+            return _Tile(coef, [(p, f(k)) for p, k in t.terms])
+        if t.coef is not None:
+            no()
+        return _Tile(None, [(mk(op, [p, x]), k) for p, k in t.terms])
+
+    def neg(t: _Tile) -> _Tile:
+        return _Tile(None if t.coef is None else mk("neg", [t.coef]), [(mk("neg", [p]), k) for p, k in t.terms])
+
+    def add(a: _Tile, b: _Tile) -> _Tile:
+        coef = a.coef if b.coef is None else (b.coef if a.coef is None else mk("add", [a.coef, b.coef]))
+        terms = list(a.terms)
+        for p, k in b.terms:
+            for i, (p2, k2) in enumerate(terms):
+                if k2 == k:
+                    terms[i] = (mk("add", [p2, p]), k)
+                    break
+            else:
+                terms.append((p, k))
+        return _Tile(coef, terms)
+
+    def diag(k: Arg) -> Arg:
+        if not isinstance(k, str) or cls(k) != N1:
+            no()
+        f, k = factors(k)
+        if f != 1.0:
+            return mk("mul", [f, diag(k)])
+        if k not in diags:
+            diags.append(k)
+            nm = f"dg{diags.index(k)}"
+            shape[nm] = S11
+            rowset.add(nm)
+        return f"dg{diags.index(k)}"
+
+    for i in in_names:
+        val[i] = i
+        if shape[i] == MN:
+            no()
+    val[st_name] = _Tile(1.0, [])
+    for n in g.nodes:
+        vs = [val[a] if isinstance(a, str) else a for a in n.args]
+        tiles = [isinstance(v, _Tile) for v in vs]
+        if n.op == "copy":
+            val[n.name] = vs[0]
+        elif n.op == "const":
+            val[n.name] = n.args[0]
+        elif n.op == "sum":
+            if n.over_m or not n.over_n:
+                no()
+            if tiles[0]:
+                t = vs[0]
+                acc: Arg = 0.0
+                if t.coef is not None:
+                    if not isinstance(t.coef, str) or cls(t.coef) != N1:
+                        no()
+                    f, v = factors(t.coef)
+                    if v not in alphas:
+                        alphas.append(v)
+                        shape[f"sig{alphas.index(v)}"] = M1
+                        rowset.add(f"sig{alphas.index(v)}")
+                    acc = mk("mul", [f, f"sig{alphas.index(v)}"])
+                for p, k in t.terms:
+                    acc = mk("add", [acc, mk("mul", [p, diag(k)])])
+                val[n.name] = acc
+            else:
+                no()                        # sums of plain column vectors are not hoisted
+        elif any(tiles):
+            if n.op == "mul" and sum(tiles) == 1:
+                t, x = (vs[0], vs[1]) if tiles[0] else (vs[1], vs[0])
+                val[n.name] = scale(t, x)
+            elif n.op == "div" and tiles[0] and not tiles[1]:
+                val[n.name] = scale(vs[0], vs[1], "div")
+            elif n.op == "neg":
+                val[n.name] = neg(vs[0])
+            elif n.op in ("add", "sub") and all(tiles):
+                val[n.name] = add(vs[0], vs[1] if n.op == "add" else neg(vs[1]))
+            else:
+                no()
+        elif n.shape == MN:
+            if n.op != "mul":
+                no()
+            ca, cb = cls(vs[0]), cls(vs[1])
+            if (ca, cb) == (M1, N1):
+                val[n.name] = _Tile(None, [(vs[0], vs[1])])
+            elif (ca, cb) == (N1, M1):
+                val[n.name] = _Tile(None, [(vs[1], vs[0])])
+            else:
+                no()
+        else:
+            val[n.name] = mk(n.op, vs)
+    ys = [val[o] for o in g.outputs[:n_out]]
+    new = tile_of(val[g.outputs[n_out]])
+    if any(isinstance(y, _Tile) or not isinstance(y, str) or cls(y) != M1 for y in ys):
+        no()
+    terms = []
+    for p, k in new.terms:
+        if p == 0.0 or k == 0.0:
+            continue
+        f, v = factors(k)
+        p = mk("mul", [f, p])
+        same = next((i for i, t in enumerate(terms) if t[1] == v), None)
+        if same is None:
+            terms.append((p, v))
+        else:
+            terms[same] = (mk("add", [terms[same][0], p]), v)
+    if not terms or new.coef is None or any(not isinstance(k, str) or cls(k) != N1 or not isinstance(p, str) or cls(p) != M1
+                                            for p, k in terms):
+        no()
+    decay = new.coef
+    if decay == 1.0:
+        decay = None
+    elif not isinstance(decay, str):
+        no()
+    ps = [p for p, _ in terms]
+    kap = [k for _, k in terms]
+    by_name = {n.name: n for n in hoist}
+    diag_at = []
+    for z in diags:
+        n = by_name.get(z)
+        if n is None or n.op != "mul":
+            no()
+        at = None
+        for k, x in ((n.args[0], n.args[1]), (n.args[1], n.args[0])):
+            a = mk("mul", [decay, x]) if decay is not None and cls(decay) == N1 else x
+            if k in kap and a in alphas:
+                at = (alphas.index(a), kap.index(k))
+        diag_at.append(at if at is not None else no())
+    # only what the outputs and the state need
+    need = set(ps) | set(ys) | set(alphas) | set(kap) | set(diags) | ({decay} if decay else set())
+    for nodes in (row, hoist):
+        for n in reversed(nodes):
+            if n.name in need:
+                need.update(n.value_args())
+    used_sig = [f"sig{d}" in need for d in range(len(alphas))]
+    if not alphas or not all(used_sig) or any(f"dg{k}" not in need for k in range(len(diags))):
+        no()
+    return Normal(in_names, shape, [n for n in hoist if n.name in need], [n for n in row if n.name in need], alphas, kap, ps, ys,
+                  decay, diags, diag_at)
+
+
+_TORCH_OPS: Dict[str, Callable] = {
+    "mul": th.mul, "add": th.add, "sub": th.sub, "div": th.div, "neg": th.neg, "exp": th.exp, "log": th.log, "sqrt": th.sqrt,
+    "rsqrt": th.rsqrt, "reciprocal": th.reciprocal, "abs": th.abs, "sigmoid": th.sigmoid, "tanh": th.tanh,
+    "log1p": th.log1p, "expm1": th.expm1, "relu": th.relu, "erf": th.erf, "pow": th.pow,
+    "copy": lambda x: x,
+}
+
+
+def local_vjp(nf: Normal, M: int, N: int) -> Optional[Tuple[StepGraph, bool]]:
+    """The vector-Jacobian product of the row functions and of the vectors, traced: a graph with inputs [*inputs, *sig,
+    *dg, *ga, *gk, (gw), *gp, *gy] (cotangents of alpha, kappa, decay, p, y) and outputs [*d inputs, *d sig], and
+    whether the decay is an exponential and gw the cotangent of its exponent; None where an operation has no derivative
+    here."""
+    from torch.fx.experimental.proxy_tensor import make_fx
+    from .graph import UnsupportedStepOp, from_fx
+    from .trace import clean_dispatch
+    if any(n.op not in _TORCH_OPS for n in nf.hoist + nf.row):
+        return None
+    extra = [f"sig{d}" for d in range(len(nf.alphas))] + [f"dg{k}" for k in range(len(nf.diags))]
+    names = list(nf.inputs) + extra
+    dims = (max(2, M), max(2, N))
+    nin = len(nf.inputs)
+    by_name = {n.name: n for n in nf.hoist}
+    dn = by_name.get(nf.decay)
+    log_decay = dn is not None and dn.op == "exp" and isinstance(dn.args[0], str)
+    vectors = nf.alphas + nf.kappas + ([dn.args[0] if log_decay else nf.decay] if nf.decay else [])
+
+    def evaluate(a, outs, diags):
+        env: Dict[str, th.Tensor] = dict(zip(names, a))
+        get = lambda x: env[x] if isinstance(x, str) else x
+        for n in nf.hoist + (nf.row if len(a) == len(names) else []):
+            args = [get(x) for x in n.args]
+            if not any(isinstance(x, th.Tensor) for x in args):
+                raise UnsupportedStepOp("literal operands only")
+            if n.op in ("mul", "add", "sub", "div") and not isinstance(args[0], th.Tensor):
+                args[0] = th.full((1, 1), args[0], device="meta")
+            env[n.name] = _TORCH_OPS[n.op](*args)
+        return tuple(env[o] * 1.0 for o in outs) + tuple(env[z].sum(-1, True) for z in diags)
+
+    try:
+        with clean_dispatch():
+            args = [th.empty(dims[0] if nf.shape[n][0] else 1, dims[1] if nf.shape[n][1] else 1, device="meta") for n in names]
+
+            def joint(*a):
+                x, gv, gr = a[:len(args)], a[len(args):len(args) + len(vectors)], a[len(args) + len(vectors):]
+                _, pull = th.func.vjp(lambda *z: evaluate(z, nf.ps + nf.ys, ()), *x)
+                d_row = pull(tuple(gr))
+                _, pull = th.func.vjp(lambda *z: evaluate(z, vectors, nf.diags), *x[:nin])
+                d_vec = pull(tuple(gv) + tuple(d_row[nin + len(nf.alphas):]))
+                return tuple(r + v for r, v in zip(d_row, d_vec)) + tuple(d_row[nin:nin + len(nf.alphas)])
+            outs = evaluate(args[:nin], vectors, ()) + evaluate(args, nf.ps + nf.ys, ())
+            gm = make_fx(joint)(*args, *[th.empty_like(o) for o in outs])
+        gj = from_fx(gm, "local_vjp", dims)
+    except (UnsupportedStepOp, KeyError):
+        return None
+    ren = dict(zip(gj.inputs, names + [f"ga{d}" for d in range(len(nf.alphas))] + [f"gk{r}" for r in range(len(nf.kappas))]
+                   + (["gw"] if nf.decay else []) + [f"gp{r}" for r in range(len(nf.ps))] + [f"gy{j}" for j in range(len(nf.ys))]))
+    for n in gj.nodes:
+        ren[n.name] = "b_" + n.name
+    f = lambda a: ren.get(a, a) if isinstance(a, str) else a
+    return simplified(StepGraph("local_vjp", [f(i) for i in gj.inputs],
+                                [Node(f(n.name), n.op, [f(a) for a in n.args], n.shape, n.over_m, n.over_n) for n in gj.nodes],
+                                [f(o) for o in gj.outputs], {f(k): v for k, v in gj.shape.items()})), log_decay
+
+
+def simplified(g: StepGraph) -> StepGraph:
+    """``g`` without multiplications by one or zero, copies, repeated expressions and dead nodes."""
+    alias: Dict[str, Arg] = {}
+    known: Dict[tuple, str] = {}
+    nodes: List[Node] = []
+    f = lambda a: alias.get(a, a) if isinstance(a, str) else a
+    for n in g.nodes:
+        args = [f(a) for a in n.args]
+        if n.op == "copy" or (n.op == "mul" and 1.0 in args and any(isinstance(a, str) for a in args)):
+            rest = [a for a in args if a != 1.0]
+            alias[n.name] = rest[0]
+            continue
+        if n.op == "const":
+            alias[n.name] = n.args[0]
+            continue
+        if n.op == "mul" and 0.0 in args or (n.op == "sum" and args[0] == 0.0) or (n.op == "neg" and args[0] == 0.0):
+            alias[n.name] = 0.0
+            continue
+        if n.op == "add" and 0.0 in args:
+            alias[n.name] = args[1] if args[0] == 0.0 else args[0]
+            continue
+        key = (n.op, n.over_m, n.over_n, *args)
+        if key in known:
+            alias[n.name] = known[key]
+            continue
+        known[key] = n.name
+        nodes.append(Node(n.name, n.op, args, n.shape, n.over_m, n.over_n))
+    g2 = StepGraph(g.name, list(g.inputs), nodes, [f(o) for o in g.outputs], dict(g.shape))
+    return g2.pruned(g2.outputs, g2.name)
+
+
+# ---------------------------------------------------------------------------
+# the scan over chunks
+# ---------------------------------------------------------------------------
+
+_CHUNK_PRELUDE: Optional[str] = None
+
+
+def chunk_prelude() -> str:
+    global _CHUNK_PRELUDE
+    if _CHUNK_PRELUDE is None:
+        import os
+        from .twopass import prelude
+        with open(os.path.join(os.path.dirname(os.path.abspath(__file__)), "csrc", "frnn_chunk.cuh")) as f:
+            _CHUNK_PRELUDE = prelude() + f.read()
+    return _CHUNK_PRELUDE
+
+
+@dataclass
+class Staged:
+    """One per-timestep vector a chunked kernel reads: see ``KernelBuilder.add_item``."""
+    key: str
+    cls: Shape
+    spec: TensorSpec
+    ptr: str
+    dims: Dict[str, int]
+    const_off: int = 0
+
+
+@dataclass
+class ScanSpec:
+    """What ``emit_scan`` makes a kernel of: a recurrence in the chunked form (module docstring)."""
+    name: str
+    params: List[Tuple[str, str, bool, int]]         # (name, C type, read only, bytes)
+    items: List[Staged]
+    const_scalars: List[Tuple[str, TensorSpec, str]]  # time-invariant [1,1] inputs: (name, spec, pointer)
+    shape: Dict[str, Shape]
+    hoist: List[Node]
+    row: List[Node]
+    alphas: List[str]
+    kappas: List[str]
+    ps: List[str]
+    decay: Optional[str]
+    diags: List[str]
+    diag_at: List[Tuple[int, int]]
+    outs: List[Tuple[str, int, str, Callable[[str], str], int]]   # (row value, dtype, pointer, element offset of row m0's head at time t, row stride)
+    init: Tuple[TensorSpec, str]
+    final: Tuple[TensorSpec, str]
+    dg_out: Optional[str]                            # where to keep the dg<k>, [k, B, H, T] fp32
+    ckpt: Optional[str]                              # state at each chunk's start (in processing order), [B, H, chunk, N, M] fp32
+    reverse: bool
+
+
+SCAN_PREP = 256          # threads that prepare the vectors (beside the 128 that own the state's rows)
+TMEM_COLS = 512
+
+
+def _tmem_pow2(cols: int) -> int:
+    c = 32
+    while c < cols:
+        c *= 2
+    return c
+
+
+class ColumnCode:
+    """Code for one column n of the hoisted column vectors at one timestep, read from the raw stage buffer: the
+    vectors are evaluated where they are used, in registers, and never stored as fp32."""
+
+    def __init__(self, kb: KernelBuilder, hoist: Sequence[Node], shape: Dict[str, Shape], scalar: Callable[[str], str]):
+        self.kb, self.shape, self.scalar = kb, shape, scalar
+        self.nodes = {n.name: n for n in hoist}
+
+    def scalars(self, names: Sequence[str]) -> List[str]:
+        """The [1,1] values that the vectors ``names`` are made of."""
+        out: List[str] = []
+
+        def visit(a):
+            if not isinstance(a, str):
+                return
+            if self.shape[a] == S11:
+                if a not in out:
+                    out.append(a)
+            elif a in self.nodes:
+                for x in self.nodes[a].args:
+                    visit(x)
+        for n in names:
+            visit(n)
+        return out
+
+    def emit(self, names: Sequence[str], stage: str, tl: str, n: str, pre: str) -> Dict[str, str]:
+        """Declare the values of ``names`` (and what they need) as floats with prefix ``pre``."""
+        w, done = self.kb.w, {}
+
+        def visit(a) -> str:
+            if not isinstance(a, str):
+                return lower.flit(a)
+            if a in done:
+                return done[a]
+            v = pre + a.replace(".", "_")
+            if self.shape[a] == S11:
+                w(f"const float {v} = {self.scalar(a)};")
+            elif a in self.nodes:
+                ops = [visit(x) for x in self.nodes[a].args]
+                w(f"const float {v} = {op_expr(self.nodes[a], ops)};")
+            else:
+                it = self.kb.item_by_key[a]
+                w(f"const float {v} = frnn_io<{it.dt}>::ld({stage} + {it.off} + ({tl}) * {it.rowb}, {n});")
+            done[a] = v
+            return v
+        for nm in names:
+            visit(nm)
+        return done
+
+
+def exact_vectors(names: Sequence[str], items: Sequence[Staged], decay_vec: bool) -> bool:
+    """Whether the vectors are plain 16-bit inputs, which tf32 holds exactly."""
+    dt = {it.key: it.spec.dt for it in items}
+    return not decay_vec and all(dt.get(n) in (lower.DT_BF16, lower.DT_F16) for n in names)
+
+
+def emit_scan(p: Problem, s: ScanSpec, C: int, MB: int, use_tma: bool = True, state_unroll: int = 2) -> KernelSource:
+    """Scan over chunks of ``C`` timesteps; a CTA owns ``MB`` <= 128 rows of one (b, h).
+
+    Row m of the state lives in lane m of Tensor Memory (columns: S, then what tf32 truncation leaves out of it), and
+    state thread m does everything that concerns the row.  Per chunk:
+
+      products 1   S . alpha for all C steps: [S and rest of S] x [alpha | rest of alpha]
+      rows         forward substitution over the steps: sigma, row functions, outputs; p goes to Tensor Memory
+      products 2   sum_i p_i (x) kappa_i
+      state        S = S * W_C + that, in fp32 registers; rest of S; checkpoint
+
+    One warp issues all products.  Products 1 start on the first columns of the new state while the state threads are
+    still at the others.  Eight more warps keep a chunk ahead: raw inputs by TMA, row vectors and scalars in fp32, the
+    operands alpha and kappa in the tensor cores' layout (thread n converts column n), and the C x C inner products Gram
+    of the vectors, on the tensor cores too, while the state threads are at the substitution.  Decays over columns are folded into the operands (alpha W_j-1, kappa W_C/W_i), decays per head
+    stay scalars on the row side, so that vectors that are plain 16-bit inputs remain exact in tf32 and need no second
+    term.  Gram needs the ratios W_j-1/W_i: as kappa/W_i where no W of the chunk is tiny, else (a reset, an extreme
+    decay) as running products, by a slower path for that chunk alone.
+
+    The chain of one chunk - products 1, substitution, products 2, state - bounds the kernel; a product of up to 64
+    columns takes 46 cycles whatever its width, so hi and rest of alpha share one.
+    """
+    import types
+    from .lower import Body
+    N, nd, nr = p.N, len(s.alphas), len(s.kappas)
+    Np = (N + 15) // 16 * 16
+    PT = SCAN_PREP
+    Tl = types.SimpleNamespace(MB=MB, NT=PT, R=1, C=1)
+    kb = KernelBuilder(p, Tl, C, use_tma)
+    w = kb.w
+    for nm, ct, const, nb in s.params:
+        kb.add_param(nm, ct, const, nb)
+    for nm, spec, ptr in s.const_scalars:
+        kb.const_scalars[nm] = f"{lower.vname(nm)}[0]"
+    for it in s.items:
+        kb.add_item(it.key, it.cls, it.spec, it.ptr, it.dims, it.const_off)
+    dec_vec = bool(s.decay) and s.shape[s.decay] == N1
+    dec_sc = bool(s.decay) and not dec_vec
+    xa, xk = exact_vectors(s.alphas, s.items, dec_vec), exact_vectors(s.kappas, s.items, dec_vec)
+    row_names = {n.name for n in s.row}
+    special = {f"sig{d}" for d in range(nd)} | {f"dg{k}" for k in range(len(s.diags))}
+    col = ColumnCode(kb, s.hoist, s.shape, lambda a: "")
+    need: List[str] = []            # hoisted row vectors and scalars
+    for a in [a for n in s.row for a in n.value_args()] + list(s.ps) + [o[0] for o in s.outs]:
+        if a not in row_names and a not in special and a not in need:
+            need.append(a)
+    row_in = list(need)
+    vec_names = s.alphas + s.kappas + ([s.decay] if dec_vec else []) + s.diags
+    for a in col.scalars(vec_names) + ([s.decay] if dec_sc else []):
+        if a not in need:
+            need.append(a)
+    if any(nm in kb.const_scalars for nm in need):
+        raise lower.LoweringError("a time-invariant scalar is read directly")
+    g = StepGraph("vec", [it.key for it in s.items] + list(kb.const_scalars), list(s.hoist), need, dict(s.shape))
+    kb.plan([g.pruned(need)], need)
+    mk_row = 0
+    for want, ln in ((M1, MB), (S11, 1)):
+        mk_row = (mk_row + 3) // 4 * 4
+        for nm, (cls, _) in list(kb.wk.items()):
+            if cls == want:
+                kb.wk[nm] = (cls, mk_row)
+                mk_row += ln
+    mk_row = (mk_row + 3) // 4 * 4
+    # shared memory
+    al = lambda x: (x + 127) // 128 * 128
+    nA, nK = nd * C, nr * C
+    RA, RK = nA * (1 if xa else 2), nK * (1 if xk else 2)
+    GS = C + 4
+    gram_f = nd * nr * C * GS
+    dec_f = Np if dec_vec else (3 * C if dec_sc else 0)        # W_C; or, per head, W_j-1 | W_C/W_i | W_C: three of them, the
+    o_dec = 0                                                  # state threads still read one when gram is free again
+    o_dg = gram_f
+    o_end = o_dg + (len(s.diags) * C + 3) // 4 * 4
+    lboA, lboH, lboK = RA * 16 + 16, RK * 16 + 16, Np * 16
+    off_stage = 256
+    off_mk = off_stage + 2 * al(kb.stage_bytes)
+    mk_bytes = al(mk_row * C * 4)
+    off_gr = off_mk + 2 * mk_bytes
+    gr_bytes = al(o_end * 4)
+    off_dec = off_gr + 2 * gr_bytes
+    off_al = off_dec + al(3 * dec_f * 4)
+    al_bytes = al((N // 4 - 1) * lboA + max(2048 + 16, lboA))     # Gram reads 128 rows of alpha, whatever is there
+    off_ka = off_al + 2 * al_bytes
+    ka_bytes = al(nK // 4 * lboK)
+    off_kh = off_ka + (1 if xk else 2) * ka_bytes
+    smem_bytes = off_kh + al(N // 4 * lboH)
+    # Tensor Memory columns: S | rest of S | products 2 | p | rest of p, over products 1 (read before p is written) | Gram
+    colS, colL, colD, colP = 0, Np, 2 * Np, 3 * Np
+    colA = colP
+    colG = colP + max(2 * nK, RA)
+    tm_cols = _tmem_pow2(colG + RK)
+    if tm_cols > TMEM_COLS:
+        raise lower.LoweringError("the chunk's operands do not fit Tensor Memory")
+    nchunk = (p.T + C - 1) // C
+    B_RAW, B_AF, B_AE, B_HF, B_KF, B_KE, B_GF, B_GE, B_M1, B_M2, B_SB, B_PB, B_HS, B_MG, B_SE = 0, 2, 4, 6, 7, 8, 9, 11, 13, 14, 15, 19, 20, 21, 25
+    nblk = Np // 16
+    quarters = [(nblk * q // min(4, nblk) * 16, nblk * (q + 1) // min(4, nblk) * 16) for q in range(min(4, nblk))]
+    whole = p.T % C == 0
+    ERR = lower.ERR_STAGE_TIMEOUT
+
+    w(lower._header(chunk_prelude()))
+    w(f"// chunked scan {s.name}: B={p.B} T={p.T} H={p.H} M={p.M} N={N}; {MB} rows per CTA, {C} steps per chunk, {nd} row sums, "
+      f"{nr} rank-1 terms" + (", reversed" if s.reverse else ""))
+    kb.emit_tma_issue("sc_issue")
+    w(f'extern "C" __global__ void __launch_bounds__({128 + PT + 128}, 1)')
+    w.open(f"{s.name}({', '.join(kb.param_decl)})")
+    w("FRNN_DYN_SMEM(smem);")
+    w("const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5; (void)lane;")
+    w(f"const int m0 = blockIdx.x * {MB}, h = blockIdx.y, b = blockIdx.z; (void)m0; (void)h; (void)b;")
+    kb.emit_bounds_prologue()
+    w("u64* bar = (u64*)smem;")
+    w(f"unsigned char* kappaB = smem + {off_ka};")
+    w.open("if (tid == 0)")
+    for bi, cnt in ((B_RAW, 1), (B_RAW + 1, 1), (B_AF, 128), (B_AF + 1, 128), (B_AE, 1), (B_AE + 1, 1), (B_HF, 128), (B_KF, 128),
+                    (B_KE, 1), (B_GF, PT), (B_GF + 1, PT), (B_GE, 128), (B_GE + 1, 128), (B_M1, 1), (B_M2, 1), (B_SB, 128),
+                    (B_SB + 1, 128), (B_SB + 2, 128), (B_SB + 3, 128), (B_PB, 128), (B_HS, PT), (B_MG, 1), (B_SE, PT), (B_SE + 1, PT)):
+        w(f"frnn_mbar_init(&bar[{bi}], {cnt});")
+    w("((int*)&bar[23])[0] = 0;      // warps that are done with Tensor Memory")
+    w("bar[24] = 0;                  // two ints: a chunk (even, odd) whose decays are too small to divide by, its number plus one")
+    w("frnn_mbar_init_fence();")
+    w.close()
+    w.open("if (warp == 0)")
+    w(f"frnn_tmem_alloc((u32*)&bar[22], {tm_cols}u);")
+    w("frnn_tmem_fence_before_sync();")
+    w.close()
+    w("frnn_block_sync();")
+    w("frnn_tmem_fence_after_sync();")
+    w("const u32 tm = *(volatile u32*)&bar[22];")
+    tma_call = (", " + kb.tma_issue_call) if kb.tma_items else ""
+
+    def chunk_head():
+        """kc: the chunk in time order, t0 / nv: its first timestep and length."""
+        w(f"const int kc = {f'{nchunk - 1} - c' if s.reverse else 'c'}, t0 = kc * {C}, nv = min({C}, {p.T} - t0), buf = c & 1; (void)kc;")
+        w(f"{{0}}float* mk = ({{0}}float*)(smem + {off_mk} + buf * {mk_bytes}); (void)mk;")
+        w(f"{{0}}float* gram = ({{0}}float*)(smem + {off_gr} + buf * {gr_bytes});")
+        if dec_f:
+            w(f"{{0}}float* dec = ({{0}}float*)(smem + {off_dec} + (c % 3) * {dec_f * 4}); (void)dec;")
+
+    def head(const: str):
+        n0 = len(w.lines)
+        chunk_head()
+        for i in range(n0, len(w.lines)):
+            w.lines[i] = w.lines[i].replace("{0}", const)
+    pos = (lambda q: f"(nv - 1 - ({q}))") if s.reverse else (lambda q: f"({q})")
+
+    # ------------------------------------------------------------------ preparing warps
+    # registers: 512 threads start with 128 each; the state's rows need more, the products' warpgroup hardly any
+    w("auto work = [&]() -> void {")
+    w.ind += 1
+    w.open(f"if (tid >= 128 && tid < {128 + PT})")
+    w("frnn_regs_release<104>();")
+    w("const int hl = tid - 128, hw = hl >> 5; (void)hw;")
+    w("u32 hs_par = 0; (void)hs_par;")
+    w(f"float k[{nr}][{C}];     // kappa of the last chunk: stored when the products of the chunk before are complete")
+
+    def put_kappa():
+        """Column hl of kappa of chunk c - 1, from registers to the operand."""
+        w(f"if (c > 1 && !frnn_mbar_wait(&bar[{B_KE}], c & 1, err, {ERR})) return;      // products 2 of chunk c - 2 are complete")
+        w.open(f"if (hl < {Np})")
+        w("#pragma unroll")
+        w.open(f"for (int q = 0; q < {C}; q += 4)")
+        for r in range(nr):
+            w(f"unsigned char* dst{r} = kappaB + (({r * C} + q) >> 2) * {lboK} + (hl >> 3) * 128 + (hl & 7) * 16;")
+            if xk:
+                w(f"frnn_stv<0,4>(dst{r}, 0, &k[{r}][q]);")
+            else:
+                w(f"{{ float hi[4]; for (int e = 0; e < 4; e++) {{ hi[e] = k[{r}][q + e]; k[{r}][q + e] = frnn_tf32_rest(hi[e]); }}")
+                w(f"frnn_stv<0,4>(dst{r}, 0, hi); frnn_stv<0,4>(dst{r} + {ka_bytes}, 0, &k[{r}][q]); }}")
+        w.close()
+        w.close()
+        w("frnn_async_proxy_fence();")
+        w(f"frnn_mbar_arrive(&bar[{B_KF}]);")
+    for nm, spec, ptr in s.const_scalars:
+        kb.emit_const_input(Body(w, Tl, {}, False, False), nm, S11, spec, ptr, lower.IN_DIMS)
+
+    def hsync():
+        w(f"frnn_mbar_arrive(&bar[{B_HS}]); if (!frnn_mbar_wait(&bar[{B_HS}], hs_par, err, {ERR})) return; hs_par ^= 1;")
+
+    def h_issue(t0e, nve, be):
+        """Plain copies of one chunk into stage buffer ``be`` (inputs no tensor copy reaches)."""
+        if kb.plain_items:
+            w.open("")
+            w(f"unsigned char* stage = smem + {off_stage} + ({be}) * {al(kb.stage_bytes)}; (void)stage;")
+            kb.emit_plain_direct("stage", t0e, nve, "hl", PT)
+            w.close()
+    first = nchunk - 1 if s.reverse else 0
+    h_issue(str(first * C), str(min(C, p.T - first * C)), "0")
+    w("#pragma unroll 1")
+    w.open(f"for (int c = 0; c < {nchunk}; c++)")
+    head("")
+    w(f"const unsigned char* stage = smem + {off_stage} + buf * {al(kb.stage_bytes)};")
+    w(f"unsigned char* alphaB = smem + {off_al} + buf * {al_bytes};")
+    w.open(f"if (c + 1 < {nchunk})" if kb.plain_items else "")
+    nxt = f"(kc {'-' if s.reverse else '+'} 1)"
+    h_issue(f"{nxt} * {C}", f"min({C}, {p.T} - {nxt} * {C})", "(c + 1) & 1")
+    w.close()
+    if kb.tma_items:
+        w(f"if (!frnn_mbar_wait(&bar[{B_RAW} + buf], (c >> 1) & 1, err, {ERR})) return;")
+    if kb.plain_items:
+        hsync()
+    w(f"if (c >= 2 && !frnn_mbar_wait(&bar[{B_GE} + buf], ((c >> 1) - 1) & 1, err, {ERR})) return;")
+    if kb.wk:
+        kb.emit_convert("stage", "mk", "nv", "hl", PT, rows={M1: ("mk", mk_row), S11: ("mk", mk_row)})
+        w(f"for (int e = hl; e < ({C} - nv) * {mk_row}; e += {PT}) mk[nv * {mk_row} + e] = 0.0f;")
+    col.scalar = lambda a: f"mk[tl * {mk_row} + {kb.wk[a][1]}]"
+    if col.scalars(vec_names) or dec_sc:
+        hsync()
+    if dec_sc:
+        od = kb.wk[s.decay][1]
+        w.open("if (hl == 0)")
+        w("float W = 1.0f;")
+        w("#pragma unroll")
+        w(f"for (int q = 0; q < {C}; q++) {{ dec[{o_dec} + q] = W; if (q < nv) W *= mk[{pos('q')} * {mk_row} + {od}]; }}")
+        w(f"dec[{o_dec + 2 * C}] = W;")
+        w.close()
+        w.open("if (hl == 32)")
+        w("float W = 1.0f;")
+        w("#pragma unroll")
+        w(f"for (int q = {C - 1}; q >= 0; q--) {{ dec[{o_dec + C} + q] = W; if (q < nv) W *= mk[{pos('q')} * {mk_row} + {od}]; }}")
+        w.close()
+
+    def live(names, q, n, pre):
+        if whole:
+            w(f"const bool live = true; const int tl = {pos(q)}; (void)live;")
+        else:
+            w(f"const bool live = {q} < nv; const int tl = live ? {pos(q)} : 0;")
+        return col.emit(names, "stage", "tl", n, pre)
+
+    def put_km(base, lbo, row, n, val):
+        """Store into a K-major operand over columns: element (row, n)."""
+        w(f"*(float*)({base} + ({n} >> 2) * {lbo} + (({row}) >> 3) * 128 + (({row}) & 7) * 16 + ({n} & 3) * 4) = {val};")
+    # --- thread n of the first four warps: column n of alpha (times the decays before the step) and of kappa (times those
+    # after it)
+    w.open("if (hl < 128)")
+    w.open("if (c > 0)")
+    put_kappa()
+    w.close()
+    w(f"if (c >= 2 && !frnn_mbar_wait(&bar[{B_AE} + buf], ((c >> 1) - 1) & 1, err, {ERR})) return;   // products 1 two chunks back are complete")
+    w(f"float x[{C if dec_vec else 1}]; (void)x;")
+    w.open(f"if (hl < {N})")
+    w("float W = 1.0f; (void)W;")
+    w("#pragma unroll")
+    w.open(f"for (int q = 0; q < {C}; q++)")
+    v = live(s.alphas + s.kappas + ([s.decay] if dec_vec else []), "q", "hl", "x_")
+    for d, nm in enumerate(s.alphas):
+        w(f"const float a{d} = live ? {v[nm]}{' * W' if dec_vec else ''} : 0.0f;")
+        if xa:
+            put_km("alphaB", lboA, f"{d * C} + q", "hl", f"a{d}")
+        else:
+            put_km("alphaB", lboA, f"{d * C} + q", "hl", f"a{d}")
+            put_km("alphaB", lboA, f"{nA + d * C} + q", "hl", f"frnn_tf32_rest(a{d})")
+    for r, nm in enumerate(s.kappas):
+        w(f"k[{r}][q] = live ? {v[nm]} : 0.0f;")
+    if dec_vec:
+        w(f"x[q] = live ? {v[s.decay]} : 1.0f; W *= x[q];")
+    w.close()
+    if dec_vec:
+        w(f"dec[{o_dec} + hl] = W;")
+    w.close()
+    w.open("else")
+    w("#pragma unroll")
+    w(f"for (int q = 0; q < {C}; q++) {{ " + " ".join(f"k[{r}][q] = 0.0f;" for r in range(nr)) + " }")
+    if dec_vec:
+        w("#pragma unroll")
+        w(f"for (int q = 0; q < {C}; q++) x[q] = 1.0f;")
+        if Np > N:
+            w(f"if (hl < {Np}) dec[{o_dec} + hl] = 1.0f;")
+    w.close()
+    w("frnn_async_proxy_fence();")
+    w(f"frnn_mbar_arrive(&bar[{B_AF} + buf]);")
+    if dec_vec:
+        w("float S = 1.0f;")
+        w("#pragma unroll")
+        w(f"for (int q = {C - 1}; q >= 0; q--) {{ " + " ".join(f"k[{r}][q] *= S;" for r in range(nr)) + " S *= x[q]; }")
+    w.close()
+    # --- thread n of the last four warps: column n of kappa over W, for Gram (its previous products are complete: below)
+    w.open("else")
+    w("const int n = hl - 128;")
+    w.open(f"if (n < {N})")
+    if dec_vec:
+        w("float W = 1.0f, R = 1.0f; bool tiny = false;")
+    w("#pragma unroll")
+    w.open(f"for (int q = 0; q < {C}; q++)")
+    v = live(s.kappas + ([s.decay] if dec_vec else []), "q", "n", "x_")
+    if dec_vec:
+        w(f"const float x = live ? {v[s.decay]} : 1.0f;")
+        w("W *= x; R *= frnn_rcp1(x); tiny = tiny || !(fabsf(W) > 1e-25f && fabsf(W) < 1e25f);")
+    for r, nm in enumerate(s.kappas):
+        w(f"const float y{r} = live ? {v[nm]}{' * R' if dec_vec else ''} : 0.0f;")
+        if xk:
+            put_km(f"(smem + {off_kh})", lboH, f"{r * C} + q", "n", f"y{r}")
+        else:
+            put_km(f"(smem + {off_kh})", lboH, f"{r * C} + q", "n", f"y{r}")
+            put_km(f"(smem + {off_kh})", lboH, f"{nK + r * C} + q", "n", f"frnn_tf32_rest(y{r})")
+    w.close()
+    if dec_vec:
+        w("if (tiny) ((volatile int*)&bar[24])[buf] = c + 1;")
+    w.close()
+    w("frnn_async_proxy_fence();")
+    w(f"frnn_mbar_arrive(&bar[{B_HF}]);")
+    w.close()
+    # --- Gram: alpha against kappa, rows (d, j), columns (r, i)
+    w(f"if (!frnn_mbar_wait(&bar[{B_MG}], c & 1, err, {ERR})) return;")
+    slow = "((volatile int*)&bar[24])[buf] == c + 1"
+    if dec_vec:
+        w(f"const bool slow = {slow};")
+        w.open("if (!slow)")
+    w("frnn_tmem_fence_after_sync();")
+    w("const u32 gt = tm + frnn_tmem_lane_base(hw);")
+    w("const int d = hl / %d, j = hl %% %d; (void)d; (void)j;" % (C, C))
+
+    def gram_at(i):
+        return f"gram[((d * {nr} + {i} / {C}) * {C} + {i} % {C}) * {GS} + j]"
+    if not xa:
+        w("// rows of the rest of alpha")
+        w.open(f"if (hl >= {nA // 32 * 32} && hl < {(2 * nA + 31) // 32 * 32})")
+        w(f"float v[{nK}];")
+        w(f"frnn_tmem_ld<{nK}>(gt + {colG}u, v); frnn_tmem_wait_ld();")
+        w.open(f"if (hl >= {nA} && hl < {2 * nA})")
+        w(f"const int d = (hl - {nA}) / {C}, j = (hl - {nA}) % {C};")
+        w("#pragma unroll")
+        w(f"for (int i = 0; i < {nK}; i++) {gram_at('i')} = v[i];")
+        w.close()
+        w.close()
+        hsync()
+    w.open(f"if (hl < {(nA + 31) // 32 * 32})")
+    w(f"float v[{nK}];")
+    w(f"frnn_tmem_ld<{nK}>(gt + {colG}u, v);")
+    if not xk:
+        w(f"float u[{nK}];")
+        w(f"frnn_tmem_ld<{nK}>(gt + {colG + nK}u, u);")
+    w("frnn_tmem_wait_ld();")
+    w.open(f"if (hl < {nA})")
+    w("#pragma unroll")
+    w(f"for (int i = 0; i < {nK}; i++) v[i] = v[i]{' + u[i]' if not xk else ''}{f' + {gram_at(chr(105))}' if not xa else ''};")
+    for k in range(len(s.diags)):
+        d_, r_ = s.diag_at[k]
+        w(f"if (d == {d_}) {{ float z = 0.0f;")
+        w("#pragma unroll")
+        w(f"for (int i = 0; i < {C}; i++) z = i == j ? v[{r_ * C} + i] : z;")
+        w(f"gram[{o_dg + k * C} + j] = z;" + (f" if (j < nv) frnn_st_raw<float>({s.dg_out}, {dg_off(p, k, f't0 + {pos(chr(106))}')}, z);" if s.dg_out else "") + " }")
+    if dec_sc:
+        w("float W = 1.0f;")
+        w("#pragma unroll")
+        w.open(f"for (int i = {C - 1}; i >= 0; i--)")
+        w.open("if (i < j)")
+        w(" ".join(f"v[{r * C} + i] *= W;" for r in range(nr)))
+        w(f"if (i < nv) W *= mk[{pos('i')} * {mk_row} + {od}];")
+        w.close()
+        w.close()
+    w("#pragma unroll")
+    w(f"for (int i = 0; i < {nK}; i++) {gram_at('i')} = v[i];")
+    w.close()
+    w.close()
+    if dec_vec:
+        w.close()
+        w.open("else")
+        NE = (N + 31) // 32
+        w("#pragma unroll 1")
+        w.open(f"for (int j = hw; j < {C}; j += {PT // 32})")
+        w(f"float A[{nd}][{NE}], acc[{nd * nr}];")
+        w("#pragma unroll 1")
+        w.open("for (int i = j; i >= 0; i--)")
+        w(" ".join(f"acc[{x}] = 0.0f;" for x in range(nd * nr)))
+        w("#pragma unroll")
+        w.open(f"for (int e = 0; e < {NE}; e++)")
+        w("const int n = lane + 32 * e;")
+        w.open(f"if (n < {N} && j < nv)")
+        w.open("if (i == j)")
+        w(f"const int tl = {pos('j')};")
+        v = col.emit(s.alphas, "stage", "tl", "n", "x_")
+        for d, nm in enumerate(s.alphas):
+            w(f"A[{d}][e] = {v[nm]};")
+        w.close()
+        w.open("else")
+        w(f"const int tl = {pos('i')};")
+        v = col.emit(s.kappas + [s.decay], "stage", "tl", "n", "x_")
+        for d in range(nd):
+            for r, nm in enumerate(s.kappas):
+                w(f"acc[{d * nr + r}] = fmaf(A[{d}][e], {v[nm]}, acc[{d * nr + r}]);")
+        for d in range(nd):
+            w(f"A[{d}][e] *= {v[s.decay]};")
+        w.close()
+        w.close()
+        w.close()
+        w("#pragma unroll")
+        w.open(f"for (int x = 0; x < {nd * nr}; x++)")
+        w("float z = acc[x];")
+        w("#pragma unroll")
+        w("for (int o = 16; o > 0; o >>= 1) z += frnn_shfl_xor(z, o);")
+        w(f"if (lane == 0 && i < j) gram[(x * {C} + i) * {GS} + j] = z;")
+        w.close()
+        w.close()
+        for k, zn in enumerate(s.diags):
+            w.open("")
+            w("float z = 0.0f;")
+            w("#pragma unroll")
+            w.open(f"for (int e = 0; e < {NE}; e++)")
+            w("const int n = lane + 32 * e;")
+            w.open(f"if (n < {N} && j < nv)")
+            w(f"const int tl = {pos('j')};")
+            v = col.emit([zn], "stage", "tl", "n", "x_")
+            w(f"z += {v[zn]};")
+            w.close()
+            w.close()
+            w("#pragma unroll")
+            w("for (int o = 16; o > 0; o >>= 1) z += frnn_shfl_xor(z, o);")
+            w(f"if (lane == 0) gram[{o_dg + k * C} + j] = z;")
+            if s.dg_out:
+                w(f"if (lane == 0 && j < nv) frnn_st_raw<float>({s.dg_out}, {dg_off(p, k, f't0 + {pos(chr(106))}')}, z);")
+            w.close()
+        w.close()
+        w.close()
+    w("frnn_tmem_fence_before_sync();")
+    w(f"frnn_mbar_arrive(&bar[{B_GF} + buf]); frnn_mbar_arrive(&bar[{B_SE} + buf]);")
+    if kb.plain_items:
+        hsync()
+    w.close()     # chunk loop
+    w.open("if (hl < 128)")
+    w(f"const int c = {nchunk};")
+    put_kappa()
+    w.close()
+    w("return;")
+    w.close()     # preparing warps
+
+    # ------------------------------------------------------------------ the warp that starts the copies of the inputs
+    w.open(f"if (tid >= {128 + PT})")
+    w("frnn_regs_release<104>();")
+    w.close()
+    w.open(f"if (tid >= {128 + PT + 32})")
+    if kb.tma_items:
+        w(f"if (tid >= {128 + PT + 64}) return;")
+        w("#pragma unroll 1")
+        w.open(f"for (int c = 0; c < {nchunk}; c++)")
+        chunk_head_line = f"const int kc = {f'{nchunk - 1} - c' if s.reverse else 'c'}, t0 = kc * {C}, nv = min({C}, {p.T} - t0);"
+        w(chunk_head_line)
+        w(f"if (c >= 2 && !frnn_mbar_wait(&bar[{B_SE} + (c & 1)], ((c >> 1) - 1) & 1, err, {ERR})) return;")
+        w(f"sc_issue(smem + {off_stage} + (c & 1) * {al(kb.stage_bytes)}, &bar[{B_RAW} + (c & 1)], t0, nv, lane, b, h, m0{tma_call});")
+        w.close()
+    w("return;")
+    w.close()
+
+    # ------------------------------------------------------------------ the warp that issues the products
+    w.open(f"if (tid >= {128 + PT} && tid < {128 + PT + 32})")
+    w("if (lane) return;")
+
+    for nm, off, lbo in (("dA", off_al, lboA), ("dH", off_kh, lboH), ("dK", off_ka, lboK)):
+        w(f"const u64 {nm} = frnn_mma_desc(smem + {off}, {lbo});")
+    w(f"const u64 dKlo = frnn_mma_desc(smem + {off_ka + (0 if xk else ka_bytes)}, {lboK}), dA1 = frnn_mma_desc(smem + {off_al + al_bytes}, {lboA}); (void)dKlo;")
+
+    def gram_products(c: str):
+        w("frnn_tmem_fence_after_sync();")
+        w(f"const u64 da = (({c}) & 1) ? dA1 : dA;")
+        w("#pragma unroll 4")
+        w(f"for (int k = 0; k < {N // 8}; k++) frnn_mma_ss_d(tm + {colG}u, frnn_mma_next(da, {lboA}, k), frnn_mma_next(dH, {lboH}, k), FRNN_MMA_IDESC({RK}), k > 0);")
+        w(f"frnn_mma_commit(&bar[{B_MG}]);")
+    w.open("")
+    w(f"if (!frnn_mbar_wait(&bar[{B_AF}], 0, err, {ERR}) || !frnn_mbar_wait(&bar[{B_HF}], 0, err, {ERR})) return;")
+    gram_products("0")
+    w.close()
+    w("#pragma unroll 1")
+    w.open(f"for (int c = 0; c < {nchunk}; c++)")
+    w("const u64 da = (c & 1) ? dA1 : dA;")
+    for qi, (n0, n1) in enumerate(quarters):
+        w(f"if (!frnn_mbar_wait(&bar[{B_SB + qi}], c & 1, err, {ERR})) return;")
+        w("frnn_tmem_fence_after_sync();")
+        k0, k1 = n0 // 8, min(n1, N) // 8
+        for a, n_, first_ in ((colS, RA, "k > 0"), (colL, RA, "true")):
+            w("#pragma unroll")
+            w(f"for (int k = {k0}; k < {k1}; k++) frnn_mma_ts_d(tm + {colA}u, tm + {a}u + k * 8, frnn_mma_next(da, {lboA}, k), FRNN_MMA_IDESC({n_}), {first_});")
+    w(f"frnn_mma_commit(&bar[{B_M1}]); frnn_mma_commit(&bar[{B_AE} + (c & 1)]);")
+    # Gram of the next chunk as soon as its operands are there, but never in the way of products 2
+    w(f"bool gram = c + 1 >= {nchunk};")
+    w("const u64 t_wait = frnn_now_ns();")
+    w.open("for (;;)")
+    w.open(f"if (!gram && frnn_mbar_try(&bar[{B_AF} + ((c + 1) & 1)], ((c + 1) >> 1) & 1) && frnn_mbar_try(&bar[{B_HF}], (c + 1) & 1))")
+    gram_products("c + 1")
+    w("gram = true;")
+    w.close()
+    w(f"if (frnn_mbar_try(&bar[{B_PB}], c & 1)) break;")
+    w(f"if (frnn_now_ns() - t_wait > FRNN_WAIT_LIMIT_NS) {{ frnn_report(err, {ERR}); return; }}")
+    w.close()
+    w(f"if (!frnn_mbar_wait(&bar[{B_KF}], c & 1, err, {ERR})) return;")
+    w("frnn_tmem_fence_after_sync();")
+    passes = ([] if xk else [(colP + nK, "dKlo"), (colP, "dKlo")]) + [(colP + nK, "dK"), (colP, "dK")]
+    for i, (a, dsc) in enumerate(passes):
+        w("#pragma unroll")
+        w(f"for (int k = 0; k < {nK // 8}; k++) frnn_mma_ts_d(tm + {colD}u, tm + {a}u + k * 8, frnn_mma_next({dsc}, {lboK}, k), FRNN_MMA_IDESC({Np}), {'k > 0' if i == 0 else 'true'});")
+    w(f"frnn_mma_commit(&bar[{B_M2}]); frnn_mma_commit(&bar[{B_KE}]);")
+    w.open("if (!gram)")
+    w(f"if (!frnn_mbar_wait(&bar[{B_AF} + ((c + 1) & 1)], ((c + 1) >> 1) & 1, err, {ERR}) || !frnn_mbar_wait(&bar[{B_HF}], (c + 1) & 1, err, {ERR})) return;")
+    gram_products("c + 1")
+    w.close()
+    w.close()
+    w("return;")
+    w.close()
+
+    # ------------------------------------------------------------------ state warps
+    w("frnn_regs_acquire<200>();")
+    w("const u32 mine = tm + frnn_tmem_lane_base(warp);")
+    w(f"const int m = m0 + tid; const bool row = tid < {MB};")
+    nck = nchunk
+
+    def tile_io(spec: TensorSpec, ptr: str, n0: str, cnt: int, load: bool):
+        """``cnt`` columns from n0 of this thread's row, between x[] and a tensor of any layout."""
+        base = _elem_off(spec, [(0, "b"), (1, "h"), (2, "m")])
+        e = ELT[spec.dt]
+        fast = spec.st(3) == 1 and spec.aligned16 and all((st * e) % 16 == 0 for st in spec.stride[:-1]) and N % 16 == 0
+        w.open("if (row)")
+        if fast:
+            v = 16 // e if e < 4 else 4
+            for q in range(0, cnt, v):
+                w(f"{'frnn_ldv' if load else 'frnn_stv'}<{spec.dt},{v}>({ptr}, {base} + {n0} + {q}, &x[{q}]);")
+        else:
+            w("#pragma unroll")
+            w.open(f"for (int k = 0; k < {cnt}; k++)")
+            idx = f"{base} + (long)({n0} + k) * {spec.st(3)}L"
+            w(f"if ({n0} + k < {N}) " + (f"x[k] = frnn_io<{spec.dt}>::ld({ptr}, {idx});" if load else f"frnn_io<{spec.dt}>::st({ptr}, {idx}, x[k]);"))
+            w.close()
+        w.close()
+
+    def put_state(ck: Optional[str], guard: str = ""):
+        """Columns n0.. of the state (x[]): into Tensor Memory with their rest, and into checkpoint ``ck``."""
+        w(f"frnn_tmem_st<16>(mine + {colS}u + n0, x);")
+        if ck and s.ckpt:
+            w.open(f"if (row{guard})")
+            w(f"float* cp = {s.ckpt} + ((((long)b * {p.H} + h) * {nck} + {ck}) * {N}L + n0) * {p.M}L + m;")
+            w("#pragma unroll")
+            w(f"for (int k = 0; k < 16; k++) " + ("" if N % 16 == 0 else f"if (n0 + k < {N}) ") + f"frnn_st_raw<float>(cp, k * {p.M}L, x[k]);")
+            w.close()
+        w("#pragma unroll")
+        w("for (int k = 0; k < 16; k++) x[k] = frnn_tf32_rest(x[k]);")
+        w(f"frnn_tmem_st<16>(mine + {colL}u + n0, x);")
+    for qi, (n0, n1) in enumerate(quarters):
+        w("#pragma unroll 1")
+        w.open(f"for (int n0 = {n0}; n0 < {n1}; n0 += 16)")
+        w("float x[16];")
+        w("#pragma unroll")
+        w("for (int k = 0; k < 16; k++) x[k] = 0.0f;")
+        tile_io(s.init[0], s.init[1], "n0", 16, True)
+        put_state(str(first))
+        w.close()
+        w(f"frnn_tmem_wait_st(); frnn_tmem_fence_before_sync(); frnn_mbar_arrive(&bar[{B_SB + qi}]);")
+    w("#pragma unroll 1")
+    w.open(f"for (int c = 0; c < {nchunk}; c++)")
+    head("const ")
+    w(f"if (!frnn_mbar_wait(&bar[{B_GF} + buf], (c >> 1) & 1, err, {ERR})) return;")
+    w(f"if (!frnn_mbar_wait(&bar[{B_M1}], c & 1, err, {ERR})) return;")
+    w("frnn_tmem_fence_after_sync();")
+    w.open("")
+    w(f"float g[{nA}], ph[{nr}][{C}];")
+    for k in range(len(s.outs)):
+        w(f"float o{k}[{C}];")
+    w.open("")
+    w(f"frnn_tmem_ld<{nA}>(mine + {colA}u, g);")
+    if not xa:
+        w(f"float lo[{nA}];")
+        w(f"frnn_tmem_ld<{nA}>(mine + {colA + nA}u, lo);")
+    w("frnn_tmem_wait_ld();")
+    if not xa or dec_sc:
+        w("#pragma unroll")
+        e = "g[k] + lo[k]" if not xa else "g[k]"
+        w(f"for (int k = 0; k < {nA}; k++) g[k] = " + (f"({e}) * dec[{o_dec} + k % {C}];" if dec_sc else f"{e};"))
+    w.close()
+    w("#pragma unroll")
+    w.open(f"for (int q = 0; q < {C}; q++)")
+    w(f"const bool live = {'true' if whole else 'q < nv'}; const int tl = {pos('q')}; (void)live;")
+
+    def rv(a: Arg) -> str:
+        if not isinstance(a, str):
+            return lower.flit(a)
+        if a.startswith("sig") and a in special:
+            return f"g[{int(a[3:]) * C} + q]"
+        if a.startswith("dg") and a in special:
+            return f"gram[{o_dg + int(a[2:]) * C} + q]"
+        if a in row_names:
+            return lower.vname(a)
+        return "i_" + a.replace(".", "_")
+    for nm in row_in:
+        cls, o = kb.wk[nm]
+        idx = (f"max(tl, 0)" if s.reverse and not whole else "tl") + f" * {mk_row} + {o}"
+        w(f"const float {rv(nm)} = " + (f"mk[{idx} + " + (f"min(tid, {MB - 1})" if MB < 128 else "tid") + "];" if cls == M1 else f"mk[{idx}];"))
+    for n in s.row:
+        w(f"const float {lower.vname(n.name)} = {op_expr(n, [rv(a) for a in n.args])};")
+    for r, nm in enumerate(s.ps):
+        w(f"ph[{r}][q] = " + (f"{rv(nm)};" if whole and MB == 128 else f"(live && row) ? {rv(nm)} : 0.0f;"))
+    for k, o in enumerate(s.outs):
+        w(f"o{k}[q] = {rv(o[0])};")
+    w("#pragma unroll")
+    w.open(f"for (int j4 = 0; j4 < {C}; j4 += 4)")
+    w.open("if (j4 + 3 > q)")
+    for d in range(nd):
+        for r in range(nr):
+            w(f"{{ float x[4]; frnn_ldv<0,4>(gram, ({(d * nr + r) * C} + q) * {GS} + j4, x);")
+            w("#pragma unroll")
+            w(f"for (int k = 0; k < 4; k++) if (j4 + k > q) g[{d * C} + j4 + k] = fmaf(ph[{r}][q], x[k], g[{d * C} + j4 + k]); }}")
+    w.close()
+    w.close()
+    w.close()     # q
+    for r in range(nr):
+        if dec_sc:
+            w("#pragma unroll")
+            w(f"for (int q = 0; q < {C}; q++) ph[{r}][q] *= dec[{o_dec + C} + q];")
+        w(f"frnn_tmem_st<{C}>(mine + {colP + r * C}u, ph[{r}]);")
+        w("#pragma unroll")
+        w(f"for (int q = 0; q < {C}; q++) ph[{r}][q] = frnn_tf32_rest(ph[{r}][q]);")
+        w(f"frnn_tmem_st<{C}>(mine + {colP + nK + r * C}u, ph[{r}]);")
+    w("frnn_tmem_wait_st(); frnn_tmem_fence_before_sync();")
+    w(f"frnn_mbar_arrive(&bar[{B_PB}]); frnn_mbar_arrive(&bar[{B_GE} + buf]);")
+    # the outputs leave while products 2 run
+    w.open("if (row)" if MB < 128 else "")
+    w("#pragma unroll")
+    w.open(f"for (int q = 0; q < {C}; q++)")
+    w(f"const int tl = {pos('q')};")
+    w.open("" if whole else "if (q < nv)")
+    for k, (nm, dt, ptr, at, sm) in enumerate(s.outs):
+        w(f"frnn_io<{dt}>::st({ptr}, {at('t0 + tl')} + (long)m * {sm}L, o{k}[q]);")
+    w.close()
+    w.close()
+    w.close()
+    w.close()
+    w(f"if (!frnn_mbar_wait(&bar[{B_M2}], c & 1, err, {ERR})) return;")
+    w("frnn_tmem_fence_after_sync();")
+    if dec_sc:
+        w(f"const float y = dec[{o_dec + 2 * C}];")
+    w("float x[16], u[16];")
+    w(f"frnn_tmem_ld<16>(mine + {colS}u, x); frnn_tmem_ld<16>(mine + {colD}u, u);")
+    for qi, (n0, n1) in enumerate(quarters):
+        w(f"#pragma unroll {state_unroll}")
+        w.open(f"for (int n0 = {n0}; n0 < {n1}; n0 += 16)")
+        if dec_vec:
+            w("float y[16];")
+            w("#pragma unroll")
+            w(f"for (int k = 0; k < 16; k += 4) frnn_ldv<0,4>(dec, n0 + k, &y[k]);")
+        w("frnn_tmem_wait_ld();")
+        w("#pragma unroll")
+        w("for (int k = 0; k < 16; k++) x[k] = " + ("fmaf(x[k], y[k], u[k]);" if dec_vec else "fmaf(x[k], y, u[k]);" if dec_sc else "x[k] + u[k];"))
+        # the next columns come in while these are split and stored
+        w("float z[16];")
+        w(f"if (n0 + 16 < {Np}) {{ frnn_tmem_ld<16>(mine + {colS}u + n0 + 16, z); frnn_tmem_ld<16>(mine + {colD}u + n0 + 16, u); }}")
+        put_state("(kc - 1)" if s.reverse else "(kc + 1)", f" && c + 1 < {nchunk}")
+        w("#pragma unroll")
+        w("for (int k = 0; k < 16; k++) x[k] = z[k];")
+        w.close()
+        w(f"frnn_tmem_wait_st(); frnn_tmem_fence_before_sync(); frnn_mbar_arrive(&bar[{B_SB + qi}]);")
+    w.close()     # chunk loop
+    w("frnn_tmem_wait_st();")
+    w("#pragma unroll 1")
+    w.open(f"for (int n0 = 0; n0 < {Np}; n0 += 16)")
+    w("float x[16];")
+    w(f"frnn_tmem_ld<16>(mine + {colS}u + n0, x);")
+    w("frnn_tmem_wait_ld();")
+    tile_io(s.final[0], s.final[1], "n0", 16, False)
+    w.close()
+    w.ind -= 1
+    w("};")
+    w("work();")
+    w("// done, normally or after a timed-out wait: check in, and the allocating warp frees Tensor Memory")
+    w("frnn_tmem_fence_before_sync();")
+    w("frnn_warp_sync();")
+    w("if (lane == 0) frnn_smem_add((int*)&bar[23], 1);")
+    w.open("if (warp == 0)")
+    w("const u64 t_exit = frnn_now_ns();")
+    w(f"while (frnn_smem_add((int*)&bar[23], 0) < {(128 + PT) // 32 + 4} && frnn_now_ns() - t_exit < 2 * FRNN_WAIT_LIMIT_NS) {{}}")
+    w("frnn_tmem_fence_after_sync();")
+    w(f"frnn_tmem_dealloc(tm, {tm_cols}u);")
+    w.close()
+    w.close()
+    return KernelSource(s.name, w.text().replace("@SMEM_BYTES@", str(smem_bytes)), (p.M // MB, p.H, p.B), 128 + PT + 128, smem_bytes,
+                        kb.params, kb.param_decl, {"chunk": C, "tile": [MB, N, C], "packed": False, "tmem_cols": tm_cols, "nck": nck,
+                                                   "tma_items": len(kb.tma_items), "plain_items": len(kb.plain_items)}, kb.tmaps)
+
+
+#: timesteps per chunk when the chunk boundaries are also the checkpoints of the backward pass
+CHUNK = 16
+
+
+def ck_bytes(p: Problem) -> int:
+    return p.B * p.H * ((p.T + CHUNK - 1) // CHUNK) * p.N * p.M * 4
+
+
+def rows_per_cta(M: int) -> Optional[int]:
+    """State rows of one CTA: all up to the 128 lanes of Tensor Memory, else a divisor of M."""
+    for mb in range(min(M, 128), 0, -1):
+        if M % mb == 0:
+            return mb if mb >= 16 or mb == M else None
+    return None
+
+
+def forward_spec(p: Problem, nf: Normal, saved: Sequence[int], train: bool) -> ScanSpec:
+    """The forward scan.  Parameters, in order: used inputs, initial state, outputs, final state and, for training,
+    checkpoints [B, H, chunk, N, M] and the row sums ``saved`` [len, B, H, T, M]; error word."""
+    yshape = (p.B, p.T, p.H, p.M)
+    used = nf_inputs(nf)
+    params = [(f"in{i}", "void", True, _spec_bytes(p.inputs[i])) for i in range(len(p.inputs)) if used[i]]
+    params.append(("s0", "void", True, _spec_bytes(p.states[0])))
+    params += [(f"out{j}", "void", False, p.B * p.T * p.H * p.M * ELT[p.out_dt[j]]) for j in range(len(nf.ys))]
+    params.append(("sT", "void", False, _spec_bytes(p.res_states[0])))
+    if train:
+        params.append(("ck", "float", False, ck_bytes(p)))
+        params.append(("aux", "float", False, len(saved) * p.B * p.H * p.T * p.M * 4))
+    params.append(("err", "int", False, 4))
+    outs = []
+    for j, y in enumerate(nf.ys):
+        ys = TensorSpec(yshape, _contig(yshape), p.out_dt[j])
+        outs.append((y, p.out_dt[j], f"out{j}", lambda t, ys=ys: _elem_off(ys, [(0, "b"), (1, t), (2, "h")]), 1))
+    if train:
+        for k, d in enumerate(saved):
+            outs.append((f"sig{d}", DT_F32, "aux", lambda t, k=k: aux_off(p, k, t), 1))
+    items, consts = staged_inputs(p, nf, used)
+    return ScanSpec("frnn_cfw", params, items, consts, nf.shape, nf.hoist, nf.row, nf.alphas, nf.kappas, nf.ps, nf.decay, nf.diags, nf.diag_at,
+                    outs, (p.states[0], "s0"), (p.res_states[0], "sT"), None, "ck" if train else None, False)
+
+
+def aux_off(p: Problem, k: int, t: str) -> str:
+    """Element offset of time t in the k-th member of a [*, B, H, T, M] fp32 buffer."""
+    return f"(((({k}L * {p.B} + b) * {p.H} + h) * {p.T}L + ({t})) * {p.M}L)"
+
+
+def dg_off(p: Problem, k: int, t: str) -> str:
+    """Element offset of dg<k> at time t in a [*, B, H, T] fp32 buffer."""
+    return f"((({k}L * {p.B} + b) * {p.H} + h) * {p.T}L + ({t}))"
+
+
+def aux_item(p: Problem, key: str, ptr: str, k: int) -> Staged:
+    sh = (p.B, p.H, p.T, p.M)
+    return Staged(key, M1, TensorSpec(sh, _contig(sh), DT_F32), ptr, {"b": 0, "h": 1, "t": 2, "v": 3}, k * p.B * p.H * p.T * p.M)
+
+
+def nf_inputs(nf: Normal) -> List[bool]:
+    read = {a for n in nf.hoist + nf.row for a in n.value_args()} | set(nf.ps) | set(nf.ys) | set(nf.alphas) | set(nf.kappas) | {nf.decay}
+    return [i in read for i in nf.inputs]
+
+
+def staged_inputs(p: Problem, nf: Normal, used: Sequence[bool]):
+    items, consts = [], []
+    for i, spec in enumerate(p.inputs):
+        if not used[i]:
+            continue
+        cls = p.in_cls(i)
+        if spec.shape[1] == 1 and p.T > 1:
+            if cls != S11:
+                raise lower.LoweringError("time-invariant vectors are not staged")
+            consts.append((nf.inputs[i], spec, f"in{i}"))
+        else:
+            items.append(Staged(nf.inputs[i], cls, spec, f"in{i}", lower._in_dims(cls)))
+    return items, consts
+
+
+# ---------------------------------------------------------------------------
+# backward: the scan of the state gradient, then the gradients of the vectors
+# ---------------------------------------------------------------------------
+
+@dataclass
+class BackwardPlan:
+    """How the backward pass of a normal form is divided.  ``vjp``: ``local_vjp``.  ``saved``: row sums the forward has to
+    keep; ``kept``: row sums of the state gradient that its scan keeps for the vector gradients."""
+    vjp: StepGraph
+    saved: List[int]
+    kept: List[int]
+    kept_dg: bool                             # the scan of the state gradient also keeps the dg<k>
+    dsig: List[Arg]
+    row_grads: List[Tuple[int, Arg]]          # (input, value): gradients of row-vector inputs
+    grads: List[Tuple[int, Arg]]              # the others
+    log_decay: bool
+
+
+def backward_plan(p: Problem, nf: Normal, v: StepGraph, log_decay: bool) -> Optional[BackwardPlan]:
+    """None when the gradients do not divide into row functions, vectors and scalars as the two kernels need it."""
+    nin, nd, nr = len(nf.inputs), len(nf.alphas), len(nf.kappas)
+    nodes = v.node_map()
+    late = [f"ga{d}" for d in range(nd)] + [f"gk{r}" for r in range(nr)] + ["gw"]
+    dep_late = v.depends_on([x for x in late if x in v.inputs])
+    msums = [n.name for n in v.nodes if n.op == "sum" and n.over_m]
+    nsums = [n.name for n in v.nodes if n.op == "sum" and n.over_n]
+    after_m = v.depends_on(msums)
+    after_n = v.depends_on(nsums + (["gw"] if nf.decay and nf.shape[nf.decay] == S11 else []))
+    for n in v.nodes:
+        if n.shape == MN or (n.op == "sum" and n.over_m and n.over_n):
+            return None
+        if n.shape == M1 and (n.name in dep_late or n.name in after_m or n.name in after_n):
+            return None
+        if n.shape == N1 and n.name in after_n:
+            return None
+        if n.op == "sum" and n.over_m and v.shape.get(n.args[0]) != M1:
+            return None
+        if n.op == "sum" and n.over_n and v.shape.get(n.args[0]) != N1:
+            return None
+    dsig = list(v.outputs[nin:])
+    row_grads, grads = [], []
+    for i in range(nin):
+        cls, o = p.in_cls(i), v.outputs[i]
+        s = v.shape[o] if isinstance(o, str) else S11
+        if cls == M1:
+            if isinstance(o, str) and s != M1:
+                return None
+            row_grads.append((i, o))
+        else:
+            if isinstance(o, str) and s != cls:
+                return None
+            grads.append((i, o))
+    if any(not isinstance(x, str) or v.shape[x] != M1 for x in dsig):
+        return None
+
+    def leaves(outs) -> set:
+        need = set(o for o in outs if isinstance(o, str))
+        for n in reversed(v.nodes):
+            if n.name in need:
+                need.update(n.value_args())
+        return need
+    k2 = leaves(dsig + [o for _, o in row_grads])
+    k3 = leaves(dsig + [o for _, o in grads])
+    rowdep = set()
+    pn = {n.name: n for n in nf.row}
+    todo = [x for x in nf.ps]
+    while todo:
+        a = todo.pop()
+        if isinstance(a, str) and a not in rowdep:
+            rowdep.add(a)
+            if a in pn:
+                todo += pn[a].value_args()
+    if any(f"dg{k}" in rowdep for k in range(len(nf.diags))):
+        return None
+    saved = [d for d in range(nd) if f"sig{d}" in (k2 | k3 | rowdep)]
+    kept = [r for r in range(nr) if f"gp{r}" in k3]
+    return BackwardPlan(v, saved, kept, any(f"dg{k}" in k3 for k in range(len(nf.diags))), dsig, row_grads, grads, log_decay)
+
+
+def backward_scan_spec(p: Problem, nf: Normal, bp: BackwardPlan, dspec: Sequence[TensorSpec]) -> ScanSpec:
+    """The scan of the state gradient E: E' = E * w + sum_d dsig_d (x) alpha_d with the row sums E . kappa_r, from the
+    last timestep to the first.  Parameters, in order: used inputs, d outputs, d final state, forward row sums, d initial
+    state, gradients of the row-vector inputs, checkpoints of E, kept row sums, error word."""
+    v, nin = bp.vjp, len(nf.inputs)
+    fs = {f"sig{d}": f"fsig{d}" for d in range(len(nf.alphas))}
+    fs.update({f"gp{r}": f"sig{r}" for r in range(len(nf.kappas))})
+    f = lambda a: fs.get(a, a) if isinstance(a, str) else a
+    outs = [o for o in bp.dsig + [o for _, o in bp.row_grads] if isinstance(o, str)]
+    g = v.pruned(outs)
+    shape = dict(nf.shape)
+    shape.update({f(k): s for k, s in v.shape.items()})
+    for d in range(len(nf.alphas)):
+        shape[f"fsig{d}"] = M1
+    for r in range(len(nf.kappas)):
+        shape[f"sig{r}"] = M1
+    dyn = {f"sig{r}" for r in range(len(nf.kappas))} | {f"dg{k}" for k in range(len(nf.diags))}
+    row, hoist = [], list(nf.hoist)
+    for n in g.nodes:
+        m = Node(f(n.name), n.op, [f(a) for a in n.args], n.shape)
+        if any(a in dyn for a in m.value_args()):
+            dyn.add(m.name)
+            row.append(m)
+        else:
+            hoist.append(m)
+    read = {a for n in hoist + row for a in n.value_args()} | {f(o) for o in outs} | set(nf.alphas) | set(nf.kappas) | {nf.decay}
+    # hoisted nodes that nothing here reads (row functions of the forward) are pruned by the emitter
+    keep, need = [], {a for n in row for a in n.value_args()} | {f(o) for o in outs} | set(nf.alphas) | set(nf.kappas) | set(nf.diags) | {nf.decay}
+    for n in reversed(hoist):
+        if n.name in need:
+            need.update(n.value_args())
+            keep.append(n)
+    hoist = keep[::-1]
+    used = [i in need for i in nf.inputs]
+    items, consts = staged_inputs(p, nf, used)
+    yshape = (p.B, p.T, p.H, p.M)
+    params = [(f"in{i}", "void", True, _spec_bytes(p.inputs[i])) for i in range(nin) if used[i]]
+    dys = [j for j in range(len(nf.ys)) if f"gy{j}" in need]
+    for j in dys:
+        params.append((f"dy{j}", "void", True, p.B * p.T * p.H * p.M * ELT[p.out_dt[j]]))
+        items.append(Staged(f"gy{j}", M1, TensorSpec(yshape, _contig(yshape), p.out_dt[j]), f"dy{j}", {"b": 0, "t": 1, "h": 2, "v": 3}))
+    sshape = (p.B, p.H, p.M, p.N)
+    params.append(("dsT", "void", True, p.B * p.H * p.M * p.N * ELT[p.states[0].dt]))
+    aux = [d for d in bp.saved if f"fsig{d}" in need]
+    if aux:
+        params.append(("aux", "float", True, len(bp.saved) * p.B * p.H * p.T * p.M * 4))
+        for d in aux:
+            items.append(aux_item(p, f"fsig{d}", "aux", bp.saved.index(d)))
+    params.append(("ds0", "void", False, _spec_bytes(p.res_states[0])))
+    louts = []
+    for i, o in bp.row_grads:
+        params.append((f"dx{i}", "void", False, _spec_bytes(dspec[i])))
+        if not isinstance(o, str):
+            raise lower.LoweringError("a constant gradient")
+        louts.append((f(o), dspec[i].dt, f"dx{i}", lambda t, sp=dspec[i]: _elem_off(sp, [(0, "b"), (1, t), (2, "h")]), dspec[i].st(3)))
+    params.append(("eck", "float", False, ck_bytes(p)))
+    if bp.kept:
+        params.append(("tau", "float", False, len(bp.kept) * p.B * p.H * p.T * p.M * 4))
+        for k, r in enumerate(bp.kept):
+            louts.append((f"sig{r}", DT_F32, "tau", lambda t, k=k: aux_off(p, k, t), 1))
+    if bp.kept_dg:
+        params.append(("dgk", "float", False, len(nf.diags) * p.B * p.H * p.T * 4))
+    params.append(("err", "int", False, 4))
+    return ScanSpec("frnn_cbw", params, items, consts, shape, hoist, row, nf.kappas, nf.alphas, [f(x) for x in bp.dsig], nf.decay,
+                    nf.diags, [(r, d) for d, r in nf.diag_at], louts, (TensorSpec(sshape, _contig(sshape), p.states[0].dt), "dsT"),
+                    (p.res_states[0], "ds0"), "dgk" if bp.kept_dg else None, "eck", True)
+
+
+VG_THREADS = 256
+
+
+def emit_vector_grads(p: Problem, nf: Normal, bp: BackwardPlan, dspec: Sequence[TensorSpec], atomic: Sequence[bool], C: int) -> KernelSource:
+    """Gradients of the column vectors and scalars, one CTA per chunk of ``C`` timesteps: with the state S_0 at the
+    chunk's start, the state gradient E_C at its end, X = dsig and Z = p (vectors over the rows, per timestep),
+
+      d alpha_d,j = W_j-1 * (S_0^T X_d,j) + sum_{i<j,r} L_dj,ri kappa_r,i W_j-1/W_i          L = X Z^T (over the rows)
+      d kappa_r,i = W_C/W_i * (E_C^T Z_r,i) + sum_{j>i,d} L_dj,ri alpha_d,j W_j-1/W_i
+      w_j d w_j   = R_j - sum_r kappa_r,j * d kappa_r,j,   R_j-1 = w_j d w_j + sum_d alpha_d,j * d alpha_d,j
+
+    (R_j: sums over the rows of E_j * S_j, at the chunk's end from S_0 and E_C), then the chain rule to the inputs
+    (``local_vjp``).  All products run on the tensor cores.  Where a decay of the chunk is too small to divide by, the
+    chunk takes a slower path of plain loops with running products instead.
+
+    Bound by HBM: S_0 and E_C are 2 x 4 M N bytes per C timesteps.  Two CTAs share an SM, so that one loads while the
+    other computes.  Parameters, in order: inputs, d outputs, forward row sums, kept row sums, checkpoints of S, of E,
+    gradients, error word.
+    """
+    v = bp.vjp
+    M, N, B, T, H = p.M, p.N, p.B, p.T, p.H
+    nd, nr = len(nf.alphas), len(nf.kappas)
+    nA, nK = nd * C, nr * C
+    dec_vec = bool(nf.decay) and nf.shape[nf.decay] == N1
+    dec_sc = bool(nf.decay) and not dec_vec
+    w = W()
+    nin = len(nf.inputs)
+    shape = dict(nf.shape)
+    shape.update(v.shape)
+    MS = 16 if M % 16 == 0 else 8
+    nsl = M // MS
+    # ---- stages
+    msums = [n for n in v.nodes if n.op == "sum" and n.over_m]
+    nsums = [n for n in v.nodes if n.op == "sum" and n.over_n]
+    gouts = [o for _, o in bp.grads if isinstance(o, str)]
+    need = set(gouts) | set(x for x in bp.dsig)
+    live_nodes = []
+    for n in reversed(v.nodes):
+        if n.name in need:
+            need.update(n.value_args())
+            live_nodes.append(n)
+    live_nodes.reverse()
+    msums = [n for n in msums if n.name in need]
+    nsums = [n for n in nsums if n.name in need]
+    g = StepGraph("v", v.inputs, live_nodes, gouts, dict(v.shape))
+    after_m = g.depends_on([n.name for n in msums])
+    after_n = g.depends_on([n.name for n in nsums] + (["gw"] if dec_sc else []))
+    # the forward's own nodes, and those of p
+    fnodes = {n.name: n for n in nf.hoist + nf.row}
+    # scalars of the first stage: forward ones and those of the vjp that depend on inputs and dg only
+    first_s = [n for n in list(nf.hoist) + live_nodes if n.shape == S11 and n.op != "sum" and n.name not in after_m and n.name not in after_n]
+    second_s = [n for n in live_nodes if n.shape == S11 and n.op != "sum" and n.name in after_m and n.name not in after_n]
+    third_s = [n for n in live_nodes if n.shape == S11 and n.op != "sum" and n.name in after_n]
+    s_inputs = [i for i in range(nin) if p.in_cls(i) == S11]
+    use_dg = [k for k in range(len(nf.diags)) if f"dg{k}" in need]
+    # ---- parameters
+    params, decl, nbytes = [], [], {}
+
+    def param(nm, ct, const, nb):
+        params.append(nm)
+        decl.append(f"{'const ' if const else ''}{ct}*{' __restrict__' if const else ''} {nm}")
+        nbytes[nm] = nb
+    for i in range(nin):
+        param(f"in{i}", "void", True, _spec_bytes(p.inputs[i]))
+    for j in range(len(nf.ys)):
+        param(f"dy{j}", "void", True, B * T * H * M * ELT[p.out_dt[j]])
+    if bp.saved:
+        param("aux", "float", True, len(bp.saved) * B * H * T * M * 4)
+    if bp.kept:
+        param("tau", "float", True, len(bp.kept) * B * H * T * M * 4)
+    if bp.kept_dg:
+        param("dgk", "float", True, len(nf.diags) * B * H * T * 4)
+    nchunk = (T + C - 1) // C
+    param("ck", "float", True, ck_bytes(p))
+    param("eck", "float", True, ck_bytes(p))
+    for i, _ in bp.grads:
+        param(f"dx{i}", "void", False, _spec_bytes(dspec[i]))
+    param("err", "int", False, 4)
+    # ---- shared memory
+    al = lambda x: (x + 127) // 128 * 128
+    sc_slots: Dict[str, int] = {}           # scalar arrays [C]
+
+    def slot(nm: str) -> str:
+        if nm not in sc_slots:
+            sc_slots[nm] = len(sc_slots)
+        return f"sc[{sc_slots[nm] * C}"
+    for i in s_inputs:
+        slot(nf.inputs[i])
+    for n in first_s + second_s + third_s:
+        slot(n.name)
+    for k in use_dg:
+        slot(f"dg{k}")
+    for n in msums:
+        slot(n.name)
+    want_gw = bool(nf.decay) and "gw" in need
+    n_nsum = len(nsums) + (2 if dec_sc and want_gw else 0)
+    for x in ("Wp", "Ws", "gw"):
+        slot(x)
+    npart = max(len(msums), n_nsum) + 1
+    HC = C // 2                              # timesteps of one thread: 128 rows or columns times two halves of the chunk
+    off_sc = 256
+    off_part = off_sc + al(len(sc_slots) * C * 4)
+    off_z0 = off_part + al(npart * 4 * C * 4)
+    off_xr = off_z0 + al(128 * 4)            # what the halves of a column exchange
+    off_X = off_xr + al(3 * 128 * 4)
+    lboX, lboZ, lboS = 2 * nA * 16 + 16, 2 * nK * 16 + 16, 128 * 16 + 16
+    off_Z = off_X + al((M // 4 - 1) * lboX + max(2048 + 16, lboX))
+    off_sl = off_Z + al(M // 4 * lboZ)
+    sl_bytes = al(MS // 4 * lboS)
+    end1 = off_sl + 4 * sl_bytes
+    # second phase, over the same memory
+    lboT, lbo1, lbo2 = 128 * 16, 2 * nA * 16, 2 * nK * 16
+    off_kT = off_X
+    kT_b, aT_b = nK // 4 * lboT, nA // 4 * lboT
+    off_aT = off_kT + 2 * kT_b
+    off_L1 = off_aT + 2 * aT_b
+    off_L2 = off_L1 + nK // 4 * lbo1
+    off_Lr = off_L2 + nA // 4 * lbo2
+    LS = nK + 1
+    off_slow = off_kT                        # the slow path's results, over the operands: (nA + nK + C) x 128 floats
+    smem_bytes = al(max(end1, off_Lr + nA * LS * 4))
+    slow_path = bool(nf.decay) and (dec_vec or want_gw)
+    if slow_path:
+        off_Lr = max(off_Lr, off_slow + (nA + nK + C) * 512)
+        smem_bytes = al(max(smem_bytes, off_Lr + nA * LS * 4))
+    cD1, cD2 = 0, 2 * nA
+    cL = cD2 + 2 * nK
+    # the parts from S_0 and E_C and those from L are scaled differently: decays per head keep both of L's apart, decays
+    # over columns (in the operands already) only kappa's; L itself is read before its space is written again
+    cD1b = cL if dec_sc else cD1
+    cD2b = (cL + (2 * nA if dec_sc else 0)) if nf.decay else cD2
+    tm_cols = _tmem_pow2(max(cL + 2 * nK, cD2b + 2 * nK))
+    if tm_cols > 256:
+        raise lower.LoweringError("the vector gradients of a chunk do not fit half of Tensor Memory")
+    ERR = lower.ERR_STAGE_TIMEOUT
+    full_n = N == 128
+    # loads are never predicated (the compiler would wait for each in turn): past the ends they repeat the last timestep,
+    # row or column, and a select drops what they bring
+    whole = T % C == 0
+    tq = lambda q: f"t0 + {q}" if whole else f"t0 + min({q}, nv - 1)"
+    live_n = " && ".join(([] if whole else ["q < nv"]) + ([] if full_n else ["ncol"])) or "true"
+    live_m = " && ".join(([] if whole else ["q < nv"]) + ([] if M == 128 else ["mrow"])) or "true"
+    sel = lambda live, e, z="0.0f": e if live == "true" else f"(live ? {e} : {z})"
+
+    w(lower._header(chunk_prelude()))
+    w(f"// vector gradients: B={B} T={T} H={H} M={M} N={N}; {C} steps per chunk, {nd} row sums, {nr} rank-1 terms")
+    w(f'extern "C" __global__ void __launch_bounds__({VG_THREADS}, 2)')
+    w.open(f"frnn_cvg({', '.join(decl)})")
+    w("FRNN_DYN_SMEM(smem);")
+    w("const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;")
+    w(f"const int kc = blockIdx.x, h = blockIdx.y, b = blockIdx.z, t0 = kc * {C}, nv = min({C}, {T} - t0); (void)nv;")
+    w("#ifdef FRNN_BOUNDS")
+    w.open("if (tid == 0)")
+    w("frnn_bounds_begin(err, smem, @SMEM_BYTES@L);")
+    for nm, nb in nbytes.items():
+        w(f"frnn_bounds_add({nm}, {nb}L);")
+    w.close()
+    w("frnn_block_sync();")
+    w("#endif")
+    w("u64* bar = (u64*)smem;")
+    w(f"float* sc = (float*)(smem + {off_sc});")
+    w(f"float* part = (float*)(smem + {off_part});")
+    w(f"float* z0 = (float*)(smem + {off_z0}); (void)z0;")
+    w(f"float* xr = (float*)(smem + {off_xr}); (void)xr;")
+
+    def in_off(i: int, t: str, extra: str = "") -> str:
+        sp = p.inputs[i]
+        o = _elem_off(sp, [(0, "b"), (1, t), (2, "h")])
+        return o + (f" + (long)({extra}) * {sp.st(4 if p.in_cls(i) == N1 else 3)}L" if extra else "")
+    by_in = {nm: i for i, nm in enumerate(nf.inputs)}
+
+    def leaf(a: str, t: str, idx: str) -> Optional[str]:
+        """Load expression of a per-timestep vector that comes from global memory."""
+        if a in by_in:
+            i = by_in[a]
+            return f"frnn_io<{p.inputs[i].dt}>::ld(in{i}, {in_off(i, t, idx)})"
+        if a.startswith("gy"):
+            j = int(a[2:])
+            return f"frnn_io<{p.out_dt[j]}>::ld(dy{j}, ((((long)b * {T} + {t}) * {H} + h) * {M}L + {idx}))"
+        if a.startswith("sig") or a.startswith("gp"):
+            k, ptr = (bp.saved.index(int(a[3:])), "aux") if a.startswith("sig") else (bp.kept.index(int(a[2:])), "tau")
+            return f"frnn_ld_raw<float>({ptr}, (((({k}L * {B} + b) * {H} + h) * {T}L + {t}) * {M}L + {idx}))"
+        return None
+    all_nodes = {n.name: n for n in live_nodes}
+    all_nodes.update(fnodes)
+
+    def leaves_of(names: Sequence[Arg], cls: Shape, given: Sequence[str] = ()) -> List[str]:
+        out: List[str] = []
+
+        def visit(a):
+            if not isinstance(a, str) or a in given or shape[a] != cls:
+                return
+            if a in all_nodes:
+                for x in all_nodes[a].args:
+                    visit(x)
+            elif a not in out:
+                out.append(a)
+        for a in names:
+            visit(a)
+        return out
+
+    class Stage:
+        """Values of one timestep: scalars from shared memory, vectors from the registers ``regs`` names."""
+
+        def __init__(self, pre: str, q: str, cls: Shape, regs: Dict[str, str]):
+            self.pre, self.q, self.cls, self.done = pre, q, cls, dict(regs)
+
+        def get(self, a) -> str:
+            if not isinstance(a, str):
+                return lower.flit(a)
+            if a in self.done:
+                return self.done[a]
+            if shape[a] == S11:
+                if a not in sc_slots:
+                    raise lower.LoweringError(f"scalar {a} is not available at this stage")
+                self.done[a] = f"{slot(a)} + {self.q}]"
+                return self.done[a]
+            if shape[a] != self.cls or a not in all_nodes:
+                raise lower.LoweringError(f"{a} is not available at this stage")
+            nm = self.pre + a.replace(".", "_")
+            ops = [self.get(x) for x in all_nodes[a].args]
+            w(f"const float {nm} = {op_expr(all_nodes[a], ops)};")
+            self.done[a] = nm
+            return nm
+
+    def reduce_lanes(arr: str, cnt: int, dst: str):
+        """Sum ``arr[cnt]`` over the lanes of a warp, all values at once; ``dst`` receives value @."""
+        c, o, idx = cnt, 16, []
+        while c > 1 and o >= 1:
+            hf = c // 2
+            w("#pragma unroll")
+            w(f"for (int k = 0; k < {hf}; k++) {{ const bool up = lane & {o}; const float snd = up ? {arr}[k] : {arr}[k + {hf}], own = up ? {arr}[k + {hf}] : {arr}[k]; "
+              f"{arr}[k] = own + frnn_shfl_xor(snd, {o}); }}")
+            idx.append((o, hf))
+            c, o = hf, o // 2
+        mask = 0
+        while o >= 1:
+            w(f"{arr}[0] += frnn_shfl_xor({arr}[0], {o});")
+            mask |= o
+            o //= 2
+        e = " + ".join(f"((lane & {o_}) ? {hf} : 0)" for o_, hf in idx) or "0"
+        w(f"if ((lane & {mask}) == 0) {dst.replace('@', '(' + e + ')')} = {arr}[0];")
+
+    def scalar_nodes(nodes, q="q"):
+        for n in nodes:
+            w(f"{slot(n.name)} + {q}] = {op_expr(n, [lower.flit(a) if not isinstance(a, str) else f'{slot(a)} + {q}]' for a in n.args])};")
+
+    # ---- what can be loaded at once: the rows' vectors, the first slices of S_0 and E_C
+    w(f"const int x128 = tid & 127, hf = tid >> 7, q0 = hf * {HC};")
+    w(f"const int mc = {'x128' if M == 128 else f'min(x128, {M - 1})'}, nc = {'x128' if full_n else f'min(x128, {N - 1})'};")
+    w(f"const bool mrow = x128 < {M}, ncol = x128 < {N}; (void)mrow; (void)ncol; (void)nc;")
+    mleaves = leaves_of(list(bp.dsig) + list(nf.ps) + [n.args[0] for n in msums], M1)
+    reg = lambda a: "r_" + a.replace(".", "_")
+    for a in mleaves:
+        w(f"float {reg(a)}[{HC}];")
+    w("#pragma unroll")
+    w.open(f"for (int k = 0; k < {HC}; k++)")
+    w(f"const int t = {tq('q0 + k')};")
+    for a in mleaves:
+        w(f"{reg(a)}[k] = {leaf(a, 't', 'mc')};")
+    w.close()
+    q4 = MS // 4
+    per = 128 // (VG_THREADS // q4)        # columns per thread and slice
+    w(f"const int sm4 = tid % {q4}, sn = tid / {q4};")
+    w(f"const float* ckp = ck + (((long)b * {H} + h) * {nchunk} + kc) * {N}L * {M}L; const float* ekp = eck + (((long)b * {H} + h) * {nchunk} + kc) * {N}L * {M}L;")
+    w(f"float zz[{per}], sv[2][{per}][4], ev[2][{per}][4];")
+    w("#pragma unroll")
+    w(f"for (int i = 0; i < {per}; i++) zz[i] = 0.0f;")
+
+    def load_slice(sx, u):
+        w("#pragma unroll")
+        w.open(f"for (int i = 0; i < {per}; i++)")
+        w(f"const int n = {'sn' if full_n else 'min(sn'} + i * {VG_THREADS // q4}{'' if full_n else f', {N - 1})'};")
+        w(f"frnn_ldv<0,4>(ckp, n * {M}L + ({sx}) * {MS} + sm4 * 4, sv[{u}][i]);")
+        w(f"frnn_ldv<0,4>(ekp, n * {M}L + ({sx}) * {MS} + sm4 * 4, ev[{u}][i]);")
+        w.close()
+    load_slice("0", "0")
+    if nsl > 1:
+        load_slice("1", "1")
+    w("if (tid == 0) { frnn_mbar_init(&bar[0], 1); frnn_mbar_init(&bar[1], 1); frnn_mbar_init(&bar[2], 1); ((int*)&bar[4])[0] = 0; frnn_mbar_init_fence(); }")
+    w.open("if (warp == 0)")
+    w(f"frnn_tmem_alloc((u32*)&bar[3], {tm_cols}u);")
+    w("frnn_tmem_fence_before_sync();")
+    w.close()
+    # ---- scalars of the inputs, decay products
+    w.open(f"if (tid >= 32 && tid < {32 + C})")
+    w(f"const int q = tid - 32, t = {'t0 + q' if whole else 't0 + min(q, nv - 1)'}; (void)t;")
+    for i in s_inputs:
+        w(f"{slot(nf.inputs[i])} + q] = frnn_io<{p.inputs[i].dt}>::ld(in{i}, {in_off(i, 't')});")
+    for k in use_dg:
+        w(f"{slot(f'dg{k}')} + q] = frnn_ld_raw<float>(dgk, {dg_off(p, k, 't')});")
+    scalar_nodes(first_s)
+    if dec_sc:
+        w("frnn_half_warp_sync();")
+        w("float a = 1.0f, c = 1.0f;")
+        w("#pragma unroll")
+        w(f"for (int l = 0; l < {C}; l++) {{ const float x = {slot(nf.decay)} + l]; if (l < q) a *= x; if (l > q && l < nv) c *= x; }}")
+        w(f"{slot('Wp')} + q] = a; {slot('Ws')} + q] = c;")
+        if want_gw:
+            # the gradient of a decay per head divides by it only where the step reads it as it is (an exponential's does not)
+            cond = f"!(fabsf({slot(nf.decay)} + q]) > 0.0009765625f)"
+            if not bp.log_decay:
+                w(f"if (q < nv && {cond}) *(volatile int*)&bar[4] = 1;")
+    w.close()
+    w("frnn_block_sync();")
+    w("frnn_tmem_fence_after_sync();")
+    w("const u32 tm = *(volatile u32*)&bar[3];")
+    # ---- rows: X, Z and the sums over the rows
+    w.open("")
+    for x in range(len(msums)):
+        w(f"float e{x}[{HC}];")
+    w("#pragma unroll")
+    w.open(f"for (int k = 0; k < {HC}; k++)")
+    w(f"const int q = q0 + k; const bool live = {live_m}; (void)live;")
+    st = Stage("x_", "q", M1, {a: f"{reg(a)}[k]" for a in mleaves})
+    vals = [(f"{d * C}", st.get(x), "X") for d, x in enumerate(bp.dsig)] + [(f"{r * C}", st.get(x), "Z") for r, x in enumerate(nf.ps)]
+    for x, n in enumerate(msums):
+        w(f"e{x}[k] = {sel(live_m, st.get(n.args[0]))};")
+    w.open(f"if (mrow)" if M < 128 else "")
+    for base, val, which in vals:
+        lbo, off, n2 = (lboX, off_X, nA) if which == "X" else (lboZ, off_Z, nK)
+        w(f"{{ const float a = {sel(live_m, val)}, hi = a; unsigned char* dst = smem + {off} + (x128 >> 2) * {lbo} + (x128 & 3) * 4; "
+          f"const int r0 = {base} + q, r1 = r0 + {n2}; *(float*)(dst + (r0 >> 3) * 128 + (r0 & 7) * 16) = hi; *(float*)(dst + (r1 >> 3) * 128 + (r1 & 7) * 16) = frnn_tf32_rest(a); }}")
+    w.close()
+    w.close()
+    for x in range(len(msums)):
+        reduce_lanes(f"e{x}", HC, f"part[{x * 4 * C} + (warp & 3) * {C} + q0 + @]")
+    w.close()
+    w("frnn_async_proxy_fence();")
+    w("frnn_block_sync();")
+    w(f"const u64 dX = frnn_mma_desc(smem + {off_X}, {lboX}), dZ = frnn_mma_desc(smem + {off_Z}, {lboZ});")
+    w.open("if (tid == 0)")
+    w("#pragma unroll")
+    w(f"for (int k = 0; k < {M // 8}; k++) frnn_mma_ss_d(tm + {cL}u, frnn_mma_next(dX, {lboX}, k), frnn_mma_next(dZ, {lboZ}, k), FRNN_MMA_IDESC({2 * nK}), k > 0);")
+    w("frnn_mma_commit(&bar[0]);")
+    w.close()
+    # ---- second-stage scalars
+    w.open(f"if (tid >= 32 && tid < {32 + C})")
+    w("const int q = tid - 32; (void)q;")
+    for x, n in enumerate(msums):
+        w(f"{slot(n.name)} + q] = (part[{x * 4 * C} + q] + part[{x * 4 * C + C} + q]) + (part[{x * 4 * C + 2 * C} + q] + part[{x * 4 * C + 3 * C} + q]);")
+    scalar_nodes(second_s)
+    w.close()
+    # ---- S_0 and E_C, a slice of rows at a time, loaded two slices ahead
+    colv = nf.alphas + nf.kappas + ([nf.decay] if dec_vec else [])
+    ngiven = [f"ga{d}" for d in range(nd)] + [f"gk{r}" for r in range(nr)] + ["gw"]
+    n_outs = [o for i, o in bp.grads if p.in_cls(i) == N1]
+    nleaves = leaves_of(list(colv) + [n.args[0] for n in nsums] + n_outs, N1, ngiven)
+    wleaves = leaves_of([nf.decay], N1) if dec_vec else []
+    for a in nleaves:
+        w(f"float {reg(a)}[{HC}];")
+    for a in wleaves:
+        w(f"float o_{reg(a)}[{HC}];          // the other half's timesteps")
+    w.open(f"for (int s2 = 0; s2 < {nsl}; s2 += 2)")
+    for u in (0, 1):
+        w.open(f"if (s2 + {u} < {nsl})")
+        w(f"const int s = s2 + {u};")
+        w(f"if (s > 0 && !frnn_mbar_wait(&bar[1], (s - 1) & 1, err, {ERR})) break;     // products of the previous slice are complete")
+        w("#pragma unroll")
+        w.open(f"for (int i = 0; i < {per}; i++)")
+        w(f"const int n = sn + i * {VG_THREADS // q4};")
+        w(f"unsigned char* dst = smem + {off_sl} + sm4 * {lboS} + (n >> 3) * 128 + (n & 7) * 16;")
+        w("float r[4];")
+        w("#pragma unroll")
+        w(f"for (int k = 0; k < 4; k++) {{ r[k] = frnn_tf32_rest(sv[{u}][i][k]); zz[i] = fmaf(sv[{u}][i][k], ev[{u}][i][k], zz[i]); }}")
+        w(f"frnn_stv<0,4>(dst, 0, sv[{u}][i]); frnn_stv<0,4>(dst + {sl_bytes}, 0, r);")
+        w("#pragma unroll")
+        w(f"for (int k = 0; k < 4; k++) r[k] = frnn_tf32_rest(ev[{u}][i][k]);")
+        w(f"frnn_stv<0,4>(dst + {2 * sl_bytes}, 0, ev[{u}][i]); frnn_stv<0,4>(dst + {3 * sl_bytes}, 0, r);")
+        w.close()
+        w(f"if (s + 2 < {nsl}) {{")
+        w.ind += 1
+        load_slice("s + 2", str(u))
+        w.ind -= 1
+        w("}")
+        w("frnn_async_proxy_fence();")
+        w("frnn_block_sync();")
+        w.open("if (tid == 0)")
+        for k in range(MS // 8):
+            for which, (col_, dsc, lbo, n2) in enumerate(((cD1, "dX", lboX, nA), (cD2, "dZ", lboZ, nK))):
+                sb = off_sl + 2 * which * sl_bytes + k * 2 * lboS
+                bexp = f"frnn_mma_next({dsc}, {lbo}, s * {MS // 8} + {k})"
+                w(f"frnn_mma_ss_d(tm + {col_}u, frnn_mma_desc(smem + {sb}, {lboS}), {bexp}, FRNN_MMA_IDESC({2 * n2}), {'s > 0' if k == 0 else 'true'});")
+                w(f"frnn_mma_ss_d(tm + {col_}u, frnn_mma_desc(smem + {sb + sl_bytes}, {lboS}), {bexp}, FRNN_MMA_IDESC({2 * n2}), true);")
+        w("frnn_mma_commit(&bar[1]);")
+        w.close()
+        w.close()
+    w.close()
+    # the columns' vectors come in while the last products run
+    w("#pragma unroll")
+    w.open(f"for (int k = 0; k < {HC}; k++)")
+    w(f"const int t = {tq('q0 + k')};")
+    for a in nleaves:
+        w(f"{reg(a)}[k] = {leaf(a, 't', 'nc')};")
+    if wleaves:
+        w(f"const int to = {tq(f'({HC} - q0) + k')};")
+        for a in wleaves:
+            w(f"o_{reg(a)}[k] = {leaf(a, 'to', 'nc')};")
+    w.close()
+    if nf.decay:
+        w("#pragma unroll")
+        w.open(f"for (int i = 0; i < {per}; i++)")
+        w("#pragma unroll")
+        w(f"for (int o = {q4 // 2}; o > 0; o >>= 1) zz[i] += frnn_shfl_xor(zz[i], o);")
+        w(f"if (sm4 == 0) z0[sn + i * {VG_THREADS // q4}] = zz[i];")
+        w.close()
+    w(f"bool ok = frnn_mbar_wait(&bar[0], 0, err, {ERR}) && frnn_mbar_wait(&bar[1], {(nsl - 1) & 1}, err, {ERR});")
+    w("frnn_tmem_fence_after_sync();")
+    w("frnn_block_sync();       // X, Z and the slices are no longer read")
+    w("const u32 lanes = tm + frnn_tmem_lane_base(warp);")
+    w(f"float* Lr = (float*)(smem + {off_Lr});")
+    # ---- L: rows (d, j) of hi and of rest, columns (r, i) of hi and of rest
+    w.open(f"if (tid >= {nA // 32 * 32} && tid < {(2 * nA + 31) // 32 * 32})")
+    w(f"float u[{nK}];")
+    w(f"frnn_tmem_ld<{nK}>(lanes + {cL}u, u); frnn_tmem_wait_ld();")
+    w("#pragma unroll")
+    w(f"for (int i = 0; i < {nK}; i++) if (tid >= {nA} && tid < {2 * nA}) Lr[(tid - {nA}) * {LS} + i] = u[i];")
+    w.close()
+    w("frnn_block_sync();")
+    w.open(f"if (tid < {(nA + 31) // 32 * 32})")
+    w(f"float u[{nK}], x[{nK}];")
+    w(f"frnn_tmem_ld<{nK}>(lanes + {cL}u, u); frnn_tmem_ld<{nK}>(lanes + {cL + nK}u, x); frnn_tmem_wait_ld();")
+    w.open(f"if (tid < {nA})")
+    w(f"const int j = tid % {C};")
+    if dec_sc:
+        w("float D = 1.0f;")
+    w("#pragma unroll")
+    w.open(f"for (int i = {C - 1}; i >= 0; i--)")
+    w("#pragma unroll")
+    w.open(f"for (int r = 0; r < {nr}; r++)")
+    w(f"const int ri = r * {C} + i;")
+    w(f"float a = i < j ? u[ri] + x[ri] + Lr[tid * {LS} + ri] : 0.0f;")
+    w(f"Lr[tid * {LS} + ri] = a;")
+    if dec_sc:
+        w("a *= D;")
+    w("const float hi = a, lo = frnn_tf32_rest(a);")
+    w(f"unsigned char* d1 = smem + {off_L1} + (ri >> 2) * {lbo1} + (ri & 3) * 4; const int ra = tid, rb = tid + {nA};")
+    w("*(float*)(d1 + (ra >> 3) * 128 + (ra & 7) * 16) = hi; *(float*)(d1 + (rb >> 3) * 128 + (rb & 7) * 16) = lo;")
+    w(f"unsigned char* d2 = smem + {off_L2} + (tid >> 2) * {lbo2} + (tid & 3) * 4; const int rc = ri, rd = ri + {nK};")
+    w("*(float*)(d2 + (rc >> 3) * 128 + (rc & 7) * 16) = hi; *(float*)(d2 + (rd >> 3) * 128 + (rd & 7) * 16) = lo;")
+    w.close()
+    if dec_sc:
+        w(f"if (i < j && i < nv) D *= {slot(nf.decay)} + i];")
+    w.close()
+    w.close()
+    w.close()
+    # ---- operands over the columns: kappa (over W) and alpha (times W), this thread's half of the timesteps
+    if dec_vec:
+        w(f"float xw[{HC}], pre = 1.0f, post = 1.0f, rpre = 1.0f; bool tiny = false;   // decays; products of the other half's")
+        w("#pragma unroll")
+        w.open(f"for (int k = 0; k < {HC}; k++)")
+        w.open("")
+        w(f"const int q = q0 + k; const bool live = {live_n}; (void)live;")
+        e = Stage("x_", "q", N1, {a: f"{reg(a)}[k]" for a in nleaves}).get(nf.decay)
+        w(f"xw[k] = {sel(live_n, e, '1.0f')};")
+        tiny = "1e-25f" if bp.log_decay or not want_gw else "0.0009765625f"
+        w(f"tiny = tiny || !(fabsf(xw[k]) > {tiny});")
+        w.close()
+        w.open("")
+        w(f"const int q = ({HC} - q0) + k; const bool live = {live_n}; (void)live;")
+        e = Stage("x_", "q", N1, {a: f"o_{reg(a)}[k]" for a in wleaves}).get(nf.decay)
+        w(f"const float y = {sel(live_n, e, '1.0f')};")
+        w("if (hf) { pre *= y; rpre *= frnn_rcp1(y); } else post *= y;")
+        w.close()
+        w.close()
+        w("float rw = rpre, pw = pre;")
+    w("#pragma unroll")
+    w.open(f"for (int k4 = 0; k4 < {HC}; k4 += 4)")
+    names = nf.kappas + nf.alphas
+    w(f"float x[{len(names)}][4];")
+    w("#pragma unroll")
+    w.open("for (int k = 0; k < 4; k++)")
+    w(f"const int q = q0 + k4 + k; const bool live = {live_n}; (void)live; (void)q;")
+    st = Stage("x_", "q", N1, {a: f"{reg(a)}[k4 + k]" for a in nleaves})
+    if dec_vec:
+        w("rw *= frnn_rcp1(xw[k4 + k]); tiny = tiny || !(fabsf(rw) < 1e25f);")
+    for x, nm in enumerate(names):
+        f = "" if not dec_vec else (" * rw" if x < nr else " * pw")
+        w(f"x[{x}][k] = {sel(live_n, st.get(nm) + f)};")
+    if dec_vec:
+        w("pw *= xw[k4 + k];")
+    w.close()
+    for x in range(len(names)):
+        off, tb, r = (off_kT, kT_b, x) if x < nr else (off_aT, aT_b, x - nr)
+        w(f"{{ float hi[4]; unsigned char* dst = smem + {off} + (({r * C} + q0 + k4) >> 2) * {lboT} + (x128 >> 3) * 128 + (x128 & 7) * 16;")
+        w("#pragma unroll")
+        w(f"for (int k = 0; k < 4; k++) {{ hi[k] = x[{x}][k]; x[{x}][k] = frnn_tf32_rest(hi[k]); }}")
+        w(f"frnn_stv<0,4>(dst, 0, hi); frnn_stv<0,4>(dst + {tb}, 0, x[{x}]); }}")
+    w.close()
+    if dec_vec:
+        w("if (tiny) *(volatile int*)&bar[4] = 1;")
+    w("frnn_async_proxy_fence(); frnn_tmem_fence_before_sync();")
+    w("frnn_block_sync();")
+    w("const bool slow = *(volatile int*)&bar[4] != 0; (void)slow;")
+    w.open("if (tid == 0 && ok)" if not dec_vec else "if (tid == 0 && ok && !slow)")
+    w("frnn_tmem_fence_after_sync();")
+    for (cd, offA, tb, nk, offB, lboB, n2) in ((cD1b, off_kT, kT_b, nK, off_L1, lbo1, nA), (cD2b, off_aT, aT_b, nA, off_L2, lbo2, nK)):
+        acc0 = "k > 0" if cd not in (cD1, cD2) else "true"
+        for part_, n_, acc in ((offA, 2 * n2, acc0), (offA + tb, 2 * n2, "true")):
+            w(f"{{ const u64 da = frnn_mma_desc(smem + {part_}, {lboT}), db = frnn_mma_desc(smem + {offB}, {lboB});")
+            w("#pragma unroll")
+            w(f"for (int k = 0; k < {nk // 8}; k++) frnn_mma_ss_d(tm + {cd}u, frnn_mma_next(da, {lboT}, k), frnn_mma_next(db, {lboB}, k), FRNN_MMA_IDESC({n_}), {acc}); }}")
+    w.close()
+    w("if (tid == 0) frnn_mma_commit(&bar[2]);")
+    w(f"ok = frnn_mbar_wait(&bar[2], 0, err, {ERR}) && ok;")
+    w("frnn_tmem_fence_after_sync();")
+    # ---- columns: this thread's half of the timesteps
+    w(f"float da[{nd * HC}], dk[{nr * HC}], R = 0.0f; (void)R;")
+
+    def ld_half(dst: str, vecs: int, col0: int, rest: int, add: bool = False):
+        """dst[v * HC + k] = value of vector v at timestep q0 + k: the sum of two accumulator columns."""
+        w.open("")
+        w(f"float u[{vecs * HC}], lo[{vecs * HC}];")
+        for x in range(vecs):
+            w(f"frnn_tmem_ld<{HC}>(lanes + {col0 + x * C}u + (u32)q0, &u[{x * HC}]); frnn_tmem_ld<{HC}>(lanes + {col0 + rest + x * C}u + (u32)q0, &lo[{x * HC}]);")
+        w("frnn_tmem_wait_ld();")
+        w("#pragma unroll")
+        w(f"for (int k = 0; k < {vecs * HC}; k++) {dst}[k] {'+=' if add else '='} u[k] + lo[k];")
+        w.close()
+    if slow_path:
+        emit_slow_columns(w, C, nd, nr, nA, nK, tq, live_n, sel, nf, bp, dec_vec, want_gw, Stage, leaf, leaves_of, slot, LS, cD1, cD2, off_slow)
+    ld_half("da", nd, cD1, nA)
+    ld_half("dk", nr, cD2, nK)
+    if nf.decay:
+        if dec_sc:
+            w(f"float xw[{HC}], pre = {slot('Wp')} + q0], post = {slot('Ws')} + q0 + {HC - 1}];")
+            w("#pragma unroll")
+            w.open(f"for (int k = 0; k < {HC}; k++)")
+            w(f"xw[k] = " + (f"{slot(nf.decay)} + q0 + k];" if whole else f"q0 + k < nv ? {slot(nf.decay)} + q0 + k] : 1.0f;"))
+            w.close()
+        w.open("")
+        w("float a = post;")
+        w("#pragma unroll")
+        w(f"for (int k = {HC - 1}; k >= 0; k--) {{ " + " ".join(f"dk[{r * HC} + k] *= a;" for r in range(nr)) + " a *= xw[k]; }")
+        if want_gw:
+            # R_C = W_C Z + sum kappa (W_C / W) (E^T p)
+            w("R = (ncol && hf == 0) ? z0[x128] * a : 0.0f;")
+            w("#pragma unroll")
+            w.open(f"for (int k = 0; k < {HC}; k++)")
+            w(f"const int q = q0 + k; const bool live = {live_n}; (void)live; (void)q;")
+            st = Stage("x_", "q", N1, {a: f"{reg(a)}[k]" for a in nleaves})
+            for r, nm in enumerate(nf.kappas):
+                w(f"R = fmaf({st.get(nm)}, {sel(live_n, f'dk[{r * HC} + k]')}, R);")
+            w.close()
+        w("a = pre;")
+        w("#pragma unroll")
+        w(f"for (int k = 0; k < {HC}; k++) {{ " + " ".join(f"da[{d * HC} + k] *= a;" for d in range(nd)) + " a *= xw[k]; }")
+        if dec_vec:
+            w(f"float y[{nr * HC}], ra = rpre;")
+            ld_half("y", nr, cD2b, nK)
+            w("#pragma unroll")
+            w(f"for (int k = 0; k < {HC}; k++) {{ ra *= frnn_rcp1(xw[k]); " + " ".join(f"dk[{r * HC} + k] = fmaf(y[{r * HC} + k], ra, dk[{r * HC} + k]);" for r in range(nr)) + " }")
+        else:
+            ld_half("da", nd, cD1b, nA, add=True)
+            ld_half("dk", nr, cD2b, nK, add=True)
+        w.close()
+    if slow_path:
+        w(f"const float* sl = (const float*)(smem + {off_slow});")
+    if dec_vec:
+        w.open("if (slow)")
+        w("#pragma unroll")
+        w.open(f"for (int k = 0; k < {HC}; k++)")
+        w(" ".join(f"da[{d * HC} + k] = sl[({d * C} + q0 + k) * 128 + x128];" for d in range(nd)) + " "
+          + " ".join(f"dk[{r * HC} + k] = sl[({nA + r * C} + q0 + k) * 128 + x128];" for r in range(nr)))
+        w.close()
+        w.close()
+    if dec_vec and want_gw:
+        # the upper half's part of the sums that lead from R_C to the lower half
+        w("float P = 0.0f;")
+        w("#pragma unroll")
+        w.open(f"for (int k = 0; k < {HC}; k++)")
+        w(f"const int q = q0 + k; const bool live = {live_n}; (void)live; (void)q;")
+        st = Stage("x_", "q", N1, {a: f"{reg(a)}[k]" for a in nleaves})
+        kd = " + ".join(f"{st.get(nm)} * dk[{r * HC} + k]" for r, nm in enumerate(nf.kappas))
+        ad = " + ".join(f"{st.get(nm)} * da[{d * HC} + k]" for d, nm in enumerate(nf.alphas))
+        w(f"P += {sel(live_n, f'(({ad}) - ({kd}))')};")
+        w.close()
+        w("xr[hf * 128 + x128] = R; if (hf) xr[256 + x128] = P;")
+        w("frnn_block_sync();")
+        w("R = xr[x128] + xr[128 + x128] + (hf ? 0.0f : xr[256 + x128]);")
+    for x in range(n_nsum):
+        w(f"float e{x}[{HC}];")
+    w("#pragma unroll")
+    w.open(f"for (int k = {HC - 1}; k >= 0; k--)")
+    w(f"const int q = q0 + k, t = t0 + q; const bool live = {live_n}; (void)t; (void)live;")
+    given = {f"ga{d}": f"da[{d * HC} + k]" for d in range(nd)}
+    given.update({f"gk{r}": f"dk[{r * HC} + k]" for r in range(nr)})
+    given.update({a: f"{reg(a)}[k]" for a in nleaves})
+    st = Stage("x_", "q", N1, given)
+    if want_gw:
+        kd = " + ".join(f"{st.get(nm)} * dk[{r * HC} + k]" for r, nm in enumerate(nf.kappas))
+        ad = " + ".join(f"{st.get(nm)} * da[{d * HC} + k]" for d, nm in enumerate(nf.alphas))
+        gws = f"sl[({nA + nK} + q) * 128 + x128]"
+        if dec_vec:
+            w(f"const float wdw = R - {sel(live_n, f'({kd})')};")
+            w(f"R = wdw + {sel(live_n, f'({ad})')};")
+            w(f"const float gw = slow ? {gws} : " + ("wdw;" if bp.log_decay else "frnn_divf(wdw, xw[k]);"))
+            st.done["gw"] = "gw"
+        else:
+            w(f"e{n_nsum - 2}[k] = {sel(live_n, f'(slow ? {gws} : {kd})')}; e{n_nsum - 1}[k] = {sel(live_n, f'({ad})')};")
+    for x, n in enumerate(nsums):
+        w(f"e{x}[k] = {sel(live_n, st.get(n.args[0]))};")
+    for i, o in bp.grads:
+        if p.in_cls(i) != N1:
+            continue
+        val = st.get(o)
+        sp = dspec[i]
+        w(f"{'' if live_n == 'true' else 'if (live) '}frnn_io<{sp.dt}>::st(dx{i}, {_elem_off(sp, [(0, 'b'), (1, 't'), (2, 'h')])} + (long)x128 * {sp.st(4)}L, {val});")
+    w.close()
+    for x in range(n_nsum):
+        reduce_lanes(f"e{x}", HC, f"part[{x * 4 * C} + (warp & 3) * {C} + q0 + @]")
+    if dec_sc and want_gw:
+        w("#pragma unroll")
+        w("for (int o = 16; o > 0; o >>= 1) R += frnn_shfl_xor(R, o);")
+        w(f"if (lane == 0) part[{n_nsum * 4 * C} + warp] = R;")
+    w("frnn_tmem_fence_before_sync();")
+    w("frnn_block_sync();")
+    w(f"if (warp == 0) frnn_tmem_dealloc(tm, {tm_cols}u);")
+    # ---- scalars
+    total = lambda x, q: f"((part[{x * 4 * C} + {q}] + part[{x * 4 * C + C} + {q}]) + (part[{x * 4 * C + 2 * C} + {q}] + part[{x * 4 * C + 3 * C} + {q}]))"
+    sgrads = [(i, o) for i, o in bp.grads if p.in_cls(i) == S11]
+    if sgrads:
+        w.open(f"if (tid >= 32 && tid < {32 + C})")
+        w("const int q = tid - 32, t = t0 + q; const bool live = q < nv; (void)t;")
+        for x, n in enumerate(nsums):
+            w(f"{slot(n.name)} + q] = {total(x, 'q')};")
+        if dec_sc and want_gw:
+            w("float R = 0.0f, wdw = 0.0f;")
+            w("#pragma unroll")
+            w(f"for (int k = 0; k < {VG_THREADS // 32}; k++) R += part[{n_nsum * 4 * C} + k];")
+            w(f"for (int l = nv - 1; l >= q; l--) {{ wdw = R - {total(n_nsum - 2, 'l')}; R = wdw + {total(n_nsum - 1, 'l')}; }}")
+            w(f"{slot('gw')} + q] = slow ? {total(n_nsum - 2, 'q')} : " + ("wdw;" if bp.log_decay else f"frnn_divf(wdw, {slot(nf.decay)} + q]);"))
+        scalar_nodes(third_s)
+        for i, o in sgrads:
+            sp = dspec[i]
+            val = f"{slot(o)} + q]" if isinstance(o, str) else lower.flit(o)
+            off = _elem_off(sp, [(0, "b"), (1, "t"), (2, "h")])
+            if atomic[i]:
+                w(f"if (live) frnn_atomic_add_c((float*)dx{i} + ({off}), {val});")
+            else:
+                w(f"if (live) frnn_io<{sp.dt}>::st(dx{i}, {off}, {val});")
+        w.close()
+    w("(void)ok;")
+    w.close()
+    return KernelSource("frnn_cvg", w.text().replace("@SMEM_BYTES@", str(smem_bytes)), (nchunk, H, B), VG_THREADS, smem_bytes, params, decl,
+                        {"chunk": C, "tile": [M, N, C], "packed": False, "tmem_cols": tm_cols}, [])
+
+
+def emit_slow_columns(w, C, nd, nr, nA, nK, tq, live_n, sel, nf, bp, dec_vec, want_gw, Stage, leaf, leaves_of, slot, LS, cD1, cD2, off_slow):
+    """Columns of a chunk with a decay too small to divide by: running products in plain loops, by the first four warps;
+    the results (d alpha, d kappa, d decay for all timesteps) go through shared memory."""
+    w.open("if (slow)")
+    w("frnn_tmem_fence_before_sync();")
+    w("frnn_block_sync();         // the operands are no longer read")
+    w.open("if (tid < 128)")
+    w(f"float* sl = (float*)(smem + {off_slow});")
+    w(f"float ka[{nK}], aa[{nA}], ta[{nA}], tk[{nK}], xs[{C}];")
+    for arr, cnt, colx in (("ta", nA, cD1), ("tk", nK, cD2)):
+        w.open("")
+        w(f"float u[{cnt}], lo[{cnt}];")
+        w(f"frnn_tmem_ld<{cnt}>(lanes + {colx}u, u); frnn_tmem_ld<{cnt}>(lanes + {colx + cnt}u, lo); frnn_tmem_wait_ld();")
+        w("#pragma unroll")
+        w(f"for (int k = 0; k < {cnt}; k++) {arr}[k] = u[k] + lo[k];")
+        w.close()
+    names = nf.alphas + nf.kappas + [nf.decay]
+    lv = leaves_of(names, (0, 1))
+    w("#pragma unroll 1")
+    w.open(f"for (int q = 0; q < {C}; q++)")
+    w(f"const int t = {tq('q')}; const bool live = {live_n}; (void)live; (void)t;")
+    for a in lv:
+        w(f"const float l_{a.replace('.', '_')} = {leaf(a, 't', 'nc')};")
+    st = Stage("x_", "q", (0, 1), {a: f"l_{a.replace('.', '_')}" for a in lv})
+    for r, nm in enumerate(nf.kappas):
+        w(f"ka[{r * C} + q] = {sel(live_n, st.get(nm))};")
+    for d, nm in enumerate(nf.alphas):
+        w(f"aa[{d * C} + q] = {sel(live_n, st.get(nm))};")
+    w(f"xs[q] = {sel(live_n, st.get(nf.decay), '1.0f')};")
+    w.close()
+    if want_gw:
+        w("const float Z = ncol ? z0[x128] : 0.0f;")
+        w("#pragma unroll 1")
+        w.open(f"for (int j = 0; j < {C}; j++)")
+        w("float A = 1.0f, Bj = 1.0f, g = 0.0f, s0 = 0.0f, Q = 1.0f;")
+        w("for (int l = 0; l < j; l++) A *= xs[l];")
+        w(f"for (int l = j + 1; l < {C}; l++) Bj *= xs[l];")
+        w("#pragma unroll 1")
+        w(f"for (int i = j + 1; i < {C}; i++) {{ " + " ".join(f"s0 += aa[{d * C} + i] * ta[{d * C} + i] * Q;" for d in range(nd)) + " Q *= xs[i]; }")
+        w("g = A * (Bj * Z + s0);")
+        w("float P = 1.0f;")
+        w("#pragma unroll 1")
+        w.open("for (int l = j - 1; l >= 0; l--)")
+        w("#pragma unroll 1")
+        w.open(f"for (int r = 0; r < {nr}; r++)")
+        w(f"float e = Bj * tk[r * {C} + l]; Q = 1.0f;")
+        w("#pragma unroll 1")
+        w(f"for (int i = j + 1; i < {C}; i++) {{ " + " ".join(f"e += Lr[({d * C} + i) * {LS} + r * {C} + l] * aa[{d * C} + i] * Q;" for d in range(nd)) + " Q *= xs[i]; }")
+        w(f"g += ka[r * {C} + l] * P * e;")
+        w.close()
+        w("P *= xs[l];")
+        w.close()
+        w(f"sl[({nA + nK} + j) * 128 + x128] = g" + (" * xs[j];" if bp.log_decay else ";"))
+        w.close()
+    if dec_vec:
+        w("float a = 1.0f;")
+        w("#pragma unroll 1")
+        w(f"for (int q = 0; q < {C}; q++) {{ for (int d = 0; d < {nd}; d++) ta[d * {C} + q] *= a; a *= xs[q]; }}")
+        w("a = 1.0f;")
+        w("#pragma unroll 1")
+        w(f"for (int q = {C - 1}; q >= 0; q--) {{ for (int r = 0; r < {nr}; r++) tk[r * {C} + q] *= a; a *= xs[q]; }}")
+        w("#pragma unroll 1")
+        w.open(f"for (int i = 0; i < {C}; i++)")
+        w("a = 1.0f;")
+        w("#pragma unroll 1")
+        w.open(f"for (int j = i + 1; j < {C}; j++)")
+        w("#pragma unroll 1")
+        w(f"for (int dr = 0; dr < {nd * nr}; dr++) {{ const int d = dr / {nr}, r = dr % {nr}; const float L = Lr[(d * {C} + j) * {LS} + r * {C} + i] * a; "
+          f"ta[d * {C} + j] += L * ka[r * {C} + i]; tk[r * {C} + i] += L * aa[d * {C} + j]; }}")
+        w("a *= xs[j];")
+        w.close()
+        w.close()
+        w("#pragma unroll 1")
+        w(f"for (int k = 0; k < {nA}; k++) sl[k * 128 + x128] = ta[k];")
+        w("#pragma unroll 1")
+        w(f"for (int k = 0; k < {nK}; k++) sl[({nA} + k) * 128 + x128] = tk[k];")
+    w.close()
+    w("frnn_block_sync();")
+    w("frnn_tmem_fence_after_sync();")
+    w.close()
+
+
+# ---------------------------------------------------------------------------
+# planning
+# ---------------------------------------------------------------------------
+
+@dataclass
+class ChunkPlan:
+    """The chunked kernels of one specialisation."""
+    problem: Problem
+    nf: Normal
+    bp: Optional[BackwardPlan]                # None: only calls without gradients are chunked
+    dspec: List[TensorSpec]
+    atomic: List[bool]
+
+    def forward(self, **kw) -> KernelSource:
+        p = self.problem
+        return emit_scan(p, forward_spec(p, self.nf, self.bp.saved, True), CHUNK, rows_per_cta(p.M), **kw)
+
+    def infer(self, **kw) -> KernelSource:
+        p = self.problem
+        return emit_scan(p, forward_spec(p, self.nf, [], False), CHUNK, rows_per_cta(p.M), **kw)
+
+    def backward_scan(self, **kw) -> KernelSource:
+        p = self.problem
+        return emit_scan(p, backward_scan_spec(p, self.nf, self.bp, self.dspec), CHUNK, rows_per_cta(p.M), **kw)
+
+    def vector_grads(self) -> KernelSource:
+        return emit_vector_grads(self.problem, self.nf, self.bp, self.dspec, self.atomic, CHUNK)
+
+    def variants(self) -> List[dict]:
+        """Keyword arguments of the scans worth timing; member 0 is the default."""
+        return [dict(state_unroll=2), dict(state_unroll=1), dict(state_unroll=4)]
+
+
+def chunk_plan(plan) -> Optional[ChunkPlan]:
+    """The chunked form of a specialisation (a ``twopass.Plan``), where it applies and is the faster one:
+
+    * one state, in the normal form, of at most 128 columns (a multiple of 8: one tf32 product takes 8) - the state, its
+      rest and the products of a chunk then fit Tensor Memory; training also wants the rows of a head in one CTA;
+    * 16-bit inputs.  fp32 inputs keep the recurrent kernels, whose sums are fp32 throughout (relative error 1e-7 against
+      5e-7 of the split products here);
+    * at least two chunks: shorter sequences are done before the first chunk's operands are ready.
+    """
+    p = plan.problem
+    if plan.n_st != 1 or p.N % 8 or not 16 <= p.N <= 128 or p.T < 2 * CHUNK or p.naux < 0:
+        return None
+    if any(s.dt not in (lower.DT_BF16, lower.DT_F16) for s in p.inputs) or p.states[0].dt == lower.DT_F64:
+        return None
+    if p.M < 8 or rows_per_cta(p.M) is None or 0 in (p.B, p.T, p.H):
+        return None
+    for s in p.inputs:
+        cls = (int(s.shape[3] > 1), int(s.shape[4] > 1))
+        if list(s.shape[:3]) != [p.B, p.T, p.H] and not (cls == S11 and s.shape[1] == 1):
+            return None
+    nf = normal_form(plan.g_fw, p.in_names, p.st_names[0], plan.n_out)
+    if nf is None or not all(nf_inputs(nf)):
+        return None
+    cp = ChunkPlan(p, nf, None, [g.spec for g in plan.grads], [g.atomic for g in plan.grads])
+    try:
+        cp.infer()
+        if p.M <= 128 and p.M % 8 == 0:
+            v = local_vjp(nf, p.M, p.N)
+            cp.bp = backward_plan(p, nf, *v) if v is not None else None
+            if cp.bp is not None:
+                for ks in (cp.forward(), cp.backward_scan(), cp.vector_grads()):
+                    if ks.smem_bytes > 227 * 1024:
+                        cp.bp = None
+    except lower.LoweringError:
+        return None
+    return cp

@@ -936,9 +936,11 @@ class KernelBuilder:
             w(f"if (tl < {self.D}) (({CTYPE[it.dt]}*)({stage} + {it.off} + tl * {it.rowb}))[j] = pl{k}[q];")
             w.close()
 
-    def emit_convert(self, raw: str, wk: str, nv: str, tidv: str = "tid", nthr: Optional[int] = None):
+    def emit_convert(self, raw: str, wk: str, nv: str, tidv: str = "tid", nthr: Optional[int] = None,
+                     rows: Optional[Dict[Shape, Tuple[str, int]]] = None):
         """Threads ``tidv`` in [0, nthr) (default: the whole CTA): raw chunk -> fp32
-        work buffer, evaluating hoisted nodes."""
+        work buffer, evaluating hoisted nodes.  ``rows`` gives some shape classes a
+        work buffer of their own: (base pointer, floats per timestep)."""
         w, t = self.w, self.t
         nthr = nthr or t.NT
         hoisted = {n.name: n for n in self.hoisted}
@@ -963,6 +965,7 @@ class KernelBuilder:
             if not targets:
                 continue
             order = closure(targets)
+            dst, dst_row = (rows or {}).get(cls, (wk, self.wk_row))
             vw = 4 if ln % 4 == 0 else (2 if ln % 2 == 0 else 1)   # elements per thread and iteration
             w.open(f"for (int e = {tidv}; e < {nv} * {ln // vw}; e += {nthr})")
             w(f"const int tl = e / {ln // vw}, i = (e % {ln // vw}) * {vw}; (void)i;")
@@ -997,9 +1000,9 @@ class KernelBuilder:
             for nm in targets:
                 hn = "h_" + nm.replace(".", "_")
                 if cls == S11:
-                    w(f"{wk}[tl * {self.wk_row} + {self.wk[nm][1]}] = {hn}[0];")
+                    w(f"{dst}[tl * {dst_row} + {self.wk[nm][1]}] = {hn}[0];")
                 else:
-                    w(f"frnn_stv<0,{vw}>({wk}, tl * {self.wk_row} + {self.wk[nm][1]} + i, {hn});")
+                    w(f"frnn_stv<0,{vw}>({dst}, tl * {dst_row} + {self.wk[nm][1]} + i, {hn});")
             w.close()
 
     def emit_wk_read(self, body: Body, name: str, wkt: str):

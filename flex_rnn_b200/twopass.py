@@ -26,7 +26,7 @@ from typing import Callable, Dict, List, Optional, Sequence, Tuple
 
 import torch as th
 
-from . import lower
+from . import chunk, lower
 from .graph import MN, M1, N1, S11, StepGraph
 from .lower import (DT_BF16, DT_F16, DT_F32, DT_F64, GradOut, Problem, TensorSpec, choose_tile,
                     emit_backward, emit_forward)
@@ -119,6 +119,7 @@ class Tuning:
     bounds: int = 0          # 1 = checked build of both kernels: every access is tested against the extents of the
                              # kernel's buffers, one outside is skipped and reported through the error word (debugging)
     use_tma: bool = True
+    chunk: int = 0           # chunked form on the tensor cores where the step function has it (see chunk.chunk_plan)
 
 
 SMEM_LIMIT = 227 * 1024
@@ -865,6 +866,15 @@ def build_twopass(step, inputs, state, dryrun=False, tuning: Optional[Tuning] = 
     if Mp is not None:
         return _build_row_padded(step, inputs, state, Mp, dryrun, tuning, _launcher)
     plan, fw_meta, bw_meta = make_plan(step, inputs, state, tuning)
+    p = plan.problem
+    nin, nst, nout = len(inputs), plan.n_st, plan.n_out
+    cplan = chunk.chunk_plan(plan) if plan.tuning.chunk else None
+    ctrain = cplan is not None and cplan.bp is not None
+    if ctrain:
+        # checkpoints are the states at the chunks' starts, transposed; the saved row sums are the chunked form's
+        nck = (p.T + chunk.CHUNK - 1) // chunk.CHUNK
+        fw_meta = fw_meta[:nout + nst] + get_meta([th.empty(p.B, p.H, nck, p.N, p.M, device="meta"),
+                                                   th.empty(len(cplan.bp.saved), p.B, p.H, p.T, p.M, device="meta")])
     if dryrun:
         return fw_meta, bw_meta
 
@@ -875,18 +885,19 @@ def build_twopass(step, inputs, state, dryrun=False, tuning: Optional[Tuning] = 
                            "use the .naive method for a CPU evaluation of the step function")
     if 0 in (plan.problem.B, plan.problem.T, plan.problem.H):
         return (*_build_empty(plan, fw_meta, bw_meta, inputs, state), fw_meta, bw_meta)
-    fw_src, bw_src = generate(plan)
+    fw_src, bw_src = generate(plan) if not ctrain else (None, None)
     tu0 = plan.tuning
     forced_fw, forced_bw = tu0.fw_variant >= 0, tu0.bw_variant >= 0
-    if forced_fw and tu0.fw_variant > 0:
+    if forced_fw and tu0.fw_variant > 0 and not ctrain:
         fw_src = generate_forward(plan, **forward_variants(plan)[tu0.fw_variant])
-    if forced_bw and tu0.bw_variant > 0:
+    if forced_bw and tu0.bw_variant > 0 and not ctrain:
         bw_src = generate_backward(plan, **backward_variants(plan)[tu0.bw_variant])
         if bw_src is None:
             raise lower.LoweringError("the requested backward variant does not fit shared memory")
-    p = plan.problem
-    nin, nst, nout = len(inputs), plan.n_st, plan.n_out
     make = _launcher or _CudaLauncher
+    if ctrain:
+        fw_src, bw_src = _checked(cplan.forward(), tu0), _checked(cplan.backward_scan(), tu0)
+        launch_vg = make(_checked(cplan.vector_grads(), tu0))
     launch_fw, launch_bw = make(fw_src), make(bw_src)
 
     in_meta = tuple(th.empty_strided(x.shape, x.stride(), dtype=x.dtype, device="meta") for x in inputs)
@@ -975,14 +986,16 @@ def build_twopass(step, inputs, state, dryrun=False, tuning: Optional[Tuning] = 
         """Time the alternative backward kernels once, writing into throw-away
         gradient buffers (the kernel accumulates into some of its outputs)."""
         tuned["bw"] = True
-        nouts = len(dxs) + len(ds0)
-        first_out = len(ptrs) - 1 - nouts
-        scratch = [th.zeros_like(t) for t in list(ds0) + list(dxs)]
-        trial = list(ptrs[:first_out]) + [t.data_ptr() for t in scratch] + [ptrs[-1]]
+        trial = ptrs                 # the chunked scan accumulates nowhere
+        if not ctrain:
+            nouts = len(dxs) + len(ds0)
+            first_out = len(ptrs) - 1 - nouts
+            scratch = [th.zeros_like(t) for t in list(ds0) + list(dxs)]
+            trial = list(ptrs[:first_out]) + [t.data_ptr() for t in scratch] + [ptrs[-1]]
         best, log = None, []
-        for k, kw in enumerate(backward_variants(plan)):
+        for k, kw in enumerate(cplan.variants() if ctrain else backward_variants(plan)):
             try:
-                ks = bw_src if k == 0 else generate_backward(plan, **kw)
+                ks = bw_src if k == 0 else cplan.backward_scan(**kw) if ctrain else generate_backward(plan, **kw)
                 if ks is None:
                     continue
                 launcher = launch_bw if k == 0 else make(ks)
@@ -1002,9 +1015,13 @@ def build_twopass(step, inputs, state, dryrun=False, tuning: Optional[Tuning] = 
         forward kernel only writes its outputs) and keep the fastest."""
         first = infer_kernel() if infer else (fw_src, launch_fw)
         best, log = None, []
-        for k, kw in enumerate(forward_variants(plan)):
+        chunked = cplan is not None if infer else ctrain
+        for k, kw in enumerate(cplan.variants() if chunked else forward_variants(plan)):
             try:
-                ks = first[0] if k == 0 else generate_forward(plan, infer=infer, **kw)
+                if chunked:
+                    ks = first[0] if k == 0 else cplan.infer(**kw) if infer else cplan.forward(**kw)
+                else:
+                    ks = first[0] if k == 0 else generate_forward(plan, infer=infer, **kw)
                 launcher = first[1] if k == 0 else make(ks)
                 ms = timed(launcher, ptrs, device)
             except (lower.LoweringError, RuntimeError):
@@ -1026,8 +1043,8 @@ def build_twopass(step, inputs, state, dryrun=False, tuning: Optional[Tuning] = 
     def infer_kernel():
         """(source, launcher) of the planned kernel for calls without gradients, made on first use."""
         if "launch_infer" not in tuned:
-            kw = forward_variants(plan)[tu0.fw_variant] if tu0.fw_variant > 0 else {}
-            tuned["infer_src"] = generate_forward(plan, infer=True, **kw)
+            kw = forward_variants(plan)[tu0.fw_variant] if tu0.fw_variant > 0 and cplan is None else {}
+            tuned["infer_src"] = generate_forward(plan, infer=True, **kw) if cplan is None else _checked(cplan.infer(), tu0)
             tuned["launch_infer"] = make(tuned["infer_src"])
         return tuned["infer_src"], tuned["launch_infer"]
 
@@ -1050,9 +1067,9 @@ def build_twopass(step, inputs, state, dryrun=False, tuning: Optional[Tuning] = 
         with _device_ctx(device):
             check_before(device)
             outs, stT = alloc_results(state0, device)
-            store = tuple(alloc(f"checkpoints of state #{k + 1}", *cont(p.B, p.H, plan.nck, p.M, p.N), th.float32, device)
+            store = tuple(alloc(f"checkpoints of state #{k + 1}", *cont(*fw_meta[nout + nst + k][0]), th.float32, device)
                           for k, _ in enumerate(state0))
-            aux = alloc("saved row sums", *cont(len(plan.aux), p.B, p.H, p.T, p.M), th.float32, device)
+            aux = alloc("saved row sums", *cont(*fw_meta[-1][0]), th.float32, device)
             ew = err_word(device)
             ptrs = [x.data_ptr() for x, u in zip(inputs_, fw_used[:nin]) if u]
             ptrs += [s.data_ptr() for s in state0] + [o.data_ptr() for o in outs] + [s.data_ptr() for s in stT]
@@ -1082,6 +1099,16 @@ def build_twopass(step, inputs, state, dryrun=False, tuning: Optional[Tuning] = 
             check_guard(device)
         return (*outs, *stT)
 
+    # buffers of the chunked backward, by parameter name: inputs, upstream gradients, saved tensors, gradients, scratch
+    chunk_temps, chunk_where = [], {}
+    if ctrain:
+        chunk_temps = [("state gradients at the chunks' ends", fw_meta[nout + nst][0]),
+                       ("kept row sums", (len(cplan.bp.kept), p.B, p.H, p.T, p.M)),
+                       ("kept inner products", (len(cplan.nf.diags) if cplan.bp.kept_dg else 0, p.B, p.H, p.T))]
+        names = [f"in{i}" for i in range(nin)] + [f"dy{j}" for j in range(nout)] + ["dsT", "ck", "aux"] + \
+                [f"dx{i}" for i in range(nin)] + ["ds0", "eck", "tau", "dgk", "err"]
+        chunk_where = {nm: i for i, nm in enumerate(names)}
+
     def backward(doutput, dstateT, inputs_, state_store, aux_):
         doutput = tuple(d.contiguous() for d in doutput)
         dstateT = tuple(d.contiguous() for d in dstateT)
@@ -1099,6 +1126,15 @@ def build_twopass(step, inputs, state, dryrun=False, tuning: Optional[Tuning] = 
                     dxs.append(alloc_like(f"gradient of input #{i + 1}", x, device))
             ds0 = tuple(alloc_like(f"gradient of initial state #{k + 1}", s, device) for k, s in enumerate(st_meta))
             ew = err_word(device)
+            if ctrain:
+                tmp = [alloc(nm, *cont(*sh), th.float32, device) for nm, sh in chunk_temps]
+                every = [*inputs_, *doutput, *dstateT, *state_store, aux, *dxs, *ds0, *tmp, ew]
+                ptr = lambda ks: [every[chunk_where[nm]].data_ptr() for nm in ks.params if nm in chunk_where]
+                if not tuned["bw"]:
+                    autotune_backward(ptr(bw_src), device, dxs, ds0)
+                tuned["launch_bw"](ptr(bw_src), device)
+                launch_vg(ptr(launch_vg.ks), device)
+                return finish_backward(dxs, ds0, inputs_, device)
             ptrs = [x.data_ptr() for x, u in zip(inputs_, bw_used[:nin]) if u]
             ptrs += [d.data_ptr() for d in doutput] + [d.data_ptr() for d in dstateT]
             ptrs += [s.data_ptr() for s in state_store] + [aux.data_ptr()]
@@ -1106,11 +1142,14 @@ def build_twopass(step, inputs, state, dryrun=False, tuning: Optional[Tuning] = 
             if not tuned["bw"]:
                 autotune_backward(ptrs, device, dxs, ds0)
             tuned["launch_bw"](ptrs, device)
-            check_status(device, "backward")
-            check_guard(device)
-            for i, go in enumerate(plan.grads):
-                if go.atomic:          # accumulated in fp32: now in the input's dtype and layout
-                    dxs[i] = th.empty_like(inputs_[i]).copy_(dxs[i])
+            return finish_backward(dxs, ds0, inputs_, device)
+
+    def finish_backward(dxs, ds0, inputs_, device):
+        check_status(device, "backward")
+        check_guard(device)
+        for i, go in enumerate(plan.grads):
+            if go.atomic:          # accumulated in fp32: now in the input's dtype and layout
+                dxs[i] = th.empty_like(inputs_[i]).copy_(dxs[i])
         return tuple(dxs), ds0
 
     def kernel_status(device=None) -> int:
@@ -1135,6 +1174,12 @@ def build_twopass(step, inputs, state, dryrun=False, tuning: Optional[Tuning] = 
         idx = dev.index if dev.index is not None else th.cuda.current_device()
         if not isinstance(launcher, _CudaLauncher) or idx not in launcher.mods:
             return None
+        def kernel(launcher, params):
+            ks = launcher.ks
+            assert len(params) + len(ks.tmaps) == len(ks.params)
+            return {"module": launcher.mods[idx]._h.value, "grid": list(ks.grid), "block": ks.block, "smem": ks.smem_bytes,
+                    "params": params, "maps": ks.tmaps}
+
         st = list(range(nin, nin + nst))
         zeroed, cast_from = [], []
         if which == "backward":
@@ -1150,6 +1195,17 @@ def build_twopass(step, inputs, state, dryrun=False, tuning: Optional[Tuning] = 
                     metas.append((bw_meta[i][0], lower._contig(bw_meta[i][0]), th.float32))
             params = [i for i in range(nin) if bw_used[i]] + list(range(nin, given)) + where[nin:] + where[:nin]
             returned = nin + nst
+            if ctrain:
+                if idx not in launch_vg.mods:
+                    return None
+                at = {nm: given + len(metas) + k for k, nm in enumerate(("eck", "tau", "dgk", "err"))}
+                metas += [(tuple(sh), lower._contig(sh), th.float32) for _, sh in chunk_temps]
+                at.update({f"dx{i}": where[i] for i in range(nin)})
+                at["ds0"] = where[nin]
+                at.update({nm: i for nm, i in chunk_where.items() if i < given})
+                kernels = [kernel(x, [at[nm] for nm in x.ks.params if nm in at]) for x in (launcher, launch_vg)]
+                return {"kernels": kernels, "zeroed": zeroed, "cast_from": cast_from, "returned": returned,
+                        "alloc": [(tuple(s), tuple(t), d) for s, t, d in metas]}
         else:
             given = nin + nst
             metas = list(fw_meta if which == "forward" else fw_meta[:nout + nst])
@@ -1157,11 +1213,7 @@ def build_twopass(step, inputs, state, dryrun=False, tuning: Optional[Tuning] = 
             params = [i for i in range(nin) if used[i]] + st + list(range(given, given + len(metas)))
             returned = len(metas)
         params.append(given + len(metas))
-        ks = launcher.ks
-        assert len(params) + len(ks.tmaps) == len(ks.params)
-        kernel = {"module": launcher.mods[idx]._h.value, "grid": list(ks.grid), "block": ks.block, "smem": ks.smem_bytes,
-                  "params": params, "maps": ks.tmaps}
-        return {"kernels": [kernel], "zeroed": zeroed, "cast_from": cast_from, "returned": returned,
+        return {"kernels": [kernel(launcher, params)], "zeroed": zeroed, "cast_from": cast_from, "returned": returned,
                 "alloc": [(tuple(s), tuple(t), d) for s, t, d in metas]}
 
     def host_checks():

@@ -41,10 +41,12 @@ struct emu_cta {
     std::barrier<>* block_bar;
     std::vector<std::barrier<>*> warp_bar;
     std::barrier<>* group_bar[16] = {nullptr};   // named barriers, created on first use with that use's thread count
+    std::barrier<>* half_bar[32] = {nullptr};    // the first 16 lanes of each warp, created on first use
     std::vector<float> xchg;          // [nthreads]
     std::vector<float> tmem;          // Tensor Memory: 128 lanes x 512 columns (allocated on first use)
     int tmem_cols = 0;                // columns the CTA has allocated (0: none)
     unsigned char* smem;
+    size_t smem_bytes = 0;
     std::mutex mtx;
 };
 static thread_local emu_dim3 threadIdx, blockIdx;
@@ -180,6 +182,46 @@ FRNN_DEV float* emu_tmem_at(u32 taddr, int n) {
     FRNN_DEV void frnn_tmem_st##N(u32 taddr, const float* v) { memcpy(emu_tmem_at(taddr, N), v, 4 * N); } \
     FRNN_DEV void frnn_tmem_ld##N(u32 taddr, float* v) { memcpy(v, emu_tmem_at(taddr, N), 4 * N); }
 EMU_TMEM_FN(1) EMU_TMEM_FN(2) EMU_TMEM_FN(4) EMU_TMEM_FN(8) EMU_TMEM_FN(16)
+FRNN_DEV void frnn_half_warp_sync() {
+    emu_cta* c = emu_ctx;
+    const int w = threadIdx.x >> 5;
+    {
+        std::lock_guard<std::mutex> g(c->mtx);
+        if (!c->half_bar[w]) c->half_bar[w] = new std::barrier<>((std::ptrdiff_t)16);
+    }
+    c->half_bar[w]->arrive_and_wait();
+}
+// tf32 matrix products on Tensor Memory (csrc/frnn_chunk.cuh): done at issue, operands truncated like the hardware does
+FRNN_DEV u32 frnn_f32_bits(float x) { return emu_f2u(x); }
+FRNN_DEV float frnn_bits_f32(u32 x) { return emu_u2f(x); }
+FRNN_DEV float frnn_tf32_trunc(float x) { return emu_u2f(emu_f2u(x) & 0xffffe000u); }
+FRNN_DEV float emu_mma_smem(const void* p, u32 lbo, int row, int k) {
+    if ((uintptr_t)p & 15 || lbo & 15) { fprintf(stderr, "emu: misaligned matrix operand\n"); abort(); }
+    const unsigned char* a = (const unsigned char*)p + (k / 4) * (size_t)lbo + (row / 8) * 128 + (row % 8) * 16 + (k % 4) * 4;
+    if (a < emu_ctx->smem || a + 4 > emu_ctx->smem + emu_ctx->smem_bytes) { fprintf(stderr, "emu: matrix operand outside shared memory\n"); abort(); }
+    return frnn_tf32_trunc(*(const float*)a);
+}
+template <class A> FRNN_DEV void emu_mma(u32 d, A a, const void* b, u32 lbo_b, u32 n, bool acc) {
+    std::lock_guard<std::mutex> g(emu_ctx->mtx);
+    if (n % 16 || n < 16 || n > 256 || (int)(d + n) > emu_ctx->tmem_cols || d >> 16) { fprintf(stderr, "emu: bad matrix product shape n %u d %u\n", n, d); abort(); }
+    for (int m = 0; m < 128; m++)
+        for (u32 j = 0; j < n; j++) {
+            float s = acc ? emu_ctx->tmem[(size_t)m * 512 + d + j] : 0.0f;
+            for (int k = 0; k < 8; k++) s += a(m, k) * emu_mma_smem(b, lbo_b, (int)j, k);
+            emu_ctx->tmem[(size_t)m * 512 + d + j] = s;
+        }
+}
+#define FRNN_MMA_IDESC(n) ((u32)(n))
+FRNN_DEV u64 frnn_mma_desc(const void* p, u32 lbo) { return (u64)((const unsigned char*)p - emu_ctx->smem) | ((u64)lbo << 32); }
+FRNN_DEV u64 frnn_mma_next(u64 desc, u32 lbo, int k) { return desc + (u64)k * 2 * lbo; }
+FRNN_DEV void frnn_mma_ts_d(u32 d, u32 a, u64 b, u32 n, bool acc) {
+    if ((int)a + 8 > emu_ctx->tmem_cols) { fprintf(stderr, "emu: matrix operand outside Tensor Memory\n"); abort(); }
+    emu_mma(d, [=](int m, int k) { return frnn_tf32_trunc(emu_ctx->tmem[(size_t)m * 512 + a + k]); }, emu_ctx->smem + (u32)b, (u32)(b >> 32), n, acc);
+}
+FRNN_DEV void frnn_mma_ss_d(u32 d, u64 a, u64 b, u32 n, bool acc) {
+    emu_mma(d, [=](int m, int k) { return emu_mma_smem(emu_ctx->smem + (u32)a, (u32)(a >> 32), m, k); }, emu_ctx->smem + (u32)b, (u32)(b >> 32), n, acc);
+}
+FRNN_DEV void frnn_mma_commit(u64* bar) { frnn_mbar_arrive(bar); }
 FRNN_DEV int frnn_smem_add(int* p, int v) { std::lock_guard<std::mutex> g(emu_atomic_mtx); int o = *p; *p = o + v; return o; }
 template <int N> FRNN_DEV void frnn_regs_release() {}
 template <int N> FRNN_DEV void frnn_regs_acquire() {}
@@ -225,6 +267,7 @@ static void emu_launch(emu_entry_t fn, const unsigned grid[3], unsigned nthreads
                 unsigned char* raw = (unsigned char*)aligned_alloc(128, ((size_t)smem_bytes + 255) / 128 * 128);
                 memset(raw, 0xCD, smem_bytes);
                 cta.smem = raw;
+                cta.smem_bytes = smem_bytes;
                 std::vector<std::thread> th;
                 for (unsigned t = 0; t < nthreads; t++)
                     th.emplace_back([&, t] {
@@ -235,6 +278,7 @@ static void emu_launch(emu_entry_t fn, const unsigned grid[3], unsigned nthreads
                     });
                 for (auto& t : th) t.join();
                 for (auto* b : wb) delete b;
+                for (auto*& hb : cta.half_bar) { delete hb; hb = nullptr; }
                 for (auto*& gb : cta.group_bar) { delete gb; gb = nullptr; }
                 free(raw);
             }
