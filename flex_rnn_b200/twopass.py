@@ -119,7 +119,7 @@ class Tuning:
     bounds: int = 0          # 1 = checked build of both kernels: every access is tested against the extents of the
                              # kernel's buffers, one outside is skipped and reported through the error word (debugging)
     use_tma: bool = True
-    chunk: int = 0           # chunked form on the tensor cores where the step function has it (see chunk.chunk_plan)
+    chunk: int = 1           # chunked form on the tensor cores where the step function has it (see chunk.chunk_plan)
 
 
 SMEM_LIMIT = 227 * 1024
@@ -868,7 +868,9 @@ def build_twopass(step, inputs, state, dryrun=False, tuning: Optional[Tuning] = 
     plan, fw_meta, bw_meta = make_plan(step, inputs, state, tuning)
     p = plan.problem
     nin, nst, nout = len(inputs), plan.n_st, plan.n_out
-    cplan = chunk.chunk_plan(plan) if plan.tuning.chunk else None
+    # a pinned variant names one of the recurrent kernels
+    pinned = plan.tuning.fw_variant >= 0 or plan.tuning.bw_variant >= 0
+    cplan = chunk.chunk_plan(plan) if plan.tuning.chunk and not pinned else None
     ctrain = cplan is not None and cplan.bp is not None
     if ctrain:
         # checkpoints are the states at the chunks' starts, transposed; the saved row sums are the chunked form's
@@ -888,9 +890,9 @@ def build_twopass(step, inputs, state, dryrun=False, tuning: Optional[Tuning] = 
     fw_src, bw_src = generate(plan) if not ctrain else (None, None)
     tu0 = plan.tuning
     forced_fw, forced_bw = tu0.fw_variant >= 0, tu0.bw_variant >= 0
-    if forced_fw and tu0.fw_variant > 0 and not ctrain:
+    if forced_fw and tu0.fw_variant > 0:
         fw_src = generate_forward(plan, **forward_variants(plan)[tu0.fw_variant])
-    if forced_bw and tu0.bw_variant > 0 and not ctrain:
+    if forced_bw and tu0.bw_variant > 0:
         bw_src = generate_backward(plan, **backward_variants(plan)[tu0.bw_variant])
         if bw_src is None:
             raise lower.LoweringError("the requested backward variant does not fit shared memory")
@@ -1043,7 +1045,7 @@ def build_twopass(step, inputs, state, dryrun=False, tuning: Optional[Tuning] = 
     def infer_kernel():
         """(source, launcher) of the planned kernel for calls without gradients, made on first use."""
         if "launch_infer" not in tuned:
-            kw = forward_variants(plan)[tu0.fw_variant] if tu0.fw_variant > 0 and cplan is None else {}
+            kw = forward_variants(plan)[tu0.fw_variant] if tu0.fw_variant > 0 else {}
             tuned["infer_src"] = generate_forward(plan, infer=True, **kw) if cplan is None else _checked(cplan.infer(), tu0)
             tuned["launch_infer"] = make(tuned["infer_src"])
         return tuned["infer_src"], tuned["launch_infer"]

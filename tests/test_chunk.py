@@ -1,0 +1,86 @@
+"""The chunked form (chunk.py): which step functions have it, and its kernels against the naive scan in fp64 at the
+edges of chunks, columns and rows, with decays that vanish inside a chunk.  CPU: under the host emulation; GPU: the
+public API."""
+import pytest
+import torch
+
+import flex_rnn_b200
+from flex_rnn_b200 import chunk
+from flex_rnn_b200 import examples as X
+from flex_rnn_b200 import workloads as W
+from flex_rnn_b200.twopass import build_twopass, make_plan
+from oracle import naive_oracle as O
+
+
+def case(op, B, T, H, M, N, dt, reset=False):
+    """16-bit inputs and an fp32 state, so that outputs and final states show the kernels' own accuracy."""
+    if op in W.STEPS:
+        *ins, s = W.synthetic(op, B, T, H, M, N, dt)[0]
+        step = W.STEPS[op]
+    else:
+        (ins, (s,)), step = X.zoo_case(op, B, T, H, M, N, dt), X.ZOO[op]
+    if reset:
+        g = torch.Generator().manual_seed(3)
+        k = {"gated_delta_rule": 3, "rwkv7": 1, "gla": 3}[op]
+        hit = torch.rand(ins[k].shape, generator=g) < 0.05
+        ins[k] = torch.where(hit, torch.full_like(ins[k], -200.0 if op == "gla" else 0.0), ins[k])
+    g = torch.Generator().manual_seed(1)
+    s = 0.1 * torch.randn(s.shape, generator=g)
+    dy, dS = torch.randn(B, T, H, M, generator=g), torch.randn(s.shape, generator=g)
+    return step, ins, s, dy, dS
+
+
+def check(got, step, ins, s, dy, dS, dt):
+    ry, rS, rgx, rgs = O.fwd_bwd(step, ins, [s], [dy], [dS], dtype=torch.float64)
+    tol = {torch.bfloat16: 1e-2, torch.float16: 2e-3}[dt]
+    for a, b in zip(got, [*ry, *rS, *rgx, *rgs]):
+        assert a.shape == b.shape
+        assert O.rel_err(a.cpu(), b) < (2e-6 if a.dtype == torch.float32 else tol), (a.dtype, O.rel_err(a.cpu(), b))
+
+
+CASES = [("delta_rule", 1, 32, 1, 32, 16, torch.bfloat16, False), ("gated_delta_rule", 2, 37, 1, 8, 40, torch.float16, True),
+         ("rwkv7", 1, 33, 1, 24, 24, torch.bfloat16, True), ("mamba2", 1, 49, 2, 16, 128, torch.bfloat16, False),
+         ("gla", 1, 50, 1, 128, 80, torch.float16, True), ("retention", 1, 47, 2, 40, 32, torch.bfloat16, False)]
+
+
+def test_which_steps_have_the_form():
+    for op, want in [("delta_rule", True), ("gated_delta_rule", True), ("rwkv7", True), ("mamba2", True), ("gla", True),
+                     ("retention", True), ("longhorn", False), ("hgrn", False), ("mamba", False)]:
+        step, ins, s, _, _ = case(op, 1, 64, 2, 32, 1 if op == "hgrn" else 32, torch.bfloat16)
+        cp = chunk.chunk_plan(make_plan(step, ins, [s])[0])
+        assert (cp is not None and cp.bp is not None) == want, op
+    step, ins, s, _, _ = case("delta_rule", 1, 64, 1, 256, 64, torch.bfloat16)
+    cp = chunk.chunk_plan(make_plan(step, ins, [s])[0])
+    assert cp is not None and cp.bp is None            # rows over several CTAs: calls without gradients only
+
+
+@pytest.mark.parametrize("op,B,T,H,M,N,dt,reset", CASES)
+def test_emulated(op, B, T, H, M, N, dt, reset):
+    from emu.emu import EmuLauncher
+    step, ins, s, dy, dS = case(op, B, T, H, M, N, dt, reset)
+    fwd, bwd, fm, bm = build_twopass(step, tuple(ins), (s,), _launcher=EmuLauncher)
+    assert [ks.name for ks in fwd.sources] == ["frnn_cfw", "frnn_cbw"]
+    assert build_twopass(step, tuple(ins), (s,), dryrun=True) == (fm, bm)
+    y, sT, ck, aux = fwd(tuple(ins), (s,))
+    assert [tuple(m[0]) for m in fm] == [tuple(t.shape) for t in (y, sT, ck, aux)]
+    dx, ds = bwd((dy.to(y.dtype),), (dS,), tuple(ins), (ck,), (aux,))
+    check([y, sT, *dx, *ds], step, ins, s, dy, dS, dt)
+    assert all(torch.equal(a, b) for a, b in zip(fwd.infer(tuple(ins), (s,)), (y, sT)))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("op,B,T,H,M,N,dt,reset", CASES + [
+    ("delta_rule", 3, 200, 2, 128, 128, torch.bfloat16, False), ("gated_delta_rule", 2, 64, 3, 64, 128, torch.bfloat16, True),
+    ("rwkv7", 1, 100, 2, 128, 128, torch.bfloat16, True), ("mamba2", 2, 300, 2, 64, 64, torch.float16, False),
+    ("gla", 2, 130, 2, 96, 128, torch.bfloat16, True)])
+def test_gpu(op, B, T, H, M, N, dt, reset):
+    step, ins, s, dy, dS = case(op, B, T, H, M, N, dt, reset)
+    f = flex_rnn_b200.jit(step)
+    leaves = [x.cuda().requires_grad_() for x in [*ins, s]]
+    for _ in range(2):
+        y, sT = f(*leaves)
+        grads = torch.autograd.grad((y, sT), leaves, (dy.cuda().to(y.dtype), dS.cuda()))
+        assert f.forward_func.kernel_status("cuda:0") == 0
+        check([y.detach(), sT.detach(), *grads], step, ins, s, dy, dS, dt)
+    with torch.no_grad():
+        assert all(torch.equal(a, b) for a, b in zip(f(*leaves), (y, sT)))
