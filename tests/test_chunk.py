@@ -40,7 +40,7 @@ def check(got, step, ins, s, dy, dS, dt):
 
 CASES = [("delta_rule", 1, 32, 1, 32, 16, torch.bfloat16, False), ("gated_delta_rule", 2, 37, 1, 8, 40, torch.float16, True),
          ("rwkv7", 1, 33, 1, 24, 24, torch.bfloat16, True), ("mamba2", 1, 49, 2, 16, 128, torch.bfloat16, False),
-         ("gla", 1, 50, 1, 128, 80, torch.float16, True), ("retention", 1, 47, 2, 40, 32, torch.bfloat16, False)]
+         ("gla", 1, 50, 1, 128, 80, torch.float16, True), ("retention", 1, 70, 2, 40, 32, torch.bfloat16, False)]
 
 
 def test_which_steps_have_the_form():
@@ -65,7 +65,7 @@ def test_emulated(op, B, T, H, M, N, dt, reset):
     assert [tuple(m[0]) for m in fm] == [tuple(t.shape) for t in (y, sT, ck, aux)]
     dx, ds = bwd((dy.to(y.dtype),), (dS,), tuple(ins), (ck,), (aux,))
     check([y, sT, *dx, *ds], step, ins, s, dy, dS, dt)
-    assert all(torch.equal(a, b) for a, b in zip(fwd.infer(tuple(ins), (s,)), (y, sT)))
+    check([*fwd.infer(tuple(ins), (s,))], step, ins, s, dy, dS, dt)
 
 
 @pytest.mark.gpu
@@ -83,4 +83,4 @@ def test_gpu(op, B, T, H, M, N, dt, reset):
         assert f.forward_func.kernel_status("cuda:0") == 0
         check([y.detach(), sT.detach(), *grads], step, ins, s, dy, dS, dt)
     with torch.no_grad():
-        assert all(torch.equal(a, b) for a, b in zip(f(*leaves), (y, sT)))
+        check([*f(*leaves)], step, ins, s, dy, dS, dt)
