@@ -1186,8 +1186,9 @@ def emit_scan(p: Problem, s: ScanSpec, C: int, MB: int, use_tma: bool = True, st
 CHUNK = 16
 
 
-def ck_bytes(p: Problem) -> int:
-    return p.B * p.H * ((p.T + CHUNK - 1) // CHUNK) * p.N * p.M * 4
+def ck_bytes(p: Problem, C: int) -> int:
+    """Bytes of the fp32 states at the starts of chunks of C timesteps."""
+    return p.B * p.H * ((p.T + C - 1) // C) * p.N * p.M * 4
 
 
 def rows_per_cta(M: int) -> Optional[int]:
@@ -1198,7 +1199,7 @@ def rows_per_cta(M: int) -> Optional[int]:
     return None
 
 
-def forward_spec(p: Problem, nf: Normal, saved: Sequence[int], train: bool) -> ScanSpec:
+def forward_spec(p: Problem, nf: Normal, saved: Sequence[int], train: bool, C: int) -> ScanSpec:
     """The forward scan.  Parameters, in order: used inputs, initial state, outputs, final state and, for training,
     checkpoints [B, H, chunk, N, M] and the row sums ``saved`` [len, B, H, T, M]; error word."""
     yshape = (p.B, p.T, p.H, p.M)
@@ -1208,7 +1209,7 @@ def forward_spec(p: Problem, nf: Normal, saved: Sequence[int], train: bool) -> S
     params += [(f"out{j}", "void", False, p.B * p.T * p.H * p.M * ELT[p.out_dt[j]]) for j in range(len(nf.ys))]
     params.append(("sT", "void", False, _spec_bytes(p.res_states[0])))
     if train:
-        params.append(("ck", "float", False, ck_bytes(p)))
+        params.append(("ck", "float", False, ck_bytes(p, C)))
         params.append(("aux", "float", False, len(saved) * p.B * p.H * p.T * p.M * 4))
     params.append(("err", "int", False, 4))
     outs = []
@@ -1337,7 +1338,7 @@ def backward_plan(p: Problem, nf: Normal, v: StepGraph, log_decay: bool) -> Opti
     return BackwardPlan(v, saved, kept, any(f"dg{k}" in k3 for k in range(len(nf.diags))), dsig, row_grads, grads, log_decay)
 
 
-def backward_scan_spec(p: Problem, nf: Normal, bp: BackwardPlan, dspec: Sequence[TensorSpec]) -> ScanSpec:
+def backward_scan_spec(p: Problem, nf: Normal, bp: BackwardPlan, dspec: Sequence[TensorSpec], C: int) -> ScanSpec:
     """The scan of the state gradient E: E' = E * w + sum_d dsig_d (x) alpha_d with the row sums E . kappa_r, from the
     last timestep to the first.  Parameters, in order: used inputs, d outputs, d final state, forward row sums, d initial
     state, gradients of the row-vector inputs, checkpoints of E, kept row sums, error word."""
@@ -1392,7 +1393,7 @@ def backward_scan_spec(p: Problem, nf: Normal, bp: BackwardPlan, dspec: Sequence
         if not isinstance(o, str):
             raise lower.LoweringError("a constant gradient")
         louts.append((f(o), dspec[i].dt, f"dx{i}", lambda t, sp=dspec[i]: _elem_off(sp, [(0, "b"), (1, t), (2, "h")]), dspec[i].st(3)))
-    params.append(("eck", "float", False, ck_bytes(p)))
+    params.append(("eck", "float", False, ck_bytes(p, C)))
     if bp.kept:
         params.append(("tau", "float", False, len(bp.kept) * p.B * p.H * p.T * p.M * 4))
         for k, r in enumerate(bp.kept):
@@ -1478,8 +1479,8 @@ def emit_vector_grads(p: Problem, nf: Normal, bp: BackwardPlan, dspec: Sequence[
     if bp.kept_dg:
         param("dgk", "float", True, len(nf.diags) * B * H * T * 4)
     nchunk = (T + C - 1) // C
-    param("ck", "float", True, ck_bytes(p))
-    param("eck", "float", True, ck_bytes(p))
+    param("ck", "float", True, ck_bytes(p, C))
+    param("eck", "float", True, ck_bytes(p, C))
     for i, _ in bp.grads:
         param(f"dx{i}", "void", False, _spec_bytes(dspec[i]))
     param("err", "int", False, 4)
@@ -1524,19 +1525,18 @@ def emit_vector_grads(p: Problem, nf: Normal, bp: BackwardPlan, dspec: Sequence[
     off_L2 = off_L1 + nK // 4 * lbo1
     off_Lr = off_L2 + nA // 4 * lbo2
     LS = nK + 1
-    off_slow = off_kT                        # the slow path's results, over the operands: (nA + nK + C) x 128 floats
+    off_slow = off_kT                        # the slow path's results, over the operands it does without: (nA + nK + C) x 128 floats
     smem_bytes = al(max(end1, off_Lr + nA * LS * 4))
     slow_path = bool(nf.decay) and (dec_vec or want_gw)
-    if slow_path:
+    if slow_path and dec_vec:
         off_Lr = max(off_Lr, off_slow + (nA + nK + C) * 512)
         smem_bytes = al(max(smem_bytes, off_Lr + nA * LS * 4))
+    elif slow_path:                          # the gradients of a decay per head only: beside the operands, which stay
+        off_slow = al(off_Lr + nA * LS * 4) - (nA + nK) * 512
+        smem_bytes = al(max(smem_bytes, off_slow + (nA + nK + C) * 512))
     cD1, cD2 = 0, 2 * nA
     cL = cD2 + 2 * nK
-    # the parts from S_0 and E_C and those from L are scaled differently: decays per head keep both of L's apart, decays
-    # over columns (in the operands already) only kappa's; L itself is read before its space is written again
-    cD1b = cL if dec_sc else cD1
-    cD2b = (cL + (2 * nA if dec_sc else 0)) if nf.decay else cD2
-    tm_cols = _tmem_pow2(max(cL + 2 * nK, cD2b + 2 * nK))
+    tm_cols = _tmem_pow2(cL + 2 * nK)
     if tm_cols > 256:
         raise lower.LoweringError("the vector gradients of a chunk do not fit half of Tensor Memory")
     ERR = lower.ERR_STAGE_TIMEOUT
@@ -1698,7 +1698,7 @@ def emit_vector_grads(p: Problem, nf: Normal, bp: BackwardPlan, dspec: Sequence[
         w(f"{slot(f'dg{k}')} + q] = frnn_ld_raw<float>(dgk, {dg_off(p, k, 't')});")
     scalar_nodes(first_s)
     if dec_sc:
-        w("frnn_half_warp_sync();")
+        w("frnn_warp_sync();" if C == 32 else "frnn_half_warp_sync();")
         w("float a = 1.0f, c = 1.0f;")
         w("#pragma unroll")
         w(f"for (int l = 0; l < {C}; l++) {{ const float x = {slot(nf.decay)} + l]; if (l < q) a *= x; if (l > q && l < nv) c *= x; }}")
@@ -1896,25 +1896,10 @@ def emit_vector_grads(p: Problem, nf: Normal, bp: BackwardPlan, dspec: Sequence[
     w.close()
     if dec_vec:
         w("if (tiny) *(volatile int*)&bar[4] = 1;")
-    w("frnn_async_proxy_fence(); frnn_tmem_fence_before_sync();")
-    w("frnn_block_sync();")
-    w("const bool slow = *(volatile int*)&bar[4] != 0; (void)slow;")
-    w.open("if (tid == 0 && ok)" if not dec_vec else "if (tid == 0 && ok && !slow)")
-    w("frnn_tmem_fence_after_sync();")
-    for (cd, offA, tb, nk, offB, lboB, n2) in ((cD1b, off_kT, kT_b, nK, off_L1, lbo1, nA), (cD2b, off_aT, aT_b, nA, off_L2, lbo2, nK)):
-        acc0 = "k > 0" if cd not in (cD1, cD2) else "true"
-        for part_, n_, acc in ((offA, 2 * n2, acc0), (offA + tb, 2 * n2, "true")):
-            w(f"{{ const u64 da = frnn_mma_desc(smem + {part_}, {lboT}), db = frnn_mma_desc(smem + {offB}, {lboB});")
-            w("#pragma unroll")
-            w(f"for (int k = 0; k < {nk // 8}; k++) frnn_mma_ss_d(tm + {cd}u, frnn_mma_next(da, {lboT}, k), frnn_mma_next(db, {lboB}, k), FRNN_MMA_IDESC({n_}), {acc}); }}")
-    w.close()
-    w("if (tid == 0) frnn_mma_commit(&bar[2]);")
-    w(f"ok = frnn_mbar_wait(&bar[2], 0, err, {ERR}) && ok;")
-    w("frnn_tmem_fence_after_sync();")
-    # ---- columns: this thread's half of the timesteps
-    w(f"float da[{nd * HC}], dk[{nr * HC}], R = 0.0f; (void)R;")
+    # ---- the parts of the accumulators so far, from S_0 and E_C, scaled to what those from L need
+    w("float R = 0.0f; (void)R;")
 
-    def ld_half(dst: str, vecs: int, col0: int, rest: int, add: bool = False):
+    def ld_half(dst: str, vecs: int, col0: int, rest: int):
         """dst[v * HC + k] = value of vector v at timestep q0 + k: the sum of two accumulator columns."""
         w.open("")
         w(f"float u[{vecs * HC}], lo[{vecs * HC}];")
@@ -1922,21 +1907,33 @@ def emit_vector_grads(p: Problem, nf: Normal, bp: BackwardPlan, dspec: Sequence[
             w(f"frnn_tmem_ld<{HC}>(lanes + {col0 + x * C}u + (u32)q0, &u[{x * HC}]); frnn_tmem_ld<{HC}>(lanes + {col0 + rest + x * C}u + (u32)q0, &lo[{x * HC}]);")
         w("frnn_tmem_wait_ld();")
         w("#pragma unroll")
-        w(f"for (int k = 0; k < {vecs * HC}; k++) {dst}[k] {'+=' if add else '='} u[k] + lo[k];")
+        w(f"for (int k = 0; k < {vecs * HC}; k++) {dst}[k] = u[k] + lo[k];")
         w.close()
+
+    def st_half(src: str, vecs: int, col0: int, rest: int):
+        for x in range(vecs):
+            w(f"frnn_tmem_st<{HC}>(lanes + {col0 + x * C}u + (u32)q0, &{src}[{x * HC}]); frnn_tmem_st<{HC}>(lanes + {col0 + rest + x * C}u + (u32)q0, zero);")
+    if dec_sc:
+        w(f"float xw[{HC}], pre = {slot('Wp')} + q0], post = {slot('Ws')} + q0 + {HC - 1}];")
+        w("#pragma unroll")
+        w.open(f"for (int k = 0; k < {HC}; k++)")
+        w("xw[k] = " + (f"{slot(nf.decay)} + q0 + k];" if whole else f"q0 + k < nv ? {slot(nf.decay)} + q0 + k] : 1.0f;"))
+        w.close()
+    w("frnn_block_sync();")
+    w("const bool slow = *(volatile int*)&bar[4] != 0; (void)slow;")
     if slow_path:
         emit_slow_columns(w, C, nd, nr, nA, nK, tq, live_n, sel, nf, bp, dec_vec, want_gw, Stage, leaf, leaves_of, slot, LS, cD1, cD2, off_slow)
-    ld_half("da", nd, cD1, nA)
-    ld_half("dk", nr, cD2, nK)
     if nf.decay:
-        if dec_sc:
-            w(f"float xw[{HC}], pre = {slot('Wp')} + q0], post = {slot('Ws')} + q0 + {HC - 1}];")
-            w("#pragma unroll")
-            w.open(f"for (int k = 0; k < {HC}; k++)")
-            w(f"xw[k] = " + (f"{slot(nf.decay)} + q0 + k];" if whole else f"q0 + k < nv ? {slot(nf.decay)} + q0 + k] : 1.0f;"))
-            w.close()
-        w.open("")
+        w.open("if (!slow)" if dec_vec else "")
+        w(f"float dk[{nr * HC}], zero[{HC}];")
+        w("#pragma unroll")
+        w(f"for (int k = 0; k < {HC}; k++) zero[k] = 0.0f;")
+        ld_half("dk", nr, cD2, nK)
         w("float a = post;")
+        if dec_vec:
+            w(f"float y[{nr * HC}];")
+            w("#pragma unroll")
+            w(f"for (int k = 0; k < {nr * HC}; k++) y[k] = dk[k];")
         w("#pragma unroll")
         w(f"for (int k = {HC - 1}; k >= 0; k--) {{ " + " ".join(f"dk[{r * HC} + k] *= a;" for r in range(nr)) + " a *= xw[k]; }")
         if want_gw:
@@ -1949,17 +1946,46 @@ def emit_vector_grads(p: Problem, nf: Normal, bp: BackwardPlan, dspec: Sequence[
             for r, nm in enumerate(nf.kappas):
                 w(f"R = fmaf({st.get(nm)}, {sel(live_n, f'dk[{r * HC} + k]')}, R);")
             w.close()
-        w("a = pre;")
-        w("#pragma unroll")
-        w(f"for (int k = 0; k < {HC}; k++) {{ " + " ".join(f"da[{d * HC} + k] *= a;" for d in range(nd)) + " a *= xw[k]; }")
         if dec_vec:
-            w(f"float y[{nr * HC}], ra = rpre;")
-            ld_half("y", nr, cD2b, nK)
+            # kappa's: times W_C, over W_j at the end; alpha's: as they are, times W_j-1 at the end
+            w("const float wc = a * pre;")
             w("#pragma unroll")
-            w(f"for (int k = 0; k < {HC}; k++) {{ ra *= frnn_rcp1(xw[k]); " + " ".join(f"dk[{r * HC} + k] = fmaf(y[{r * HC} + k], ra, dk[{r * HC} + k]);" for r in range(nr)) + " }")
+            w(f"for (int k = 0; k < {nr * HC}; k++) dk[k] = y[k] * wc;")
+            st_half("dk", nr, cD2, nK)
         else:
-            ld_half("da", nd, cD1b, nA, add=True)
-            ld_half("dk", nr, cD2b, nK, add=True)
+            st_half("dk", nr, cD2, nK)
+            w(f"float da[{nd * HC}];")
+            ld_half("da", nd, cD1, nA)
+            w("a = pre;")
+            w("#pragma unroll")
+            w(f"for (int k = 0; k < {HC}; k++) {{ " + " ".join(f"da[{d * HC} + k] *= a;" for d in range(nd)) + " a *= xw[k]; }")
+            st_half("da", nd, cD1, nA)
+        w("frnn_tmem_wait_st();")
+        w.close()
+    w("frnn_async_proxy_fence(); frnn_tmem_fence_before_sync();")
+    w("frnn_block_sync();")
+    w.open("if (tid == 0 && ok)" if not dec_vec else "if (tid == 0 && ok && !slow)")
+    w("frnn_tmem_fence_after_sync();")
+    for (cd, offA, tb, nk, offB, lboB, n2) in ((cD1, off_kT, kT_b, nK, off_L1, lbo1, nA), (cD2, off_aT, aT_b, nA, off_L2, lbo2, nK)):
+        for part_, n_ in ((offA, 2 * n2), (offA + tb, 2 * n2)):
+            w(f"{{ const u64 da = frnn_mma_desc(smem + {part_}, {lboT}), db = frnn_mma_desc(smem + {offB}, {lboB});")
+            w("#pragma unroll")
+            w(f"for (int k = 0; k < {nk // 8}; k++) frnn_mma_ss_d(tm + {cd}u, frnn_mma_next(da, {lboT}, k), frnn_mma_next(db, {lboB}, k), FRNN_MMA_IDESC({n_}), true); }}")
+    w.close()
+    w("if (tid == 0) frnn_mma_commit(&bar[2]);")
+    w(f"ok = frnn_mbar_wait(&bar[2], 0, err, {ERR}) && ok;")
+    w("frnn_tmem_fence_after_sync();")
+    # ---- columns: this thread's half of the timesteps
+    w(f"float da[{nd * HC}], dk[{nr * HC}];")
+    ld_half("da", nd, cD1, nA)
+    ld_half("dk", nr, cD2, nK)
+    if dec_vec:
+        # the accumulators held W_C/W_j of kappa's part times W_j and alpha's part over W_j-1
+        w.open("if (!slow)")
+        w("float a = pre, ra = rpre;")
+        w("#pragma unroll")
+        w(f"for (int k = 0; k < {HC}; k++) {{ ra *= frnn_rcp1(xw[k]); " + " ".join(f"da[{d * HC} + k] *= a;" for d in range(nd)) + " "
+          + " ".join(f"dk[{r * HC} + k] *= ra;" for r in range(nr)) + " a *= xw[k]; }")
         w.close()
     if slow_path:
         w(f"const float* sl = (const float*)(smem + {off_slow});")
@@ -2147,10 +2173,11 @@ class ChunkPlan:
     bp: Optional[BackwardPlan]                # None: only calls without gradients are chunked
     dspec: List[TensorSpec]
     atomic: List[bool]
+    C: int = CHUNK                            # timesteps per chunk of the training kernels
 
     def forward(self, **kw) -> KernelSource:
         p = self.problem
-        return emit_scan(p, forward_spec(p, self.nf, self.bp.saved, True), CHUNK, rows_per_cta(p.M), **kw)
+        return emit_scan(p, forward_spec(p, self.nf, self.bp.saved, True, self.C), self.C, rows_per_cta(p.M), **kw)
 
     def infer(self, **kw) -> KernelSource:
         """Without checkpoints a chunk may be longer: its chain costs about 3000 cycles whatever its length and the
@@ -2159,23 +2186,31 @@ class ChunkPlan:
         p = self.problem
         if len(self.nf.alphas) * len(self.nf.kappas) <= 2 and p.T >= 4 * CHUNK:
             try:
-                ks = emit_scan(p, forward_spec(p, self.nf, [], False), 2 * CHUNK, rows_per_cta(p.M), **kw)
+                ks = emit_scan(p, forward_spec(p, self.nf, [], False, 2 * CHUNK), 2 * CHUNK, rows_per_cta(p.M), **kw)
                 if ks.smem_bytes <= SMEM_BYTES:
                     return ks
             except lower.LoweringError:
                 pass
-        return emit_scan(p, forward_spec(p, self.nf, [], False), CHUNK, rows_per_cta(p.M), **kw)
+        return emit_scan(p, forward_spec(p, self.nf, [], False, CHUNK), CHUNK, rows_per_cta(p.M), **kw)
 
     def backward_scan(self, **kw) -> KernelSource:
         p = self.problem
-        return emit_scan(p, backward_scan_spec(p, self.nf, self.bp, self.dspec), CHUNK, rows_per_cta(p.M), **kw)
+        return emit_scan(p, backward_scan_spec(p, self.nf, self.bp, self.dspec, self.C), self.C, rows_per_cta(p.M), **kw)
 
     def vector_grads(self) -> KernelSource:
-        return emit_vector_grads(self.problem, self.nf, self.bp, self.dspec, self.atomic, CHUNK)
+        return emit_vector_grads(self.problem, self.nf, self.bp, self.dspec, self.atomic, self.C)
 
     def variants(self) -> List[dict]:
         """Keyword arguments of the scans worth timing; member 0 is the default."""
         return [dict(state_unroll=2), dict(state_unroll=1), dict(state_unroll=4)]
+
+
+def _fits(cp: ChunkPlan) -> bool:
+    """Whether the training kernels fit an SM."""
+    try:
+        return all(ks.smem_bytes <= SMEM_BYTES for ks in (cp.forward(), cp.backward_scan(), cp.vector_grads()))
+    except lower.LoweringError:
+        return False
 
 
 def chunk_plan(plan) -> Optional[ChunkPlan]:
@@ -2208,10 +2243,8 @@ def chunk_plan(plan) -> Optional[ChunkPlan]:
         if p.M <= 128 and p.M % 8 == 0:
             v = local_vjp(nf, p.M, p.N)
             cp.bp = backward_plan(p, nf, *v) if v is not None else None
-            if cp.bp is not None:
-                for ks in (cp.forward(), cp.backward_scan(), cp.vector_grads()):
-                    if ks.smem_bytes > SMEM_BYTES:
-                        cp.bp = None
+            if cp.bp is not None and not _fits(cp):
+                cp.bp = None
     except lower.LoweringError:
         return None
     return cp

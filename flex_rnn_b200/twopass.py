@@ -874,7 +874,7 @@ def build_twopass(step, inputs, state, dryrun=False, tuning: Optional[Tuning] = 
     ctrain = cplan is not None and cplan.bp is not None
     if ctrain:
         # checkpoints are the states at the chunks' starts, transposed; the saved row sums are the chunked form's
-        nck = (p.T + chunk.CHUNK - 1) // chunk.CHUNK
+        nck = (p.T + cplan.C - 1) // cplan.C
         fw_meta = fw_meta[:nout + nst] + get_meta([th.empty(p.B, p.H, nck, p.N, p.M, device="meta"),
                                                    th.empty(len(cplan.bp.saved), p.B, p.H, p.T, p.M, device="meta")])
     if dryrun:
