@@ -119,6 +119,7 @@ class Tuning:
     bounds: int = 0          # 1 = checked build of both kernels: every access is tested against the extents of the
                              # kernel's buffers, one outside is skipped and reported through the error word (debugging)
     use_tma: bool = True
+    fill: int = 1            # smaller tiles and rows over more CTAs where there are fewer (batch, head) pairs than SMs
     chunk: int = 1           # chunked form on the tensor cores where the step function has it (see chunk.chunk_plan)
 
 
@@ -365,12 +366,41 @@ def make_plan(step: Callable, inputs: Sequence[th.Tensor], state: Sequence[th.Te
             mb, t = t2.MB, t2
         return t
 
-    fw_tile = fitted_tile(fr, fc, tu.fw_mb, fw_tiles, 0)
-    if fw_tile.NT < 128 and fc >= 32:
+    def filling_tile(min_rows):
+        """A tile for fewer (batch, head) pairs than the GPU has SMs: the rows of a head go to as many CTAs as it takes
+        to give every SM one (but ``min_rows`` each), and a thread to 4 x 8 elements or fewer, so that a CTA has four
+        warps; a step is a chain of latencies then, and shorter with little work per thread.  None if no such tile.
+        (B1 H16 T128 128x128 fp32 Gated Delta: forward 121 -> 47 us, backward 175 -> 110 us with 32 rows per CTA;
+        B2 H16 T512 128x16 Mamba: 152 -> 66 us and 411 -> 192 us; HGRN, 8 states of 4096x1: 154 -> 86 us and
+        1362 -> 156 us.)"""
+        mb = M
+        while mb % 2 == 0 and mb // 2 >= min_rows and (mb > 1024 or B * H * (M // mb) < n_sm):
+            mb //= 2
+        r, c = 4, 8
+        try:
+            while True:
+                t = choose_tile(M, N, r, c, mb)
+                if t.NT >= 128 or r * c <= 4 or (r == 1 and c <= 4):
+                    return t if t.MB == mb and t.NT <= 512 else None
+                r, c = (r // 2, c) if r > 1 else (r, c // 2)
+        except lower.LoweringError:
+            return None
+
+    default_tiles = (tu.fw_r, tu.fw_c, tu.fw_mb, tu.bw_r, tu.bw_c, tu.bw_mb) == (4, 32, 128, 8, 8, 0)
+    idle_sms = default_tiles and bool(tu.fill) and B * H < n_sm
+    fw_tile = filling_tile(32 if N > 1 else 128) if idle_sms else None
+    if fw_tile is None:
+        fw_tile = fitted_tile(fr, fc, tu.fw_mb, fw_tiles, 0)
+    if fw_tile.NT < 128 and fc >= 32 and not idle_sms:
         # a forward CTA of fewer than four warps leaves schedulers with a single warp: halve the columns per
         # thread instead (Mamba-2's 64x128 state: R4xC16, 128 threads, measured 4 % faster than R4xC32)
         fw_tile = fitted_tile(fr, fc // 2, tu.fw_mb, fw_tiles, 0)
-    bw_tile = fitted_tile(br, bc, tu.bw_mb or None, bw_tiles, 128 if tu.bw_helper else 0)
+    # the backward's rows only go to several CTAs where no gradient is summed over rows, or where the sequence is long
+    # enough to pay for the fp32 buffers of such sums (zeroed, accumulated atomically, converted: about 10 us)
+    row_sums = any(c in (N1, S11) for c in in_cls)
+    bw_tile = filling_tile(M if row_sums and T < 128 else 32 if N > 1 else 128) if idle_sms else None
+    if bw_tile is None:
+        bw_tile = fitted_tile(br, bc, tu.bw_mb or None, bw_tiles, 128 if tu.bw_helper else 0)
     rows_split = bw_tile.MB < M
     # additive state update S' = S +/- X with X free of the state (given the saved row sums):
     # the backward can step the state backwards instead of recomputing it from checkpoints
