@@ -478,9 +478,30 @@ class ColumnCode:
             visit(n)
         return out
 
-    def emit(self, names: Sequence[str], stage: str, tl: str, n: str, pre: str) -> Dict[str, str]:
-        """Declare the values of ``names`` (and what they need) as floats with prefix ``pre``."""
-        w, done = self.kb.w, {}
+    def leaves(self, names: Sequence[str]) -> List[str]:
+        """The staged vectors that the vectors ``names`` are made of."""
+        out: List[str] = []
+
+        def visit(a):
+            if not isinstance(a, str) or self.shape[a] == S11:
+                return
+            if a in self.nodes:
+                for x in self.nodes[a].args:
+                    visit(x)
+            elif a not in out:
+                out.append(a)
+        for n in names:
+            visit(n)
+        return out
+
+    def load(self, a: str, stage: str, tl: str, n: str) -> str:
+        it = self.kb.item_by_key[a]
+        return f"frnn_io<{it.dt}>::ld({stage} + {it.off} + ({tl}) * {it.rowb}, {n})"
+
+    def emit(self, names: Sequence[str], stage: str, tl: str, n: str, pre: str, given: Optional[Dict[str, str]] = None) -> Dict[str, str]:
+        """Declare the values of ``names`` (and what they need) as floats with prefix ``pre``; ``given``: staged vectors
+        that are in registers already."""
+        w, done = self.kb.w, dict(given or {})
 
         def visit(a) -> str:
             if not isinstance(a, str):
@@ -494,8 +515,7 @@ class ColumnCode:
                 ops = [visit(x) for x in self.nodes[a].args]
                 w(f"const float {v} = {op_expr(self.nodes[a], ops)};")
             else:
-                it = self.kb.item_by_key[a]
-                w(f"const float {v} = frnn_io<{it.dt}>::ld({stage} + {it.off} + ({tl}) * {it.rowb}, {n});")
+                w(f"const float {v} = {self.load(a, stage, tl, n)};")
             done[a] = v
             return v
         for nm in names:
@@ -599,7 +619,10 @@ def emit_scan(p: Problem, s: ScanSpec, C: int, MB: int, use_tma: bool = True, st
     colS, colL, colD, colP = 0, Np, 2 * Np, 3 * Np
     colA = colP
     colG = colP + max(2 * nK, RA)
-    tm_cols = _tmem_pow2(colG + RK)
+    late_gram = colG + RK > TMEM_COLS and RA + RK <= 2 * nK
+    if late_gram:                     # Gram over p as well: read before p is written, computed once products 2 have read p
+        colG = colP + RA
+    tm_cols = _tmem_pow2(max(colG + RK, colP + 2 * nK))
     if tm_cols > TMEM_COLS:
         raise lower.LoweringError("the chunk's operands do not fit Tensor Memory")
     nchunk = (p.T + C - 1) // C
@@ -718,24 +741,41 @@ def emit_scan(p: Problem, s: ScanSpec, C: int, MB: int, use_tma: bool = True, st
         hsync()
     if dec_sc:
         od = kb.wk[s.decay][1]
-        w.open("if (hl == 0)")
-        w("float W = 1.0f;")
+        # thread q: the products of the decays before step q and after it; thread 32 + q of the next warp
+        w.open(f"if (hl < {C} || (hl >= 32 && hl < {32 + C}))")
+        w("const int j = hl & 31;")
+        w(f"float xs[{C}], W = 1.0f;")
         w("#pragma unroll")
-        w(f"for (int q = 0; q < {C}; q++) {{ dec[{o_dec} + q] = W; if (q < nv) W *= mk[{pos('q')} * {mk_row} + {od}]; }}")
-        w(f"dec[{o_dec + 2 * C}] = W;")
-        w.close()
-        w.open("if (hl == 32)")
-        w("float W = 1.0f;")
+        w(f"for (int q = 0; q < {C}; q++) xs[q] = mk[max({pos('q')}, 0) * {mk_row} + {od}];")
         w("#pragma unroll")
-        w(f"for (int q = {C - 1}; q >= 0; q--) {{ dec[{o_dec + C} + q] = W; if (q < nv) W *= mk[{pos('q')} * {mk_row} + {od}]; }}")
+        w(f"for (int q = 0; q < {C}; q++) if (q < nv && (hl < 32 ? q < j : q > j)) W *= xs[q];")
+        w(f"dec[{o_dec} + (hl < 32 ? 0 : {C}) + j] = W;")
+        w(f"if (hl == {C - 1}) dec[{o_dec + 2 * C}] = nv == {C} ? W * xs[{C - 1}] : W;")
         w.close()
 
-    def live(names, q, n, pre):
-        if whole:
-            w(f"const bool live = true; const int tl = {pos(q)}; (void)live;")
-        else:
-            w(f"const bool live = {q} < nv; const int tl = live ? {pos(q)} : 0;")
-        return col.emit(names, "stage", "tl", n, pre)
+    def steps(names, n, body):
+        """``body(values)`` for the steps q of the chunk in order, eight at a time: their loads come before the first
+        store, which the compiler would not move them across (a step at a time cost 240 cycles, all of them latencies)."""
+        lv = col.leaves(names)
+        where = (lambda q: f"const bool live = true; const int tl = {pos(q)}; (void)live; (void)tl;") if whole else \
+            (lambda q: f"const bool live = {q} < nv; const int tl = live ? {pos(q)} : 0; (void)live; (void)tl;")
+        for q8 in range(0, C, 8):
+            w.open("")
+            for a in lv:
+                w(f"float l_{a.replace('.', '_')}[8];")
+            w("#pragma unroll")
+            w.open("for (int e = 0; e < 8; e++)")
+            w(where(f"({q8} + e)"))
+            for a in lv:
+                w(f"l_{a.replace('.', '_')}[e] = {col.load(a, 'stage', 'tl', n)};")
+            w.close()
+            w("#pragma unroll")
+            w.open("for (int e = 0; e < 8; e++)")
+            w(f"const int q = {q8} + e;")
+            w(where("q"))
+            body(col.emit(names, "stage", "tl", n, "x_", {a: f"l_{a.replace('.', '_')}[e]" for a in lv}))
+            w.close()
+            w.close()
 
     def put_km(base, lbo, row, n, val):
         """Store into a K-major operand over columns: element (row, n)."""
@@ -750,21 +790,18 @@ def emit_scan(p: Problem, s: ScanSpec, C: int, MB: int, use_tma: bool = True, st
     w(f"float x[{C if dec_vec else 1}]; (void)x;")
     w.open(f"if (hl < {N})")
     w("float W = 1.0f; (void)W;")
-    w("#pragma unroll")
-    w.open(f"for (int q = 0; q < {C}; q++)")
-    v = live(s.alphas + s.kappas + ([s.decay] if dec_vec else []), "q", "hl", "x_")
-    for d, nm in enumerate(s.alphas):
-        w(f"const float a{d} = live ? {v[nm]}{' * W' if dec_vec else ''} : 0.0f;")
-        if xa:
+
+    def alpha_step(v):
+        for d, nm in enumerate(s.alphas):
+            w(f"const float a{d} = live ? {v[nm]}{' * W' if dec_vec else ''} : 0.0f;")
             put_km("alphaB", lboA, f"{d * C} + q", "hl", f"a{d}")
-        else:
-            put_km("alphaB", lboA, f"{d * C} + q", "hl", f"a{d}")
-            put_km("alphaB", lboA, f"{nA + d * C} + q", "hl", f"frnn_tf32_rest(a{d})")
-    for r, nm in enumerate(s.kappas):
-        w(f"k[{r}][q] = live ? {v[nm]} : 0.0f;")
-    if dec_vec:
-        w(f"x[q] = live ? {v[s.decay]} : 1.0f; W *= x[q];")
-    w.close()
+            if not xa:
+                put_km("alphaB", lboA, f"{nA + d * C} + q", "hl", f"frnn_tf32_rest(a{d})")
+        for r, nm in enumerate(s.kappas):
+            w(f"k[{r}][q] = live ? {v[nm]} : 0.0f;")
+        if dec_vec:
+            w(f"x[q] = live ? {v[s.decay]} : 1.0f; W *= x[q];")
+    steps(s.alphas + s.kappas + ([s.decay] if dec_vec else []), "hl", alpha_step)
     if dec_vec:
         w(f"dec[{o_dec} + hl] = W;")
     w.close()
@@ -790,20 +827,17 @@ def emit_scan(p: Problem, s: ScanSpec, C: int, MB: int, use_tma: bool = True, st
     w.open(f"if (n < {N})")
     if dec_vec:
         w("float W = 1.0f, R = 1.0f; bool tiny = false;")
-    w("#pragma unroll")
-    w.open(f"for (int q = 0; q < {C}; q++)")
-    v = live(s.kappas + ([s.decay] if dec_vec else []), "q", "n", "x_")
-    if dec_vec:
-        w(f"const float x = live ? {v[s.decay]} : 1.0f;")
-        w("W *= x; R *= frnn_rcp1(x); tiny = tiny || !(fabsf(W) > 1e-25f && fabsf(W) < 1e25f);")
-    for r, nm in enumerate(s.kappas):
-        w(f"const float y{r} = live ? {v[nm]}{' * R' if dec_vec else ''} : 0.0f;")
-        if xk:
+
+    def kappa_step(v):
+        if dec_vec:
+            w(f"const float x = live ? {v[s.decay]} : 1.0f;")
+            w("W *= x; R *= frnn_rcp1(x); tiny = tiny || !(fabsf(W) > 1e-25f && fabsf(W) < 1e25f);")
+        for r, nm in enumerate(s.kappas):
+            w(f"const float y{r} = live ? {v[nm]}{' * R' if dec_vec else ''} : 0.0f;")
             put_km(f"(smem + {off_kh})", lboH, f"{r * C} + q", "n", f"y{r}")
-        else:
-            put_km(f"(smem + {off_kh})", lboH, f"{r * C} + q", "n", f"y{r}")
-            put_km(f"(smem + {off_kh})", lboH, f"{nK + r * C} + q", "n", f"frnn_tf32_rest(y{r})")
-    w.close()
+            if not xk:
+                put_km(f"(smem + {off_kh})", lboH, f"{nK + r * C} + q", "n", f"frnn_tf32_rest(y{r})")
+    steps(s.kappas + ([s.decay] if dec_vec else []), "n", kappa_step)
     if dec_vec:
         w("if (tiny) ((volatile int*)&bar[24])[buf] = c + 1;")
     w.close()
@@ -981,10 +1015,10 @@ def emit_scan(p: Problem, s: ScanSpec, C: int, MB: int, use_tma: bool = True, st
             w(f"for (int k = {k0}; k < {k1}; k++) frnn_mma_ts_d(tm + {colA}u, tm + {a}u + k * 8, frnn_mma_next(da, {lboA}, k), FRNN_MMA_IDESC({n_}), {first_});")
     w(f"frnn_mma_commit(&bar[{B_M1}]); frnn_mma_commit(&bar[{B_AE} + (c & 1)]);")
     # Gram of the next chunk as soon as its operands are there, but never in the way of products 2
-    w(f"bool gram = c + 1 >= {nchunk};")
+    w(f"bool gram = c + 1 >= {nchunk}; (void)gram;")
     w("const u64 t_wait = frnn_now_ns();")
     w.open("for (;;)")
-    w.open(f"if (!gram && frnn_mbar_try(&bar[{B_AF} + ((c + 1) & 1)], ((c + 1) >> 1) & 1) && frnn_mbar_try(&bar[{B_HF}], (c + 1) & 1))")
+    w.open(f"if ({'false' if late_gram else '!gram'} && frnn_mbar_try(&bar[{B_AF} + ((c + 1) & 1)], ((c + 1) >> 1) & 1) && frnn_mbar_try(&bar[{B_HF}], (c + 1) & 1))")
     gram_products("c + 1")
     w("gram = true;")
     w.close()
@@ -999,6 +1033,8 @@ def emit_scan(p: Problem, s: ScanSpec, C: int, MB: int, use_tma: bool = True, st
         w(f"for (int k = 0; k < {nK // 8}; k++) frnn_mma_ts_d(tm + {colD}u, tm + {a}u + k * 8, frnn_mma_next({dsc}, {lboK}, k), FRNN_MMA_IDESC({Np}), {'k > 0' if i == 0 else 'true'});")
     w(f"frnn_mma_commit(&bar[{B_M2}]); frnn_mma_commit(&bar[{B_KE}]);")
     w.open("if (!gram)")
+    if late_gram:
+        w(f"if (!frnn_mbar_wait(&bar[{B_M2}], c & 1, err, {ERR})) return;")
     w(f"if (!frnn_mbar_wait(&bar[{B_AF} + ((c + 1) & 1)], ((c + 1) >> 1) & 1, err, {ERR}) || !frnn_mbar_wait(&bar[{B_HF}], (c + 1) & 1, err, {ERR})) return;")
     gram_products("c + 1")
     w.close()
@@ -1515,7 +1551,11 @@ def emit_vector_grads(p: Problem, nf: Normal, bp: BackwardPlan, dspec: Sequence[
     off_Z = off_X + al((M // 4 - 1) * lboX + max(2048 + 16, lboX))
     off_sl = off_Z + al(M // 4 * lboZ)
     sl_bytes = al(MS // 4 * lboS)
-    end1 = off_sl + 4 * sl_bytes
+    # two CTAs per SM hide each other's latencies; where X and Z are too large for that, the one CTA keeps two buffers of
+    # slices and loads four slices ahead instead of two
+    ctas = 2 if C <= 16 else 1
+    NB, DP = (1, 2) if ctas == 2 else (2, 4)
+    end1 = off_sl + 4 * NB * sl_bytes
     # second phase, over the same memory
     lboT, lbo1, lbo2 = 128 * 16, 2 * nA * 16, 2 * nK * 16
     off_kT = off_X
@@ -1551,7 +1591,7 @@ def emit_vector_grads(p: Problem, nf: Normal, bp: BackwardPlan, dspec: Sequence[
 
     w(lower._header(chunk_prelude()))
     w(f"// vector gradients: B={B} T={T} H={H} M={M} N={N}; {C} steps per chunk, {nd} row sums, {nr} rank-1 terms")
-    w(f'extern "C" __global__ void __launch_bounds__({VG_THREADS}, 2)')
+    w(f'extern "C" __global__ void __launch_bounds__({VG_THREADS}, {ctas})')
     w.open(f"frnn_cvg({', '.join(decl)})")
     w("FRNN_DYN_SMEM(smem);")
     w("const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;")
@@ -1670,7 +1710,7 @@ def emit_vector_grads(p: Problem, nf: Normal, bp: BackwardPlan, dspec: Sequence[
     per = 128 // (VG_THREADS // q4)        # columns per thread and slice
     w(f"const int sm4 = tid % {q4}, sn = tid / {q4};")
     w(f"const float* ckp = ck + (((long)b * {H} + h) * {nchunk} + kc) * {N}L * {M}L; const float* ekp = eck + (((long)b * {H} + h) * {nchunk} + kc) * {N}L * {M}L;")
-    w(f"float zz[{per}], sv[2][{per}][4], ev[2][{per}][4];")
+    w(f"float zz[{per}], sv[{DP}][{per}][4], ev[{DP}][{per}][4];")
     w("#pragma unroll")
     w(f"for (int i = 0; i < {per}; i++) zz[i] = 0.0f;")
 
@@ -1681,10 +1721,9 @@ def emit_vector_grads(p: Problem, nf: Normal, bp: BackwardPlan, dspec: Sequence[
         w(f"frnn_ldv<0,4>(ckp, n * {M}L + ({sx}) * {MS} + sm4 * 4, sv[{u}][i]);")
         w(f"frnn_ldv<0,4>(ekp, n * {M}L + ({sx}) * {MS} + sm4 * 4, ev[{u}][i]);")
         w.close()
-    load_slice("0", "0")
-    if nsl > 1:
-        load_slice("1", "1")
-    w("if (tid == 0) { frnn_mbar_init(&bar[0], 1); frnn_mbar_init(&bar[1], 1); frnn_mbar_init(&bar[2], 1); ((int*)&bar[4])[0] = 0; frnn_mbar_init_fence(); }")
+    for u in range(min(DP, nsl)):
+        load_slice(str(u), str(u))
+    w("if (tid == 0) { frnn_mbar_init(&bar[0], 1); frnn_mbar_init(&bar[1], 1); frnn_mbar_init(&bar[2], 1); frnn_mbar_init(&bar[5], 1); ((int*)&bar[4])[0] = 0; frnn_mbar_init_fence(); }")
     w.open("if (warp == 0)")
     w(f"frnn_tmem_alloc((u32*)&bar[3], {tm_cols}u);")
     w("frnn_tmem_fence_before_sync();")
@@ -1758,15 +1797,18 @@ def emit_vector_grads(p: Problem, nf: Normal, bp: BackwardPlan, dspec: Sequence[
         w(f"float {reg(a)}[{HC}];")
     for a in wleaves:
         w(f"float o_{reg(a)}[{HC}];          // the other half's timesteps")
-    w.open(f"for (int s2 = 0; s2 < {nsl}; s2 += 2)")
-    for u in (0, 1):
+    w("#pragma unroll 1")
+    w.open(f"for (int s2 = 0; s2 < {nsl}; s2 += {DP})")
+    for u in range(DP):
+        bb = 5 if u % NB else 1
         w.open(f"if (s2 + {u} < {nsl})")
         w(f"const int s = s2 + {u};")
-        w(f"if (s > 0 && !frnn_mbar_wait(&bar[1], (s - 1) & 1, err, {ERR})) break;     // products of the previous slice are complete")
+        w(f"if (s >= {NB} && !frnn_mbar_wait(&bar[{bb}], (s / {NB} - 1) & 1, err, {ERR})) break;     // the products that read this buffer are complete")
         w("#pragma unroll")
         w.open(f"for (int i = 0; i < {per}; i++)")
         w(f"const int n = sn + i * {VG_THREADS // q4};")
-        w(f"unsigned char* dst = smem + {off_sl} + sm4 * {lboS} + (n >> 3) * 128 + (n & 7) * 16;")
+        off_b = off_sl + (u % NB) * 4 * sl_bytes
+        w(f"unsigned char* dst = smem + {off_b} + sm4 * {lboS} + (n >> 3) * 128 + (n & 7) * 16;")
         w("float r[4];")
         w("#pragma unroll")
         w(f"for (int k = 0; k < 4; k++) {{ r[k] = frnn_tf32_rest(sv[{u}][i][k]); zz[i] = fmaf(sv[{u}][i][k], ev[{u}][i][k], zz[i]); }}")
@@ -1775,9 +1817,9 @@ def emit_vector_grads(p: Problem, nf: Normal, bp: BackwardPlan, dspec: Sequence[
         w(f"for (int k = 0; k < 4; k++) r[k] = frnn_tf32_rest(ev[{u}][i][k]);")
         w(f"frnn_stv<0,4>(dst + {2 * sl_bytes}, 0, ev[{u}][i]); frnn_stv<0,4>(dst + {3 * sl_bytes}, 0, r);")
         w.close()
-        w(f"if (s + 2 < {nsl}) {{")
+        w(f"if (s + {DP} < {nsl}) {{")
         w.ind += 1
-        load_slice("s + 2", str(u))
+        load_slice(f"s + {DP}", str(u))
         w.ind -= 1
         w("}")
         w("frnn_async_proxy_fence();")
@@ -1785,11 +1827,11 @@ def emit_vector_grads(p: Problem, nf: Normal, bp: BackwardPlan, dspec: Sequence[
         w.open("if (tid == 0)")
         for k in range(MS // 8):
             for which, (col_, dsc, lbo, n2) in enumerate(((cD1, "dX", lboX, nA), (cD2, "dZ", lboZ, nK))):
-                sb = off_sl + 2 * which * sl_bytes + k * 2 * lboS
+                sb = off_b + 2 * which * sl_bytes + k * 2 * lboS
                 bexp = f"frnn_mma_next({dsc}, {lbo}, s * {MS // 8} + {k})"
                 w(f"frnn_mma_ss_d(tm + {col_}u, frnn_mma_desc(smem + {sb}, {lboS}), {bexp}, FRNN_MMA_IDESC({2 * n2}), {'s > 0' if k == 0 else 'true'});")
                 w(f"frnn_mma_ss_d(tm + {col_}u, frnn_mma_desc(smem + {sb + sl_bytes}, {lboS}), {bexp}, FRNN_MMA_IDESC({2 * n2}), true);")
-        w("frnn_mma_commit(&bar[1]);")
+        w(f"frnn_mma_commit(&bar[{bb}]);")
         w.close()
         w.close()
     w.close()
@@ -1811,7 +1853,10 @@ def emit_vector_grads(p: Problem, nf: Normal, bp: BackwardPlan, dspec: Sequence[
         w(f"for (int o = {q4 // 2}; o > 0; o >>= 1) zz[i] += frnn_shfl_xor(zz[i], o);")
         w(f"if (sm4 == 0) z0[sn + i * {VG_THREADS // q4}] = zz[i];")
         w.close()
-    w(f"bool ok = frnn_mbar_wait(&bar[0], 0, err, {ERR}) && frnn_mbar_wait(&bar[1], {(nsl - 1) & 1}, err, {ERR});")
+    w(f"bool ok = frnn_mbar_wait(&bar[0], 0, err, {ERR});")
+    for u in range(min(NB, nsl)):
+        uses = (nsl - u + NB - 1) // NB
+        w(f"ok = frnn_mbar_wait(&bar[{5 if u else 1}], {(uses - 1) & 1}, err, {ERR}) && ok;")
     w("frnn_tmem_fence_after_sync();")
     w("frnn_block_sync();       // X, Z and the slices are no longer read")
     w("const u32 lanes = tm + frnn_tmem_lane_base(warp);")
@@ -2243,6 +2288,12 @@ def chunk_plan(plan) -> Optional[ChunkPlan]:
         if p.M <= 128 and p.M % 8 == 0:
             v = local_vjp(nf, p.M, p.N)
             cp.bp = backward_plan(p, nf, *v) if v is not None else None
+            # 32 steps per chunk halve the traffic of the chunk boundaries and the chains of the scans, but not the
+            # substitution: for large states and few pairs of vectors (TIMES)
+            if cp.bp is not None and len(nf.alphas) * len(nf.kappas) <= 2 and p.M * p.N >= 8192 and p.T >= 4 * CHUNK:
+                cp.C = 2 * CHUNK
+                if not _fits(cp):
+                    cp.C = CHUNK
             if cp.bp is not None and not _fits(cp):
                 cp.bp = None
     except lower.LoweringError:
