@@ -603,18 +603,22 @@ def emit_scan(p: Problem, s: ScanSpec, C: int, MB: int, use_tma: bool = True, st
     o_dg = gram_f
     o_end = o_dg + (len(s.diags) * C + 3) // 4 * 4
     lboA, lboH, lboK = RA * 16 + 16, RK * 16 + 16, Np * 16
-    off_stage = 256
-    off_mk = off_stage + 2 * al(kb.stage_bytes)
-    mk_bytes = al(mk_row * C * 4)
-    off_gr = off_mk + 2 * mk_bytes
-    gr_bytes = al(o_end * 4)
-    off_dec = off_gr + 2 * gr_bytes
-    off_al = off_dec + al(3 * dec_f * 4)
-    al_bytes = al((N // 4 - 1) * lboA + max(2048 + 16, lboA))     # Gram reads 128 rows of alpha, whatever is there
-    off_ka = off_al + 2 * al_bytes
-    ka_bytes = al(nK // 4 * lboK)
-    off_kh = off_ka + (1 if xk else 2) * ka_bytes
-    smem_bytes = off_kh + al(N // 4 * lboH)
+    # two buffers of raw inputs, or one where two do not fit (the next copies then wait for the last column to be read)
+    for NS in (2, 1):
+        off_stage = 256
+        off_mk = off_stage + NS * al(kb.stage_bytes)
+        mk_bytes = al(mk_row * C * 4)
+        off_gr = off_mk + 2 * mk_bytes
+        gr_bytes = al(o_end * 4)
+        off_dec = off_gr + 2 * gr_bytes
+        off_al = off_dec + al(3 * dec_f * 4)
+        al_bytes = al((N // 4 - 1) * lboA + max(2048 + 16, lboA))     # Gram reads 128 rows of alpha, whatever is there
+        off_ka = off_al + 2 * al_bytes
+        ka_bytes = al(nK // 4 * lboK)
+        off_kh = off_ka + (1 if xk else 2) * ka_bytes
+        smem_bytes = off_kh + al(N // 4 * lboH)
+        if smem_bytes <= SMEM_BYTES:
+            break
     # Tensor Memory columns: S | rest of S | products 2 | p | rest of p, over products 1 (read before p is written) | Gram
     colS, colL, colD, colP = 0, Np, 2 * Np, 3 * Np
     colA = colP
@@ -714,7 +718,7 @@ def emit_scan(p: Problem, s: ScanSpec, C: int, MB: int, use_tma: bool = True, st
         """Plain copies of one chunk into stage buffer ``be`` (inputs no tensor copy reaches)."""
         if kb.plain_items:
             w.open("")
-            w(f"unsigned char* stage = smem + {off_stage} + ({be}) * {al(kb.stage_bytes)}; (void)stage;")
+            w(f"unsigned char* stage = smem + {off_stage} + (({be}) % {NS}) * {al(kb.stage_bytes)}; (void)stage;")
             kb.emit_plain_direct("stage", t0e, nve, "hl", PT)
             w.close()
     first = nchunk - 1 if s.reverse else 0
@@ -722,14 +726,18 @@ def emit_scan(p: Problem, s: ScanSpec, C: int, MB: int, use_tma: bool = True, st
     w("#pragma unroll 1")
     w.open(f"for (int c = 0; c < {nchunk}; c++)")
     head("")
-    w(f"const unsigned char* stage = smem + {off_stage} + buf * {al(kb.stage_bytes)};")
+    w(f"const unsigned char* stage = smem + {off_stage} + (c % {NS}) * {al(kb.stage_bytes)};")
     w(f"unsigned char* alphaB = smem + {off_al} + buf * {al_bytes};")
-    w.open(f"if (c + 1 < {nchunk})" if kb.plain_items else "")
-    nxt = f"(kc {'-' if s.reverse else '+'} 1)"
-    h_issue(f"{nxt} * {C}", f"min({C}, {p.T} - {nxt} * {C})", "(c + 1) & 1")
-    w.close()
+    def next_plain():
+        if kb.plain_items:
+            nxt = f"(kc {'-' if s.reverse else '+'} 1)"
+            w.open(f"if (c + 1 < {nchunk})")
+            h_issue(f"{nxt} * {C}", f"min({C}, {p.T} - {nxt} * {C})", "c + 1")
+            w.close()
+    if NS == 2:
+        next_plain()
     if kb.tma_items:
-        w(f"if (!frnn_mbar_wait(&bar[{B_RAW} + buf], (c >> 1) & 1, err, {ERR})) return;")
+        w(f"if (!frnn_mbar_wait(&bar[{B_RAW} + c % {NS}], (c / {NS}) & 1, err, {ERR})) return;")
     if kb.plain_items:
         hsync()
     w(f"if (c >= 2 && !frnn_mbar_wait(&bar[{B_GE} + buf], ((c >> 1) - 1) & 1, err, {ERR})) return;")
@@ -844,6 +852,8 @@ def emit_scan(p: Problem, s: ScanSpec, C: int, MB: int, use_tma: bool = True, st
     w("frnn_async_proxy_fence();")
     w(f"frnn_mbar_arrive(&bar[{B_HF}]);")
     w.close()
+    if not dec_vec:
+        w(f"frnn_mbar_arrive(&bar[{B_SE} + c % {NS}]);       // the raw inputs are read")
     # --- Gram: alpha against kappa, rows (d, j), columns (r, i)
     w(f"if (!frnn_mbar_wait(&bar[{B_MG}], c & 1, err, {ERR})) return;")
     slow = "((volatile int*)&bar[24])[buf] == c + 1"
@@ -957,9 +967,11 @@ def emit_scan(p: Problem, s: ScanSpec, C: int, MB: int, use_tma: bool = True, st
         w.close()
         w.close()
     w("frnn_tmem_fence_before_sync();")
-    w(f"frnn_mbar_arrive(&bar[{B_GF} + buf]); frnn_mbar_arrive(&bar[{B_SE} + buf]);")
+    w(f"frnn_mbar_arrive(&bar[{B_GF} + buf]);" + (f" frnn_mbar_arrive(&bar[{B_SE} + c % {NS}]);" if dec_vec else ""))
     if kb.plain_items:
         hsync()
+    if NS == 1:
+        next_plain()
     w.close()     # chunk loop
     w.open("if (hl < 128)")
     w(f"const int c = {nchunk};")
@@ -979,8 +991,8 @@ def emit_scan(p: Problem, s: ScanSpec, C: int, MB: int, use_tma: bool = True, st
         w.open(f"for (int c = 0; c < {nchunk}; c++)")
         chunk_head_line = f"const int kc = {f'{nchunk - 1} - c' if s.reverse else 'c'}, t0 = kc * {C}, nv = min({C}, {p.T} - t0);"
         w(chunk_head_line)
-        w(f"if (c >= 2 && !frnn_mbar_wait(&bar[{B_SE} + (c & 1)], ((c >> 1) - 1) & 1, err, {ERR})) return;")
-        w(f"sc_issue(smem + {off_stage} + (c & 1) * {al(kb.stage_bytes)}, &bar[{B_RAW} + (c & 1)], t0, nv, lane, b, h, m0{tma_call});")
+        w(f"if (c >= {NS} && !frnn_mbar_wait(&bar[{B_SE} + c % {NS}], (c / {NS} - 1) & 1, err, {ERR})) return;")
+        w(f"sc_issue(smem + {off_stage} + (c % {NS}) * {al(kb.stage_bytes)}, &bar[{B_RAW} + c % {NS}], t0, nv, lane, b, h, m0{tma_call});")
         w.close()
     w("return;")
     w.close()
@@ -2281,7 +2293,7 @@ def chunk_plan(plan) -> Optional[ChunkPlan]:
     nf = normal_form(plan.g_fw, p.in_names, p.st_names[0], plan.n_out)
     if nf is None or not all(nf_inputs(nf)):
         return None
-    cp = ChunkPlan(p, nf, None, [g.spec for g in plan.grads], [g.atomic for g in plan.grads])
+    cp = ChunkPlan(p, nf, None, [g.spec for g in plan.whole_grads], [g.atomic for g in plan.whole_grads])
     try:
         if cp.infer().smem_bytes > SMEM_BYTES:
             return None

@@ -559,6 +559,7 @@ def make_plan(step: Callable, inputs: Sequence[th.Tensor], state: Sequence[th.Te
                 g_fw0.count_mn_ops(), joint.pruned(jout, "all").count_mn_ops(), reverse, post_split, choice)
     plan.dy_names, plan.dnext_names = dy_names, dnext_names   # type: ignore[attr-defined]
     plan.n_sm = n_sm                                            # type: ignore[attr-defined]
+    plan.whole_grads = make_grads(False)                        # type: ignore[attr-defined]  (no rows over several CTAs)
     return plan, fw_meta, bw_meta
 
 
@@ -903,6 +904,7 @@ def build_twopass(step, inputs, state, dryrun=False, tuning: Optional[Tuning] = 
     cplan = chunk.chunk_plan(plan) if plan.tuning.chunk and not pinned else None
     ctrain = cplan is not None and cplan.bp is not None
     if ctrain:
+        plan.grads = plan.whole_grads
         # checkpoints are the states at the chunks' starts, transposed; the saved row sums are the chunked form's
         nck = (p.T + cplan.C - 1) // cplan.C
         fw_meta = fw_meta[:nout + nst] + get_meta([th.empty(p.B, p.H, nck, p.N, p.M, device="meta"),
