@@ -1565,7 +1565,8 @@ def emit_vector_grads(p: Problem, nf: Normal, bp: BackwardPlan, dspec: Sequence[
     sl_bytes = al(MS // 4 * lboS)
     # two CTAs per SM hide each other's latencies; where X and Z are too large for that, the one CTA keeps two buffers of
     # slices and loads four slices ahead instead of two
-    ctas = 2 if C <= 16 else 1
+    single = max(off_sl + 4 * sl_bytes, off_X + 2 * (nK + nA) // 4 * 128 * 16 + 16 * (nA * nK // 2 + nA))
+    ctas = 2 if single <= SMEM_BYTES // 2 - 1024 else 1
     NB, DP = (1, 2) if ctas == 2 else (2, 4)
     end1 = off_sl + 4 * NB * sl_bytes
     # second phase, over the same memory
