@@ -490,7 +490,15 @@ def make_plan(step: Callable, inputs: Sequence[th.Tensor], state: Sequence[th.Te
         tu.bw_tmem_slots = 0
         if reverse is None and tu.bw_helper and tu.bw_tmem and T >= 8:
             # segment bases in Tensor Memory: as many slots as fit, one step fewer to recompute per slot more
-            for nsl in (8, 4):
+            # (a thread with few elements is done with 8 steps before the next chunk's checkpoint and inputs are there: 32 or
+            # 16 of its states, one per step, fit as well)
+            small = idle_sms and bw_tile.R * bw_tile.C * nst <= 8
+            for nsl in ([n for n in (32, 16) if n <= T] if small else []) + [8, 4]:
+                if nsl > 8 and fits(1, nsl, max(1, tu.kflush), 2 if tu.bw_helper else 1, 1, tmem=nsl):
+                    tu.bw_tmem_slots = nsl
+                    return (1, max(1, tu.kflush), 2), nsl, 1
+                if nsl > 8:
+                    continue
                 for kflush, bufs in flush_options(1):
                     if fits(8 // nsl, nsl, kflush, bufs, 1, tmem=nsl):
                         tu.bw_tmem_slots = nsl
@@ -573,8 +581,9 @@ def generate_forward(plan: Plan, tile: Optional[lower.Tile] = None, pack: Option
     p, tu = plan.problem, plan.tuning
     pack2 = bool(tu.pack2 & 2) if pack is None else bool(pack)
     tile = tile or plan.fw_tile
-    # keep the per-CTA shared memory small enough for all CTAs of an SM to be resident
-    stage = max(1, min(stage or tu.fw_stage, p.T))
+    # keep the per-CTA shared memory small enough for all CTAs of an SM to be resident; where a thread has few elements
+    # the steps of a chunk must still take longer than the copies of the next one
+    stage = max(1, min(stage or (tu.fw_stage * 2 if tile.R * tile.C * plan.n_st <= 4 else tu.fw_stage), p.T))
     if unroll is None:
         # bound the code size of the unrolled step loop: about 0.55 instructions of 16 bytes per counted [M,N]
         # operation and tile element, plus the per-step overhead (larger bodies measured no faster)
