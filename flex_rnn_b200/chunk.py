@@ -2232,6 +2232,7 @@ class ChunkPlan:
     dspec: List[TensorSpec]
     atomic: List[bool]
     C: int = CHUNK                            # timesteps per chunk of the training kernels
+    short: bool = True                        # whether calls without gradients are chunked
 
     def forward(self, **kw) -> KernelSource:
         p = self.problem
@@ -2272,43 +2273,51 @@ def _fits(cp: ChunkPlan) -> bool:
 
 
 def chunk_plan(plan) -> Optional[ChunkPlan]:
-    """The chunked form of a specialisation (a ``twopass.Plan``), where it applies and is the faster one:
+    """The chunked form of a specialisation (a ``twopass.Plan``), where it applies and is the faster one.
 
-    * one state, in the normal form, of at most 128 columns (a multiple of 8: one tf32 product takes 8) - the state, its
-      rest and the products of a chunk then fit Tensor Memory; training also wants the rows of a head in one CTA;
-    * 16-bit inputs.  fp32 inputs keep the recurrent kernels, whose sums are fp32 throughout (relative error 1e-7 against
-      5e-7 of the split products here);
-    * at least two chunks: shorter sequences are done before the first chunk's operands are ready.
-    """
+    It applies to one state in the normal form, of at most 128 columns (a multiple of 8: one tf32 product takes 8) - the
+    state, its rest and the products of a chunk then fit Tensor Memory; training also wants the rows of a head in one
+    CTA.  The inputs have 16 bits; for fp32 inputs the recurrent kernels stay, whose sums are fp32 throughout.
+
+    A chunk costs a CTA the same chain whatever the state's size, and only one CTA fits an SM; the recurrent kernels' time
+    grows with the state and they share an SM.  So: where every SM has at most one CTA (T128 Delta Rule, forward +
+    backward: 16 heads of 128x128 82 us against 126 us, 128 heads of 64x64 106 us against 146 us), and beyond that for
+    large states (256 heads T1024 128x128: 1.65 ms against 2.57 ms; 512 heads of 64x128, T128: 434 against 436 us, Mamba-2
+    412 against 485 us; but 512 heads of 64x64 376 against 321 us).  Calls without gradients beyond one CTA per SM also
+    want more than half of Tensor Memory's 128 lanes in use (512 heads of 64x128, Mamba-2: 114 against 94 us)."""
     p = plan.problem
-    if plan.n_st != 1 or p.N % 8 or not 16 <= p.N <= 128 or p.T < 2 * CHUNK or p.naux < 0:
+    if plan.n_st != 1 or p.N % 8 or not 16 <= p.N <= 128 or p.T < 2 * CHUNK or 0 in (p.B, p.T, p.H):
         return None
     if any(s.dt not in (lower.DT_BF16, lower.DT_F16) for s in p.inputs) or p.states[0].dt == lower.DT_F64:
         return None
-    if p.M < 8 or rows_per_cta(p.M) is None or 0 in (p.B, p.T, p.H):
+    if p.M < 8 or rows_per_cta(p.M) is None:
         return None
     for s in p.inputs:
         cls = (int(s.shape[3] > 1), int(s.shape[4] > 1))
         if list(s.shape[:3]) != [p.B, p.T, p.H] and not (cls == S11 and s.shape[1] == 1):
             return None
+    one_wave = p.B * p.H * (p.M // rows_per_cta(p.M)) <= plan.n_sm
+    if not one_wave and p.M * p.N < 8192:
+        return None
     nf = normal_form(plan.g_fw, p.in_names, p.st_names[0], plan.n_out)
     if nf is None or not all(nf_inputs(nf)):
         return None
     cp = ChunkPlan(p, nf, None, [g.spec for g in plan.whole_grads], [g.atomic for g in plan.whole_grads])
     try:
-        if cp.infer().smem_bytes > SMEM_BYTES:
-            return None
+        cp.short = (one_wave or p.M > 64) and cp.infer().smem_bytes <= SMEM_BYTES
         if p.M <= 128 and p.M % 8 == 0:
             v = local_vjp(nf, p.M, p.N)
             cp.bp = backward_plan(p, nf, *v) if v is not None else None
-            # 32 steps per chunk halve the traffic of the chunk boundaries and the chains of the scans, but not the
-            # substitution: for large states and few pairs of vectors (TIMES)
-            if cp.bp is not None and len(nf.alphas) * len(nf.kappas) <= 2 and p.M * p.N >= 8192 and p.T >= 4 * CHUNK:
-                cp.C = 2 * CHUNK
-                if not _fits(cp):
-                    cp.C = CHUNK
-            if cp.bp is not None and not _fits(cp):
-                cp.bp = None
     except lower.LoweringError:
         return None
-    return cp
+    if cp.bp is not None:
+        # 32 steps per chunk halve the traffic of the chunk boundaries and the chains of the scans, but not the
+        # substitution: for large states and few pairs of vectors (B8 T1024 H32 128x128, forward + backward: Delta Rule
+        # 1.66 ms against 1.91 ms, Mamba-2 1.30 ms against 1.67 ms; 512 heads of 32x32, T512: 1.18 against 1.05 ms)
+        if len(nf.alphas) * len(nf.kappas) <= 2 and p.M * p.N >= 8192 and p.T >= 4 * CHUNK:
+            cp.C = 2 * CHUNK
+            if not _fits(cp):
+                cp.C = CHUNK
+        if not _fits(cp):
+            cp.bp = None
+    return cp if cp.short or cp.bp is not None else None

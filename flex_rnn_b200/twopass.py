@@ -912,6 +912,7 @@ def build_twopass(step, inputs, state, dryrun=False, tuning: Optional[Tuning] = 
     pinned = plan.tuning.fw_variant >= 0 or plan.tuning.bw_variant >= 0
     cplan = chunk.chunk_plan(plan) if plan.tuning.chunk and not pinned else None
     ctrain = cplan is not None and cplan.bp is not None
+    cshort = cplan is not None and cplan.short
     if ctrain:
         plan.grads = plan.whole_grads
         # checkpoints are the states at the chunks' starts, transposed; the saved row sums are the chunked form's
@@ -1058,7 +1059,7 @@ def build_twopass(step, inputs, state, dryrun=False, tuning: Optional[Tuning] = 
         forward kernel only writes its outputs) and keep the fastest."""
         first = infer_kernel() if infer else (fw_src, launch_fw)
         best, log = None, []
-        chunked = cplan is not None if infer else ctrain
+        chunked = cshort if infer else ctrain
         for k, kw in enumerate(cplan.variants() if chunked else forward_variants(plan)):
             try:
                 if chunked:
@@ -1087,7 +1088,7 @@ def build_twopass(step, inputs, state, dryrun=False, tuning: Optional[Tuning] = 
         """(source, launcher) of the planned kernel for calls without gradients, made on first use."""
         if "launch_infer" not in tuned:
             kw = forward_variants(plan)[tu0.fw_variant] if tu0.fw_variant > 0 else {}
-            tuned["infer_src"] = generate_forward(plan, infer=True, **kw) if cplan is None else _checked(cplan.infer(), tu0)
+            tuned["infer_src"] = _checked(cplan.infer(), tu0) if cshort else generate_forward(plan, infer=True, **kw)
             tuned["launch_infer"] = make(tuned["infer_src"])
         return tuned["infer_src"], tuned["launch_infer"]
 

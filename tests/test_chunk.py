@@ -53,7 +53,13 @@ def test_which_steps_have_the_form():
         assert (cp is not None and cp.bp is not None) == want, op
     step, ins, s, _, _ = case("delta_rule", 1, 64, 1, 256, 64, torch.bfloat16)
     cp = chunk.chunk_plan(make_plan(step, ins, [s])[0])
-    assert cp is not None and cp.bp is None            # rows over several CTAs: calls without gradients only
+    assert cp is not None and cp.short and cp.bp is None            # rows over several CTAs: calls without gradients only
+    for H, M, N, short, train in [(64, 64, 64, True, True), (400, 64, 64, False, False), (400, 64, 128, False, True),
+                                  (400, 128, 64, True, True), (400, 256, 128, True, False), (4, 64, 256, False, False)]:
+        args = [torch.empty(1, 64, H, *x, dtype=torch.bfloat16, device="meta") for x in ((1, N), (1, N), (M, 1), (1, 1))]
+        plan = make_plan(W.delta_rule, args, [torch.empty(1, H, M, N, dtype=torch.bfloat16, device="meta")])[0]
+        cp = chunk.chunk_plan(plan)
+        assert (cp is not None and cp.short, cp is not None and cp.bp is not None) == (short, train), (H, M, N)
 
 
 @pytest.mark.parametrize("op,B,T,H,M,N,dt,reset", CASES)
