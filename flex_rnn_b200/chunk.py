@@ -1874,34 +1874,48 @@ def emit_vector_grads(p: Problem, nf: Normal, bp: BackwardPlan, dspec: Sequence[
     w("frnn_block_sync();       // X, Z and the slices are no longer read")
     w("const u32 lanes = tm + frnn_tmem_lane_base(warp);")
     w(f"float* Lr = (float*)(smem + {off_Lr});")
-    # ---- L: rows (d, j) of hi and of rest, columns (r, i) of hi and of rest
-    w.open(f"if (tid >= {nA // 32 * 32} && tid < {(2 * nA + 31) // 32 * 32})")
-    w(f"float u[{nK}];")
-    w(f"frnn_tmem_ld<{nK}>(lanes + {cL}u, u); frnn_tmem_wait_ld();")
+    # ---- L: rows (d, j) of hi and of rest, columns (r, i) of hi and of rest; each half of the threads takes half of the i
+    def ld_L(dst):
+        w(f"float {dst}[{nr * HC}];")
+        w.open("")
+        w(f"float lo[{nr * HC}];")
+        for r in range(nr):
+            w(f"frnn_tmem_ld<{HC}>(lanes + {cL + r * C}u + (u32)q0, &{dst}[{r * HC}]); frnn_tmem_ld<{HC}>(lanes + {cL + nK + r * C}u + (u32)q0, &lo[{r * HC}]);")
+        w("frnn_tmem_wait_ld();")
+        w("#pragma unroll")
+        w(f"for (int k = 0; k < {nr * HC}; k++) {dst}[k] += lo[k];")
+        w.close()
+    w.open(f"if (x128 >= {nA // 32 * 32} && x128 < {(2 * nA + 31) // 32 * 32})")
+    ld_L("u")
+    w.open(f"if (x128 >= {nA} && x128 < {2 * nA})")
     w("#pragma unroll")
-    w(f"for (int i = 0; i < {nK}; i++) if (tid >= {nA} && tid < {2 * nA}) Lr[(tid - {nA}) * {LS} + i] = u[i];")
+    w(f"for (int k = 0; k < {nr * HC}; k++) Lr[(x128 - {nA}) * {LS} + (k / {HC}) * {C} + q0 + k % {HC}] = u[k];")
+    w.close()
     w.close()
     w("frnn_block_sync();")
-    w.open(f"if (tid < {(nA + 31) // 32 * 32})")
-    w(f"float u[{nK}], x[{nK}];")
-    w(f"frnn_tmem_ld<{nK}>(lanes + {cL}u, u); frnn_tmem_ld<{nK}>(lanes + {cL + nK}u, x); frnn_tmem_wait_ld();")
-    w.open(f"if (tid < {nA})")
-    w(f"const int j = tid % {C};")
-    if dec_sc:
-        w("float D = 1.0f;")
+    w.open(f"if (x128 < {(nA + 31) // 32 * 32})")
+    ld_L("u")
+    w.open(f"if (x128 < {nA})")
+    w(f"const int j = x128 % {C};")
     w("#pragma unroll")
-    w.open(f"for (int i = {C - 1}; i >= 0; i--)")
+    w(f"for (int k = 0; k < {nr * HC}; k++) u[k] += Lr[x128 * {LS} + (k / {HC}) * {C} + q0 + k % {HC}];")
+    if dec_sc:
+        w(f"float D = 1.0f;          // decays between step j and the last of this half")
+        w(f"if (hf == 0) for (int l = {HC}; l < {C}; l++) if (l < j && l < nv) D *= {slot(nf.decay)} + l];")
+    w("#pragma unroll")
+    w.open(f"for (int k = {HC - 1}; k >= 0; k--)")
+    w("const int i = q0 + k;")
     w("#pragma unroll")
     w.open(f"for (int r = 0; r < {nr}; r++)")
     w(f"const int ri = r * {C} + i;")
-    w(f"float a = i < j ? u[ri] + x[ri] + Lr[tid * {LS} + ri] : 0.0f;")
-    w(f"Lr[tid * {LS} + ri] = a;")
+    w(f"float a = i < j ? u[r * {HC} + k] : 0.0f;")
+    w(f"Lr[x128 * {LS} + ri] = a;")
     if dec_sc:
         w("a *= D;")
     w("const float hi = a, lo = frnn_tf32_rest(a);")
-    w(f"unsigned char* d1 = smem + {off_L1} + (ri >> 2) * {lbo1} + (ri & 3) * 4; const int ra = tid, rb = tid + {nA};")
+    w(f"unsigned char* d1 = smem + {off_L1} + (ri >> 2) * {lbo1} + (ri & 3) * 4; const int ra = x128, rb = x128 + {nA};")
     w("*(float*)(d1 + (ra >> 3) * 128 + (ra & 7) * 16) = hi; *(float*)(d1 + (rb >> 3) * 128 + (rb & 7) * 16) = lo;")
-    w(f"unsigned char* d2 = smem + {off_L2} + (tid >> 2) * {lbo2} + (tid & 3) * 4; const int rc = ri, rd = ri + {nK};")
+    w(f"unsigned char* d2 = smem + {off_L2} + (x128 >> 2) * {lbo2} + (x128 & 3) * 4; const int rc = ri, rd = ri + {nK};")
     w("*(float*)(d2 + (rc >> 3) * 128 + (rc & 7) * 16) = hi; *(float*)(d2 + (rd >> 3) * 128 + (rd & 7) * 16) = lo;")
     w.close()
     if dec_sc:
