@@ -834,12 +834,12 @@ def emit_scan(p: Problem, s: ScanSpec, C: int, MB: int, use_tma: bool = True, st
     w("const int n = hl - 128;")
     w.open(f"if (n < {N})")
     if dec_vec:
-        w("float W = 1.0f, R = 1.0f; bool tiny = false;")
+        w("float W = 1.0f, R = 1.0f, wlo = 1.0f, whi = 1.0f;")
 
     def kappa_step(v):
         if dec_vec:
             w(f"const float x = live ? {v[s.decay]} : 1.0f;")
-            w("W *= x; R *= frnn_rcp1(x); tiny = tiny || !(fabsf(W) > 1e-25f && fabsf(W) < 1e25f);")
+            w("W *= x; R *= frnn_rcp1(x); wlo = fminf(wlo, fabsf(W)); whi = fmaxf(whi, fabsf(W));")
         for r, nm in enumerate(s.kappas):
             w(f"const float y{r} = live ? {v[nm]}{' * R' if dec_vec else ''} : 0.0f;")
             put_km(f"(smem + {off_kh})", lboH, f"{r * C} + q", "n", f"y{r}")
@@ -847,7 +847,7 @@ def emit_scan(p: Problem, s: ScanSpec, C: int, MB: int, use_tma: bool = True, st
                 put_km(f"(smem + {off_kh})", lboH, f"{nK + r * C} + q", "n", f"frnn_tf32_rest(y{r})")
     steps(s.kappas + ([s.decay] if dec_vec else []), "n", kappa_step)
     if dec_vec:
-        w("if (tiny) ((volatile int*)&bar[24])[buf] = c + 1;")
+        w("if (!(wlo > 1e-25f && whi < 1e25f)) ((volatile int*)&bar[24])[buf] = c + 1;")
     w.close()
     w("frnn_async_proxy_fence();")
     w(f"frnn_mbar_arrive(&bar[{B_HF}]);")
@@ -862,49 +862,49 @@ def emit_scan(p: Problem, s: ScanSpec, C: int, MB: int, use_tma: bool = True, st
         w.open("if (!slow)")
     w("frnn_tmem_fence_after_sync();")
     w("const u32 gt = tm + frnn_tmem_lane_base(hw);")
-    w("const int d = hl / %d, j = hl %% %d; (void)d; (void)j;" % (C, C))
-
-    def gram_at(i):
-        return f"gram[((d * {nr} + {i} / {C}) * {C} + {i} % {C}) * {GS} + j]"
-    if not xa:
-        w("// rows of the rest of alpha")
-        w.open(f"if (hl >= {nA // 32 * 32} && hl < {(2 * nA + 31) // 32 * 32})")
-        w(f"float v[{nK}];")
-        w(f"frnn_tmem_ld<{nK}>(gt + {colG}u, v); frnn_tmem_wait_ld();")
-        w.open(f"if (hl >= {nA} && hl < {2 * nA})")
-        w(f"const int d = (hl - {nA}) / {C}, j = (hl - {nA}) % {C};")
-        w("#pragma unroll")
-        w(f"for (int i = 0; i < {nK}; i++) {gram_at('i')} = v[i];")
-        w.close()
-        w.close()
-        hsync()
-    w.open(f"if (hl < {(nA + 31) // 32 * 32})")
-    w(f"float v[{nK}];")
-    w(f"frnn_tmem_ld<{nK}>(gt + {colG}u, v);")
+    # the rows' two halves of the threads take half of the columns each, where that is whole vectors or half of the only one
+    parts = 2 if nr == 1 or nr % 2 == 0 else 1
+    KC = nK // parts
+    w(f"const int ml = hl & 127, half = hl >> 7, d = ml / {C}, j = ml % {C}; (void)d; (void)j; (void)half;")
+    w.open(f"if (ml < {(nA + 31) // 32 * 32}" + (" && half == 0)" if parts == 1 else ")"))
+    w(f"const int i0 = half * {KC if parts == 2 else 0}; (void)i0;")
+    w(f"float v[{KC}];")
+    w(f"frnn_tmem_ld<{KC}>(gt + {colG}u + (u32)i0, v);")
     if not xk:
-        w(f"float u[{nK}];")
-        w(f"frnn_tmem_ld<{nK}>(gt + {colG + nK}u, u);")
+        w(f"float u[{KC}];")
+        w(f"frnn_tmem_ld<{KC}>(gt + {colG + nK}u + (u32)i0, u);")
+    if dec_sc:
+        w(f"float xs[{C}];")
+        w("#pragma unroll")
+        w(f"for (int q = 0; q < {C}; q++) xs[q] = mk[max({pos('q')}, 0) * {mk_row} + {od}];")
     w("frnn_tmem_wait_ld();")
-    w.open(f"if (hl < {nA})")
-    w("#pragma unroll")
-    w(f"for (int i = 0; i < {nK}; i++) v[i] = v[i]{' + u[i]' if not xk else ''}{f' + {gram_at(chr(105))}' if not xa else ''};")
+    w.open(f"if (ml < {nA})")
+    if not xk:
+        w("#pragma unroll")
+        w(f"for (int i = 0; i < {KC}; i++) v[i] += u[i];")
     for k in range(len(s.diags)):
         d_, r_ = s.diag_at[k]
-        w(f"if (d == {d_}) {{ float z = 0.0f;")
+        w.open(f"if (d == {d_} && j >= i0 - {r_ * C} && j < i0 - {r_ * C} + {KC})")
+        w("float z = 0.0f;")
         w("#pragma unroll")
-        w(f"for (int i = 0; i < {C}; i++) z = i == j ? v[{r_ * C} + i] : z;")
-        w(f"gram[{o_dg + k * C} + j] = z;" + (f" if (j < nv) frnn_st_raw<float>({s.dg_out}, {dg_off(p, k, f't0 + {pos(chr(106))}')}, z);" if s.dg_out else "") + " }")
+        w(f"for (int i = 0; i < {KC}; i++) z = i0 + i == {r_ * C} + j ? v[i] : z;")
+        w(f"gram[{o_dg + k * C} + j] = z;")
+        if s.dg_out:
+            w(f"if (j < nv) frnn_st_raw<float>({s.dg_out}, {dg_off(p, k, f't0 + {pos(chr(106))}')}, z);")
+        w.close()
     if dec_sc:
         w("float W = 1.0f;")
-        w("#pragma unroll")
-        w.open(f"for (int i = {C - 1}; i >= 0; i--)")
-        w.open("if (i < j)")
-        w(" ".join(f"v[{r * C} + i] *= W;" for r in range(nr)))
-        w(f"if (i < nv) W *= mk[{pos('i')} * {mk_row} + {od}];")
-        w.close()
-        w.close()
+        per = min(KC, C)                 # positions of one vector that a half holds
+        if per < C:
+            w("#pragma unroll")
+            w(f"for (int i = {C - 1}; i >= {per}; i--) if (half == 0 && i < j && i < nv) W *= xs[i];")
+            w("#pragma unroll")
+            w(f"for (int i = {per - 1}; i >= 0; i--) {{ if (i0 + i < j) {{ v[i] *= W; if (i0 + i < nv) W *= half ? xs[i + {per}] : xs[i]; }} }}")
+        else:
+            w("#pragma unroll")
+            w(f"for (int i = {C - 1}; i >= 0; i--) {{ if (i < j) {{ " + " ".join(f"v[{x * C} + i] *= W;" for x in range(KC // C)) + " if (i < nv) W *= xs[i]; } }")
     w("#pragma unroll")
-    w(f"for (int i = 0; i < {nK}; i++) {gram_at('i')} = v[i];")
+    w(f"for (int i = 0; i < {KC}; i++) {{ const int ci = i0 + i; gram[((d * {nr} + ci / {C}) * {C} + ci % {C}) * {GS} + j] = v[i]; }}")
     w.close()
     w.close()
     if dec_vec:
@@ -1010,6 +1010,9 @@ def emit_scan(p: Problem, s: ScanSpec, C: int, MB: int, use_tma: bool = True, st
         w(f"const u64 da = (({c}) & 1) ? dA1 : dA;")
         w("#pragma unroll 4")
         w(f"for (int k = 0; k < {N // 8}; k++) frnn_mma_ss_d(tm + {colG}u, frnn_mma_next(da, {lboA}, k), frnn_mma_next(dH, {lboH}, k), FRNN_MMA_IDESC({RK}), k > 0);")
+        if not xa:      # the rest of alpha, nA rows further on, onto the same rows of the result
+            w("#pragma unroll 4")
+            w(f"for (int k = 0; k < {N // 8}; k++) frnn_mma_ss_d(tm + {colG}u, frnn_mma_next(da, {lboA}, k) + {nA // 8 * 128 // 16}ull, frnn_mma_next(dH, {lboH}, k), FRNN_MMA_IDESC({RK}), true);")
         w(f"frnn_mma_commit(&bar[{B_MG}]);")
     w.open("")
     w(f"if (!frnn_mbar_wait(&bar[{B_AF}], 0, err, {ERR}) || !frnn_mbar_wait(&bar[{B_HF}], 0, err, {ERR})) return;")
@@ -1925,7 +1928,7 @@ def emit_vector_grads(p: Problem, nf: Normal, bp: BackwardPlan, dspec: Sequence[
     w.close()
     # ---- operands over the columns: kappa (over W) and alpha (times W), this thread's half of the timesteps
     if dec_vec:
-        w(f"float xw[{HC}], pre = 1.0f, post = 1.0f, rpre = 1.0f; bool tiny = false;   // decays; products of the other half's")
+        w(f"float xw[{HC}], pre = 1.0f, post = 1.0f, rpre = 1.0f, wlo = 1.0f, whi = 1.0f;   // decays; products of the other half's")
         w("#pragma unroll")
         w.open(f"for (int k = 0; k < {HC}; k++)")
         w.open("")
@@ -1933,7 +1936,7 @@ def emit_vector_grads(p: Problem, nf: Normal, bp: BackwardPlan, dspec: Sequence[
         e = Stage("x_", "q", N1, {a: f"{reg(a)}[k]" for a in nleaves}).get(nf.decay)
         w(f"xw[k] = {sel(live_n, e, '1.0f')};")
         tiny = "1e-25f" if bp.log_decay or not want_gw else "0.0009765625f"
-        w(f"tiny = tiny || !(fabsf(xw[k]) > {tiny});")
+        w("wlo = fminf(wlo, fabsf(xw[k]));")
         w.close()
         w.open("")
         w(f"const int q = ({HC} - q0) + k; const bool live = {live_n}; (void)live;")
@@ -1952,7 +1955,7 @@ def emit_vector_grads(p: Problem, nf: Normal, bp: BackwardPlan, dspec: Sequence[
     w(f"const int q = q0 + k4 + k; const bool live = {live_n}; (void)live; (void)q;")
     st = Stage("x_", "q", N1, {a: f"{reg(a)}[k4 + k]" for a in nleaves})
     if dec_vec:
-        w("rw *= frnn_rcp1(xw[k4 + k]); tiny = tiny || !(fabsf(rw) < 1e25f);")
+        w("rw *= frnn_rcp1(xw[k4 + k]); whi = fmaxf(whi, fabsf(rw));")
     for x, nm in enumerate(names):
         f = "" if not dec_vec else (" * rw" if x < nr else " * pw")
         w(f"x[{x}][k] = {sel(live_n, st.get(nm) + f)};")
@@ -1967,7 +1970,7 @@ def emit_vector_grads(p: Problem, nf: Normal, bp: BackwardPlan, dspec: Sequence[
         w(f"frnn_stv<0,4>(dst, 0, hi); frnn_stv<0,4>(dst + {tb}, 0, x[{x}]); }}")
     w.close()
     if dec_vec:
-        w("if (tiny) *(volatile int*)&bar[4] = 1;")
+        w(f"if (!(wlo > {tiny} && whi < 1e25f)) *(volatile int*)&bar[4] = 1;")
     # ---- the parts of the accumulators so far, from S_0 and E_C, scaled to what those from L need
     w("float R = 0.0f; (void)R;")
 

@@ -212,14 +212,15 @@ template <class A> FRNN_DEV void emu_mma(u32 d, A a, const void* b, u32 lbo_b, u
         }
 }
 #define FRNN_MMA_IDESC(n) ((u32)(n))
-FRNN_DEV u64 frnn_mma_desc(const void* p, u32 lbo) { return (u64)((const unsigned char*)p - emu_ctx->smem) | ((u64)lbo << 32); }
-FRNN_DEV u64 frnn_mma_next(u64 desc, u32 lbo, int k) { return desc + (u64)k * 2 * lbo; }
+// addresses in units of 16 bytes, as in the hardware's descriptors
+FRNN_DEV u64 frnn_mma_desc(const void* p, u32 lbo) { return (u64)((const unsigned char*)p - emu_ctx->smem) / 16 | ((u64)lbo << 32); }
+FRNN_DEV u64 frnn_mma_next(u64 desc, u32 lbo, int k) { return desc + (u64)k * (2 * lbo / 16); }
 FRNN_DEV void frnn_mma_ts_d(u32 d, u32 a, u64 b, u32 n, bool acc) {
     if ((int)a + 8 > emu_ctx->tmem_cols) { fprintf(stderr, "emu: matrix operand outside Tensor Memory\n"); abort(); }
-    emu_mma(d, [=](int m, int k) { return frnn_tf32_trunc(emu_ctx->tmem[(size_t)m * 512 + a + k]); }, emu_ctx->smem + (u32)b, (u32)(b >> 32), n, acc);
+    emu_mma(d, [=](int m, int k) { return frnn_tf32_trunc(emu_ctx->tmem[(size_t)m * 512 + a + k]); }, emu_ctx->smem + (u32)b * 16ul, (u32)(b >> 32), n, acc);
 }
 FRNN_DEV void frnn_mma_ss_d(u32 d, u64 a, u64 b, u32 n, bool acc) {
-    emu_mma(d, [=](int m, int k) { return emu_mma_smem(emu_ctx->smem + (u32)a, (u32)(a >> 32), m, k); }, emu_ctx->smem + (u32)b, (u32)(b >> 32), n, acc);
+    emu_mma(d, [=](int m, int k) { return emu_mma_smem(emu_ctx->smem + (u32)a * 16ul, (u32)(a >> 32), m, k); }, emu_ctx->smem + (u32)b * 16ul, (u32)(b >> 32), n, acc);
 }
 FRNN_DEV void frnn_mma_commit(u64* bar) { frnn_mbar_arrive(bar); }
 FRNN_DEV int frnn_smem_add(int* p, int v) { std::lock_guard<std::mutex> g(emu_atomic_mtx); int o = *p; *p = o + v; return o; }
