@@ -686,7 +686,7 @@ def emit_scan(p: Problem, s: ScanSpec, C: int, MB: int, use_tma: bool = True, st
     w("auto work = [&]() -> void {")
     w.ind += 1
     w.open(f"if (tid >= 128 && tid < {128 + PT})")
-    w("frnn_regs_release<104>();")
+    w("frnn_regs_release<112>();")
     w("const int hl = tid - 128, hw = hl >> 5; (void)hw;")
     w("u32 hs_par = 0; (void)hs_par;")
     w(f"float k[{nr}][{C}];     // kappa of the last chunk: stored when the products of the chunk before are complete")
@@ -873,10 +873,6 @@ def emit_scan(p: Problem, s: ScanSpec, C: int, MB: int, use_tma: bool = True, st
     if not xk:
         w(f"float u[{KC}];")
         w(f"frnn_tmem_ld<{KC}>(gt + {colG + nK}u + (u32)i0, u);")
-    if dec_sc:
-        w(f"float xs[{C}];")
-        w("#pragma unroll")
-        w(f"for (int q = 0; q < {C}; q++) xs[q] = mk[max({pos('q')}, 0) * {mk_row} + {od}];")
     w("frnn_tmem_wait_ld();")
     w.open(f"if (ml < {nA})")
     if not xk:
@@ -894,15 +890,16 @@ def emit_scan(p: Problem, s: ScanSpec, C: int, MB: int, use_tma: bool = True, st
         w.close()
     if dec_sc:
         w("float W = 1.0f;")
+        xs = lambda q: f"mk[max({pos(q)}, 0) * {mk_row} + {od}]"
         per = min(KC, C)                 # positions of one vector that a half holds
         if per < C:
             w("#pragma unroll")
-            w(f"for (int i = {C - 1}; i >= {per}; i--) if (half == 0 && i < j && i < nv) W *= xs[i];")
+            w(f"for (int i = {C - 1}; i >= {per}; i--) if (half == 0 && i < j && i < nv) W *= {xs('i')};")
             w("#pragma unroll")
-            w(f"for (int i = {per - 1}; i >= 0; i--) {{ if (i0 + i < j) {{ v[i] *= W; if (i0 + i < nv) W *= half ? xs[i + {per}] : xs[i]; }} }}")
+            w(f"for (int i = {per - 1}; i >= 0; i--) {{ if (i0 + i < j) {{ v[i] *= W; if (i0 + i < nv) W *= {xs('i0 + i')}; }} }}")
         else:
             w("#pragma unroll")
-            w(f"for (int i = {C - 1}; i >= 0; i--) {{ if (i < j) {{ " + " ".join(f"v[{x * C} + i] *= W;" for x in range(KC // C)) + " if (i < nv) W *= xs[i]; } }")
+            w(f"for (int i = {C - 1}; i >= 0; i--) {{ if (i < j) {{ " + " ".join(f"v[{x * C} + i] *= W;" for x in range(KC // C)) + f" if (i < nv) W *= {xs('i')}; }} }}")
     w("#pragma unroll")
     w(f"for (int i = 0; i < {KC}; i++) {{ const int ci = i0 + i; gram[((d * {nr} + ci / {C}) * {C} + ci % {C}) * {GS} + j] = v[i]; }}")
     w.close()
@@ -982,7 +979,7 @@ def emit_scan(p: Problem, s: ScanSpec, C: int, MB: int, use_tma: bool = True, st
 
     # ------------------------------------------------------------------ the warp that starts the copies of the inputs
     w.open(f"if (tid >= {128 + PT})")
-    w("frnn_regs_release<104>();")
+    w("frnn_regs_release<96>();")
     w.close()
     w.open(f"if (tid >= {128 + PT + 32})")
     if kb.tma_items:
@@ -1005,18 +1002,27 @@ def emit_scan(p: Problem, s: ScanSpec, C: int, MB: int, use_tma: bool = True, st
         w(f"const u64 {nm} = frnn_mma_desc(smem + {off}, {lbo});")
     w(f"const u64 dKlo = frnn_mma_desc(smem + {off_ka + (0 if xk else ka_bytes)}, {lboK}), dA1 = frnn_mma_desc(smem + {off_al + al_bytes}, {lboA}); (void)dKlo;")
 
-    def gram_products(c: str):
-        w("frnn_tmem_fence_after_sync();")
-        w(f"const u64 da = (({c}) & 1) ? dA1 : dA;")
-        w("#pragma unroll 4")
-        w(f"for (int k = 0; k < {N // 8}; k++) frnn_mma_ss_d(tm + {colG}u, frnn_mma_next(da, {lboA}, k), frnn_mma_next(dH, {lboH}, k), FRNN_MMA_IDESC({RK}), k > 0);")
+    # Gram in up to four pieces, so that products the state threads wait for never queue behind all of it
+    pieces = 4 if N % 32 == 0 else 1
+
+    def gram_piece(c: str, g: str):
+        """Piece ``g`` of Gram of chunk ``c``."""
+        kp = N // 8 // pieces
+        w.open("")
+        w(f"const u64 dga = frnn_mma_next((({c}) & 1) ? dA1 : dA, {lboA}, ({g}) * {kp}), dgh = frnn_mma_next(dH, {lboH}, ({g}) * {kp});")
+        w("#pragma unroll")
+        w.open(f"for (int k = 0; k < {kp}; k++)")
+        w(f"frnn_mma_ss_d(tm + {colG}u, frnn_mma_next(dga, {lboA}, k), frnn_mma_next(dgh, {lboH}, k), FRNN_MMA_IDESC({RK}), ({g}) > 0 || k > 0);")
         if not xa:      # the rest of alpha, nA rows further on, onto the same rows of the result
-            w("#pragma unroll 4")
-            w(f"for (int k = 0; k < {N // 8}; k++) frnn_mma_ss_d(tm + {colG}u, frnn_mma_next(da, {lboA}, k) + {nA // 8 * 128 // 16}ull, frnn_mma_next(dH, {lboH}, k), FRNN_MMA_IDESC({RK}), true);")
-        w(f"frnn_mma_commit(&bar[{B_MG}]);")
-    w.open("")
+            w(f"frnn_mma_ss_d(tm + {colG}u, frnn_mma_next(dga, {lboA}, k) + {nA // 8 * 128 // 16}ull, frnn_mma_next(dgh, {lboH}, k), FRNN_MMA_IDESC({RK}), true);")
+        w.close()
+        w(f"if (({g}) == {pieces - 1}) frnn_mma_commit(&bar[{B_MG}]);")
+        w.close()
     w(f"if (!frnn_mbar_wait(&bar[{B_AF}], 0, err, {ERR}) || !frnn_mbar_wait(&bar[{B_HF}], 0, err, {ERR})) return;")
-    gram_products("0")
+    w("frnn_tmem_fence_after_sync();")
+    w("#pragma unroll 1")
+    w.open(f"for (int g = 0; g < {pieces}; g++)")
+    gram_piece("0", "g")
     w.close()
     w("#pragma unroll 1")
     w.open(f"for (int c = 0; c < {nchunk}; c++)")
@@ -1030,13 +1036,20 @@ def emit_scan(p: Problem, s: ScanSpec, C: int, MB: int, use_tma: bool = True, st
             w(f"for (int k = {k0}; k < {k1}; k++) frnn_mma_ts_d(tm + {colA}u, tm + {a}u + k * 8, frnn_mma_next(da, {lboA}, k), FRNN_MMA_IDESC({n_}), {first_});")
     w(f"frnn_mma_commit(&bar[{B_M1}]); frnn_mma_commit(&bar[{B_AE} + (c & 1)]);")
     # Gram of the next chunk as soon as its operands are there, but never in the way of products 2
-    w(f"bool gram = c + 1 >= {nchunk}; (void)gram;")
+    w(f"int g = c + 1 < {nchunk} ? 0 : {pieces}; bool ready = false; (void)ready;")
     w("const u64 t_wait = frnn_now_ns();")
     w.open("for (;;)")
-    w.open(f"if ({'false' if late_gram else '!gram'} && frnn_mbar_try(&bar[{B_AF} + ((c + 1) & 1)], ((c + 1) >> 1) & 1) && frnn_mbar_try(&bar[{B_HF}], (c + 1) & 1))")
-    gram_products("c + 1")
-    w("gram = true;")
-    w.close()
+    if not late_gram:
+        w.open(f"if (g < {pieces})")
+        w.open("if (!ready)")
+        w(f"ready = frnn_mbar_try(&bar[{B_AF} + ((c + 1) & 1)], ((c + 1) >> 1) & 1) && frnn_mbar_try(&bar[{B_HF}], (c + 1) & 1);")
+        w("if (ready) frnn_tmem_fence_after_sync();")
+        w.close()
+        w.open("if (ready)")
+        gram_piece("c + 1", "g")
+        w("g++;")
+        w.close()
+        w.close()
     w(f"if (frnn_mbar_try(&bar[{B_PB}], c & 1)) break;")
     w(f"if (frnn_now_ns() - t_wait > FRNN_WAIT_LIMIT_NS) {{ frnn_report(err, {ERR}); return; }}")
     w.close()
@@ -1047,18 +1060,22 @@ def emit_scan(p: Problem, s: ScanSpec, C: int, MB: int, use_tma: bool = True, st
         w("#pragma unroll")
         w(f"for (int k = 0; k < {nK // 8}; k++) frnn_mma_ts_d(tm + {colD}u, tm + {a}u + k * 8, frnn_mma_next({dsc}, {lboK}, k), FRNN_MMA_IDESC({Np}), {'k > 0' if i == 0 else 'true'});")
     w(f"frnn_mma_commit(&bar[{B_M2}]); frnn_mma_commit(&bar[{B_KE}]);")
-    w.open("if (!gram)")
+    w.open(f"if (g < {pieces})")
     if late_gram:
         w(f"if (!frnn_mbar_wait(&bar[{B_M2}], c & 1, err, {ERR})) return;")
     w(f"if (!frnn_mbar_wait(&bar[{B_AF} + ((c + 1) & 1)], ((c + 1) >> 1) & 1, err, {ERR}) || !frnn_mbar_wait(&bar[{B_HF}], (c + 1) & 1, err, {ERR})) return;")
-    gram_products("c + 1")
+    w("frnn_tmem_fence_after_sync();")
+    w("#pragma unroll 1")
+    w.open(f"for (; g < {pieces}; g++)")
+    gram_piece("c + 1", "g")
+    w.close()
     w.close()
     w.close()
     w("return;")
     w.close()
 
     # ------------------------------------------------------------------ state warps
-    w("frnn_regs_acquire<200>();")
+    w("frnn_regs_acquire<192>();")
     w("const u32 mine = tm + frnn_tmem_lane_base(warp);")
     w(f"const int m = m0 + tid; const bool row = tid < {MB};")
     nck = nchunk
