@@ -1018,54 +1018,40 @@ def emit_scan(p: Problem, s: ScanSpec, C: int, MB: int, use_tma: bool = True, st
         w.close()
         w(f"if (({g}) == {pieces - 1}) frnn_mma_commit(&bar[{B_MG}]);")
         w.close()
-    def gram_ready(c: str) -> str:
-        return (f"frnn_mbar_try(&bar[{B_AF} + (({c}) & 1)], (({c}) >> 1) & 1) && frnn_mbar_try(&bar[{B_HF}], ({c}) & 1)"
-                + (f" && (({c}) == 0 || frnn_mbar_try(&bar[{B_M2}], (({c}) - 1) & 1))" if late_gram else ""))
-
-    def try_gram(c: str):
-        """A piece of Gram of chunk ``c`` if its operands are there."""
-        w.open(f"if (g < {pieces})")
-        w.open("if (!ready)")
-        w(f"ready = {gram_ready(c)};")
-        w("if (ready) frnn_tmem_fence_after_sync();")
-        w.close()
-        w.open("if (ready)")
-        gram_piece(c, "g")
-        w("g++;")
-        w.close()
-        w.close()
-
-    def give_up():
-        w(f"if (frnn_now_ns() - t_wait > FRNN_WAIT_LIMIT_NS) {{ frnn_report(err, {ERR}); return; }}")
-    w("int g = 0; bool ready = false;          // pieces of the current chunk's Gram issued so far, and whether they can be")
+    w(f"if (!frnn_mbar_wait(&bar[{B_AF}], 0, err, {ERR}) || !frnn_mbar_wait(&bar[{B_HF}], 0, err, {ERR})) return;")
+    w("frnn_tmem_fence_after_sync();")
+    w("#pragma unroll 1")
+    w.open(f"for (int g = 0; g < {pieces}; g++)")
+    gram_piece("0", "g")
+    w.close()
     w("#pragma unroll 1")
     w.open(f"for (int c = 0; c < {nchunk}; c++)")
     w("const u64 da = (c & 1) ? dA1 : dA;")
-    w("u64 t_wait = frnn_now_ns();")
     for qi, (n0, n1) in enumerate(quarters):
-        # products 1 of the columns the state threads have finished, a piece of Gram where they have not
-        cond = f"frnn_mbar_try(&bar[{B_SB + qi}], c & 1)" + (f" && frnn_mbar_try(&bar[{B_AF} + (c & 1)], (c >> 1) & 1)" if qi == 0 else "")
-        w.open(f"while (!({cond}))")
-        try_gram("c")
-        give_up()
-        w.close()
+        w(f"if (!frnn_mbar_wait(&bar[{B_SB + qi}], c & 1, err, {ERR})) return;")
         w("frnn_tmem_fence_after_sync();")
         k0, k1 = n0 // 8, min(n1, N) // 8
         for a, n_, first_ in ((colS, RA, "k > 0"), (colL, RA, "true")):
             w("#pragma unroll")
             w(f"for (int k = {k0}; k < {k1}; k++) frnn_mma_ts_d(tm + {colA}u, tm + {a}u + k * 8, frnn_mma_next(da, {lboA}, k), FRNN_MMA_IDESC({n_}), {first_});")
-    w(f"frnn_mma_commit(&bar[{B_M1}]);")
-    w.open(f"while (g < {pieces})")
-    try_gram("c")
-    give_up()
-    w.close()
-    w(f"frnn_mma_commit(&bar[{B_AE} + (c & 1)]);")
-    w(f"g = c + 1 < {nchunk} ? 0 : {pieces}; ready = false;")
-    w("t_wait = frnn_now_ns();")
-    w.open(f"while (!frnn_mbar_try(&bar[{B_PB}], c & 1))")
+    w(f"frnn_mma_commit(&bar[{B_M1}]); frnn_mma_commit(&bar[{B_AE} + (c & 1)]);")
+    # Gram of the next chunk as soon as its operands are there, but never in the way of products 2
+    w(f"int g = c + 1 < {nchunk} ? 0 : {pieces}; bool ready = false; (void)ready;")
+    w("const u64 t_wait = frnn_now_ns();")
+    w.open("for (;;)")
     if not late_gram:
-        try_gram("c + 1")
-    give_up()
+        w.open(f"if (g < {pieces})")
+        w.open("if (!ready)")
+        w(f"ready = frnn_mbar_try(&bar[{B_AF} + ((c + 1) & 1)], ((c + 1) >> 1) & 1) && frnn_mbar_try(&bar[{B_HF}], (c + 1) & 1);")
+        w("if (ready) frnn_tmem_fence_after_sync();")
+        w.close()
+        w.open("if (ready)")
+        gram_piece("c + 1", "g")
+        w("g++;")
+        w.close()
+        w.close()
+    w(f"if (frnn_mbar_try(&bar[{B_PB}], c & 1)) break;")
+    w(f"if (frnn_now_ns() - t_wait > FRNN_WAIT_LIMIT_NS) {{ frnn_report(err, {ERR}); return; }}")
     w.close()
     w(f"if (!frnn_mbar_wait(&bar[{B_KF}], c & 1, err, {ERR})) return;")
     w("frnn_tmem_fence_after_sync();")
@@ -1074,6 +1060,16 @@ def emit_scan(p: Problem, s: ScanSpec, C: int, MB: int, use_tma: bool = True, st
         w("#pragma unroll")
         w(f"for (int k = 0; k < {nK // 8}; k++) frnn_mma_ts_d(tm + {colD}u, tm + {a}u + k * 8, frnn_mma_next({dsc}, {lboK}, k), FRNN_MMA_IDESC({Np}), {'k > 0' if i == 0 else 'true'});")
     w(f"frnn_mma_commit(&bar[{B_M2}]); frnn_mma_commit(&bar[{B_KE}]);")
+    w.open(f"if (g < {pieces})")
+    if late_gram:
+        w(f"if (!frnn_mbar_wait(&bar[{B_M2}], c & 1, err, {ERR})) return;")
+    w(f"if (!frnn_mbar_wait(&bar[{B_AF} + ((c + 1) & 1)], ((c + 1) >> 1) & 1, err, {ERR}) || !frnn_mbar_wait(&bar[{B_HF}], (c + 1) & 1, err, {ERR})) return;")
+    w("frnn_tmem_fence_after_sync();")
+    w("#pragma unroll 1")
+    w.open(f"for (; g < {pieces}; g++)")
+    gram_piece("c + 1", "g")
+    w.close()
+    w.close()
     w.close()
     w("return;")
     w.close()
