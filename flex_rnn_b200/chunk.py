@@ -1477,7 +1477,7 @@ def backward_scan_spec(p: Problem, nf: Normal, bp: BackwardPlan, dspec: Sequence
 VG_THREADS = 256
 
 
-def emit_vector_grads(p: Problem, nf: Normal, bp: BackwardPlan, dspec: Sequence[TensorSpec], atomic: Sequence[bool], C: int, n_sm: int) -> KernelSource:
+def emit_vector_grads(p: Problem, nf: Normal, bp: BackwardPlan, dspec: Sequence[TensorSpec], atomic: Sequence[bool], C: int) -> KernelSource:
     """Gradients of the column vectors and scalars, one CTA per chunk of ``C`` timesteps: with the state S_0 at the
     chunk's start, the state gradient E_C at its end, X = dsig and Z = p (vectors over the rows, per timestep),
 
@@ -1729,11 +1729,6 @@ def emit_vector_grads(p: Problem, nf: Normal, bp: BackwardPlan, dspec: Sequence[
     w(f"const int x128 = tid & 127, hf = tid >> 7, q0 = hf * {HC};")
     w(f"const int mc = {'x128' if M == 128 else f'min(x128, {M - 1})'}, nc = {'x128' if full_n else f'min(x128, {N - 1})'};")
     w(f"const bool mrow = x128 < {M}, ncol = x128 < {N}; (void)mrow; (void)ncol; (void)nc;")
-    colv = nf.alphas + nf.kappas + ([nf.decay] if dec_vec else [])
-    ngiven = [f"ga{d}" for d in range(nd)] + [f"gk{r}" for r in range(nr)] + ["gw"]
-    n_outs = [o for i, o in bp.grads if p.in_cls(i) == N1]
-    nleaves = leaves_of(list(colv) + [n.args[0] for n in nsums] + n_outs, N1, ngiven)
-    wleaves = leaves_of([nf.decay], N1) if dec_vec else []
     mleaves = leaves_of(list(bp.dsig) + list(nf.ps) + [n.args[0] for n in msums], M1)
     reg = lambda a: "r_" + a.replace(".", "_")
     for a in mleaves:
@@ -1761,38 +1756,6 @@ def emit_vector_grads(p: Problem, nf: Normal, bp: BackwardPlan, dspec: Sequence[
         w.close()
     for u in range(min(DP, nsl)):
         load_slice(str(u), str(u))
-    # the chunk that will take this CTA's place comes into L2 meanwhile: its loads then cost L2's latency, not DRAM's
-    w.open("")
-    w(f"const int nid = ((int)blockIdx.z * {H} + (int)blockIdx.y) * {nchunk} + (int)blockIdx.x + {ctas * n_sm};")
-    w.open(f"if (nid < {nchunk * H * B})")
-    w(f"const int kc2 = nid % {nchunk}, h2 = nid / {nchunk} % {H}, b2 = nid / {nchunk * H};")
-    cb = N * M * 4
-    w(f"if (tid < 2) frnn_prefetch_l2_c((tid ? eck : ck) + (((long)b2 * {H} + h2) * {nchunk} + kc2) * {N * M}L, {cb}u);")
-    rows = []                             # (pointer expression of the row of timestep t2, bytes)
-    for a in dict.fromkeys(mleaves + nleaves):
-        if a in by_in:
-            i = by_in[a]
-            sp, e, ln = p.inputs[i], ELT[p.inputs[i].dt], N if p.in_cls(i) == N1 else M
-            dims = {0: "b2", 1: "t2", 2: "h2"}
-            if sp.st(4 if p.in_cls(i) == N1 else 3) == 1 and sp.aligned16 and (ln * e) % 16 == 0 and all((sp.st(d) * e) % 16 == 0 for d in dims):
-                rows.append((f"(const char*)in{i} + ({_elem_off(sp, list(dims.items()))}) * {e}", ln * e))
-        elif a.startswith("gy"):
-            e = ELT[p.out_dt[int(a[2:])]]
-            if (M * e) % 16 == 0:
-                rows.append((f"(const char*)dy{a[2:]} + (((long)b2 * {T} + t2) * {H} + h2) * {M * e}L", M * e))
-        else:
-            k, ptr = (bp.saved.index(int(a[3:])), "aux") if a.startswith("sig") else (bp.kept.index(int(a[2:])), "tau")
-            rows.append((f"(const char*)({ptr} + ((({k}L * {B} + b2) * {H} + h2) * {T}L + t2) * {M}L)", M * 4))
-    if rows:
-        w.open(f"for (int it = tid - 32; it < {len(rows) * C}; it += {VG_THREADS - 32})")
-        w(f"const int t2 = kc2 * {C} + it % {C};")
-        w.open(f"if (it >= 0 && t2 < {T})")
-        for x, (ptr, nb) in enumerate(rows):
-            w(f"if (it / {C} == {x}) frnn_prefetch_l2_c({ptr}, {nb}u);")
-        w.close()
-        w.close()
-    w.close()
-    w.close()
     w("if (tid == 0) { frnn_mbar_init(&bar[0], 1); frnn_mbar_init(&bar[1], 1); frnn_mbar_init(&bar[2], 1); frnn_mbar_init(&bar[5], 1); ((int*)&bar[4])[0] = 0; frnn_mbar_init_fence(); }")
     w.open("if (warp == 0)")
     w(f"frnn_tmem_alloc((u32*)&bar[3], {tm_cols}u);")
@@ -1858,6 +1821,11 @@ def emit_vector_grads(p: Problem, nf: Normal, bp: BackwardPlan, dspec: Sequence[
     scalar_nodes(second_s)
     w.close()
     # ---- S_0 and E_C, a slice of rows at a time, loaded two slices ahead
+    colv = nf.alphas + nf.kappas + ([nf.decay] if dec_vec else [])
+    ngiven = [f"ga{d}" for d in range(nd)] + [f"gk{r}" for r in range(nr)] + ["gw"]
+    n_outs = [o for i, o in bp.grads if p.in_cls(i) == N1]
+    nleaves = leaves_of(list(colv) + [n.args[0] for n in nsums] + n_outs, N1, ngiven)
+    wleaves = leaves_of([nf.decay], N1) if dec_vec else []
     for a in nleaves:
         w(f"float {reg(a)}[{HC}];")
     for a in wleaves:
@@ -2298,7 +2266,6 @@ class ChunkPlan:
     dspec: List[TensorSpec]
     atomic: List[bool]
     C: int = CHUNK                            # timesteps per chunk of the training kernels
-    n_sm: int = 148
     short: bool = True                        # whether calls without gradients are chunked
 
     def forward(self, **kw) -> KernelSource:
@@ -2324,7 +2291,7 @@ class ChunkPlan:
         return emit_scan(p, backward_scan_spec(p, self.nf, self.bp, self.dspec, self.C), self.C, rows_per_cta(p.M), **kw)
 
     def vector_grads(self) -> KernelSource:
-        return emit_vector_grads(self.problem, self.nf, self.bp, self.dspec, self.atomic, self.C, self.n_sm)
+        return emit_vector_grads(self.problem, self.nf, self.bp, self.dspec, self.atomic, self.C)
 
     def variants(self) -> List[dict]:
         """Keyword arguments of the scans worth timing; member 0 is the default."""
@@ -2369,7 +2336,7 @@ def chunk_plan(plan) -> Optional[ChunkPlan]:
     nf = normal_form(plan.g_fw, p.in_names, p.st_names[0], plan.n_out)
     if nf is None or not all(nf_inputs(nf)):
         return None
-    cp = ChunkPlan(p, nf, None, [g.spec for g in plan.whole_grads], [g.atomic for g in plan.whole_grads], n_sm=plan.n_sm)
+    cp = ChunkPlan(p, nf, None, [g.spec for g in plan.whole_grads], [g.atomic for g in plan.whole_grads])
     try:
         cp.short = (one_wave or p.M > 64) and cp.infer().smem_bytes <= SMEM_BYTES
         if p.M <= 128 and p.M % 8 == 0:

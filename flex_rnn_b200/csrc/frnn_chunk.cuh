@@ -32,10 +32,6 @@ FRNN_DEV void frnn_mma_ss_d(u32 d, u64 a, u64 b, u32 idesc, bool accumulate) {
 FRNN_DEV void frnn_mma_commit(u64* bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(frnn_smem_addr(bar)) : "memory");
 }
-// start bringing a range into L2; 16-byte aligned, a multiple of 16 bytes
-FRNN_DEV void frnn_prefetch_l2(const void* p, u32 bytes) {
-    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(__cvta_generic_to_global(p)), "r"(bytes) : "memory");
-}
 FRNN_DEV void frnn_half_warp_sync() { __syncwarp(0xffffu); }      // the first 16 lanes of a warp
 #endif
 // What tf32 truncation leaves out of x (13 bits), rounded to the 11 that tf32 holds: hi + rest is x to 2^-22, unbiased.
@@ -47,7 +43,4 @@ FRNN_DEV float frnn_tf32_rest(float x) {
 FRNN_DEV float frnn_rcp1(float x) {
     const float r = frnn_divf(1.0f, x);
     return fmaf(r, fmaf(-x, r, 1.0f), r);
-}
-FRNN_DEV void frnn_prefetch_l2_c(const void* p, u32 bytes) {
-    if (FRNN_ACCESS_OK(p, bytes)) frnn_prefetch_l2(p, bytes);
 }

@@ -182,10 +182,6 @@ FRNN_DEV float* emu_tmem_at(u32 taddr, int n) {
     FRNN_DEV void frnn_tmem_st##N(u32 taddr, const float* v) { memcpy(emu_tmem_at(taddr, N), v, 4 * N); } \
     FRNN_DEV void frnn_tmem_ld##N(u32 taddr, float* v) { memcpy(v, emu_tmem_at(taddr, N), 4 * N); }
 EMU_TMEM_FN(1) EMU_TMEM_FN(2) EMU_TMEM_FN(4) EMU_TMEM_FN(8) EMU_TMEM_FN(16)
-FRNN_DEV void frnn_prefetch_l2(const void* p, u32 bytes) {
-    if (((uintptr_t)p & 15) || (bytes & 15) || !bytes) { fprintf(stderr, "emu: misaligned prefetch %p %u\n", p, bytes); abort(); }
-    volatile char c = ((const char*)p)[0]; c = ((const char*)p)[bytes - 1]; (void)c;
-}
 FRNN_DEV void frnn_half_warp_sync() {
     emu_cta* c = emu_ctx;
     const int w = threadIdx.x >> 5;
