@@ -1825,11 +1825,8 @@ def emit_vector_grads(p: Problem, nf: Normal, bp: BackwardPlan, dspec: Sequence[
     ngiven = [f"ga{d}" for d in range(nd)] + [f"gk{r}" for r in range(nr)] + ["gw"]
     n_outs = [o for i, o in bp.grads if p.in_cls(i) == N1]
     nleaves = leaves_of(list(colv) + [n.args[0] for n in nsums] + n_outs, N1, ngiven)
-    wleaves = leaves_of([nf.decay], N1) if dec_vec else []
     for a in nleaves:
         w(f"float {reg(a)}[{HC}];")
-    for a in wleaves:
-        w(f"float o_{reg(a)}[{HC}];          // the other half's timesteps")
     w("#pragma unroll 1")
     w.open(f"for (int s2 = 0; s2 < {nsl}; s2 += {DP})")
     for u in range(DP):
@@ -1874,10 +1871,6 @@ def emit_vector_grads(p: Problem, nf: Normal, bp: BackwardPlan, dspec: Sequence[
     w(f"const int t = {tq('q0 + k')};")
     for a in nleaves:
         w(f"{reg(a)}[k] = {leaf(a, 't', 'nc')};")
-    if wleaves:
-        w(f"const int to = {tq(f'({HC} - q0) + k')};")
-        for a in wleaves:
-            w(f"o_{reg(a)}[k] = {leaf(a, 'to', 'nc')};")
     w.close()
     if nf.decay:
         w("#pragma unroll")
@@ -1945,7 +1938,7 @@ def emit_vector_grads(p: Problem, nf: Normal, bp: BackwardPlan, dspec: Sequence[
     w.close()
     # ---- operands over the columns: kappa (over W) and alpha (times W), this thread's half of the timesteps
     if dec_vec:
-        w(f"float xw[{HC}], pre = 1.0f, post = 1.0f, rpre = 1.0f, wlo = 1.0f, whi = 1.0f;   // decays; products of the other half's")
+        w(f"float xw[{HC}], pre = 1.0f, post = 1.0f, rpre = 1.0f, wlo = 1.0f, whi = 1.0f, prod = 1.0f;   // decays; products of the other half's")
         w("#pragma unroll")
         w.open(f"for (int k = 0; k < {HC}; k++)")
         w.open("")
@@ -1955,13 +1948,13 @@ def emit_vector_grads(p: Problem, nf: Normal, bp: BackwardPlan, dspec: Sequence[
         tiny = "1e-25f" if bp.log_decay or not want_gw else "0.0009765625f"
         w("wlo = fminf(wlo, fabsf(xw[k]));")
         w.close()
-        w.open("")
-        w(f"const int q = ({HC} - q0) + k; const bool live = {live_n}; (void)live;")
-        e = Stage("x_", "q", N1, {a: f"o_{reg(a)}[k]" for a in wleaves}).get(nf.decay)
-        w(f"const float y = {sel(live_n, e, '1.0f')};")
-        w("if (hf) { pre *= y; rpre *= frnn_rcp1(y); } else post *= y;")
+        w("prod *= xw[k];")
         w.close()
-        w.close()
+        # the product of the other half's decays comes through shared memory
+        w("xr[tid] = prod;")
+        w("frnn_block_sync();")
+        w("const float other = xr[tid ^ 128];")
+        w("if (hf) { pre = other; rpre = frnn_rcp1(other); } else post = other;")
         w("float rw = rpre, pw = pre;")
     w("#pragma unroll")
     w.open(f"for (int k4 = 0; k4 < {HC}; k4 += 4)")
