@@ -376,6 +376,11 @@ def make_plan(step: Callable, inputs: Sequence[th.Tensor], state: Sequence[th.Te
         mb = M
         while mb % 2 == 0 and mb // 2 >= min_rows and (mb > 1024 or B * H * (M // mb) < n_sm):
             mb //= 2
+        if N == 1:
+            # one column: a row is a thread's, nothing is shared between rows, and whole warps of 64 to 256 of them give the
+            # GPU the most loads in flight
+            whole = [d for d in range(64, 257, 32) if M % d == 0]
+            mb = min(whole, key=lambda d: abs(d - 128), default=mb)
         r, c = 4, 8
         try:
             while True:
