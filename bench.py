@@ -418,8 +418,12 @@ class Bench:
         bytes_bw_alg = in_bytes + y_bytes + st_bytes + in_bytes + st_bytes
         # what the backward launch actually moves, from the plan: plus saved row sums and fp32 checkpoints read
         aux_bytes = len(plan.aux) * B * H * T * M * 4
-        ck_bytes = plan.nck * B * H * M * N * 4 * plan.n_st
+        chunk = m["op"].forward_func.chunk
+        nck = -(-T // chunk) if chunk else plan.nck
+        ck_bytes = nck * B * H * M * N * 4 * plan.n_st
         traffic_bw = bytes_bw_alg + aux_bytes + ck_bytes
+        if chunk:       # the second backward kernel reads inputs, dy and row sums again, and the state gradients of the first
+            traffic_bw += in_bytes + y_bytes + 2 * aux_bytes + 2 * ck_bytes
         traffic_fw = bytes_fw_alg + aux_bytes + ck_bytes
         fw_avg, bw_avg = statistics.mean(m["fw_ms"]), statistics.mean(m["bw_ms"])
         k_bw = plan.k_joint - plan.k_fwd
@@ -436,7 +440,8 @@ class Bench:
             "k_joint": plan.k_joint, "k_fwd": plan.k_fwd,
             "fp32_bound_ms": t_fp32 * 1e3, "hbm_bound_ms": t_hbm * 1e3,
             "peak_memory_gib": round(m["peak_memory_gib"], 3),
-            "checkpoint_every": plan.D, "backward": "reverse re-step" if plan.reverse else "recompute from slots",
+            "checkpoint_every": chunk or plan.D,
+            "backward": "chunked" if chunk else "reverse re-step" if plan.reverse else "recompute from slots",
             "fw_kernel": {"grid": list(fw_src.grid), "block": fw_src.block, "smem": fw_src.smem_bytes,
                           "tile": fw_src.info["tile"][:2], "packed_fp32x2": fw_src.info["packed"],
                           "variant": tuned["fw_choice"], "timed_variants": len(tuned["fw_log"])},
@@ -451,10 +456,10 @@ class Bench:
         units = B * H * (M // bw_src.info["tile"][2])
         per_wave = self.sms * max(1, plan.tuning.bw_min_blocks)
         issued = (plan.k_joint - plan.k_fwd) / 2 + (plan.n_st if plan.reverse else 0)
-        extra = {"counted_per_issued": ((plan.k_joint - plan.k_fwd) / 2) / issued if plan.reverse else None,
+        extra = {"counted_per_issued": ((plan.k_joint - plan.k_fwd) / 2) / issued if plan.reverse and not chunk else None,
                  "sm_fill": units / (-(-units // per_wave) * per_wave),
                  "bytes_fw_alg": bytes_fw_alg, "bytes_bw_alg": bytes_bw_alg, "traffic_bw": traffic_bw, "traffic_fw": traffic_fw,
-                 "achieved_bw": elems * k_bw / (bw_avg * 1e-3) / 1e12, "flops_bw": elems * k_bw, "bw_name": bw_src.name,
+                 "achieved_bw": elems * k_bw / (bw_avg * 1e-3) / 1e12, "flops_bw": elems * k_bw, "bw_name": "frnn_cbw + frnn_cvg" if chunk else bw_src.name, "chunk": chunk,
                  "stream_mb": (traffic_fw + traffic_bw) / 1e6}
         return rec, extra
 
@@ -618,9 +623,9 @@ def run_ours(args, rank, world, local):
                          "counted_per_issued_fma": extra["counted_per_issued"],
                          "sm_fill": extra["sm_fill"],
                          "ceiling_frac": (fma_kinds.get("delta_rule_backward_mix_packed", 1.0) * extra["counted_per_issued"]
-                                          * extra["sm_fill"]) if (args.op == "delta_rule" and fma_kinds) else None},
+                                          * extra["sm_fill"]) if (args.op == "delta_rule" and fma_kinds and not extra["chunk"]) else None},
             "e2e": e2e,
-            "gpu_launches": 2 * args.steps,
+            "gpu_launches": (3 if extra["chunk"] else 2) * args.steps,
             "clocks": m["clocks"],
         }
     # release the headline workload before the further records allocate theirs

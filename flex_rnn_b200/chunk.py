@@ -1246,7 +1246,7 @@ def emit_scan(p: Problem, s: ScanSpec, C: int, MB: int, use_tma: bool = True, st
     w.close()
     w.close()
     return KernelSource(s.name, w.text().replace("@SMEM_BYTES@", str(smem_bytes)), (p.M // MB, p.H, p.B), 128 + PT + 128, smem_bytes,
-                        kb.params, kb.param_decl, {"chunk": C, "tile": [MB, N, C], "packed": False, "tmem_cols": tm_cols, "nck": nck,
+                        kb.params, kb.param_decl, {"chunk": C, "tile": [1, N, MB], "packed": False, "tmem_cols": tm_cols, "nck": nck,
                                                    "tma_items": len(kb.tma_items), "plain_items": len(kb.plain_items)}, kb.tmaps)
 
 
@@ -2161,7 +2161,7 @@ def emit_vector_grads(p: Problem, nf: Normal, bp: BackwardPlan, dspec: Sequence[
     w("(void)ok;")
     w.close()
     return KernelSource("frnn_cvg", w.text().replace("@SMEM_BYTES@", str(smem_bytes)), (nchunk, H, B), VG_THREADS, smem_bytes, params, decl,
-                        {"chunk": C, "tile": [M, N, C], "packed": False, "tmem_cols": tm_cols}, [])
+                        {"chunk": C, "tile": [1, N, M], "packed": False, "tmem_cols": tm_cols}, [])
 
 
 def emit_slow_columns(w, C, nd, nr, nA, nK, tq, live_n, sel, nf, bp, dec_vec, want_gw, Stage, leaf, leaves_of, slot, LS, cD1, cD2, off_slow):

@@ -1272,6 +1272,7 @@ def build_twopass(step, inputs, state, dryrun=False, tuning: Optional[Tuning] = 
 
     forward.plan = plan                     # type: ignore[attr-defined]
     forward.infer = infer                   # type: ignore[attr-defined]
+    forward.chunk = cplan.C if ctrain else 0   # type: ignore[attr-defined]  (timesteps per chunk; 0: recurrent kernels)
     forward.host_program = host_program     # type: ignore[attr-defined]
     forward.host_checks = host_checks       # type: ignore[attr-defined]
     forward.sources = (fw_src, bw_src)      # type: ignore[attr-defined]
