@@ -2340,8 +2340,9 @@ def chunk_plan(plan) -> Optional[ChunkPlan]:
     if cp.bp is not None:
         # 32 steps per chunk halve the traffic of the chunk boundaries and the chains of the scans, but not the
         # substitution: for large states and few pairs of vectors (B8 T1024 H32 128x128, forward + backward: Delta Rule
-        # 1.66 ms against 1.91 ms, Mamba-2 1.30 ms against 1.67 ms; 512 heads of 32x32, T512: 1.18 against 1.05 ms)
-        if len(nf.alphas) * len(nf.kappas) <= 2 and p.M * p.N >= 8192 and p.T >= 4 * CHUNK:
+        # 1.66 ms against 1.91 ms, Mamba-2 1.30 ms against 1.67 ms; 32 heads of 64x64, T512: 199 against 224 us; 512 heads of
+        # 32x32, T512: 1.18 against 1.05 ms)
+        if len(nf.alphas) * len(nf.kappas) <= 2 and p.M * p.N >= (4096 if one_wave else 8192) and p.T >= 4 * CHUNK:
             cp.C = 2 * CHUNK
             if not _fits(cp):
                 cp.C = CHUNK
