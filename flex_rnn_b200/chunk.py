@@ -682,11 +682,13 @@ def emit_scan(p: Problem, s: ScanSpec, C: int, MB: int, use_tma: bool = True, st
     pos = (lambda q: f"(nv - 1 - ({q}))") if s.reverse else (lambda q: f"({q})")
 
     # ------------------------------------------------------------------ preparing warps
-    # registers: 512 threads start with 128 each; the state's rows need more, the products' warpgroup hardly any
+    # registers: 512 threads start with 128 each; the state's rows need more, the others less (state, preparing twice, products:
+    # 4 x 128 together).  64 values of kappa per preparing thread spill at 104.
+    regs = (192, 112, 96) if nK >= 64 else (200, 104, 104)
     w("auto work = [&]() -> void {")
     w.ind += 1
     w.open(f"if (tid >= 128 && tid < {128 + PT})")
-    w("frnn_regs_release<112>();")
+    w(f"frnn_regs_release<{regs[1]}>();")
     w("const int hl = tid - 128, hw = hl >> 5; (void)hw;")
     w("u32 hs_par = 0; (void)hs_par;")
     w(f"float k[{nr}][{C}];     // kappa of the last chunk: stored when the products of the chunk before are complete")
@@ -979,7 +981,7 @@ def emit_scan(p: Problem, s: ScanSpec, C: int, MB: int, use_tma: bool = True, st
 
     # ------------------------------------------------------------------ the warp that starts the copies of the inputs
     w.open(f"if (tid >= {128 + PT})")
-    w("frnn_regs_release<96>();")
+    w(f"frnn_regs_release<{regs[2]}>();")
     w.close()
     w.open(f"if (tid >= {128 + PT + 32})")
     if kb.tma_items:
@@ -1002,8 +1004,9 @@ def emit_scan(p: Problem, s: ScanSpec, C: int, MB: int, use_tma: bool = True, st
         w(f"const u64 {nm} = frnn_mma_desc(smem + {off}, {lbo});")
     w(f"const u64 dKlo = frnn_mma_desc(smem + {off_ka + (0 if xk else ka_bytes)}, {lboK}), dA1 = frnn_mma_desc(smem + {off_al + al_bytes}, {lboA}); (void)dKlo;")
 
-    # Gram in up to four pieces, so that products the state threads wait for never queue behind all of it
-    pieces = 4 if N % 32 == 0 else 1
+    # Gram of large states in four pieces, so that products the state threads wait for never queue behind all of it (RWKV-7
+    # 128x128: 795 against 785 us; with 64 columns the whole takes no longer than such a wait, and pieces cost 8 %)
+    pieces = 4 if N == 128 else 1
 
     def gram_piece(c: str, g: str):
         """Piece ``g`` of Gram of chunk ``c``."""
@@ -1075,7 +1078,7 @@ def emit_scan(p: Problem, s: ScanSpec, C: int, MB: int, use_tma: bool = True, st
     w.close()
 
     # ------------------------------------------------------------------ state warps
-    w("frnn_regs_acquire<192>();")
+    w(f"frnn_regs_acquire<{regs[0]}>();")
     w("const u32 mine = tm + frnn_tmem_lane_base(warp);")
     w(f"const int m = m0 + tid; const bool row = tid < {MB};")
     nck = nchunk

@@ -406,6 +406,10 @@ def make_plan(step: Callable, inputs: Sequence[th.Tensor], state: Sequence[th.Te
     bw_tile = filling_tile(M if row_sums and T < 128 else 32 if N > 1 else 128) if idle_sms else None
     if bw_tile is None:
         bw_tile = fitted_tile(br, bc, tu.bw_mb or None, bw_tiles, 128 if tu.bw_helper else 0)
+        if default_tiles and tu.fill and 32 < bw_tile.NT <= 64 and bw_tile.R >= 8 and B * H * (M // bw_tile.MB) > n_sm:
+            # two warps per CTA and two CTAs (shared memory) leave an SM's schedulers with one warp each: half the rows per
+            # thread (512 heads of 64x64, T128: Delta Rule 248 -> 184 us, Mamba-2 302 -> 206 us, RWKV-7 418 -> 343 us)
+            bw_tile = fitted_tile(br // 2, bc, tu.bw_mb or None, bw_tiles, 128 if tu.bw_helper else 0)
     rows_split = bw_tile.MB < M
     # additive state update S' = S +/- X with X free of the state (given the saved row sums):
     # the backward can step the state backwards instead of recomputing it from checkpoints
@@ -463,7 +467,9 @@ def make_plan(step: Callable, inputs: Sequence[th.Tensor], state: Sequence[th.Te
     if auto_blocks:
         # a (b,h) state small enough for a CTA of four warps leaves room for a second CTA on the SM
         # (Mamba-2 64x128: 7 % faster backward than one CTA of eight warps)
-        tu.bw_min_blocks = 2 if bw_tile.NT <= 128 and B * H * (M // bw_tile.MB) > n_sm else 1
+        # and a CTA of a single warp for two more (512 heads of 32x32, T128: Mamba-2 138 -> 99 us, RWKV-7 176 -> 129 us)
+        n_cta = B * H * (M // bw_tile.MB)
+        tu.bw_min_blocks = 4 if bw_tile.NT <= 32 and n_cta > 2 * n_sm else 2 if bw_tile.NT <= 128 and n_cta > n_sm else 1
 
     def flush_options(helper: int):
         ks, k = [], max(1, tu.kflush)
@@ -537,7 +543,7 @@ def make_plan(step: Callable, inputs: Sequence[th.Tensor], state: Sequence[th.Te
             tu.bw_helper, tu.nslots = helper, nsl
             break
         if auto_blocks and tu.bw_min_blocks > 1:
-            tu.bw_min_blocks = 1          # half an SM's shared memory is not enough: one CTA per SM after all
+            tu.bw_min_blocks //= 2        # that share of an SM's shared memory is not enough: fewer CTAs per SM
             continue
         # fewer rows per CTA: smaller slots and fewer row groups in the ring of gradient partials
         try:
