@@ -112,7 +112,10 @@ def choose_tile(M: int, N: int, want_r: int, want_c: int, want_mb: Optional[int]
             C //= 2
         else:
             raise LoweringError(f"state {M}x{N} is too small for a 32-thread CTA")
-    return Tile(R, C, MB, M, N)
+    try:
+        return Tile(R, C, MB, M, N)
+    except AssertionError:
+        raise LoweringError(f"no legal CTA for a {M}x{N} state at {R}x{C} elements per thread and {MB} rows") from None
 
 
 @dataclass

@@ -386,7 +386,8 @@ def make_plan(step: Callable, inputs: Sequence[th.Tensor], state: Sequence[th.Te
             while True:
                 t = choose_tile(M, N, r, c, mb)
                 if t.NT >= 128 or r * c <= 4 or (r == 1 and c <= 4):
-                    return t if t.MB == mb and t.NT <= 512 else None
+                    # (a whole head on 512 threads leaves the backward no room for its helper warps)
+                    return t if t.MB == mb and t.NT <= (256 if mb == M else 512) else None
                 r, c = (r // 2, c) if r > 1 else (r, c // 2)
         except lower.LoweringError:
             return None
@@ -401,12 +402,15 @@ def make_plan(step: Callable, inputs: Sequence[th.Tensor], state: Sequence[th.Te
         # thread instead (Mamba-2's 64x128 state: R4xC16, 128 threads, measured 4 % faster than R4xC32)
         fw_tile = fitted_tile(fr, fc // 2, tu.fw_mb, fw_tiles, 0)
     # the backward's rows only go to several CTAs where no gradient is summed over rows, or where the sequence is long
-    # enough to pay for the fp32 buffers of such sums (zeroed, accumulated atomically, converted: about 10 us)
+    # enough to pay for the fp32 buffers of such sums (zeroed, accumulated atomically, converted: about 10 us) and at least
+    # every other SM would be idle
     row_sums = any(c in (N1, S11) for c in in_cls)
-    bw_tile = filling_tile(M if row_sums and T < 128 else 32 if N > 1 else 128) if idle_sms else None
+    bw_tile = filling_tile(M if row_sums and (T < 128 or 2 * B * H > n_sm) else 32 if N > 1 else 128) if idle_sms else None
+    # (fp32 inputs stage twice the bytes: their small tiles keep the larger share of an SM's shared memory)
+    half_in = all(x.element_size() == 2 for x in inputs)
     if bw_tile is None:
         bw_tile = fitted_tile(br, bc, tu.bw_mb or None, bw_tiles, 128 if tu.bw_helper else 0)
-        if default_tiles and tu.fill and 32 < bw_tile.NT <= 64 and bw_tile.R >= 8 and B * H * (M // bw_tile.MB) > n_sm:
+        if default_tiles and tu.fill and half_in and 32 < bw_tile.NT <= 64 and bw_tile.R >= 8 and B * H * (M // bw_tile.MB) > n_sm:
             # two warps per CTA and two CTAs (shared memory) leave an SM's schedulers with one warp each: half the rows per
             # thread (512 heads of 64x64, T128: Delta Rule 248 -> 184 us, Mamba-2 302 -> 206 us, RWKV-7 418 -> 343 us)
             bw_tile = fitted_tile(br // 2, bc, tu.bw_mb or None, bw_tiles, 128 if tu.bw_helper else 0)
@@ -469,7 +473,7 @@ def make_plan(step: Callable, inputs: Sequence[th.Tensor], state: Sequence[th.Te
         # (Mamba-2 64x128: 7 % faster backward than one CTA of eight warps)
         # and a CTA of a single warp for two more (512 heads of 32x32, T128: Mamba-2 138 -> 99 us, RWKV-7 176 -> 129 us)
         n_cta = B * H * (M // bw_tile.MB)
-        tu.bw_min_blocks = 4 if bw_tile.NT <= 32 and n_cta > 2 * n_sm else 2 if bw_tile.NT <= 128 and n_cta > n_sm else 1
+        tu.bw_min_blocks = 4 if half_in and bw_tile.NT <= 32 and n_cta > 2 * n_sm else 2 if bw_tile.NT <= 128 and n_cta > n_sm else 1
 
     def flush_options(helper: int):
         ks, k = [], max(1, tu.kflush)
