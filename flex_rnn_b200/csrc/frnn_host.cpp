@@ -44,6 +44,28 @@ struct Meta {
     at::ScalarType dtype;
 };
 
+Meta meta_of(const Tensor& t) { return {t.sizes().vec(), t.strides().vec(), t.scalar_type()}; }
+
+// A saved tensor in the layout it was saved with, on a 16-byte boundary if `aligned`.  Kernels are built for that layout,
+// but a saved-tensor hook may hand back another one (torch.autograd.graph.save_on_cpu returns contiguous copies): the
+// values are then copied into it.  Another shape, data type or device is refused.
+Tensor as_saved(const Tensor& t, const Meta& m, const c10::Device& dev, bool aligned) {
+    TORCH_CHECK(t.defined() && t.layout() == at::kStrided && t.sizes().equals(m.sizes) && t.scalar_type() == m.dtype && t.device() == dev,
+                "flex_rnn_b200: a saved-tensor hook returned another shape, data type or device than was saved (shape ", at::IntArrayRef(m.sizes),
+                ", ", m.dtype, " on ", dev, ")");
+    bool same = !aligned || !((uintptr_t)t.data_ptr() & 15);
+    for (size_t d = 0; d < m.sizes.size(); d++) same = same && (m.sizes[d] <= 1 || t.stride(d) == m.strides[d]);
+    if (same) return t;
+    Tensor r = at::empty_strided(m.sizes, m.strides, t.options()), to = r, from = t;
+    for (size_t d = 0; d < m.sizes.size(); d++)
+        if (m.sizes[d] > 1 && m.strides[d] == 0) {       // an expanded dimension: one element, whose copies are all alike
+            to = to.narrow(d, 0, 1);
+            from = from.narrow(d, 0, 1);
+        }
+    to.copy_(from);
+    return r;
+}
+
 struct TensorMap {                 // a TMA tensor map to encode per call (it embeds the tensor's address)
     int src;                       // parameter whose tensor it describes
     int64_t off;                   // bytes from that tensor's first element
@@ -189,6 +211,7 @@ variable_list run_forward(Spec& s, const variable_list& args) {      // results,
 struct RecurrenceBackward : torch::autograd::Node {
     std::shared_ptr<Spec> spec;
     std::vector<torch::autograd::SavedVariable> saved;   // the arguments, then what the forward saved
+    std::vector<Meta> saved_meta;                         // what was saved, to be read back the same
     std::vector<Meta> grad_meta;                          // of the results: absent upstream gradients are zeros
 
     explicit RecurrenceBackward(torch::autograd::edge_list&& e) : Node(std::move(e)) {}
@@ -219,6 +242,7 @@ struct RecurrenceBackward : torch::autograd::Node {
             }
         }
         const int narg = s.nin + s.nst;
+        for (size_t i = 0; i < kept.size(); i++) kept[i] = as_saved(kept[i], saved_meta[i], dev, i >= (size_t)narg || s.aligned[i]);
         const Program* p = s.backward.load(std::memory_order_acquire);
         // with create_graph=True the Python closure calls the custom op, which refuses to be differentiated in its turn
         bool ok = p && !at::GradMode::is_enabled() && s.args_ok(kept, s.nin);
@@ -321,11 +345,15 @@ struct HostOp {
                 res = run_forward(*s, a);
             }
             node->spec = s;
-            for (const Tensor& t : a) node->saved.emplace_back(t, false);
-            for (size_t i = nres; i < res.size(); i++) node->saved.emplace_back(res[i], false);
+            auto save = [&](const Tensor& t) {
+                node->saved.emplace_back(t, false);
+                node->saved_meta.push_back(meta_of(t));
+            };
+            for (const Tensor& t : a) save(t);
+            for (size_t i = nres; i < res.size(); i++) save(res[i]);
             res.resize(nres);
             for (Tensor& t : res) {
-                node->grad_meta.push_back({t.sizes().vec(), t.strides().vec(), t.scalar_type()});
+                node->grad_meta.push_back(meta_of(t));
                 torch::autograd::create_gradient_edge(t, node);
             }
         }
@@ -335,7 +363,7 @@ struct HostOp {
     }
 };
 
-Meta meta_of(const py::handle& h) {
+Meta meta_from(const py::handle& h) {
     auto t = py::cast<py::tuple>(h);
     Meta m;
     m.sizes = py::cast<std::vector<int64_t>>(t[0]);
@@ -346,7 +374,7 @@ Meta meta_of(const py::handle& h) {
 
 std::unique_ptr<Program> program_of(const py::dict& d) {
     std::unique_ptr<Program> p(new Program());
-    for (auto h : d["alloc"]) p->alloc.push_back(meta_of(h));
+    for (auto h : d["alloc"]) p->alloc.push_back(meta_from(h));
     p->zeroed = py::cast<std::vector<int>>(d["zeroed"]);
     p->cast_from = py::cast<std::vector<int>>(d["cast_from"]);
     p->returned = py::cast<int>(d["returned"]);
@@ -385,6 +413,9 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
         g_launch = (launch_fn)launch;
         g_encode = (encode_fn)encode;
         g_error = (error_fn)error;
+    });
+    m.def("as_saved", [](const Tensor& t, const py::object& meta, const Tensor& device_of, bool aligned) {
+        return as_saved(t, meta_from(meta), device_of.device(), aligned);
     });
     py::class_<Spec, std::shared_ptr<Spec>>(m, "Spec")
         .def(py::init([](int nin, int nst, int nout, int device, uintptr_t err, std::vector<bool> aligned, std::vector<int64_t> reach,

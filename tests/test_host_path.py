@@ -1,5 +1,7 @@
 """The native host path of an eager call (csrc/frnn_host.cpp) and the kernels of calls without gradients: same
 results as the custom op, whatever the call looks like."""
+import contextlib
+
 import pytest
 import torch
 
@@ -83,3 +85,54 @@ def test_native_path_graph_semantics():
         y2, _ = f(*leaves)
     torch.cuda.current_stream().wait_stream(st)
     assert torch.equal(y2, f.apply(*leaves)[0])
+
+
+LAYOUTS = {"transposed": lambda g: g(2, 4, 3, 1, 8).transpose(1, 2), "sliced": lambda g: g(2, 3, 4, 1, 24)[..., 8:16],
+           "expanded": lambda g: g(2, 3, 1, 1, 8).expand(2, 3, 4, 1, 8), "windows": lambda g: g(64).as_strided((2, 3, 4, 1, 8), (24, 6, 2, 1, 1)),
+           "odd": lambda g: g(193)[1:].view(2, 3, 4, 1, 8), "reversed_dims": lambda g: g(8, 1, 4, 3, 2).permute(4, 3, 2, 1, 0)}
+
+
+@pytest.mark.parametrize("layout", list(LAYOUTS))
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_saved_tensors_come_back_as_they_were(layout, dtype):
+    """Whatever layout a saved-tensor hook returns, the backward reads the one that was saved, on its alignment."""
+    from flex_rnn_b200 import runtime
+    as_saved = runtime.host().as_saved
+    x = LAYOUTS[layout](lambda *n: torch.randn(n).to(dtype))
+    meta = (list(x.shape), list(x.stride()), x.dtype)
+    lead = torch.empty(x.numel() + 1, dtype=dtype)[1:].view(x.shape).copy_(x)       # contiguous, off a 16-byte boundary
+    for back in (x, x.contiguous(), x.transpose(0, 2).contiguous().transpose(0, 2), lead):
+        got = as_saved(back, meta, x, True)
+        assert got.data_ptr() % 16 == 0 and torch.equal(got, x)
+        assert [s for s, n in zip(got.stride(), got.shape) if n > 1] == [s for s, n in zip(x.stride(), x.shape) if n > 1]
+    assert as_saved(x, meta, x, False).data_ptr() == x.data_ptr()
+    for bad in (x[:1], x.double(), x.to("meta"), x.reshape(-1)):
+        with pytest.raises(RuntimeError, match="saved-tensor hook"):
+            as_saved(bad, meta, x, True)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dt,T", [(torch.float32, 20), (torch.bfloat16, 70)])       # recurrent and chunked kernels
+def test_saved_tensor_hooks(dt, T):
+    """Gradients do not depend on what saved-tensor hooks do to the layout of the inputs and the checkpoints."""
+    xs, dy, dS = W.synthetic("delta_rule", 2, T, 3, 64, 64, dt, device="cuda")
+    f = flex_rnn_b200.jit(W.delta_rule)
+    xs[0] = xs[0].transpose(1, 2).contiguous().transpose(1, 2)          # dense, but not in the order of its dimensions
+    xs[2] = torch.stack([xs[2], xs[2]], -1)[..., 0]
+    leaves = [x.detach().requires_grad_() for x in xs]
+
+    def off(t):                    # contiguous and off a 16-byte boundary
+        return torch.empty(t.numel() + 1, dtype=t.dtype, device=t.device)[1:].view(t.shape).copy_(t)
+
+    def grads(ctx):
+        with ctx:
+            y, S = f(*leaves)
+        return torch.autograd.grad((y, S), leaves, (dy, dS))
+    hooks = torch.autograd.graph.saved_tensors_hooks
+    for _ in range(2):             # the first call compiles (a step function cannot be traced under hooks)
+        want = grads(contextlib.nullcontext())
+    for ctx in (torch.autograd.graph.save_on_cpu(pin_memory=True), hooks(off, lambda t: t),
+                hooks(lambda t: t.transpose(0, -1).contiguous(), lambda t: t.transpose(0, -1))):
+        assert all(torch.equal(a, b) for a, b in zip(grads(ctx), want))
+    with pytest.raises(RuntimeError, match="saved-tensor hook"):
+        grads(hooks(lambda t: t.cpu(), lambda t: t))
