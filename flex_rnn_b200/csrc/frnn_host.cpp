@@ -148,7 +148,7 @@ struct Spec : std::enable_shared_from_this<Spec> {
     std::vector<char> aligned;           // argument i was 16-byte aligned at compilation
     std::vector<int64_t> reach;          // bytes from argument i's first element to the end of its last one
     std::atomic<const Program*> forward{nullptr}, infer{nullptr}, backward{nullptr};   // set once, by a Python closure's first run
-    py::object py_forward, py_infer, py_backward;    // (spec, args) -> results and saved; (spec, args) -> results; (spec, grads, args, saved) -> gradients
+    py::object py_forward, py_infer, py_backward;    // (spec, args) -> results and saved; (spec, args) -> results; (spec, grads, args, saved, whether the custom op is not needed) -> gradients
     ~Spec() {
         delete forward.load();
         delete infer.load();
@@ -207,6 +207,21 @@ variable_list run_forward(Spec& s, const variable_list& args) {      // results,
     return made;
 }
 
+// Whether something that traces or transforms calls is active, which only the custom ops serve.
+bool transformed() {
+    return c10::impl::TorchDispatchModeTLS::any_modes_set() || at::impl::torch_function_mode_enabled() ||
+           c10::impl::tls_is_dispatch_key_included(c10::DispatchKey::FuncTorchDynamicLayerFrontMode) ||
+           c10::impl::tls_is_dispatch_key_included(c10::DispatchKey::Functionalize);
+}
+
+// Whether a tensor is a wrapper of some kind (subclass, batched, lazily conjugated ...), which only the custom ops serve.
+bool wrapped(const Tensor& t) {
+    static const c10::DispatchKeySet special({c10::DispatchKey::Python, c10::DispatchKey::PythonTLSSnapshot,
+        c10::DispatchKey::FuncTorchBatched, c10::DispatchKey::FuncTorchGradWrapper, c10::DispatchKey::Functionalize,
+        c10::DispatchKey::Batched, c10::DispatchKey::ZeroTensor, c10::DispatchKey::Conjugate, c10::DispatchKey::Negative, c10::DispatchKey::BatchedNestedTensor});
+    return t.key_set().has_any(special);
+}
+
 // The node of one call in the autograd graph.
 struct RecurrenceBackward : torch::autograd::Node {
     std::shared_ptr<Spec> spec;
@@ -242,16 +257,21 @@ struct RecurrenceBackward : torch::autograd::Node {
             }
         }
         const int narg = s.nin + s.nst;
-        for (size_t i = 0; i < kept.size(); i++) kept[i] = as_saved(kept[i], saved_meta[i], dev, i >= (size_t)narg || s.aligned[i]);
+        // a gradient that is itself traced or transformed (a dispatch mode, batched upstream gradients) is the custom op's;
+        // with create_graph=True too, which refuses to be differentiated in its turn
+        bool direct = !transformed() && !at::GradMode::is_enabled();
+        for (const Tensor& t : up) direct = direct && !wrapped(t);
+        for (const Tensor& t : kept) direct = direct && t.defined() && !wrapped(t);
+        if (direct)
+            for (size_t i = 0; i < kept.size(); i++) kept[i] = as_saved(kept[i], saved_meta[i], dev, i >= (size_t)narg || s.aligned[i]);
         const Program* p = s.backward.load(std::memory_order_acquire);
-        // with create_graph=True the Python closure calls the custom op, which refuses to be differentiated in its turn
-        bool ok = p && !at::GradMode::is_enabled() && s.args_ok(kept, s.nin);
+        bool ok = p && direct && s.args_ok(kept, s.nin);
         for (const Tensor& t : up) ok = ok && t.device() == dev && !((uintptr_t)t.data_ptr() & 15);
         for (size_t i = 0; i < up.size() && ok; i++) ok = up[i].scalar_type() == grad_meta[i].dtype;
         variable_list g;
         if (!ok) {
             g = with_python([&] {
-                return to_list(s.py_backward(s.shared_from_this(), to_tuple(up, 0, up.size()), to_tuple(kept, 0, narg), to_tuple(kept, narg, kept.size())));
+                return to_list(s.py_backward(s.shared_from_this(), to_tuple(up, 0, up.size()), to_tuple(kept, 0, narg), to_tuple(kept, narg, kept.size()), direct));
             });
         } else {
             std::vector<void*> given;
@@ -285,13 +305,7 @@ struct HostOp {
     // The results of a direct call, or None: the caller then goes through the custom op.
     py::object call(py::tuple args) {
         if ((int)args.size() != nargs) return py::none();
-        if (c10::impl::TorchDispatchModeTLS::any_modes_set() || at::impl::torch_function_mode_enabled()) return py::none();
-        if (c10::impl::tls_is_dispatch_key_included(c10::DispatchKey::FuncTorchDynamicLayerFrontMode) ||
-            c10::impl::tls_is_dispatch_key_included(c10::DispatchKey::Functionalize))
-            return py::none();
-        static const c10::DispatchKeySet special({c10::DispatchKey::Python, c10::DispatchKey::PythonTLSSnapshot,
-            c10::DispatchKey::FuncTorchBatched, c10::DispatchKey::FuncTorchGradWrapper, c10::DispatchKey::Functionalize,
-            c10::DispatchKey::ZeroTensor, c10::DispatchKey::Conjugate, c10::DispatchKey::Negative, c10::DispatchKey::BatchedNestedTensor});
+        if (transformed()) return py::none();
         variable_list a;
         a.reserve(nargs);
         std::vector<int64_t> key;
@@ -301,7 +315,7 @@ struct HostOp {
             PyObject* o = PyTuple_GET_ITEM(args.ptr(), i);
             if (!THPVariable_CheckExact(o)) return py::none();
             const Tensor& t = THPVariable_Unpack(o);
-            if (!t.is_cuda() || t.layout() != at::kStrided || t.key_set().has_any(special) || t._fw_grad(0).defined()) return py::none();
+            if (!t.is_cuda() || t.layout() != at::kStrided || wrapped(t) || t._fw_grad(0).defined()) return py::none();
             if (t.device() != THPVariable_Unpack(PyTuple_GET_ITEM(args.ptr(), 0)).device()) return py::none();
             grad = grad || t.requires_grad();
             auto sz = t.sizes();

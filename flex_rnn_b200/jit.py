@@ -121,8 +121,8 @@ class jit:
 
         bw_op = self._bw_op
 
-        def backward(up, args_, saved):
-            if th.is_grad_enabled():                # create_graph=True
+        def backward(up, args_, saved, direct):
+            if not direct:                          # create_graph=True, batched upstream gradients, a dispatch mode
                 return bw_op(*up, *args_, *saved)
             dx, ds0 = bwd(up[:nout], up[nout:], args_[:nin], saved[:nst], saved[nst:])
             return (*dx, *ds0)

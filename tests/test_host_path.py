@@ -136,3 +136,27 @@ def test_saved_tensor_hooks(dt, T):
         assert all(torch.equal(a, b) for a, b in zip(grads(ctx), want))
     with pytest.raises(RuntimeError, match="saved-tensor hook"):
         grads(hooks(lambda t: t.cpu(), lambda t: t))
+
+
+@pytest.mark.gpu
+def test_transformed_backward():
+    """Batched upstream gradients and a dispatch mode around the backward find the custom op."""
+    from torch.utils._python_dispatch import TorchDispatchMode
+    xs, dy, dS = W.synthetic("delta_rule", 1, 20, 2, 64, 64, torch.float32, device="cuda")
+    f = flex_rnn_b200.jit(W.delta_rule)
+    leaves = [x.detach().requires_grad_() for x in xs]
+    want = [torch.autograd.grad(f(*leaves)[0], leaves, dy) for _ in range(2)][1]
+    up = torch.stack([dy, 0.5 * dy])
+    for a, b in zip(torch.autograd.grad(f(*leaves)[0], leaves, up, is_grads_batched=True), want):
+        assert torch.equal(a[0], b) and torch.equal(a[1], 0.5 * b)
+    seen = []
+
+    class Log(TorchDispatchMode):
+        def __torch_dispatch__(self, fn, types, args=(), kwargs=None):
+            seen.append(str(fn))
+            return fn(*args, **(kwargs or {}))
+    y = f(*leaves)[0]
+    with Log():
+        got = torch.autograd.grad(y, leaves, dy)
+    assert any("flex_rnn_b200" in s for s in seen)
+    assert all(torch.equal(a, b) for a, b in zip(got, want))
