@@ -211,7 +211,8 @@ variable_list run_forward(Spec& s, const variable_list& args) {      // results,
 bool transformed() {
     return c10::impl::TorchDispatchModeTLS::any_modes_set() || at::impl::torch_function_mode_enabled() ||
            c10::impl::tls_is_dispatch_key_included(c10::DispatchKey::FuncTorchDynamicLayerFrontMode) ||
-           c10::impl::tls_is_dispatch_key_included(c10::DispatchKey::Functionalize);
+           c10::impl::tls_is_dispatch_key_included(c10::DispatchKey::Functionalize) ||
+           c10::impl::tls_is_dispatch_key_included(c10::DispatchKey::Tracer);
 }
 
 // Whether a tensor is a wrapper of some kind (subclass, batched, lazily conjugated ...), which only the custom ops serve.

@@ -160,3 +160,17 @@ def test_transformed_backward():
         got = torch.autograd.grad(y, leaves, dy)
     assert any("flex_rnn_b200" in s for s in seen)
     assert all(torch.equal(a, b) for a, b in zip(got, want))
+
+
+@pytest.mark.gpu
+@pytest.mark.filterwarnings("ignore")
+def test_trace_records_the_op():
+    """A traced function computes from its arguments, not from those of the tracing call."""
+    xs, _, _ = W.synthetic("delta_rule", 1, 20, 2, 64, 64, torch.float32, device="cuda")
+    f = flex_rnn_b200.jit(W.delta_rule)
+    other = [0.5 * x for x in xs]
+    with torch.no_grad():
+        for _ in range(2):
+            want = f(*other)
+        traced = torch.jit.trace(lambda *a: f(*a), tuple(xs), check_trace=False)
+        assert all(torch.equal(a, b) for a, b in zip(traced(*other), want))
