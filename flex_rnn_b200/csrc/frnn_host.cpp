@@ -195,14 +195,22 @@ template <class F> variable_list with_python(F f) {
     }
 }
 
+// Run a program of a call's arguments, from a thread that holds the interpreter lock: allocations and launches may wait (a
+// full launch queue), and other Python threads go on meanwhile.
+variable_list launch(const Program& p, const variable_list& args, const Spec& s) {
+    std::vector<void*> given;
+    for (const Tensor& t : args) given.push_back(t.data_ptr());
+    variable_list made;
+    py::gil_scoped_release others;
+    run_program(p, given, made, c10::Device(c10::kCUDA, s.device), s.err);
+    return made;
+}
+
 variable_list run_forward(Spec& s, const variable_list& args) {      // results, final states, saved tensors
     const Program* p = s.forward.load(std::memory_order_acquire);
     if (!p || !s.args_ok(args, args.size()))
         return with_python([&] { return to_list(s.py_forward(s.shared_from_this(), to_tuple(args, 0, args.size()))); });
-    std::vector<void*> given;
-    for (const Tensor& t : args) given.push_back(t.data_ptr());
-    std::vector<Tensor> made;
-    run_program(*p, given, made, c10::Device(c10::kCUDA, s.device), s.err);
+    variable_list made = launch(*p, args, s);
     made.resize(p->returned);
     return made;
 }
@@ -343,13 +351,10 @@ struct HostOp {
         if (!grad) {
             at::AutoDispatchBelowADInplaceOrView below;
             const Program* p = s->infer.load(std::memory_order_acquire);
-            if (p && s->args_ok(a, a.size())) {
-                std::vector<void*> given;
-                for (const Tensor& t : a) given.push_back(t.data_ptr());
-                run_program(*p, given, res, c10::Device(c10::kCUDA, s->device), s->err);
-            } else {
+            if (p && s->args_ok(a, a.size()))
+                res = launch(*p, a, *s);
+            else
                 res = to_list(s->py_infer(s, args));
-            }
             res.resize(nres);
         } else {
             auto node = std::shared_ptr<RecurrenceBackward>(

@@ -1,6 +1,8 @@
 """The native host path of an eager call (csrc/frnn_host.cpp) and the kernels of calls without gradients: same
 results as the custom op, whatever the call looks like."""
 import contextlib
+import threading
+import time
 
 import pytest
 import torch
@@ -174,3 +176,36 @@ def test_trace_records_the_op():
             want = f(*other)
         traced = torch.jit.trace(lambda *a: f(*a), tuple(xs), check_trace=False)
         assert all(torch.equal(a, b) for a, b in zip(traced(*other), want))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("grad", [False, True])
+def test_full_launch_queue_does_not_stop_other_threads(grad):
+    """A launch that waits for room in the queue does so without the interpreter lock."""
+    xs, _, _ = W.synthetic("delta_rule", 1, 4, 1, 32, 32, torch.float32, device="cuda")
+    f = flex_rnn_b200.jit(W.delta_rule)
+    xs = [x.detach().requires_grad_(grad) for x in xs]
+    for _ in range(3):
+        f(*xs)
+    torch.cuda.synchronize()
+    gaps, done = [0.0], threading.Event()
+
+    def tick():
+        last = time.perf_counter()
+        while not done.is_set():
+            time.sleep(0.001)
+            now = time.perf_counter()
+            gaps.append(now - last)
+            last = now
+    other = threading.Thread(target=tick)
+    other.start()
+    start = time.perf_counter()
+    torch.cuda._sleep(1_500_000_000)            # about 0.8 s of GPU time in front of the queue
+    for _ in range(3000):                       # more launches than the queue holds
+        f(*xs)
+    took = time.perf_counter() - start
+    done.set()
+    other.join()
+    torch.cuda.synchronize()
+    assert took > 0.4, "the queue never filled up"
+    assert max(gaps) < 0.2, (max(gaps), took)
