@@ -1019,6 +1019,13 @@ def build_twopass(step, inputs, state, dryrun=False, tuning: Optional[Tuning] = 
             have = t.untyped_storage().nbytes() // t.element_size() - t.storage_offset()
             assert t.numel() == 0 or reach <= have, f"{what} #{i + 1}: its strides reach past the end of its storage"
 
+    def check_device(*groups):
+        """The kernels dereference every address on one device."""
+        device = groups[0][0].device
+        for t in (t for g in groups for t in g):
+            if t.device != device:
+                raise RuntimeError(f"flex_rnn_b200: all tensors of a call have to be on one device, got {device} and {t.device}")
+
     # timing alternative tilings costs a few NVRTC compilations: only worth it for work of benchmark size
     no_tune = (_launcher is not None or not plan.tuning.autotune
                or p.B * p.T * p.H * p.M * p.N < plan.tuning.autotune_min_work)
@@ -1108,6 +1115,7 @@ def build_twopass(step, inputs, state, dryrun=False, tuning: Optional[Tuning] = 
         return tuned["infer_src"], tuned["launch_infer"]
 
     def check_args(inputs_, state0):
+        check_device(inputs_, state0)
         verify_meta(inputs_, in_meta, "input Tensor metadata doesn't match compilation\n")
         verify_meta(state0, st_meta, "initial state Tensor metadata doesn't match compilation\n")
         check_align(inputs_, in_align, "input")
@@ -1169,11 +1177,12 @@ def build_twopass(step, inputs, state, dryrun=False, tuning: Optional[Tuning] = 
         chunk_where = {nm: i for i, nm in enumerate(names)}
 
     def backward(doutput, dstateT, inputs_, state_store, aux_):
+        aux = aux_[0] if isinstance(aux_, (tuple, list)) else aux_
+        check_device(inputs_, doutput, dstateT, state_store, (aux,))
         doutput = tuple(d.contiguous() for d in doutput)
         dstateT = tuple(d.contiguous() for d in dstateT)
         verify_meta(inputs_, in_meta)
         check_align(inputs_, in_align, "input")
-        aux = aux_[0] if isinstance(aux_, (tuple, list)) else aux_
         device = inputs_[0].device
         with _device_ctx(device):
             check_before(device)
