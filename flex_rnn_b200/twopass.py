@@ -1026,6 +1026,16 @@ def build_twopass(step, inputs, state, dryrun=False, tuning: Optional[Tuning] = 
             if t.device != device:
                 raise RuntimeError(f"flex_rnn_b200: all tensors of a call have to be on one device, got {device} and {t.device}")
 
+    def aligned(t):
+        """Contiguous and on a 16-byte boundary, as the kernels read upstream gradients and saved tensors."""
+        t = t.contiguous()
+        return t if t.data_ptr() % 16 == 0 else t.clone()
+
+    def saved(what, t, meta):
+        if t.shape != meta[0] or t.dtype != meta[2]:
+            raise RuntimeError(f"flex_rnn_b200: {what} were saved as {tuple(meta[0])} {meta[2]} but come back as {tuple(t.shape)} {t.dtype}")
+        return aligned(t)
+
     # timing alternative tilings costs a few NVRTC compilations: only worth it for work of benchmark size
     no_tune = (_launcher is not None or not plan.tuning.autotune
                or p.B * p.T * p.H * p.M * p.N < plan.tuning.autotune_min_work)
@@ -1179,8 +1189,9 @@ def build_twopass(step, inputs, state, dryrun=False, tuning: Optional[Tuning] = 
     def backward(doutput, dstateT, inputs_, state_store, aux_):
         aux = aux_[0] if isinstance(aux_, (tuple, list)) else aux_
         check_device(inputs_, doutput, dstateT, state_store, (aux,))
-        doutput = tuple(d.contiguous() for d in doutput)
-        dstateT = tuple(d.contiguous() for d in dstateT)
+        doutput, dstateT = tuple(aligned(d) for d in doutput), tuple(aligned(d) for d in dstateT)
+        state_store = tuple(saved("checkpoints", c, m) for c, m in zip(state_store, fw_meta[nout + nst:]))
+        aux = saved("row sums", aux, fw_meta[-1])
         verify_meta(inputs_, in_meta)
         check_align(inputs_, in_align, "input")
         device = inputs_[0].device
