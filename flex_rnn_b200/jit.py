@@ -188,11 +188,12 @@ class jit:
         def backward(ctx, *grads):
             # upstream gradients that autograd leaves out are zeros (reference: flex_rnn/jit.py:76-80)
             grads = list(grads[:nout + nst])
-            dev = ctx.saved_tensors[0].device
+            saved = ctx.saved_tensors               # read once: a checkpointed region unpacks its tensors once only
+            dev = saved[0].device
             for i, m in enumerate(ctx.out_meta):
                 if grads[i] is None:
                     grads[i] = th.zeros_like(m, device=dev)
-            return bw_op(*grads, *ctx.saved_tensors)
+            return bw_op(*grads, *saved)
 
         fw_op.register_autograd(backward, setup_context=setup_context)
         self._fw_op, self._bw_op = fw_op, bw_op

@@ -209,3 +209,18 @@ def test_full_launch_queue_does_not_stop_other_threads(grad):
     torch.cuda.synchronize()
     assert took > 0.4, "the queue never filled up"
     assert max(gaps) < 0.2, (max(gaps), took)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("native", [True, False])
+def test_checkpointed_region(native):
+    """Non-reentrant checkpointing, which recomputes through saved-tensor hooks and unpacks each tensor once."""
+    from torch.utils.checkpoint import checkpoint
+    xs, dy, _ = W.synthetic("delta_rule", 1, 20, 2, 64, 64, torch.float32, device="cuda")
+    f = flex_rnn_b200.jit(W.delta_rule)
+    leaves = [x.detach().requires_grad_() for x in xs]
+    want = torch.autograd.grad(torch.tanh(f(*leaves)[0]), leaves, dy)
+    call = f if native else f.apply
+    for _ in range(2):
+        y = checkpoint(lambda *a: torch.tanh(call(*a)[0]), *leaves, use_reentrant=False)
+        assert all(torch.equal(a, b) for a, b in zip(torch.autograd.grad(y, leaves, dy), want))
