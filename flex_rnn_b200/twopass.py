@@ -121,6 +121,8 @@ class Tuning:
     use_tma: bool = True
     fill: int = 1            # smaller tiles and rows over more CTAs where there are fewer (batch, head) pairs than SMs
     chunk: int = 1           # chunked form on the tensor cores where the step function has it (see chunk.chunk_plan)
+    chunk_variant: int = -1  # >= 0: use this member of ChunkPlan.variants() untimed for the scans of the chunked form;
+                             # fw_variant and bw_variant then pin the kernels of the calls that do not have it
 
 
 SMEM_LIMIT = 227 * 1024
@@ -923,8 +925,8 @@ def build_twopass(step, inputs, state, dryrun=False, tuning: Optional[Tuning] = 
     plan, fw_meta, bw_meta = make_plan(step, inputs, state, tuning)
     p = plan.problem
     nin, nst, nout = len(inputs), plan.n_st, plan.n_out
-    # a pinned variant names one of the recurrent kernels
-    pinned = plan.tuning.fw_variant >= 0 or plan.tuning.bw_variant >= 0
+    # a pinned forward or backward variant names one of the recurrent kernels: alone, it asks for those
+    pinned = max(plan.tuning.fw_variant, plan.tuning.bw_variant) >= 0 and plan.tuning.chunk_variant < 0
     cplan = chunk.chunk_plan(plan) if plan.tuning.chunk and not pinned else None
     ctrain = cplan is not None and cplan.bp is not None
     cshort = cplan is not None and cplan.short
@@ -946,16 +948,18 @@ def build_twopass(step, inputs, state, dryrun=False, tuning: Optional[Tuning] = 
         return (*_build_empty(plan, fw_meta, bw_meta, inputs, state), fw_meta, bw_meta)
     fw_src, bw_src = generate(plan) if not ctrain else (None, None)
     tu0 = plan.tuning
-    forced_fw, forced_bw = tu0.fw_variant >= 0, tu0.bw_variant >= 0
-    if forced_fw and tu0.fw_variant > 0:
+    fw_member, bw_member = (tu0.chunk_variant,) * 2 if ctrain else (tu0.fw_variant, tu0.bw_variant)
+    infer_member = tu0.chunk_variant if cshort else tu0.fw_variant
+    member = cplan.variants()[max(0, tu0.chunk_variant)] if cplan is not None else {}      # of the chunked scans
+    if not ctrain and tu0.fw_variant > 0:
         fw_src = generate_forward(plan, **forward_variants(plan)[tu0.fw_variant])
-    if forced_bw and tu0.bw_variant > 0:
+    if not ctrain and tu0.bw_variant > 0:
         bw_src = generate_backward(plan, **backward_variants(plan)[tu0.bw_variant])
         if bw_src is None:
             raise lower.LoweringError("the requested backward variant does not fit shared memory")
     make = _launcher or _CudaLauncher
     if ctrain:
-        fw_src, bw_src = _checked(cplan.forward(), tu0), _checked(cplan.backward_scan(), tu0)
+        fw_src, bw_src = _checked(cplan.forward(**member), tu0), _checked(cplan.backward_scan(**member), tu0)
         launch_vg = make(_checked(cplan.vector_grads(), tu0))
     launch_fw, launch_bw = make(fw_src), make(bw_src)
 
@@ -1039,9 +1043,9 @@ def build_twopass(step, inputs, state, dryrun=False, tuning: Optional[Tuning] = 
     # timing alternative tilings costs a few NVRTC compilations: only worth it for work of benchmark size
     no_tune = (_launcher is not None or not plan.tuning.autotune
                or p.B * p.T * p.H * p.M * p.N < plan.tuning.autotune_min_work)
-    tuned = {"fw": no_tune or forced_fw, "launch_fw": launch_fw, "fw_src": fw_src, "bw": no_tune or forced_bw,
-             "launch_bw": launch_bw, "bw_src": bw_src, "infer": no_tune or forced_fw,
-             "fw_choice": max(0, tu0.fw_variant), "bw_choice": max(0, tu0.bw_variant), "fw_log": [], "bw_log": []}
+    tuned = {"fw": no_tune or fw_member >= 0, "launch_fw": launch_fw, "fw_src": fw_src, "bw": no_tune or bw_member >= 0,
+             "launch_bw": launch_bw, "bw_src": bw_src, "infer": no_tune or infer_member >= 0,
+             "fw_choice": max(0, fw_member), "bw_choice": max(0, bw_member), "fw_log": [], "bw_log": []}
 
     def timed(launcher, ptrs, device, reps=5):
         """Median device time of ``reps`` launches after two warm-up launches (the first also compiles, and the
@@ -1119,8 +1123,8 @@ def build_twopass(step, inputs, state, dryrun=False, tuning: Optional[Tuning] = 
     def infer_kernel():
         """(source, launcher) of the planned kernel for calls without gradients, made on first use."""
         if "launch_infer" not in tuned:
-            kw = forward_variants(plan)[tu0.fw_variant] if tu0.fw_variant > 0 else {}
-            tuned["infer_src"] = _checked(cplan.infer(), tu0) if cshort else generate_forward(plan, infer=True, **kw)
+            kw = forward_variants(plan)[tu0.fw_variant] if tu0.fw_variant > 0 and not cshort else {}
+            tuned["infer_src"] = _checked(cplan.infer(**member), tu0) if cshort else generate_forward(plan, infer=True, **kw)
             tuned["launch_infer"] = make(tuned["infer_src"])
         return tuned["infer_src"], tuned["launch_infer"]
 

@@ -1,6 +1,8 @@
 """The chunked form (chunk.py): which step functions have it, and its kernels against the naive scan in fp64 at the
 edges of chunks, columns and rows, with decays that vanish inside a chunk.  CPU: under the host emulation; GPU: the
 public API."""
+import dataclasses
+
 import pytest
 import torch
 
@@ -8,7 +10,7 @@ import flex_rnn_b200
 from flex_rnn_b200 import chunk
 from flex_rnn_b200 import examples as X
 from flex_rnn_b200 import workloads as W
-from flex_rnn_b200.twopass import build_twopass, make_plan
+from flex_rnn_b200.twopass import build_twopass, default_tuning, make_plan
 from oracle import naive_oracle as O
 
 
@@ -74,6 +76,39 @@ def test_emulated(op, B, T, H, M, N, dt, reset):
     dx, ds = bwd((dy.to(y.dtype),), (dS,), tuple(ins), (ck,), (aux,))
     check([y, sT, *dx, *ds], step, ins, s, dy, dS, dt)
     check([*fwd.infer(tuple(ins), (s,))], step, ins, s, dy, dS, dt)
+
+
+def run_member(op, k, to, launcher=None):
+    """A pinned member of the chunked scans, with recurrent members pinned beside it: fw, bw and infer against the oracle."""
+    step, ins, s, dy, dS = case(op, 1, 40, 2, 32, 32, torch.bfloat16)
+    tu = dataclasses.replace(default_tuning(1, 40, 2, 32, 32, 1), chunk_variant=k, fw_variant=1, bw_variant=1)
+    gi, gs = [x.to(to) for x in ins], s.to(to)
+    fwd, bwd, _, _ = build_twopass(step, tuple(gi), (gs,), tuning=tu, _launcher=launcher)
+    assert [ks.name for ks in fwd.sources] == ["frnn_cfw", "frnn_cbw"] and fwd.tuned["fw_choice"] == fwd.tuned["bw_choice"] == k
+    y, sT, ck, aux = fwd(tuple(gi), (gs,))
+    dx, ds = bwd((dy.to(y),), (dS.to(sT),), tuple(gi), (ck,), (aux,))
+    check([y, sT, *dx, *ds], step, ins, s, dy, dS, torch.bfloat16)
+    check([*fwd.infer(tuple(gi), (gs,))], step, ins, s, dy, dS, torch.bfloat16)
+    return [ks.source for ks in (*fwd.sources, fwd.tuned["infer_src"])]
+
+
+def test_pinned_members():
+    """Pinning keeps the chunked form; a forward or backward member alone still asks for the recurrent kernels."""
+    from emu.emu import EmuLauncher
+    seen = [run_member("gated_delta_rule", k, "cpu", EmuLauncher) for k in range(3)]
+    assert all(len({src[i] for src in seen}) == 3 for i in range(3))
+    step, ins, s, _, _ = case("delta_rule", 1, 40, 2, 32, 32, torch.bfloat16)
+    for kw, name in [(dict(fw_variant=0), "frnn_fw"), (dict(bw_variant=0), "frnn_fw"), (dict(), "frnn_cfw"), (dict(chunk=0, chunk_variant=1), "frnn_fw")]:
+        tu = dataclasses.replace(default_tuning(1, 40, 2, 32, 32, 1), **kw)
+        fwd = build_twopass(step, tuple(ins), (s,), tuning=tu, _launcher=lambda ks: None)[0]
+        assert fwd.sources[0].name == name, kw
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("k", [0, 1, 2])
+@pytest.mark.parametrize("op", ["delta_rule", "gated_delta_rule", "rwkv7", "mamba2", "gla"])
+def test_pinned_members_gpu(op, k):
+    run_member(op, k, "cuda:0")
 
 
 @pytest.mark.gpu
