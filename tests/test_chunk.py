@@ -128,3 +128,78 @@ def test_gpu(op, B, T, H, M, N, dt, reset):
     with torch.no_grad():
         short = f(*leaves)
     check(short, step, ins, s, dy, dS, dt)
+
+
+def off(x):
+    """One element off a 16-byte boundary."""
+    return torch.empty(x.numel() + 1, dtype=x.dtype, device=x.device)[1:].view(x.shape).copy_(x)
+
+
+LAYOUTS = {
+    "packed": lambda x: torch.cat([x, x], dim=-1)[..., :x.shape[-1]],                 # sliced out of a wider tensor
+    "permuted": lambda x: x.transpose(1, 2).contiguous().transpose(1, 2),             # [B, H, T, ..] in memory
+    "heads": lambda x: x[:, :, :1].expand_as(x),                                      # the same for all heads, not copied
+    "times": lambda x: x[:, :1].expand_as(x),
+    "off": off,
+    "spread": lambda x: torch.stack([x, x], -1)[..., 0],                              # elements two apart
+    "plain": lambda x: x,
+}
+# which layout each input has, in turn; state: transposed in memory where "t", off a boundary where "o"
+LAYOUT_CASES = [
+    ("delta_rule", 2, 34, 2, 24, 40, ["packed", "off", "permuted", "spread"], "t"), ("gated_delta_rule", 1, 37, 3, 32, 32, ["heads", "times"], "o"),
+    ("rwkv7", 1, 33, 2, 24, 24, ["off", "packed", "heads", "spread", "permuted", "times"], ""), ("mamba2", 2, 49, 2, 16, 48, ["spread", "off"], "to"),
+    ("gla", 1, 70, 1, 128, 128, ["plain", "off", "packed", "permuted"], "t"), ("gated_delta_rule", 1, 65, 1, 128, 128, ["off"], ""),
+    ("gla", 1, 65, 1, 128, 128, ["off", "spread"], "o"), ("retention", 2, 33, 2, 32, 16, ["times", "off", "packed"], "t")]
+
+
+def layout_case(op, B, T, H, M, N, layouts, state, mixed):
+    step, ins, s, dy, dS = case(op, B, T, H, M, N, torch.bfloat16)
+    if mixed:                                                                         # bf16 and fp16 inputs in one call
+        ins = [x.half() if i % 2 else x for i, x in enumerate(ins)]
+    ins = [LAYOUTS[layouts[i % len(layouts)]](x) if x.shape[1] > 1 else x for i, x in enumerate(ins)]
+    if "t" in state:
+        s = s.mT.contiguous().mT
+    if "o" in state:
+        s = off(s) if "t" not in state else off(s.mT).mT
+    return step, ins, s, dy, dS
+
+
+@pytest.mark.parametrize("op,B,T,H,M,N,layouts,state", LAYOUT_CASES)
+def test_layouts_emulated(op, B, T, H, M, N, layouts, state):
+    from emu.emu import EmuLauncher
+    step, ins, s, dy, dS = layout_case(op, B, T, H, M, N, layouts, state, mixed=T % 2 == 0)
+    fwd, bwd, _, _ = build_twopass(step, tuple(ins), (s,), _launcher=EmuLauncher)
+    assert [ks.name for ks in fwd.sources] == ["frnn_cfw", "frnn_cbw"]
+    if N == 128:                   # one buffer of raw inputs: two do not fit beside the operands
+        assert "(c % 1)" in fwd.sources[1].source
+    y, sT, ck, aux = fwd(tuple(ins), (s,))
+    dx, ds = bwd((dy.to(y.dtype),), (dS,), tuple(ins), (ck,), (aux,))
+    check([y, sT, *dx, *ds], step, ins, s, dy, dS, torch.bfloat16)
+    check([*fwd.infer(tuple(ins), (s,))], step, ins, s, dy, dS, torch.bfloat16)
+    for g, x in zip([*dx, *ds], [*ins, s]):
+        assert g.dtype == x.dtype and g.stride() == torch.empty_like(x).stride()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("op,B,T,H,M,N,layouts,state", LAYOUT_CASES + [
+    ("delta_rule", 3, 130, 3, 128, 128, ["off", "spread", "heads", "permuted"], "to"), ("mamba2", 2, 200, 5, 64, 128, ["packed"], "t"),
+    ("rwkv7", 2, 100, 2, 128, 128, ["times", "off", "plain", "packed"], "o")])
+def test_layouts_gpu(op, B, T, H, M, N, layouts, state):
+    for mixed in (False, True):
+        step, ins, s, dy, dS = layout_case(op, B, T, H, M, N, layouts, state, mixed)
+        f = flex_rnn_b200.jit(step)
+        # .cuda() keeps strides but neither offsets nor expanded dimensions: the layouts are made on the GPU
+        base = case(op, B, T, H, M, N, torch.bfloat16)[1]
+        gi = [x.cuda().half() if mixed and i % 2 else x.cuda() for i, x in enumerate(base)]
+        gi = [LAYOUTS[layouts[i % len(layouts)]](x) if x.shape[1] > 1 else x for i, x in enumerate(gi)]
+        gs = s.cuda() if "o" not in state else off(s.cuda().mT).mT if "t" in state else off(s.cuda())
+        assert [x.stride() for x in [*gi, gs]] == [x.stride() for x in [*ins, s]]
+        leaves = [x.detach().requires_grad_() for x in [*gi, gs]]
+        for _ in range(2):
+            y, sT = f(*leaves)
+            grads = torch.autograd.grad((y, sT), leaves, (dy.cuda().to(y.dtype), dS.cuda()))
+            assert f.forward_func.kernel_status("cuda:0") == 0
+            check([y.detach(), sT.detach(), *grads], step, ins, s, dy, dS, torch.bfloat16)
+        with torch.no_grad():
+            short = f(*leaves)
+        check(short, step, ins, s, dy, dS, torch.bfloat16)
