@@ -1075,7 +1075,7 @@ def build_twopass(step, inputs, state, dryrun=False, tuning: Optional[Tuning] = 
         best, log = None, []
         for k, kw in enumerate(cplan.variants() if ctrain else backward_variants(plan)):
             try:
-                ks = bw_src if k == 0 else cplan.backward_scan(**kw) if ctrain else generate_backward(plan, **kw)
+                ks = bw_src if k == 0 else _checked(cplan.backward_scan(**kw), tu0) if ctrain else generate_backward(plan, **kw)
                 if ks is None:
                     continue
                 launcher = launch_bw if k == 0 else make(ks)
@@ -1099,7 +1099,7 @@ def build_twopass(step, inputs, state, dryrun=False, tuning: Optional[Tuning] = 
         for k, kw in enumerate(cplan.variants() if chunked else forward_variants(plan)):
             try:
                 if chunked:
-                    ks = first[0] if k == 0 else cplan.infer(**kw) if infer else cplan.forward(**kw)
+                    ks = first[0] if k == 0 else _checked(cplan.infer(**kw) if infer else cplan.forward(**kw), tu0)
                 else:
                     ks = first[0] if k == 0 else generate_forward(plan, infer=infer, **kw)
                 launcher = first[1] if k == 0 else make(ks)

@@ -105,8 +105,7 @@ def test_pinned_members():
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("k", [0, 1, 2])
-@pytest.mark.parametrize("op", ["delta_rule", "gated_delta_rule", "rwkv7", "mamba2", "gla"])
+@pytest.mark.parametrize("op,k", [("delta_rule", 1), ("delta_rule", 2), ("rwkv7", 1), ("rwkv7", 2), ("mamba2", 1), ("gla", 2)])
 def test_pinned_members_gpu(op, k):
     run_member(op, k, "cuda:0")
 
@@ -185,21 +184,47 @@ def test_layouts_emulated(op, B, T, H, M, N, layouts, state):
     ("delta_rule", 3, 130, 3, 128, 128, ["off", "spread", "heads", "permuted"], "to"), ("mamba2", 2, 200, 5, 64, 128, ["packed"], "t"),
     ("rwkv7", 2, 100, 2, 128, 128, ["times", "off", "plain", "packed"], "o")])
 def test_layouts_gpu(op, B, T, H, M, N, layouts, state):
-    for mixed in (False, True):
-        step, ins, s, dy, dS = layout_case(op, B, T, H, M, N, layouts, state, mixed)
-        f = flex_rnn_b200.jit(step)
-        # .cuda() keeps strides but neither offsets nor expanded dimensions: the layouts are made on the GPU
-        base = case(op, B, T, H, M, N, torch.bfloat16)[1]
-        gi = [x.cuda().half() if mixed and i % 2 else x.cuda() for i, x in enumerate(base)]
-        gi = [LAYOUTS[layouts[i % len(layouts)]](x) if x.shape[1] > 1 else x for i, x in enumerate(gi)]
-        gs = s.cuda() if "o" not in state else off(s.cuda().mT).mT if "t" in state else off(s.cuda())
-        assert [x.stride() for x in [*gi, gs]] == [x.stride() for x in [*ins, s]]
-        leaves = [x.detach().requires_grad_() for x in [*gi, gs]]
-        for _ in range(2):
-            y, sT = f(*leaves)
-            grads = torch.autograd.grad((y, sT), leaves, (dy.cuda().to(y.dtype), dS.cuda()))
-            assert f.forward_func.kernel_status("cuda:0") == 0
-            check([y.detach(), sT.detach(), *grads], step, ins, s, dy, dS, torch.bfloat16)
-        with torch.no_grad():
-            short = f(*leaves)
-        check(short, step, ins, s, dy, dS, torch.bfloat16)
+    mixed = T % 2 == 0
+    step, ins, s, dy, dS = layout_case(op, B, T, H, M, N, layouts, state, mixed)
+    f = flex_rnn_b200.jit(step)
+    # .cuda() keeps strides but neither offsets nor expanded dimensions: the layouts are made on the GPU
+    base = case(op, B, T, H, M, N, torch.bfloat16)[1]
+    gi = [x.cuda().half() if mixed and i % 2 else x.cuda() for i, x in enumerate(base)]
+    gi = [LAYOUTS[layouts[i % len(layouts)]](x) if x.shape[1] > 1 else x for i, x in enumerate(gi)]
+    gs = s.cuda() if "o" not in state else off(s.cuda().mT).mT if "t" in state else off(s.cuda())
+    assert [x.stride() for x in [*gi, gs]] == [x.stride() for x in [*ins, s]]
+    leaves = [x.detach().requires_grad_() for x in [*gi, gs]]
+    for _ in range(2):
+        y, sT = f(*leaves)
+        grads = torch.autograd.grad((y, sT), leaves, (dy.cuda().to(y.dtype), dS.cuda()))
+        assert f.forward_func.kernel_status("cuda:0") == 0
+        check([y.detach(), sT.detach(), *grads], step, ins, s, dy, dS, torch.bfloat16)
+    with torch.no_grad():
+        short = f(*leaves)
+    check(short, step, ins, s, dy, dS, torch.bfloat16)
+
+
+@pytest.mark.gpu
+def test_timed_candidates_are_checked_builds(monkeypatch):
+    """With the checked build asked for, no candidate of the timing on the first call is an unchecked one (nothing is
+    compiled or launched here)."""
+    from flex_rnn_b200 import twopass
+    made = []
+
+    class Launcher:
+        def __init__(self, ks):
+            self.ks = ks
+            made.append(ks)
+
+        def __call__(self, ptrs, device):
+            pass
+    monkeypatch.setattr(twopass, "_CudaLauncher", Launcher)
+    step, ins, s, dy, dS = case("delta_rule", 1, 64, 2, 64, 64, torch.bfloat16)
+    ins, s = tuple(x.cuda() for x in ins), s.cuda()
+    tu = dataclasses.replace(default_tuning(1, 64, 2, 64, 64, 1), bounds=1, autotune_min_work=0)
+    fwd, bwd, _, _ = build_twopass(step, ins, (s,), tuning=tu)
+    y, sT, ck, aux = fwd(ins, (s,))
+    bwd((dy.cuda().to(y),), (dS.cuda().to(sT),), ins, (ck,), (aux,))
+    fwd.infer(ins, (s,))
+    assert [sum(ks.name == n for ks in made) for n in ("frnn_cfw", "frnn_cbw", "frnn_cvg")] == [6, 3, 1]
+    assert all(ks.info.get("bounds") for ks in made)
