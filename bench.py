@@ -16,8 +16,10 @@ Printed JSON (rank 0), one line:
   value / ms_per_step   tokens/s of the whole job with inputs resident in HBM
   e2e                   the same through the public API with pinned host buffers
                         and host<->device copies in the timed region
-  roofline              the dominant kernel (the backward scan): bound = FP32
-                        CUDA-core pipe, peak measured in-run by an FMA-only probe
+  roofline              the backward kernels.  Recurrent ones: bound = FP32 CUDA-core
+                        pipe, peak measured in-run by an FMA-only probe.  Chunked ones
+                        (tensor cores): compulsory bytes at the copy rate or the busy
+                        time of the tensor cores, whichever is longer
   cpu_baseline          the reference's CPU path (its jit.naive + autograd) on a
                         bounded sample, on the host cores (one GPU only)
   workloads             (one GPU) the other benchmark configurations - RWKV-7,
@@ -38,6 +40,7 @@ importable from `baseline/_ref` (kind "reference"), else the restatement in
 """
 import argparse
 import json
+import math
 import os
 import statistics
 import subprocess
@@ -309,6 +312,11 @@ class Bench:
             pass
         self.hbm = self.peaks.get("hbm_gbs", 6650.0)
         self.fp32_peak = None
+        try:
+            self.sm_ghz = float(subprocess.run(["nvidia-smi", "--query-gpu=clocks.max.sm", "--format=csv,noheader,nounits", "-i", str(local)],
+                                               capture_output=True, text=True, timeout=60).stdout.strip().splitlines()[0]) / 1e3
+        except Exception:
+            self.sm_ghz = 1.965
 
     def sync_all(self):
         self.torch.cuda.synchronize(self.dev)
@@ -416,27 +424,49 @@ class Bench:
         # bwd reads inputs + dy + dS_T, writes the gradients + dS0
         bytes_fw_alg = in_bytes + st_bytes + y_bytes + st_bytes
         bytes_bw_alg = in_bytes + y_bytes + st_bytes + in_bytes + st_bytes
-        # what the backward launch actually moves, from the plan: plus saved row sums and fp32 checkpoints read
-        aux_bytes = len(plan.aux) * B * H * T * M * 4
-        chunk = m["op"].forward_func.chunk
-        nck = -(-T // chunk) if chunk else plan.nck
-        ck_bytes = nck * B * H * M * N * 4 * plan.n_st
-        traffic_bw = bytes_bw_alg + aux_bytes + ck_bytes
-        if chunk:       # the second backward kernel reads inputs, dy and row sums again, and the state gradients of the first
-            traffic_bw += in_bytes + y_bytes + 2 * aux_bytes + 2 * ck_bytes
+        # what the launches actually move, from the plan: plus saved row sums and fp32 checkpoints
+        fwd = m["op"].forward_func
+        chunk = fwd.chunk
+        numel = lambda shape: math.prod(shape) * 4
+        if chunk:
+            store, aux = m["op"].fw_meta[-2:]
+            ck_bytes, aux_bytes = numel(store[0]), numel(aux[0])
+            # the scan of the state gradient writes those gradients at the chunks' boundaries and its kept row sums; the second
+            # kernel reads inputs, dy, row sums, checkpoints and what the scan wrote
+            temps = sum(numel(shape) for _, shape in fwd.chunk_temps)
+            traffic_bw = bytes_bw_alg + 2 * aux_bytes + ck_bytes + 2 * temps + in_bytes + y_bytes
+        else:
+            aux_bytes = len(plan.aux) * B * H * T * M * 4
+            ck_bytes = plan.nck * B * H * M * N * 4 * plan.n_st
+            traffic_bw = bytes_bw_alg + aux_bytes + ck_bytes
         traffic_fw = bytes_fw_alg + aux_bytes + ck_bytes
         fw_avg, bw_avg = statistics.mean(m["fw_ms"]), statistics.mean(m["bw_ms"])
         k_bw = plan.k_joint - plan.k_fwd
         peak = self.fp32_peak
+        step_s = m["ms_per_step"] * 1e-3
         t_fp32 = elems * plan.k_joint / (peak * 1e12)
         t_hbm = (bytes_fw_alg + bytes_bw_alg) / (self.hbm * 1e9)
-        step_s = m["ms_per_step"] * 1e-3
+        if chunk:
+            # the FP32 pipe does not bound tensor-core kernels: the compulsory bytes do, or the cycles that the tensor cores
+            # are busy with the kernels' products (all CTAs spread evenly over the SMs)
+            busy = lambda ks: ks.info["tensor_cycles"] * math.prod(ks.grid) / self.sms / (self.sm_ghz * 1e9)
+            t_mma_fw, t_mma_bw = busy(fw_src), busy(bw_src) + busy(fwd.vector_grads)
+            bound_fw = max(bytes_fw_alg / (self.hbm * 1e9), t_mma_fw)
+            bound_bw = max(bytes_bw_alg / (self.hbm * 1e9), t_mma_bw)
+            bound = "tensor" if t_mma_bw > bytes_bw_alg / (self.hbm * 1e9) else "hbm"
+        else:
+            bound_fw, bound_bw = elems * plan.k_fwd / (peak * 1e12), elems * k_bw / (peak * 1e12)
+            bound = "fp32"
+        bound_step = bound_fw + bound_bw if chunk else max(t_fp32, t_hbm)
         rec = {
             "fw_ms": round(fw_avg, 4), "bw_ms": round(bw_avg, 4), "ms_per_step": round(m["ms_per_step"], 4),
             "tokens_per_s": self.world * B * T / step_s,
-            "roofline_fraction_step": max(t_fp32, t_hbm) / step_s,
-            "roofline_fraction_fw": elems * plan.k_fwd / (fw_avg * 1e-3) / 1e12 / peak,
-            "roofline_fraction_bw": elems * k_bw / (bw_avg * 1e-3) / 1e12 / peak,
+            "bound": bound,
+            "roofline_fraction_step": bound_step / step_s,
+            "roofline_fraction_fw": bound_fw / (fw_avg * 1e-3),
+            "roofline_fraction_bw": bound_bw / (bw_avg * 1e-3),
+            "traffic_fraction_of_hbm_fw": traffic_fw / (self.hbm * 1e9) / (fw_avg * 1e-3),
+            "traffic_fraction_of_hbm_bw": traffic_bw / (self.hbm * 1e9) / (bw_avg * 1e-3),
             "k_joint": plan.k_joint, "k_fwd": plan.k_fwd,
             "fp32_bound_ms": t_fp32 * 1e3, "hbm_bound_ms": t_hbm * 1e3,
             "peak_memory_gib": round(m["peak_memory_gib"], 3),
@@ -450,16 +480,19 @@ class Bench:
                           "variant": tuned["bw_choice"], "timed_variants": len(tuned["bw_log"])},
         }
         kref = K_JOINT_REFERENCE_TRACER.get(opname)
-        if kref and kref != plan.k_joint:
+        if chunk:
+            rec["tensor_bound_ms"] = (t_mma_fw + t_mma_bw) * 1e3
+        if kref and kref != plan.k_joint and not chunk:
             rec["roofline_fraction_step_reference_tracer_k"] = elems * kref / (peak * 1e12) / step_s
             rec["k_joint_reference_tracer"] = kref
         units = B * H * (M // bw_src.info["tile"][2])
-        per_wave = self.sms * max(1, plan.tuning.bw_min_blocks)
+        per_wave = self.sms * (1 if chunk else max(1, plan.tuning.bw_min_blocks))
         issued = (plan.k_joint - plan.k_fwd) / 2 + (plan.n_st if plan.reverse else 0)
         extra = {"counted_per_issued": ((plan.k_joint - plan.k_fwd) / 2) / issued if plan.reverse and not chunk else None,
                  "sm_fill": units / (-(-units // per_wave) * per_wave),
                  "bytes_fw_alg": bytes_fw_alg, "bytes_bw_alg": bytes_bw_alg, "traffic_bw": traffic_bw, "traffic_fw": traffic_fw,
                  "achieved_bw": elems * k_bw / (bw_avg * 1e-3) / 1e12, "flops_bw": elems * k_bw, "bw_name": "frnn_cbw + frnn_cvg" if chunk else bw_src.name, "chunk": chunk,
+                 "bound": bound, "t_mma_bw": t_mma_bw if chunk else None, "bw_s": bw_avg * 1e-3,
                  "stream_mb": (traffic_fw + traffic_bw) / 1e6}
         return rec, extra
 
@@ -551,6 +584,20 @@ class Bench:
         return rec
 
 
+def roofline_head(bench, extra):
+    """The bound of the backward kernels and what they reach of it: the FP32 pipe for the recurrent ones; for the chunked
+    ones the compulsory bytes or the busy time of the tensor cores, whichever is longer."""
+    head = {"bound": extra["bound"], "kernel": extra["bw_name"]}
+    if extra["bound"] == "fp32":
+        return {**head, "achieved": extra["achieved_bw"], "peak": bench.fp32_peak, "unit": "TFLOP/s",
+                "frac": extra["achieved_bw"] / bench.fp32_peak}
+    if extra["bound"] == "tensor":
+        return {**head, "achieved": extra["t_mma_bw"] * 1e3, "peak": extra["bw_s"] * 1e3, "unit": "ms busy of ms",
+                "frac": extra["t_mma_bw"] / extra["bw_s"]}
+    rate = extra["bytes_bw_alg"] / extra["bw_s"] / 1e9
+    return {**head, "achieved": rate, "peak": bench.hbm, "unit": "GB/s", "frac": rate / bench.hbm}
+
+
 def run_ours(args, rank, world, local):
     import torch
     from flex_rnn_b200 import workloads as W
@@ -606,13 +653,14 @@ def run_ours(args, rank, world, local):
             "roofline_fraction_step": rec["roofline_fraction_step"],
             "roofline_fraction_fw": rec["roofline_fraction_fw"],
             "peak_memory_gib": rec["peak_memory_gib"],
-            "roofline": {"bound": "fp32", "kernel": extra["bw_name"], "achieved": extra["achieved_bw"], "peak": bench.fp32_peak,
-                         "unit": "TFLOP/s", "frac": extra["achieved_bw"] / bench.fp32_peak,
+            "roofline": {**roofline_head(bench, extra),
                          "traffic": extra["traffic_bw"],
                          "traffic_source": "computed from the plan (inputs, dy, dS_T, saved row sums and fp32 checkpoints read; "
                                            "gradients and dS0 written)",
                          "algorithmic_bytes": extra["bytes_bw_alg"],
-                         "peak_source": f"measured in this run by the FMA probe kernel ({bench.sms} SMs); HBM copy peak {bench.hbm} GB/s "
+                         "peak_source": (f"measured in this run by the FMA probe kernel ({bench.sms} SMs); " if extra["bound"] == "fp32" else
+                                         "busy cycles of the tensor cores: 46 per product of 128x8 with up to 64 columns, 65 with 128 "
+                                         "(measured); " if extra["bound"] == "tensor" else "") + f"HBM copy peak {bench.hbm} GB/s "
                                         + ("of measured" if bench.peaks else "of fallback"),
                          "flops_per_launch": extra["flops_bw"], "k_joint": rec["k_joint"], "k_fwd": rec["k_fwd"],
                          "hbm_bound_ms": rec["hbm_bound_ms"], "fp32_bound_ms": rec["fp32_bound_ms"],

@@ -1248,8 +1248,11 @@ def emit_scan(p: Problem, s: ScanSpec, C: int, MB: int, use_tma: bool = True, st
     w(f"frnn_tmem_dealloc(tm, {tm_cols}u);")
     w.close()
     w.close()
+    # cycles the tensor cores are busy for one CTA: products 1 (the state and its rest), Gram, products 2, per chunk
+    busy = nchunk * (2 * (N // 8) * product_cycles(RA) + (N // 8) * (1 if xa else 2) * product_cycles(RK)
+                     + len(passes) * (nK // 8) * product_cycles(Np))
     return KernelSource(s.name, w.text().replace("@SMEM_BYTES@", str(smem_bytes)), (p.M // MB, p.H, p.B), 128 + PT + 128, smem_bytes,
-                        kb.params, kb.param_decl, {"chunk": C, "tile": [1, N, MB], "packed": False, "tmem_cols": tm_cols, "nck": nck,
+                        kb.params, kb.param_decl, {"chunk": C, "tile": [1, N, MB], "packed": False, "tmem_cols": tm_cols, "nck": nck, "tensor_cycles": busy,
                                                    "tma_items": len(kb.tma_items), "plain_items": len(kb.plain_items)}, kb.tmaps)
 
 
@@ -1260,6 +1263,12 @@ CHUNK = 16
 def ck_bytes(p: Problem, C: int) -> int:
     """Bytes of the fp32 states at the starts of chunks of C timesteps."""
     return p.B * p.H * ((p.T + C - 1) // C) * p.N * p.M * 4
+
+
+def product_cycles(n: int) -> float:
+    """Cycles of one tf32 product of 128 rows, 8 values of k and ``n`` columns (measured on a B200, one issuing thread: 46 up
+    to 64 columns, 65 with 128; between and beyond in proportion)."""
+    return 46.0 + max(0, n - 64) * 19.0 / 64.0
 
 
 def rows_per_cta(M: int) -> Optional[int]:
@@ -2165,8 +2174,11 @@ def emit_vector_grads(p: Problem, nf: Normal, bp: BackwardPlan, dspec: Sequence[
         w.close()
     w("(void)ok;")
     w.close()
+    # cycles the tensor cores are busy for one CTA: L, the slices of S_0 and E_C (each in two terms), what follows from L
+    busy = M // 8 * (product_cycles(2 * nK) + 2 * product_cycles(2 * nA) + 2 * product_cycles(2 * nK)) + \
+        2 * (nK // 8) * product_cycles(2 * nA) + 2 * (nA // 8) * product_cycles(2 * nK)
     return KernelSource("frnn_cvg", w.text().replace("@SMEM_BYTES@", str(smem_bytes)), (nchunk, H, B), VG_THREADS, smem_bytes, params, decl,
-                        {"chunk": C, "tile": [1, N, M], "packed": False, "tmem_cols": tm_cols}, [])
+                        {"chunk": C, "tile": [1, N, M], "packed": False, "tmem_cols": tm_cols, "tensor_cycles": busy}, [])
 
 
 def emit_slow_columns(w, C, nd, nr, nA, nK, tq, live_n, sel, nf, bp, dec_vec, want_gw, Stage, leaf, leaves_of, slot, LS, cD1, cD2, off_slow):

@@ -960,7 +960,8 @@ def build_twopass(step, inputs, state, dryrun=False, tuning: Optional[Tuning] = 
     make = _launcher or _CudaLauncher
     if ctrain:
         fw_src, bw_src = _checked(cplan.forward(**member), tu0), _checked(cplan.backward_scan(**member), tu0)
-        launch_vg = make(_checked(cplan.vector_grads(), tu0))
+        vg_src = _checked(cplan.vector_grads(), tu0)
+        launch_vg = make(vg_src)
     launch_fw, launch_bw = make(fw_src), make(bw_src)
 
     in_meta = tuple(th.empty_strided(x.shape, x.stride(), dtype=x.dtype, device="meta") for x in inputs)
@@ -1307,6 +1308,8 @@ def build_twopass(step, inputs, state, dryrun=False, tuning: Optional[Tuning] = 
     forward.plan = plan                     # type: ignore[attr-defined]
     forward.infer = infer                   # type: ignore[attr-defined]
     forward.chunk = cplan.C if ctrain else 0   # type: ignore[attr-defined]  (timesteps per chunk; 0: recurrent kernels)
+    forward.vector_grads = vg_src if ctrain else None   # type: ignore[attr-defined]  (the second backward kernel of the chunked form)
+    forward.chunk_temps = chunk_temps       # type: ignore[attr-defined]  (its scratch: names and shapes)
     forward.host_program = host_program     # type: ignore[attr-defined]
     forward.host_checks = host_checks       # type: ignore[attr-defined]
     forward.sources = (fw_src, bw_src)      # type: ignore[attr-defined]
