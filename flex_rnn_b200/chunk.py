@@ -683,7 +683,9 @@ def emit_scan(p: Problem, s: ScanSpec, C: int, MB: int, use_tma: bool = True, st
 
     # ------------------------------------------------------------------ preparing warps
     # registers: 512 threads start with 128 each; the state's rows need more, the others less (state, preparing twice, products:
-    # 4 x 128 together).  64 values of kappa per preparing thread spill at 104.
+    # 4 x 128 together).  A preparing thread holds nK values of kappa.  With 64 of them either split spills 10 to 100 bytes and
+    # they measure alike (backward of 256 heads T512, 128x128: Delta Rule 653 us both, Gated Delta 797 against 794 us); with 32
+    # the second is the better one (RWKV-7 forward, 128x64: 365 against 382 us) or equal within 1 %.
     regs = (192, 112, 96) if nK >= 64 else (200, 104, 104)
     w("auto work = [&]() -> void {")
     w.ind += 1
@@ -1004,8 +1006,12 @@ def emit_scan(p: Problem, s: ScanSpec, C: int, MB: int, use_tma: bool = True, st
         w(f"const u64 {nm} = frnn_mma_desc(smem + {off}, {lbo});")
     w(f"const u64 dKlo = frnn_mma_desc(smem + {off_ka + (0 if xk else ka_bytes)}, {lboK}), dA1 = frnn_mma_desc(smem + {off_al + al_bytes}, {lboA}); (void)dKlo;")
 
-    # Gram of large states in four pieces, so that products the state threads wait for never queue behind all of it (RWKV-7
-    # 128x128: 795 against 785 us; with 64 columns the whole takes no longer than such a wait, and pieces cost 8 %)
+    # Gram in pieces, so that products the state threads wait for never queue behind all of it.  256 heads T512, 128 rows,
+    # forward + backward, in one piece and in four, us: 128 columns Mamba-2 230 + 681 and 203 + 651, GLA 248 + 608 and 240 + 601,
+    # Delta Rule 17 % and 12 % less in four (two measure like four); 64 columns Mamba-2 177 + 570 and 175 + 566, GLA 213 + 517
+    # and 213 + 522, Gated Delta alike, Delta Rule 10 % and 3 % less in four.  80 to 112 columns divide into two pieces (72, 104
+    # and 120 do not), which this rule does not use although they measured faster: Mamba-2 with 96 columns 197 + 608 and
+    # 193 + 604, GLA 235 + 573 and 227 + 559, the Delta families' backward 12 to 22 %.
     pieces = 4 if N == 128 else 1
 
     def gram_piece(c: str, g: str):
@@ -2283,9 +2289,12 @@ class ChunkPlan:
         return emit_scan(p, forward_spec(p, self.nf, self.bp.saved, True, self.C), self.C, rows_per_cta(p.M), **kw)
 
     def infer(self, **kw) -> KernelSource:
-        """Without checkpoints a chunk may be longer: its chain costs about 3000 cycles whatever its length and the
-        substitution 5 nd nr C^2 (B8 T1024 H32 128x128 Delta Rule: 463 us with 16 steps, 379 us with 32; RWKV-7 with its
-        four pairs of vectors: 517 us against 611 us)."""
+        """Without checkpoints a chunk may be longer, which pays as long as its time less than doubles.  The chain of a chunk
+        takes a part that does not depend on its length (3000 to 7000 cycles, by the state's size) and a substitution of
+        2.4 to 3.8 cycles nd nr C^2.  Measured cycles a chunk with 16 and with 32 steps, one CTA per SM: Delta Rule (two pairs
+        of vectors) 128x128 6260 and 9970, 64x64 4440 and 8630, 32x32 3640 and 7550 (4 % slower); Mamba-2 (one pair) 128x128
+        7380 and 9550, 64x64 6130 and 7730; GLA (one pair) 128x128 7300 and 10510; RWKV-7 (four pairs) 64x64 7500 and
+        19200.  At 64 timesteps, two chunks, 22.0 and 20.0 us for the Delta Rule with 128x128."""
         p = self.problem
         if len(self.nf.alphas) * len(self.nf.kappas) <= 2 and p.T >= 4 * CHUNK:
             try:
