@@ -103,6 +103,8 @@ FRNN_DEV void frnn_group_sync(int id, int nthreads) {
 }
 FRNN_DEV float frnn_shfl_xor(float v, int off) { return __shfl_xor_sync(0xffffffffu, v, off); }
 FRNN_DEV void frnn_block_sync() { __syncthreads(); }
+// block barrier with a vote: whether `v` holds in every thread of the CTA
+FRNN_DEV bool frnn_block_and(bool v) { return __syncthreads_and(v); }
 FRNN_DEV void frnn_warp_sync() { __syncwarp(); }
 FRNN_DEV void frnn_atomic_add(float* p, float v) { atomicAdd(p, v); }
 // the error word may live in pinned host memory: a plain store reaches it (the first report is kept when it can be)

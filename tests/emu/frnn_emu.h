@@ -48,6 +48,7 @@ struct emu_cta {
     unsigned char* smem;
     size_t smem_bytes = 0;
     std::mutex mtx;
+    std::atomic<int> against{0};      // votes of frnn_block_and
 };
 static thread_local emu_dim3 threadIdx, blockIdx;
 static thread_local emu_cta* emu_ctx = nullptr;
@@ -227,6 +228,15 @@ FRNN_DEV int frnn_smem_add(int* p, int v) { std::lock_guard<std::mutex> g(emu_at
 template <int N> FRNN_DEV void frnn_regs_release() {}
 template <int N> FRNN_DEV void frnn_regs_acquire() {}
 FRNN_DEV void frnn_block_sync() { emu_ctx->block_bar->arrive_and_wait(); }
+FRNN_DEV bool frnn_block_and(bool v) {
+    if (!v) emu_ctx->against++;
+    frnn_block_sync();
+    const bool all = emu_ctx->against == 0;
+    frnn_block_sync();
+    if (!v) emu_ctx->against--;
+    frnn_block_sync();
+    return all;
+}
 FRNN_DEV void frnn_group_sync(int id, int nthreads) {
     emu_cta* c = emu_ctx;
     {
