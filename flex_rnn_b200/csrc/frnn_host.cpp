@@ -147,6 +147,8 @@ struct Spec : std::enable_shared_from_this<Spec> {
     int* err = nullptr;                  // the device's error word, in pinned host memory
     std::vector<char> aligned;           // argument i was 16-byte aligned at compilation
     std::vector<int64_t> reach;          // bytes from argument i's first element to the end of its last one
+    // of the results and of what a forward saves (the arguments first), the same for every call; filled by the first one
+    std::vector<Meta> result_meta, saved_meta;
     std::atomic<const Program*> forward{nullptr}, infer{nullptr}, backward{nullptr};   // set once, by a Python closure's first run
     py::object py_forward, py_infer, py_backward;    // (spec, args) -> results and saved; (spec, args) -> results; (spec, grads, args, saved, whether the custom op is not needed) -> gradients
     ~Spec() {
@@ -235,8 +237,6 @@ bool wrapped(const Tensor& t) {
 struct RecurrenceBackward : torch::autograd::Node {
     std::shared_ptr<Spec> spec;
     std::vector<torch::autograd::SavedVariable> saved;   // the arguments, then what the forward saved
-    std::vector<Meta> saved_meta;                         // what was saved, to be read back the same
-    std::vector<Meta> grad_meta;                          // of the results: absent upstream gradients are zeros
 
     explicit RecurrenceBackward(torch::autograd::edge_list&& e) : Node(std::move(e)) {}
     std::string name() const override { return "RecurrenceBackward"; }
@@ -258,7 +258,7 @@ struct RecurrenceBackward : torch::autograd::Node {
         c10::cuda::CUDAGuard guard(s.device);
         const c10::Device dev(c10::kCUDA, s.device);
         for (size_t i = 0; i < up.size(); i++) {
-            const Meta& m = grad_meta[i];
+            const Meta& m = s.result_meta[i];      // absent upstream gradients are zeros
             if (!up[i].defined()) {
                 up[i] = at::detail::empty_cuda(m.sizes, at::TensorOptions().dtype(m.dtype).device(dev)).zero_();
             } else {
@@ -272,11 +272,11 @@ struct RecurrenceBackward : torch::autograd::Node {
         for (const Tensor& t : up) direct = direct && !wrapped(t);
         for (const Tensor& t : kept) direct = direct && t.defined() && !wrapped(t);
         if (direct)
-            for (size_t i = 0; i < kept.size(); i++) kept[i] = as_saved(kept[i], saved_meta[i], dev, i >= (size_t)narg || s.aligned[i]);
+            for (size_t i = 0; i < kept.size(); i++) kept[i] = as_saved(kept[i], s.saved_meta[i], dev, i >= (size_t)narg || s.aligned[i]);
         const Program* p = s.backward.load(std::memory_order_acquire);
         bool ok = p && direct && s.args_ok(kept, s.nin);
         for (const Tensor& t : up) ok = ok && t.device() == dev && !((uintptr_t)t.data_ptr() & 15);
-        for (size_t i = 0; i < up.size() && ok; i++) ok = up[i].scalar_type() == grad_meta[i].dtype;
+        for (size_t i = 0; i < up.size() && ok; i++) ok = up[i].scalar_type() == s.result_meta[i].dtype;
         variable_list g;
         if (!ok) {
             g = with_python([&] {
@@ -365,17 +365,14 @@ struct HostOp {
                 res = run_forward(*s, a);
             }
             node->spec = s;
-            auto save = [&](const Tensor& t) {
-                node->saved.emplace_back(t, false);
-                node->saved_meta.push_back(meta_of(t));
-            };
-            for (const Tensor& t : a) save(t);
-            for (size_t i = nres; i < res.size(); i++) save(res[i]);
-            res.resize(nres);
-            for (Tensor& t : res) {
-                node->grad_meta.push_back(meta_of(t));
-                torch::autograd::create_gradient_edge(t, node);
+            if (s->result_meta.empty()) {           // (no saving hook has run yet: the interpreter lock is held throughout)
+                for (const Tensor& t : a) s->saved_meta.push_back(meta_of(t));
+                for (size_t i = 0; i < res.size(); i++) (i < nres ? s->result_meta : s->saved_meta).push_back(meta_of(res[i]));
             }
+            for (const Tensor& t : a) node->saved.emplace_back(t, false);
+            for (size_t i = nres; i < res.size(); i++) node->saved.emplace_back(res[i], false);
+            res.resize(nres);
+            for (Tensor& t : res) torch::autograd::create_gradient_edge(t, node);
         }
         py::tuple out(res.size());
         for (size_t i = 0; i < res.size(); i++) out[i] = py::reinterpret_steal<py::object>(THPVariable_Wrap(res[i]));
