@@ -548,8 +548,7 @@ def emit_scan(p: Problem, s: ScanSpec, C: int, MB: int, use_tma: bool = True, st
     term.  Gram needs the ratios W_j-1/W_i: as kappa/W_i where no W of the chunk is tiny, else (a reset, an extreme
     decay) as running products, by a slower path for that chunk alone.
 
-    The chain of one chunk - products 1, substitution, products 2, state - bounds the kernel; a product of up to 64
-    columns takes 46 cycles whatever its width, so hi and rest of alpha share one.
+    The chain of one chunk - products 1, substitution, products 2, state - bounds the kernel.
     """
     import types
     from .lower import Body
@@ -1000,7 +999,7 @@ def emit_scan(p: Problem, s: ScanSpec, C: int, MB: int, use_tma: bool = True, st
 
     # ------------------------------------------------------------------ the warp that issues the products
     w.open(f"if (tid >= {128 + PT} && tid < {128 + PT + 32})")
-    w("if (lane) return;")
+    w("if (!frnn_elect()) return;")
 
     for nm, off, lbo in (("dA", off_al, lboA), ("dH", off_kh, lboH), ("dK", off_ka, lboK)):
         w(f"const u64 {nm} = frnn_mma_desc(smem + {off}, {lbo});")
@@ -1255,7 +1254,7 @@ def emit_scan(p: Problem, s: ScanSpec, C: int, MB: int, use_tma: bool = True, st
     w.close()
     w.close()
     # cycles the tensor cores are busy for one CTA: products 1 (the state and its rest), Gram, products 2, per chunk
-    busy = nchunk * (2 * (N // 8) * product_cycles(RA) + (N // 8) * (1 if xa else 2) * product_cycles(RK)
+    busy = nchunk * (2 * (N // 8) * product_cycles(RA) + (N // 8) * (1 if xa else 2) * product_cycles(RK, True)
                      + len(passes) * (nK // 8) * product_cycles(Np))
     return KernelSource(s.name, w.text().replace("@SMEM_BYTES@", str(smem_bytes)), (p.M // MB, p.H, p.B), 128 + PT + 128, smem_bytes,
                         kb.params, kb.param_decl, {"chunk": C, "tile": [1, N, MB], "packed": False, "tmem_cols": tm_cols, "nck": nck, "tensor_cycles": busy,
@@ -1271,10 +1270,10 @@ def ck_bytes(p: Problem, C: int) -> int:
     return p.B * p.H * ((p.T + C - 1) // C) * p.N * p.M * 4
 
 
-def product_cycles(n: int) -> float:
-    """Cycles of one tf32 product of 128 rows, 8 values of k and ``n`` columns (measured on a B200, one issuing thread: 46 up
-    to 64 columns, 65 with 128; between and beyond in proportion)."""
-    return 46.0 + max(0, n - 64) * 19.0 / 64.0
+def product_cycles(n: int, smem: bool = False) -> float:
+    """Cycles of one tf32 product of 128 rows, 8 values of k and ``n`` columns (measured on a B200, see csrc/frnn_chunk.cuh),
+    its first operand in Tensor Memory or in shared memory."""
+    return max(10.0, n / 2, max(39.5, 32 + n / 4) if smem else 0.0)
 
 
 def rows_per_cta(M: int) -> Optional[int]:
@@ -1826,7 +1825,7 @@ def emit_vector_grads(p: Problem, nf: Normal, bp: BackwardPlan, dspec: Sequence[
     w("frnn_async_proxy_fence();")
     w("frnn_block_sync();")
     w(f"const u64 dX = frnn_mma_desc(smem + {off_X}, {lboX}), dZ = frnn_mma_desc(smem + {off_Z}, {lboZ});")
-    w.open("if (tid == 0)")
+    w.open("if (warp == 0 && frnn_elect())")
     w("#pragma unroll")
     w(f"for (int k = 0; k < {M // 8}; k++) frnn_mma_ss_d(tm + {cL}u, frnn_mma_next(dX, {lboX}, k), frnn_mma_next(dZ, {lboZ}, k), FRNN_MMA_IDESC({2 * nK}), k > 0);")
     w("frnn_mma_commit(&bar[0]);")
@@ -1875,7 +1874,7 @@ def emit_vector_grads(p: Problem, nf: Normal, bp: BackwardPlan, dspec: Sequence[
         w("}")
         w("frnn_async_proxy_fence();")
         w("if (!frnn_block_and(arrived)) break;")
-        w.open("if (tid == 0)")
+        w.open("if (warp == 0 && frnn_elect())")
         for k in range(MS // 8):
             for which, (col_, dsc, lbo, n2) in enumerate(((cD1, "dX", lboX, nA), (cD2, "dZ", lboZ, nK))):
                 sb = off_b + 2 * which * sl_bytes + k * 2 * lboS
@@ -2070,7 +2069,8 @@ def emit_vector_grads(p: Problem, nf: Normal, bp: BackwardPlan, dspec: Sequence[
         w.close()
     w("frnn_async_proxy_fence(); frnn_tmem_fence_before_sync();")
     w("frnn_block_sync();")
-    w.open("if (tid == 0 && ok)" if not dec_vec else "if (tid == 0 && ok && !slow)")
+    w.open("if (warp == 0 && frnn_elect())")
+    w.open("if (ok)" if not dec_vec else "if (ok && !slow)")
     w("frnn_tmem_fence_after_sync();")
     for (cd, offA, tb, nk, offB, lboB, n2) in ((cD1, off_kT, kT_b, nK, off_L1, lbo1, nA), (cD2, off_aT, aT_b, nA, off_L2, lbo2, nK)):
         for part_, n_ in ((offA, 2 * n2), (offA + tb, 2 * n2)):
@@ -2078,7 +2078,8 @@ def emit_vector_grads(p: Problem, nf: Normal, bp: BackwardPlan, dspec: Sequence[
             w("#pragma unroll")
             w(f"for (int k = 0; k < {nk // 8}; k++) frnn_mma_ss_d(tm + {cd}u, frnn_mma_next(da, {lboT}, k), frnn_mma_next(db, {lboB}, k), FRNN_MMA_IDESC({n_}), true); }}")
     w.close()
-    w("if (tid == 0) frnn_mma_commit(&bar[2]);")
+    w("frnn_mma_commit(&bar[2]);")
+    w.close()
     w(f"ok = frnn_mbar_wait(&bar[2], 0, err, {ERR}) && ok;")
     w("frnn_tmem_fence_after_sync();")
     # ---- columns: this thread's half of the timesteps
@@ -2182,8 +2183,8 @@ def emit_vector_grads(p: Problem, nf: Normal, bp: BackwardPlan, dspec: Sequence[
     w("(void)ok;")
     w.close()
     # cycles the tensor cores are busy for one CTA: L, the slices of S_0 and E_C (each in two terms), what follows from L
-    busy = M // 8 * (product_cycles(2 * nK) + 2 * product_cycles(2 * nA) + 2 * product_cycles(2 * nK)) + \
-        2 * (nK // 8) * product_cycles(2 * nA) + 2 * (nA // 8) * product_cycles(2 * nK)
+    pa, pk = product_cycles(2 * nA, True), product_cycles(2 * nK, True)
+    busy = M // 8 * (pk + 2 * pa + 2 * pk) + 2 * (nK // 8) * pa + 2 * (nA // 8) * pk
     return KernelSource("frnn_cvg", w.text().replace("@SMEM_BYTES@", str(smem_bytes)), (nchunk, H, B), VG_THREADS, smem_bytes, params, decl,
                         {"chunk": C, "tile": [1, N, M], "packed": False, "tmem_cols": tm_cols, "tensor_cycles": busy}, [])
 

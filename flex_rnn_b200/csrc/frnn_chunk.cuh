@@ -4,8 +4,9 @@
 // Shared-memory operands are K-major without swizzle: 8 x 4-element (128-byte) core matrices, element (row, k) at
 // (k / 4) * lbo + (row / 8) * 128 + (row % 8) * 16 + (k % 4) * 4 bytes; lbo is free, and padding it by 16 bytes makes
 // the producers' stores free of bank conflicts.  A product covers 8 values of k; M is 128 rows (the lanes of Tensor
-// Memory), N a multiple of 16.  Measured on a B200: 46 cycles per product up to N = 64, 65 at N = 128; operands are
-// truncated to tf32 (their low 13 bits are ignored), which the two-term splits below rely on.
+// Memory), N a multiple of 16.  Measured on a B200, cycles per product in a row: first operand in Tensor Memory N / 2
+// (N = 16: 10), in shared memory 40 up to N = 32, 48 at 64, 64 at 128 (its 4 KB and the other's 32 N bytes at 128 bytes a
+// cycle); operands are truncated to tf32 (their low 13 bits are ignored), which the two-term splits below rely on.
 #ifndef FRNN_EMU
 FRNN_DEV u32 frnn_f32_bits(float x) { return __float_as_uint(x); }
 FRNN_DEV float frnn_bits_f32(u32 x) { return __uint_as_float(x); }
@@ -17,8 +18,7 @@ FRNN_DEV u64 frnn_mma_desc(const void* smem, u32 lbo) {
 #define FRNN_MMA_IDESC(n) ((1u << 4) | (2u << 7) | (2u << 10) | (((u32)(n) >> 3) << 17) | ((128u >> 4) << 24))
 // d[128 x n] (+)= a[128 x 8] b[n x 8]^T, a in Tensor Memory (ts) or in shared memory (ss), shared-memory operands given by
 // their descriptors: consecutive k steps of an operand are 2 * lbo bytes apart, so that a loop adds a constant instead of
-// building each descriptor (one thread issues all products of a CTA; 85 cycles per product with the descriptor built
-// each time, which is more than the product takes).
+// building each descriptor (one thread issues all products of a CTA).
 FRNN_DEV u64 frnn_mma_next(u64 desc, u32 lbo, int k) { return desc + (u64)((u32)k * (2u * lbo >> 4)); }
 FRNN_DEV void frnn_mma_ts_d(u32 d, u32 a, u64 b, u32 idesc, bool accumulate) {
     asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
@@ -31,6 +31,14 @@ FRNN_DEV void frnn_mma_ss_d(u32 d, u64 a, u64 b, u32 idesc, bool accumulate) {
 // arrive on `bar` once every product this thread has issued so far is complete
 FRNN_DEV void frnn_mma_commit(u64* bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(frnn_smem_addr(bar)) : "memory");
+}
+// One thread of a whole warp, the same in every call.  The products are issued inside `if (frnn_elect())`: the compiler knows
+// from elect.sync that one thread runs there and keeps descriptors and addresses in uniform registers; inside `if (lane == 0)`
+// it moves them there for every product, one lane at a time, which takes 45 cycles whatever the product's width.
+FRNN_DEV bool frnn_elect() {
+    u32 r;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(r));
+    return r != 0;
 }
 FRNN_DEV void frnn_half_warp_sync() { __syncwarp(0xffffu); }      // the first 16 lanes of a warp
 #endif

@@ -223,6 +223,7 @@ FRNN_DEV void frnn_mma_ts_d(u32 d, u32 a, u64 b, u32 n, bool acc) {
 FRNN_DEV void frnn_mma_ss_d(u32 d, u64 a, u64 b, u32 n, bool acc) {
     emu_mma(d, [=](int m, int k) { return emu_mma_smem(emu_ctx->smem + (u32)a * 16ul, (u32)(a >> 32), m, k); }, emu_ctx->smem + (u32)b * 16ul, (u32)(b >> 32), n, acc);
 }
+FRNN_DEV bool frnn_elect() { return (threadIdx.x & 31) == 0; }
 FRNN_DEV void frnn_mma_commit(u64* bar) { frnn_mbar_arrive(bar); }
 FRNN_DEV int frnn_smem_add(int* p, int v) { std::lock_guard<std::mutex> g(emu_atomic_mtx); int o = *p; *p = o + v; return o; }
 template <int N> FRNN_DEV void frnn_regs_release() {}
