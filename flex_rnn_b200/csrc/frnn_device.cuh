@@ -202,7 +202,11 @@ template <int N> FRNN_DEV void frnn_tmem_ld(u32 taddr, float* v) {
 FRNN_DEV bool frnn_mbar_wait(u64* bar, u32 parity, int* err, int code) {
     if (frnn_mbar_try(bar, parity)) return true;
     u64 t0 = frnn_now_ns();
+    // not unrolled: 64 copies were 2 KB of code at every wait, half of a chunked kernel's, and what is beyond the 32 KB of the
+    // instruction cache slows every warp of the SM
+#pragma unroll 1
     for (;;) {
+#pragma unroll 1
         for (int i = 0; i < 64; i++)
             if (frnn_mbar_try(bar, parity)) return true;
         if (frnn_now_ns() - t0 > FRNN_WAIT_LIMIT_NS) {
