@@ -1491,9 +1491,6 @@ def backward_scan_spec(p: Problem, nf: Normal, bp: BackwardPlan, dspec: Sequence
                     (p.res_states[0], "ds0"), "dgk" if bp.kept_dg else None, "eck", True)
 
 
-VG_THREADS = 256
-
-
 def emit_vector_grads(p: Problem, nf: Normal, bp: BackwardPlan, dspec: Sequence[TensorSpec], atomic: Sequence[bool], C: int) -> KernelSource:
     """Gradients of the column vectors and scalars, one CTA per chunk of ``C`` timesteps: with the state S_0 at the
     chunk's start, the state gradient E_C at its end, X = dsig and Z = p (vectors over the rows, per timestep),
@@ -1506,8 +1503,8 @@ def emit_vector_grads(p: Problem, nf: Normal, bp: BackwardPlan, dspec: Sequence[
     (``local_vjp``).  All products run on the tensor cores.  Where a decay of the chunk is too small to divide by, the
     chunk takes a slower path of plain loops with running products instead.
 
-    Bound by HBM: S_0 and E_C are 2 x 4 M N bytes per C timesteps.  Two CTAs share an SM, so that one loads while the
-    other computes.  Parameters, in order: inputs, d outputs, forward row sums, kept row sums, checkpoints of S, of E,
+    S_0 and E_C are 2 x 4 M N bytes per C timesteps, 1.1 us at HBM's rate for 128x128; the stores that bring them and their rests
+    into the tensor cores' layout and the products' reads of them keep shared memory busy for longer.  Parameters, in order: inputs, d outputs, forward row sums, kept row sums, checkpoints of S, of E,
     gradients, error word.
     """
     v = bp.vjp
@@ -1520,8 +1517,6 @@ def emit_vector_grads(p: Problem, nf: Normal, bp: BackwardPlan, dspec: Sequence[
     nin = len(nf.inputs)
     shape = dict(nf.shape)
     shape.update(v.shape)
-    MS = 16 if M % 16 == 0 else 8
-    nsl = M // MS
     # ---- stages
     msums = [n for n in v.nodes if n.op == "sum" and n.over_m]
     nsums = [n for n in v.nodes if n.op == "sum" and n.over_n]
@@ -1590,45 +1585,71 @@ def emit_vector_grads(p: Problem, nf: Normal, bp: BackwardPlan, dspec: Sequence[
     for x in ("Wp", "Ws", "gw"):
         slot(x)
     npart = max(len(msums), n_nsum) + 1
-    HC = C // 2                              # timesteps of one thread: 128 rows or columns times two halves of the chunk
-    off_sc = 256
-    off_part = off_sc + al(len(sc_slots) * C * 4)
-    off_z0 = off_part + al(npart * 4 * C * 4)
-    off_xr = off_z0 + al(128 * 4)            # what the halves of a column exchange
-    off_X = off_xr + al(3 * 128 * 4)
-    lboX, lboZ, lboS = 2 * nA * 16 + 16, 2 * nK * 16 + 16, 128 * 16 + 16
-    off_Z = off_X + al((M // 4 - 1) * lboX + max(2048 + 16, lboX))
-    off_sl = off_Z + al(M // 4 * lboZ)
-    sl_bytes = al(MS // 4 * lboS)
-    # two CTAs per SM hide each other's latencies; where X and Z are too large for that, the one CTA keeps two buffers of
-    # slices and loads four slices ahead instead of two
-    single = max(off_sl + 4 * sl_bytes, off_X + 2 * (nK + nA) // 4 * 128 * 16 + 16 * (nA * nK // 2 + nA))
-    ctas = 2 if single <= SMEM_BYTES // 2 - 1024 else 1
-    NB, DP = (1, 2) if ctas == 2 else (2, 4)
-    end1 = off_sl + 4 * NB * sl_bytes
-    # second phase, over the same memory
-    lboT, lbo1, lbo2 = 128 * 16, 2 * nA * 16, 2 * nK * 16
-    off_kT = off_X
-    kT_b, aT_b = nK // 4 * lboT, nA // 4 * lboT
-    off_aT = off_kT + 2 * kT_b
-    off_L1 = off_aT + 2 * aT_b
-    off_L2 = off_L1 + nK // 4 * lbo1
-    off_Lr = off_L2 + nA // 4 * lbo2
-    LS = nK + 1
-    off_slow = off_kT                        # the slow path's results, over the operands it does without: (nA + nK + C) x 128 floats
-    smem_bytes = al(max(end1, off_Lr + nA * LS * 4))
+    # which operands are plain 16-bit inputs, exact in tf32: they have no second term
+    dt16 = (lower.DT_BF16, lower.DT_F16)
+    leaf_dt = {nf.inputs[i]: p.inputs[i].dt for i in range(nin)}
+    leaf_dt.update({f"gy{j}": p.out_dt[j] for j in range(len(nf.ys))})
+    is16 = lambda a: isinstance(a, str) and leaf_dt.get(a) in dt16
+    restX = [d for d in range(nd) if not is16(bp.dsig[d])]
+    restZ = [r for r in range(nr) if not is16(nf.ps[r])]
+    xa, xk = not dec_vec and all(map(is16, nf.alphas)), not dec_vec and all(map(is16, nf.kappas))
+    RX, RZ = nA + C * len(restX), nK + C * len(restZ)        # rows of X and Z: the vectors, then the rests of the inexact ones
     slow_path = bool(nf.decay) and (dec_vec or want_gw)
-    if slow_path and dec_vec:
-        off_Lr = max(off_Lr, off_slow + (nA + nK + C) * 512)
-        smem_bytes = al(max(smem_bytes, off_Lr + nA * LS * 4))
-    elif slow_path:                          # the gradients of a decay per head only: beside the operands, which stay
-        off_slow = al(off_Lr + nA * LS * 4) - (nA + nK) * 512
-        smem_bytes = al(max(smem_bytes, off_slow + (nA + nK + C) * 512))
-    cD1, cD2 = 0, 2 * nA
-    cL = cD2 + 2 * nK
-    tm_cols = _tmem_pow2(cL + 2 * nK)
+    # padding: the eight threads of a store's phase write to different banks
+    lboX, lboZ = RX * 16 + 16, RZ * 16 + 16
+    lboT, lbo1, lbo2 = 128 * 16, 2 * nA * 16, 2 * nK * 16 + 16
+    LS = nK + 1
+    kT_b, aT_b = nK // 4 * lboT, nA // 4 * lboT
+
+    class Layout:
+        """Shared memory with slices of ``MS`` rows in ``NB`` buffers and ``parts`` x 128 threads."""
+
+        def __init__(self, MS: int, NB: int, parts: int):
+            self.MS, self.NB, self.parts = MS, NB, parts
+            self.sc = 256
+            self.part = self.sc + al(len(sc_slots) * C * 4)
+            self.z0 = self.part + al(npart * 4 * C * 4)
+            self.xr = self.z0 + al(128 * 4)             # what the threads of a column exchange
+            self.X = self.xr + al(2 * 128 * parts * 4)
+            self.Z = self.X + al((M // 4 - 1) * lboX + max(2048 + 16, lboX))
+            self.sl = self.Z + al(M // 4 * lboZ)
+            self.lboS = 128 * 16 + 128 // (MS // 4)
+            self.sl_bytes = al(MS // 4 * self.lboS)
+            end1 = self.sl + 4 * NB * self.sl_bytes
+            # second phase, over the same memory
+            self.kT = self.X
+            self.aT = self.kT + (1 if xk else 2) * kT_b
+            self.L1 = self.aT + (1 if xa else 2) * aT_b
+            self.L2 = self.L1 + nK // 4 * lbo1
+            self.Lr = self.L2 + nA // 4 * lbo2
+            self.slow = self.kT                         # the slow path's results, over the operands it does without: (nA + nK + C) x 128 floats
+            if slow_path and dec_vec:
+                self.Lr = max(self.Lr, self.slow + (nA + nK + C) * 512)
+            self.bytes = al(max(end1, self.Lr + nA * LS * 4))
+            if slow_path and not dec_vec:               # the gradients of a decay per head only: beside the operands, which stay
+                self.slow = al(self.Lr + nA * LS * 4) - (nA + nK) * 512
+                self.bytes = al(max(self.bytes, self.slow + (nA + nK + C) * 512))
+            self.ctas = 2 if self.bytes <= SMEM_BYTES // 2 - 1024 else 1
+    # two CTAs of 256 threads share an SM and hide each other's latencies; where X and Z are too large for that, one of 512 with
+    # two buffers of slices (B8 T1024 H32, us: RWKV-7 128x128 1096 against 1276 with one CTA, Mamba-2 64x128 467 against 546; Delta
+    # Rule 128x128, which two CTAs fit with slices of 8 rows only, 687 against 638)
+    lay = Layout(16, 1, 2) if M % 16 == 0 else Layout(8, 1, 2)
+    if lay.ctas == 1 and M % 16 == 0:
+        lay = Layout(16, 2, 4)
+    MS, NB, parts, ctas = lay.MS, lay.NB, lay.parts, lay.ctas
+    DP = 16 * 2 * NB // MS                   # slices that are loaded ahead
+    nsl = M // MS
+    NT = 128 * parts                         # 128 rows or columns times ``parts`` parts of the chunk's timesteps
+    HC = C // parts                          # timesteps of one thread
+    lboS, sl_bytes, smem_bytes = lay.lboS, lay.sl_bytes, lay.bytes
+    off_sc, off_part, off_z0, off_xr, off_X, off_Z, off_sl = lay.sc, lay.part, lay.z0, lay.xr, lay.X, lay.Z, lay.sl
+    off_kT, off_aT, off_L1, off_L2, off_Lr, off_slow = lay.kT, lay.aT, lay.L1, lay.L2, lay.Lr, lay.slow
+    cD1, cD2 = 0, RX
+    cL = cD2 + RZ
+    tm_cols = _tmem_pow2(cL + RZ)
     if tm_cols > 256:
         raise lower.LoweringError("the vector gradients of a chunk do not fit half of Tensor Memory")
+    at_rest = lambda inexact, x, n: n + C * inexact.index(x)     # row or column where the rest of vector x begins
     ERR = lower.ERR_STAGE_TIMEOUT
     full_n = N == 128
     # loads are never predicated (the compiler would wait for each in turn): past the ends they repeat the last timestep,
@@ -1641,7 +1662,7 @@ def emit_vector_grads(p: Problem, nf: Normal, bp: BackwardPlan, dspec: Sequence[
 
     w(lower._header(chunk_prelude()))
     w(f"// vector gradients: B={B} T={T} H={H} M={M} N={N}; {C} steps per chunk, {nd} row sums, {nr} rank-1 terms")
-    w(f'extern "C" __global__ void __launch_bounds__({VG_THREADS}, {ctas})')
+    w(f'extern "C" __global__ void __launch_bounds__({NT}, {ctas})')
     w.open(f"frnn_cvg({', '.join(decl)})")
     w("FRNN_DYN_SMEM(smem);")
     w("const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;")
@@ -1757,7 +1778,7 @@ def emit_vector_grads(p: Problem, nf: Normal, bp: BackwardPlan, dspec: Sequence[
         w(f"{reg(a)}[k] = {leaf(a, 't', 'mc')};")
     w.close()
     q4 = MS // 4
-    per = 128 // (VG_THREADS // q4)        # columns per thread and slice
+    per = 128 // (NT // q4)        # columns per thread and slice
     w(f"const int sm4 = tid % {q4}, sn = tid / {q4};")
     w(f"const float* ckp = ck + (((long)b * {H} + h) * {nchunk} + kc) * {N}L * {M}L; const float* ekp = eck + (((long)b * {H} + h) * {nchunk} + kc) * {N}L * {M}L;")
     w(f"float zz[{per}], sv[{DP}][{per}][4], ev[{DP}][{per}][4];")
@@ -1767,7 +1788,7 @@ def emit_vector_grads(p: Problem, nf: Normal, bp: BackwardPlan, dspec: Sequence[
     def load_slice(sx, u):
         w("#pragma unroll")
         w.open(f"for (int i = 0; i < {per}; i++)")
-        w(f"const int n = {'sn' if full_n else 'min(sn'} + i * {VG_THREADS // q4}{'' if full_n else f', {N - 1})'};")
+        w(f"const int n = {'sn' if full_n else 'min(sn'} + i * {NT // q4}{'' if full_n else f', {N - 1})'};")
         w(f"frnn_ldv<0,4>(ckp, n * {M}L + ({sx}) * {MS} + sm4 * 4, sv[{u}][i]);")
         w(f"frnn_ldv<0,4>(ekp, n * {M}L + ({sx}) * {MS} + sm4 * 4, ev[{u}][i]);")
         w.close()
@@ -1809,14 +1830,15 @@ def emit_vector_grads(p: Problem, nf: Normal, bp: BackwardPlan, dspec: Sequence[
     w.open(f"for (int k = 0; k < {HC}; k++)")
     w(f"const int q = q0 + k; const bool live = {live_m}; (void)live;")
     st = Stage("x_", "q", M1, {a: f"{reg(a)}[k]" for a in mleaves})
-    vals = [(f"{d * C}", st.get(x), "X") for d, x in enumerate(bp.dsig)] + [(f"{r * C}", st.get(x), "Z") for r, x in enumerate(nf.ps)]
+    vals = [(d, st.get(x), "X") for d, x in enumerate(bp.dsig)] + [(r, st.get(x), "Z") for r, x in enumerate(nf.ps)]
     for x, n in enumerate(msums):
         w(f"e{x}[k] = {sel(live_m, st.get(n.args[0]))};")
     w.open(f"if (mrow)" if M < 128 else "")
-    for base, val, which in vals:
-        lbo, off, n2 = (lboX, off_X, nA) if which == "X" else (lboZ, off_Z, nK)
-        w(f"{{ const float a = {sel(live_m, val)}, hi = a; unsigned char* dst = smem + {off} + (x128 >> 2) * {lbo} + (x128 & 3) * 4; "
-          f"const int r0 = {base} + q, r1 = r0 + {n2}; *(float*)(dst + (r0 >> 3) * 128 + (r0 & 7) * 16) = hi; *(float*)(dst + (r1 >> 3) * 128 + (r1 & 7) * 16) = frnn_tf32_rest(a); }}")
+    for v_, val, which in vals:
+        lbo, off, inexact, n2 = (lboX, off_X, restX, nA) if which == "X" else (lboZ, off_Z, restZ, nK)
+        put = lambda row0, x: f"{{ const int row = {row0} + q; *(float*)(dst + (row >> 3) * 128 + (row & 7) * 16) = {x}; }}"
+        w(f"{{ const float a = {sel(live_m, val)}; unsigned char* dst = smem + {off} + (x128 >> 2) * {lbo} + (x128 & 3) * 4; {put(v_ * C, 'a')}"
+          + (" " + put(at_rest(inexact, v_, n2), "frnn_tf32_rest(a)") if v_ in inexact else "") + " }")
     w.close()
     w.close()
     for x in range(len(msums)):
@@ -1827,7 +1849,7 @@ def emit_vector_grads(p: Problem, nf: Normal, bp: BackwardPlan, dspec: Sequence[
     w(f"const u64 dX = frnn_mma_desc(smem + {off_X}, {lboX}), dZ = frnn_mma_desc(smem + {off_Z}, {lboZ});")
     w.open("if (warp == 0 && frnn_elect())")
     w("#pragma unroll")
-    w(f"for (int k = 0; k < {M // 8}; k++) frnn_mma_ss_d(tm + {cL}u, frnn_mma_next(dX, {lboX}, k), frnn_mma_next(dZ, {lboZ}, k), FRNN_MMA_IDESC({2 * nK}), k > 0);")
+    w(f"for (int k = 0; k < {M // 8}; k++) frnn_mma_ss_d(tm + {cL}u, frnn_mma_next(dX, {lboX}, k), frnn_mma_next(dZ, {lboZ}, k), FRNN_MMA_IDESC({RZ}), k > 0);")
     w("frnn_mma_commit(&bar[0]);")
     w.close()
     # ---- second-stage scalars
@@ -1856,7 +1878,7 @@ def emit_vector_grads(p: Problem, nf: Normal, bp: BackwardPlan, dspec: Sequence[
         w(f"const bool arrived = s < {NB} || frnn_mbar_wait(&bar[{bb}], (s / {NB} - 1) & 1, err, {ERR});     // the products that read this buffer are complete")
         w("#pragma unroll")
         w.open(f"for (int i = 0; i < {per}; i++)")
-        w(f"const int n = sn + i * {VG_THREADS // q4};")
+        w(f"const int n = sn + i * {NT // q4};")
         off_b = off_sl + (u % NB) * 4 * sl_bytes
         w(f"unsigned char* dst = smem + {off_b} + sm4 * {lboS} + (n >> 3) * 128 + (n & 7) * 16;")
         w("float r[4];")
@@ -1876,11 +1898,11 @@ def emit_vector_grads(p: Problem, nf: Normal, bp: BackwardPlan, dspec: Sequence[
         w("if (!frnn_block_and(arrived)) break;")
         w.open("if (warp == 0 && frnn_elect())")
         for k in range(MS // 8):
-            for which, (col_, dsc, lbo, n2) in enumerate(((cD1, "dX", lboX, nA), (cD2, "dZ", lboZ, nK))):
+            for which, (col_, dsc, lbo, n2) in enumerate(((cD1, "dX", lboX, RX), (cD2, "dZ", lboZ, RZ))):
                 sb = off_b + 2 * which * sl_bytes + k * 2 * lboS
                 bexp = f"frnn_mma_next({dsc}, {lbo}, s * {MS // 8} + {k})"
-                w(f"frnn_mma_ss_d(tm + {col_}u, frnn_mma_desc(smem + {sb}, {lboS}), {bexp}, FRNN_MMA_IDESC({2 * n2}), {'s > 0' if k == 0 else 'true'});")
-                w(f"frnn_mma_ss_d(tm + {col_}u, frnn_mma_desc(smem + {sb + sl_bytes}, {lboS}), {bexp}, FRNN_MMA_IDESC({2 * n2}), true);")
+                w(f"frnn_mma_ss_d(tm + {col_}u, frnn_mma_desc(smem + {sb}, {lboS}), {bexp}, FRNN_MMA_IDESC({n2}), {'s > 0' if k == 0 else 'true'});")
+                w(f"frnn_mma_ss_d(tm + {col_}u, frnn_mma_desc(smem + {sb + sl_bytes}, {lboS}), {bexp}, FRNN_MMA_IDESC({n2}), true);")
         w(f"frnn_mma_commit(&bar[{bb}]);")
         w.close()
         w.close()
@@ -1897,7 +1919,7 @@ def emit_vector_grads(p: Problem, nf: Normal, bp: BackwardPlan, dspec: Sequence[
         w.open(f"for (int i = 0; i < {per}; i++)")
         w("#pragma unroll")
         w(f"for (int o = {q4 // 2}; o > 0; o >>= 1) zz[i] += frnn_shfl_xor(zz[i], o);")
-        w(f"if (sm4 == 0) z0[sn + i * {VG_THREADS // q4}] = zz[i];")
+        w(f"if (sm4 == 0) z0[sn + i * {NT // q4}] = zz[i];")
         w.close()
     w(f"bool ok = frnn_mbar_wait(&bar[0], 0, err, {ERR});")
     for u in range(min(NB, nsl)):
@@ -1911,54 +1933,70 @@ def emit_vector_grads(p: Problem, nf: Normal, bp: BackwardPlan, dspec: Sequence[
     def ld_L(dst):
         w(f"float {dst}[{nr * HC}];")
         w.open("")
-        w(f"float lo[{nr * HC}];")
+        if restZ:
+            w(f"float lo[{len(restZ) * HC}];")
         for r in range(nr):
-            w(f"frnn_tmem_ld<{HC}>(lanes + {cL + r * C}u + (u32)q0, &{dst}[{r * HC}]); frnn_tmem_ld<{HC}>(lanes + {cL + nK + r * C}u + (u32)q0, &lo[{r * HC}]);")
+            w(f"frnn_tmem_ld<{HC}>(lanes + {cL + r * C}u + (u32)q0, &{dst}[{r * HC}]);")
+        for x, r in enumerate(restZ):
+            w(f"frnn_tmem_ld<{HC}>(lanes + {cL + at_rest(restZ, r, nK)}u + (u32)q0, &lo[{x * HC}]);")
         w("frnn_tmem_wait_ld();")
-        w("#pragma unroll")
-        w(f"for (int k = 0; k < {nr * HC}; k++) {dst}[k] += lo[k];")
+        for x, r in enumerate(restZ):
+            w("#pragma unroll")
+            w(f"for (int k = 0; k < {HC}; k++) {dst}[{r * HC} + k] += lo[{x * HC} + k];")
         w.close()
-    w.open(f"if (x128 >= {nA // 32 * 32} && x128 < {(2 * nA + 31) // 32 * 32})")
-    ld_L("u")
-    w.open(f"if (x128 >= {nA} && x128 < {2 * nA})")
-    w("#pragma unroll")
-    w(f"for (int k = 0; k < {nr * HC}; k++) Lr[(x128 - {nA}) * {LS} + (k / {HC}) * {C} + q0 + k % {HC}] = u[k];")
-    w.close()
-    w.close()
-    w("frnn_block_sync();")
+    if restX:
+        w.open(f"if (x128 >= {nA // 32 * 32} && x128 < {(RX + 31) // 32 * 32})")
+        ld_L("u")
+        w.open(f"if (x128 >= {nA} && x128 < {RX})")
+        w("int at = x128 - %d;%s" % (nA, "".join(f" if (x128 >= {nA + x * C} && x128 < {nA + (x + 1) * C}) at += {(d - x) * C};" for x, d in enumerate(restX) if d != x)))
+        w("#pragma unroll")
+        w(f"for (int k = 0; k < {nr * HC}; k++) Lr[at * {LS} + (k / {HC}) * {C} + q0 + k % {HC}] = u[k];")
+        w.close()
+        w.close()
+        w("frnn_block_sync();")
     w.open(f"if (x128 < {(nA + 31) // 32 * 32})")
     ld_L("u")
     w.open(f"if (x128 < {nA})")
     w(f"const int j = x128 % {C};")
-    w("#pragma unroll")
-    w(f"for (int k = 0; k < {nr * HC}; k++) u[k] += Lr[x128 * {LS} + (k / {HC}) * {C} + q0 + k % {HC}];")
+    if restX:
+        w.open(f"if ({' || '.join(f'x128 / {C} == {d}' for d in restX)})" if len(restX) < nd else "")
+        w("#pragma unroll")
+        w(f"for (int k = 0; k < {nr * HC}; k++) u[k] += Lr[x128 * {LS} + (k / {HC}) * {C} + q0 + k % {HC}];")
+        w.close()
     if dec_sc:
-        w(f"float D = 1.0f;          // decays between step j and the last of this half")
-        w(f"if (hf == 0) for (int l = {HC}; l < {C}; l++) if (l < j && l < nv) D *= {slot(nf.decay)} + l];")
+        w(f"float D = 1.0f;          // decays between step j and the last of this part")
+        w(f"for (int l = q0 + {HC}; l < {C}; l++) if (l < j && l < nv) D *= {slot(nf.decay)} + l];")
+    # four columns of a row are one store of the operand with rows (d, j), and four single ones of the other
+    w(f"unsigned char* d2 = smem + {off_L2} + (x128 >> 2) * {lbo2} + (x128 & 3) * 4;")
     w("#pragma unroll")
-    w.open(f"for (int k = {HC - 1}; k >= 0; k--)")
-    w("const int i = q0 + k;")
+    w.open(f"for (int k4 = {HC - 4}; k4 >= 0; k4 -= 4)")
+    w(f"float a[{nr}][4], lo[{nr}][4];")
+    w("#pragma unroll")
+    w.open("for (int k = 3; k >= 0; k--)")
+    w("const int i = q0 + k4 + k;")
     w("#pragma unroll")
     w.open(f"for (int r = 0; r < {nr}; r++)")
     w(f"const int ri = r * {C} + i;")
-    w(f"float a = i < j ? u[r * {HC} + k] : 0.0f;")
-    w(f"Lr[x128 * {LS} + ri] = a;")
-    if dec_sc:
-        w("a *= D;")
-    w("const float hi = a, lo = frnn_tf32_rest(a);")
-    w(f"unsigned char* d1 = smem + {off_L1} + (ri >> 2) * {lbo1} + (ri & 3) * 4; const int ra = x128, rb = x128 + {nA};")
-    w("*(float*)(d1 + (ra >> 3) * 128 + (ra & 7) * 16) = hi; *(float*)(d1 + (rb >> 3) * 128 + (rb & 7) * 16) = lo;")
-    w(f"unsigned char* d2 = smem + {off_L2} + (x128 >> 2) * {lbo2} + (x128 & 3) * 4; const int rc = ri, rd = ri + {nK};")
-    w("*(float*)(d2 + (rc >> 3) * 128 + (rc & 7) * 16) = hi; *(float*)(d2 + (rd >> 3) * 128 + (rd & 7) * 16) = lo;")
+    w(f"const float x = i < j ? u[r * {HC} + k4 + k] : 0.0f;")
+    w(f"Lr[x128 * {LS} + ri] = x;")
+    w("a[r][k] = x" + (" * D;" if dec_sc else ";") + " lo[r][k] = frnn_tf32_rest(a[r][k]);")
+    w(f"const int rd = ri + {nK};")
+    w("*(float*)(d2 + (ri >> 3) * 128 + (ri & 7) * 16) = a[r][k]; *(float*)(d2 + (rd >> 3) * 128 + (rd & 7) * 16) = lo[r][k];")
     w.close()
     if dec_sc:
         w(f"if (i < j && i < nv) D *= {slot(nf.decay)} + i];")
     w.close()
+    w("#pragma unroll")
+    w.open(f"for (int r = 0; r < {nr}; r++)")
+    w(f"unsigned char* d1 = smem + {off_L1} + ((r * {C} + q0 + k4) >> 2) * {lbo1}; const int ra = x128, rb = x128 + {nA};")
+    w("frnn_stv<0,4>(d1 + (ra >> 3) * 128 + (ra & 7) * 16, 0, a[r]); frnn_stv<0,4>(d1 + (rb >> 3) * 128 + (rb & 7) * 16, 0, lo[r]);")
     w.close()
     w.close()
-    # ---- operands over the columns: kappa (over W) and alpha (times W), this thread's half of the timesteps
+    w.close()
+    w.close()
+    # ---- operands over the columns: kappa (over W) and alpha (times W), this thread's part of the timesteps
     if dec_vec:
-        w(f"float xw[{HC}], pre = 1.0f, post = 1.0f, rpre = 1.0f, wlo = 1.0f, whi = 1.0f, prod = 1.0f;   // decays; products of the other half's")
+        w(f"float xw[{HC}], pre = 1.0f, post = 1.0f, rpre = 1.0f, wlo = 1.0f, whi = 1.0f, prod = 1.0f;   // decays; products of the other parts'")
         w("#pragma unroll")
         w.open(f"for (int k = 0; k < {HC}; k++)")
         w.open("")
@@ -1970,11 +2008,12 @@ def emit_vector_grads(p: Problem, nf: Normal, bp: BackwardPlan, dspec: Sequence[
         w.close()
         w("prod *= xw[k];")
         w.close()
-        # the product of the other half's decays comes through shared memory
+        # the products of the other parts' decays come through shared memory
         w("xr[tid] = prod;")
         w("frnn_block_sync();")
-        w("const float other = xr[tid ^ 128];")
-        w("if (hf) { pre = other; rpre = frnn_rcp1(other); } else post = other;")
+        w("#pragma unroll")
+        w(f"for (int o = 0; o < {parts}; o++) {{ const float x = xr[o * 128 + x128]; if (o < hf) pre *= x; if (o > hf) post *= x; }}")
+        w("rpre = frnn_rcp1(pre);")
         w("float rw = rpre, pw = pre;")
     w("#pragma unroll")
     w.open(f"for (int k4 = 0; k4 < {HC}; k4 += 4)")
@@ -1993,31 +2032,37 @@ def emit_vector_grads(p: Problem, nf: Normal, bp: BackwardPlan, dspec: Sequence[
         w("pw *= xw[k4 + k];")
     w.close()
     for x in range(len(names)):
-        off, tb, r = (off_kT, kT_b, x) if x < nr else (off_aT, aT_b, x - nr)
-        w(f"{{ float hi[4]; unsigned char* dst = smem + {off} + (({r * C} + q0 + k4) >> 2) * {lboT} + (x128 >> 3) * 128 + (x128 & 7) * 16;")
-        w("#pragma unroll")
-        w(f"for (int k = 0; k < 4; k++) {{ hi[k] = x[{x}][k]; x[{x}][k] = frnn_tf32_rest(hi[k]); }}")
-        w(f"frnn_stv<0,4>(dst, 0, hi); frnn_stv<0,4>(dst + {tb}, 0, x[{x}]); }}")
+        off, tb, r, exact = (off_kT, kT_b, x, xk) if x < nr else (off_aT, aT_b, x - nr, xa)
+        w(f"{{ unsigned char* dst = smem + {off} + (({r * C} + q0 + k4) >> 2) * {lboT} + (x128 >> 3) * 128 + (x128 & 7) * 16; frnn_stv<0,4>(dst, 0, x[{x}]);")
+        if not exact:
+            w("#pragma unroll")
+            w(f"for (int k = 0; k < 4; k++) x[{x}][k] = frnn_tf32_rest(x[{x}][k]);")
+            w(f"frnn_stv<0,4>(dst + {tb}, 0, x[{x}]);")
+        w("}")
     w.close()
     if dec_vec:
         w(f"if (!(wlo > {tiny} && whi < 1e25f)) *(volatile int*)&bar[4] = 1;")
     # ---- the parts of the accumulators so far, from S_0 and E_C, scaled to what those from L need
     w("float R = 0.0f; (void)R;")
 
-    def ld_half(dst: str, vecs: int, col0: int, rest: int):
-        """dst[v * HC + k] = value of vector v at timestep q0 + k: the sum of two accumulator columns."""
+    def ld_part(dst: str, vecs: int, col0: int, inexact: Sequence[int], n: int):
+        """dst[v * HC + k] = value of vector v at timestep q0 + k, with what the rest of the operand gave."""
         w.open("")
-        w(f"float u[{vecs * HC}], lo[{vecs * HC}];")
+        if inexact:
+            w(f"float lo[{len(inexact) * HC}];")
         for x in range(vecs):
-            w(f"frnn_tmem_ld<{HC}>(lanes + {col0 + x * C}u + (u32)q0, &u[{x * HC}]); frnn_tmem_ld<{HC}>(lanes + {col0 + rest + x * C}u + (u32)q0, &lo[{x * HC}]);")
+            w(f"frnn_tmem_ld<{HC}>(lanes + {col0 + x * C}u + (u32)q0, &{dst}[{x * HC}]);")
+        for k, x in enumerate(inexact):
+            w(f"frnn_tmem_ld<{HC}>(lanes + {col0 + at_rest(inexact, x, n)}u + (u32)q0, &lo[{k * HC}]);")
         w("frnn_tmem_wait_ld();")
-        w("#pragma unroll")
-        w(f"for (int k = 0; k < {vecs * HC}; k++) {dst}[k] = u[k] + lo[k];")
+        for k, x in enumerate(inexact):
+            w("#pragma unroll")
+            w(f"for (int k = 0; k < {HC}; k++) {dst}[{x * HC} + k] += lo[{k * HC} + k];")
         w.close()
 
-    def st_half(src: str, vecs: int, col0: int, rest: int):
+    def st_part(src: str, vecs: int, col0: int):
         for x in range(vecs):
-            w(f"frnn_tmem_st<{HC}>(lanes + {col0 + x * C}u + (u32)q0, &{src}[{x * HC}]); frnn_tmem_st<{HC}>(lanes + {col0 + rest + x * C}u + (u32)q0, zero);")
+            w(f"frnn_tmem_st<{HC}>(lanes + {col0 + x * C}u + (u32)q0, &{src}[{x * HC}]);")
     if dec_sc:
         w(f"float xw[{HC}], pre = {slot('Wp')} + q0], post = {slot('Ws')} + q0 + {HC - 1}];")
         w("#pragma unroll")
@@ -2027,13 +2072,11 @@ def emit_vector_grads(p: Problem, nf: Normal, bp: BackwardPlan, dspec: Sequence[
     w("frnn_block_sync();")
     w("const bool slow = *(volatile int*)&bar[4] != 0; (void)slow;")
     if slow_path:
-        emit_slow_columns(w, C, nd, nr, nA, nK, tq, live_n, sel, nf, bp, dec_vec, want_gw, Stage, leaf, leaves_of, slot, LS, cD1, cD2, off_slow)
+        emit_slow_columns(w, C, nd, nr, nA, nK, tq, live_n, sel, nf, bp, dec_vec, want_gw, Stage, leaf, leaves_of, slot, LS, ((cD1, restX), (cD2, restZ)), off_slow)
     if nf.decay:
         w.open("if (!slow)" if dec_vec else "")
-        w(f"float dk[{nr * HC}], zero[{HC}];")
-        w("#pragma unroll")
-        w(f"for (int k = 0; k < {HC}; k++) zero[k] = 0.0f;")
-        ld_half("dk", nr, cD2, nK)
+        w(f"float dk[{nr * HC}];")
+        ld_part("dk", nr, cD2, restZ, nK)
         w("float a = post;")
         if dec_vec:
             w(f"float y[{nr * HC}];")
@@ -2056,15 +2099,19 @@ def emit_vector_grads(p: Problem, nf: Normal, bp: BackwardPlan, dspec: Sequence[
             w("const float wc = a * pre;")
             w("#pragma unroll")
             w(f"for (int k = 0; k < {nr * HC}; k++) dk[k] = y[k] * wc;")
-            st_half("dk", nr, cD2, nK)
+            st_part("dk", nr, cD2)
+            if restX:
+                w(f"float da[{nd * HC}];")
+                ld_part("da", nd, cD1, restX, nA)
+                st_part("da", nd, cD1)
         else:
-            st_half("dk", nr, cD2, nK)
+            st_part("dk", nr, cD2)
             w(f"float da[{nd * HC}];")
-            ld_half("da", nd, cD1, nA)
+            ld_part("da", nd, cD1, restX, nA)
             w("a = pre;")
             w("#pragma unroll")
             w(f"for (int k = 0; k < {HC}; k++) {{ " + " ".join(f"da[{d * HC} + k] *= a;" for d in range(nd)) + " a *= xw[k]; }")
-            st_half("da", nd, cD1, nA)
+            st_part("da", nd, cD1)
         w("frnn_tmem_wait_st();")
         w.close()
     w("frnn_async_proxy_fence(); frnn_tmem_fence_before_sync();")
@@ -2072,20 +2119,21 @@ def emit_vector_grads(p: Problem, nf: Normal, bp: BackwardPlan, dspec: Sequence[
     w.open("if (warp == 0 && frnn_elect())")
     w.open("if (ok)" if not dec_vec else "if (ok && !slow)")
     w("frnn_tmem_fence_after_sync();")
-    for (cd, offA, tb, nk, offB, lboB, n2) in ((cD1, off_kT, kT_b, nK, off_L1, lbo1, nA), (cD2, off_aT, aT_b, nA, off_L2, lbo2, nK)):
-        for part_, n_ in ((offA, 2 * n2), (offA + tb, 2 * n2)):
-            w(f"{{ const u64 da = frnn_mma_desc(smem + {part_}, {lboT}), db = frnn_mma_desc(smem + {offB}, {lboB});")
-            w("#pragma unroll")
-            w(f"for (int k = 0; k < {nk // 8}; k++) frnn_mma_ss_d(tm + {cd}u, frnn_mma_next(da, {lboT}, k), frnn_mma_next(db, {lboB}, k), FRNN_MMA_IDESC({n_}), true); }}")
+    for cd, offA, tb, exact, nk, offB, lboB, n2 in ((cD1, off_kT, kT_b, xk, nK, off_L1, lbo1, nA), (cD2, off_aT, aT_b, xa, nA, off_L2, lbo2, nK)):
+        for part_ in ([offA] if exact else [offA, offA + tb]):
+            for row in (0, n2):              # L and its rest
+                w(f"{{ const u64 da = frnn_mma_desc(smem + {part_}, {lboT}), db = frnn_mma_desc(smem + {offB + row // 8 * 128}, {lboB});")
+                w("#pragma unroll")
+                w(f"for (int k = 0; k < {nk // 8}; k++) frnn_mma_ss_d(tm + {cd}u, frnn_mma_next(da, {lboT}, k), frnn_mma_next(db, {lboB}, k), FRNN_MMA_IDESC({n2}), true); }}")
     w.close()
     w("frnn_mma_commit(&bar[2]);")
     w.close()
     w(f"ok = frnn_mbar_wait(&bar[2], 0, err, {ERR}) && ok;")
     w("frnn_tmem_fence_after_sync();")
-    # ---- columns: this thread's half of the timesteps
+    # ---- columns: this thread's part of the timesteps
     w(f"float da[{nd * HC}], dk[{nr * HC}];")
-    ld_half("da", nd, cD1, nA)
-    ld_half("dk", nr, cD2, nK)
+    ld_part("da", nd, cD1, [] if nf.decay else restX, nA)
+    ld_part("dk", nr, cD2, [] if nf.decay else restZ, nK)
     if dec_vec:
         # the accumulators held W_C/W_j of kappa's part times W_j and alpha's part over W_j-1
         w.open("if (!slow)")
@@ -2105,7 +2153,7 @@ def emit_vector_grads(p: Problem, nf: Normal, bp: BackwardPlan, dspec: Sequence[
         w.close()
         w.close()
     if dec_vec and want_gw:
-        # the upper half's part of the sums that lead from R_C to the lower half
+        # the later parts' share of the sums that lead from R_C to the earlier ones
         w("float P = 0.0f;")
         w("#pragma unroll")
         w.open(f"for (int k = 0; k < {HC}; k++)")
@@ -2115,9 +2163,11 @@ def emit_vector_grads(p: Problem, nf: Normal, bp: BackwardPlan, dspec: Sequence[
         ad = " + ".join(f"{st.get(nm)} * da[{d * HC} + k]" for d, nm in enumerate(nf.alphas))
         w(f"P += {sel(live_n, f'(({ad}) - ({kd}))')};")
         w.close()
-        w("xr[hf * 128 + x128] = R; if (hf) xr[256 + x128] = P;")
+        w(f"xr[tid] = R; xr[{NT} + tid] = P;")
         w("frnn_block_sync();")
-        w("R = xr[x128] + xr[128 + x128] + (hf ? 0.0f : xr[256 + x128]);")
+        w("R = 0.0f;")
+        w("#pragma unroll")
+        w(f"for (int o = 0; o < {parts}; o++) R += xr[o * 128 + x128] + (o > hf ? xr[{NT} + o * 128 + x128] : 0.0f);")
     for x in range(n_nsum):
         w(f"float e{x}[{HC}];")
     w("#pragma unroll")
@@ -2167,7 +2217,7 @@ def emit_vector_grads(p: Problem, nf: Normal, bp: BackwardPlan, dspec: Sequence[
         if dec_sc and want_gw:
             w("float R = 0.0f, wdw = 0.0f;")
             w("#pragma unroll")
-            w(f"for (int k = 0; k < {VG_THREADS // 32}; k++) R += part[{n_nsum * 4 * C} + k];")
+            w(f"for (int k = 0; k < {NT // 32}; k++) R += part[{n_nsum * 4 * C} + k];")
             w(f"for (int l = nv - 1; l >= q; l--) {{ wdw = R - {total(n_nsum - 2, 'l')}; R = wdw + {total(n_nsum - 1, 'l')}; }}")
             w(f"{slot('gw')} + q] = slow ? {total(n_nsum - 2, 'q')} : " + ("wdw;" if bp.log_decay else f"frnn_divf(wdw, {slot(nf.decay)} + q]);"))
         scalar_nodes(third_s)
@@ -2183,13 +2233,13 @@ def emit_vector_grads(p: Problem, nf: Normal, bp: BackwardPlan, dspec: Sequence[
     w("(void)ok;")
     w.close()
     # cycles the tensor cores are busy for one CTA: L, the slices of S_0 and E_C (each in two terms), what follows from L
-    pa, pk = product_cycles(2 * nA, True), product_cycles(2 * nK, True)
-    busy = M // 8 * (pk + 2 * pa + 2 * pk) + 2 * (nK // 8) * pa + 2 * (nA // 8) * pk
-    return KernelSource("frnn_cvg", w.text().replace("@SMEM_BYTES@", str(smem_bytes)), (nchunk, H, B), VG_THREADS, smem_bytes, params, decl,
+    pa, pk = product_cycles(RX, True), product_cycles(RZ, True)
+    busy = M // 8 * (pk + 2 * pa + 2 * pk) + nK // 8 * (2 if xk else 4) * product_cycles(nA, True) + nA // 8 * (2 if xa else 4) * product_cycles(nK, True)
+    return KernelSource("frnn_cvg", w.text().replace("@SMEM_BYTES@", str(smem_bytes)), (nchunk, H, B), NT, smem_bytes, params, decl,
                         {"chunk": C, "tile": [1, N, M], "packed": False, "tmem_cols": tm_cols, "tensor_cycles": busy}, [])
 
 
-def emit_slow_columns(w, C, nd, nr, nA, nK, tq, live_n, sel, nf, bp, dec_vec, want_gw, Stage, leaf, leaves_of, slot, LS, cD1, cD2, off_slow):
+def emit_slow_columns(w, C, nd, nr, nA, nK, tq, live_n, sel, nf, bp, dec_vec, want_gw, Stage, leaf, leaves_of, slot, LS, acc, off_slow):
     """Columns of a chunk with a decay too small to divide by: running products in plain loops, by the first four warps;
     the results (d alpha, d kappa, d decay for all timesteps) go through shared memory."""
     w.open("if (slow)")
@@ -2198,12 +2248,15 @@ def emit_slow_columns(w, C, nd, nr, nA, nK, tq, live_n, sel, nf, bp, dec_vec, wa
     w.open("if (tid < 128)")
     w(f"float* sl = (float*)(smem + {off_slow});")
     w(f"float ka[{nK}], aa[{nA}], ta[{nA}], tk[{nK}], xs[{C}];")
-    for arr, cnt, colx in (("ta", nA, cD1), ("tk", nK, cD2)):
+    for arr, cnt, (colx, inexact) in (("ta", nA, acc[0]), ("tk", nK, acc[1])):
         w.open("")
-        w(f"float u[{cnt}], lo[{cnt}];")
-        w(f"frnn_tmem_ld<{cnt}>(lanes + {colx}u, u); frnn_tmem_ld<{cnt}>(lanes + {colx + cnt}u, lo); frnn_tmem_wait_ld();")
+        w(f"float u[{cnt}], lo[{max(1, len(inexact)) * C}]; (void)lo;")
+        w(f"frnn_tmem_ld<{cnt}>(lanes + {colx}u, u);" + (f" frnn_tmem_ld<{len(inexact) * C}>(lanes + {colx + cnt}u, lo);" if inexact else "") + " frnn_tmem_wait_ld();")
+        for k, x in enumerate(inexact):
+            w("#pragma unroll")
+            w(f"for (int k = 0; k < {C}; k++) u[{x * C} + k] += lo[{k * C} + k];")
         w("#pragma unroll")
-        w(f"for (int k = 0; k < {cnt}; k++) {arr}[k] = u[k] + lo[k];")
+        w(f"for (int k = 0; k < {cnt}; k++) {arr}[k] = u[k];")
         w.close()
     names = nf.alphas + nf.kappas + [nf.decay]
     lv = leaves_of(names, (0, 1))
