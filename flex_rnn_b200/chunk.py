@@ -1595,6 +1595,7 @@ def emit_vector_grads(p: Problem, nf: Normal, bp: BackwardPlan, dspec: Sequence[
     xa, xk = not dec_vec and all(map(is16, nf.alphas)), not dec_vec and all(map(is16, nf.kappas))
     RX, RZ = nA + C * len(restX), nK + C * len(restZ)        # rows of X and Z: the vectors, then the rests of the inexact ones
     slow_path = bool(nf.decay) and (dec_vec or want_gw)
+    few = dec_vec and want_gw and not bp.log_decay
     # padding: the eight threads of a store's phase write to different banks
     lboX, lboZ = RX * 16 + 16, RZ * 16 + 16
     lboT, lbo1, lbo2 = 128 * 16, 2 * nA * 16, 2 * nK * 16 + 16
@@ -1610,7 +1611,8 @@ def emit_vector_grads(p: Problem, nf: Normal, bp: BackwardPlan, dspec: Sequence[
             self.part = self.sc + al(len(sc_slots) * C * 4)
             self.z0 = self.part + al(npart * 4 * C * 4)
             self.xr = self.z0 + al(128 * 4)             # what the threads of a column exchange
-            self.X = self.xr + al(2 * 128 * parts * 4)
+            self.few = self.xr + al(2 * 128 * parts * 4)   # columns with a decay too small to divide its gradient by
+            self.X = self.few + (512 if few else 0)
             self.Z = self.X + al((M // 4 - 1) * lboX + max(2048 + 16, lboX))
             self.sl = self.Z + al(M // 4 * lboZ)
             self.lboS = 128 * 16 + 128 // (MS // 4)
@@ -1622,13 +1624,12 @@ def emit_vector_grads(p: Problem, nf: Normal, bp: BackwardPlan, dspec: Sequence[
             self.L1 = self.aT + (1 if xa else 2) * aT_b
             self.L2 = self.L1 + nK // 4 * lbo1
             self.Lr = self.L2 + nA // 4 * lbo2
-            self.slow = self.kT                         # the slow path's results, over the operands it does without: (nA + nK + C) x 128 floats
+            # the slow path's results: (nA + nK) x 128 floats over the operands it does without, gradients of the decays beside them
+            self.slow = self.kT
             if slow_path and dec_vec:
-                self.Lr = max(self.Lr, self.slow + (nA + nK + C) * 512)
-            self.bytes = al(max(end1, self.Lr + nA * LS * 4))
-            if slow_path and not dec_vec:               # the gradients of a decay per head only: beside the operands, which stay
-                self.slow = al(self.Lr + nA * LS * 4) - (nA + nK) * 512
-                self.bytes = al(max(self.bytes, self.slow + (nA + nK + C) * 512))
+                self.Lr = max(self.Lr, self.slow + (nA + nK) * 512)
+            self.gw = al(self.Lr + nA * LS * 4)
+            self.bytes = al(max(end1, self.gw + (C * 512 if slow_path and want_gw else 0)))
             self.ctas = 2 if self.bytes <= SMEM_BYTES // 2 - 1024 else 1
     # two CTAs of 256 threads share an SM and hide each other's latencies; where X and Z are too large for that, one of 512 with
     # two buffers of slices (B8 T1024 H32, us: RWKV-7 128x128 1096 against 1276 with one CTA, Mamba-2 64x128 467 against 546; Delta
@@ -1643,7 +1644,7 @@ def emit_vector_grads(p: Problem, nf: Normal, bp: BackwardPlan, dspec: Sequence[
     HC = C // parts                          # timesteps of one thread
     lboS, sl_bytes, smem_bytes = lay.lboS, lay.sl_bytes, lay.bytes
     off_sc, off_part, off_z0, off_xr, off_X, off_Z, off_sl = lay.sc, lay.part, lay.z0, lay.xr, lay.X, lay.Z, lay.sl
-    off_kT, off_aT, off_L1, off_L2, off_Lr, off_slow = lay.kT, lay.aT, lay.L1, lay.L2, lay.Lr, lay.slow
+    off_kT, off_aT, off_L1, off_L2, off_Lr, off_slow, off_gw = lay.kT, lay.aT, lay.L1, lay.L2, lay.Lr, lay.slow, lay.gw
     cD1, cD2 = 0, RX
     cL = cD2 + RZ
     tm_cols = _tmem_pow2(cL + RZ)
@@ -1794,7 +1795,10 @@ def emit_vector_grads(p: Problem, nf: Normal, bp: BackwardPlan, dspec: Sequence[
         w.close()
     for u in range(min(DP, nsl)):
         load_slice(str(u), str(u))
-    w("if (tid == 0) { frnn_mbar_init(&bar[0], 1); frnn_mbar_init(&bar[1], 1); frnn_mbar_init(&bar[2], 1); frnn_mbar_init(&bar[5], 1); ((int*)&bar[4])[0] = 0; frnn_mbar_init_fence(); }")
+    w("if (tid == 0) { frnn_mbar_init(&bar[0], 1); frnn_mbar_init(&bar[1], 1); frnn_mbar_init(&bar[2], 1); frnn_mbar_init(&bar[5], 1); bar[4] = 0; frnn_mbar_init_fence(); }")
+    if few:
+        w(f"int* fewc = (int*)(smem + {lay.few});")
+        w("if (tid < 128) fewc[tid] = 0;")
     w.open("if (warp == 0)")
     w(f"frnn_tmem_alloc((u32*)&bar[3], {tm_cols}u);")
     w("frnn_tmem_fence_before_sync();")
@@ -2003,7 +2007,6 @@ def emit_vector_grads(p: Problem, nf: Normal, bp: BackwardPlan, dspec: Sequence[
         w(f"const int q = q0 + k; const bool live = {live_n}; (void)live;")
         e = Stage("x_", "q", N1, {a: f"{reg(a)}[k]" for a in nleaves}).get(nf.decay)
         w(f"xw[k] = {sel(live_n, e, '1.0f')};")
-        tiny = "1e-25f" if bp.log_decay or not want_gw else "0.0009765625f"
         w("wlo = fminf(wlo, fabsf(xw[k]));")
         w.close()
         w("prod *= xw[k];")
@@ -2041,7 +2044,11 @@ def emit_vector_grads(p: Problem, nf: Normal, bp: BackwardPlan, dspec: Sequence[
         w("}")
     w.close()
     if dec_vec:
-        w(f"if (!(wlo > {tiny} && whi < 1e25f)) *(volatile int*)&bar[4] = 1;")
+        w("if (!(wlo > 1e-25f && whi < 1e25f)) *(volatile int*)&bar[4] = 1;")
+        if few:
+            # a decay that is merely too small for its own gradient (dW/W, by a division) does not send the chunk down the slow
+            # path, 160 us for a CTA: RWKV-7's decays fall below 2^-10 about once in two million
+            w("if (!(wlo > 0.0009765625f)) { fewc[x128] = 1; ((volatile int*)&bar[4])[1] = 1; }")
     # ---- the parts of the accumulators so far, from S_0 and E_C, scaled to what those from L need
     w("float R = 0.0f; (void)R;")
 
@@ -2071,8 +2078,10 @@ def emit_vector_grads(p: Problem, nf: Normal, bp: BackwardPlan, dspec: Sequence[
         w.close()
     w("frnn_block_sync();")
     w("const bool slow = *(volatile int*)&bar[4] != 0; (void)slow;")
+    if few:
+        w("const bool few = ((volatile int*)&bar[4])[1] != 0;")
     if slow_path:
-        emit_slow_columns(w, C, nd, nr, nA, nK, tq, live_n, sel, nf, bp, dec_vec, want_gw, Stage, leaf, leaves_of, slot, LS, ((cD1, restX), (cD2, restZ)), off_slow)
+        emit_slow_columns(w, C, nd, nr, nA, nK, tq, live_n, sel, nf, bp, dec_vec, want_gw, Stage, leaf, leaves_of, slot, LS, ((cD1, restX), (cD2, restZ)), off_slow, off_gw, few)
     if nf.decay:
         w.open("if (!slow)" if dec_vec else "")
         w(f"float dk[{nr * HC}];")
@@ -2143,7 +2152,7 @@ def emit_vector_grads(p: Problem, nf: Normal, bp: BackwardPlan, dspec: Sequence[
           + " ".join(f"dk[{r * HC} + k] *= ra;" for r in range(nr)) + " a *= xw[k]; }")
         w.close()
     if slow_path:
-        w(f"const float* sl = (const float*)(smem + {off_slow});")
+        w(f"const float* sl = (const float*)(smem + {off_slow}); const float* gwp = (const float*)(smem + {off_gw}); (void)sl; (void)gwp;")
     if dec_vec:
         w.open("if (slow)")
         w("#pragma unroll")
@@ -2180,11 +2189,11 @@ def emit_vector_grads(p: Problem, nf: Normal, bp: BackwardPlan, dspec: Sequence[
     if want_gw:
         kd = " + ".join(f"{st.get(nm)} * dk[{r * HC} + k]" for r, nm in enumerate(nf.kappas))
         ad = " + ".join(f"{st.get(nm)} * da[{d * HC} + k]" for d, nm in enumerate(nf.alphas))
-        gws = f"sl[({nA + nK} + q) * 128 + x128]"
+        gws = "gwp[q * 128 + x128]"
         if dec_vec:
             w(f"const float wdw = R - {sel(live_n, f'({kd})')};")
             w(f"R = wdw + {sel(live_n, f'({ad})')};")
-            w(f"const float gw = slow ? {gws} : " + ("wdw;" if bp.log_decay else "frnn_divf(wdw, xw[k]);"))
+            w(f"const float gw = slow{' || !(fabsf(xw[k]) > 0.0009765625f)' if few else ''} ? {gws} : " + ("wdw;" if bp.log_decay else "frnn_divf(wdw, xw[k]);"))
             st.done["gw"] = "gw"
         else:
             w(f"e{n_nsum - 2}[k] = {sel(live_n, f'(slow ? {gws} : {kd})')}; e{n_nsum - 1}[k] = {sel(live_n, f'({ad})')};")
@@ -2239,14 +2248,15 @@ def emit_vector_grads(p: Problem, nf: Normal, bp: BackwardPlan, dspec: Sequence[
                         {"chunk": C, "tile": [1, N, M], "packed": False, "tmem_cols": tm_cols, "tensor_cycles": busy}, [])
 
 
-def emit_slow_columns(w, C, nd, nr, nA, nK, tq, live_n, sel, nf, bp, dec_vec, want_gw, Stage, leaf, leaves_of, slot, LS, acc, off_slow):
+def emit_slow_columns(w, C, nd, nr, nA, nK, tq, live_n, sel, nf, bp, dec_vec, want_gw, Stage, leaf, leaves_of, slot, LS, acc, off_slow, off_gw, few):
     """Columns of a chunk with a decay too small to divide by: running products in plain loops, by the first four warps;
-    the results (d alpha, d kappa, d decay for all timesteps) go through shared memory."""
-    w.open("if (slow)")
+    the results (d alpha, d kappa, d decay for all timesteps) go through shared memory.  ``few``: where only
+    single decays are too small for their own gradients, these alone."""
+    w.open("if (slow || few)" if few else "if (slow)")
     w("frnn_tmem_fence_before_sync();")
     w("frnn_block_sync();         // the operands are no longer read")
     w.open("if (tid < 128)")
-    w(f"float* sl = (float*)(smem + {off_slow});")
+    w(f"float* sl = (float*)(smem + {off_slow}); float* gwp = (float*)(smem + {off_gw}); (void)sl; (void)gwp;")
     w(f"float ka[{nK}], aa[{nA}], ta[{nA}], tk[{nK}], xs[{C}];")
     for arr, cnt, (colx, inexact) in (("ta", nA, acc[0]), ("tk", nK, acc[1])):
         w.open("")
@@ -2258,6 +2268,8 @@ def emit_slow_columns(w, C, nd, nr, nA, nK, tq, live_n, sel, nf, bp, dec_vec, wa
         w("#pragma unroll")
         w(f"for (int k = 0; k < {cnt}; k++) {arr}[k] = u[k];")
         w.close()
+    if few:                                  # (Tensor Memory is read by whole warps)
+        w.open("if (slow || fewc[x128])")
     names = nf.alphas + nf.kappas + [nf.decay]
     lv = leaves_of(names, (0, 1))
     w("#pragma unroll 1")
@@ -2276,6 +2288,8 @@ def emit_slow_columns(w, C, nd, nr, nA, nK, tq, live_n, sel, nf, bp, dec_vec, wa
         w("const float Z = ncol ? z0[x128] : 0.0f;")
         w("#pragma unroll 1")
         w.open(f"for (int j = 0; j < {C}; j++)")
+        if few:
+            w("if (!slow && fabsf(xs[j]) > 0.0009765625f) continue;")
         w("float A = 1.0f, Bj = 1.0f, g = 0.0f, s0 = 0.0f, Q = 1.0f;")
         w("for (int l = 0; l < j; l++) A *= xs[l];")
         w(f"for (int l = j + 1; l < {C}; l++) Bj *= xs[l];")
@@ -2294,9 +2308,10 @@ def emit_slow_columns(w, C, nd, nr, nA, nK, tq, live_n, sel, nf, bp, dec_vec, wa
         w.close()
         w("P *= xs[l];")
         w.close()
-        w(f"sl[({nA + nK} + j) * 128 + x128] = g" + (" * xs[j];" if bp.log_decay else ";"))
+        w(f"gwp[j * 128 + x128] = g" + (" * xs[j];" if bp.log_decay else ";"))
         w.close()
     if dec_vec:
+        w.open("if (slow)")
         w("float a = 1.0f;")
         w("#pragma unroll 1")
         w(f"for (int q = 0; q < {C}; q++) {{ for (int d = 0; d < {nd}; d++) ta[d * {C} + q] *= a; a *= xs[q]; }}")
@@ -2318,6 +2333,9 @@ def emit_slow_columns(w, C, nd, nr, nA, nK, tq, live_n, sel, nf, bp, dec_vec, wa
         w(f"for (int k = 0; k < {nA}; k++) sl[k * 128 + x128] = ta[k];")
         w("#pragma unroll 1")
         w(f"for (int k = 0; k < {nK}; k++) sl[({nA} + k) * 128 + x128] = tk[k];")
+        w.close()
+    if few:
+        w.close()
     w.close()
     w("frnn_block_sync();")
     w("frnn_tmem_fence_after_sync();")

@@ -228,3 +228,36 @@ def test_timed_candidates_are_checked_builds(monkeypatch):
     fwd.infer(ins, (s,))
     assert [sum(ks.name == n for ks in made) for n in ("frnn_cfw", "frnn_cbw", "frnn_cvg")] == [6, 3, 1]
     assert all(ks.info.get("bounds") for ks in made)
+
+
+def small_decays(op, B, T, H, M, N, small):
+    """RWKV-7 with a few decays per chunk that are small, whose own gradients are not formed by a division, but whose
+    products over a chunk are still divided by."""
+    step, ins, s, dy, dS = case(op, B, T, H, M, N, torch.bfloat16)
+    g = torch.Generator().manual_seed(5)
+    hit = torch.rand(ins[1].shape, generator=g) < 0.02
+    ins[1] = torch.where(hit, torch.full_like(ins[1], small), ins[1])
+    return step, ins, s, dy, dS
+
+
+# 40 columns: the last two warps of a tile have threads without one; 128 rows and columns: the benchmark's state
+@pytest.mark.parametrize("T,M,N,small", [(33, 24, 40, 2e-4), (32, 16, 128, 1e-5)])
+def test_small_decays_emulated(T, M, N, small):
+    from emu.emu import EmuLauncher
+    step, ins, s, dy, dS = small_decays("rwkv7", 1, T, 1, M, N, small)
+    fwd, bwd, _, _ = build_twopass(step, tuple(ins), (s,), _launcher=EmuLauncher)
+    y, sT, ck, aux = fwd(tuple(ins), (s,))
+    dx, ds = bwd((dy.to(y.dtype),), (dS,), tuple(ins), (ck,), (aux,))
+    check([y, sT, *dx, *ds], step, ins, s, dy, dS, torch.bfloat16)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("T,M,N,small", [(33, 24, 40, 2e-4), (100, 128, 128, 1e-5)])
+def test_small_decays_gpu(T, M, N, small):
+    step, ins, s, dy, dS = small_decays("rwkv7", 2, T, 2, M, N, small)
+    f = flex_rnn_b200.jit(step)
+    leaves = [x.cuda().requires_grad_() for x in [*ins, s]]
+    y, sT = f(*leaves)
+    grads = torch.autograd.grad((y, sT), leaves, (dy.cuda().to(y.dtype), dS.cuda()))
+    assert f.forward_func.kernel_status("cuda:0") == 0
+    check([y.detach(), sT.detach(), *grads], step, ins, s, dy, dS, torch.bfloat16)
