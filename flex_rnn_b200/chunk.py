@@ -1795,7 +1795,7 @@ def emit_vector_grads(p: Problem, nf: Normal, bp: BackwardPlan, dspec: Sequence[
         w.close()
     for u in range(min(DP, nsl)):
         load_slice(str(u), str(u))
-    w("if (tid == 0) { frnn_mbar_init(&bar[0], 1); frnn_mbar_init(&bar[1], 1); frnn_mbar_init(&bar[2], 1); frnn_mbar_init(&bar[5], 1); bar[4] = 0; frnn_mbar_init_fence(); }")
+    w("if (tid == 0) { frnn_mbar_init(&bar[0], 1); frnn_mbar_init(&bar[1], 1); frnn_mbar_init(&bar[2], 1); frnn_mbar_init(&bar[5], 1); frnn_mbar_init_fence(); }")
     if few:
         w(f"int* fewc = (int*)(smem + {lay.few});")
         w("if (tid < 128) fewc[tid] = 0;")
@@ -1806,6 +1806,7 @@ def emit_vector_grads(p: Problem, nf: Normal, bp: BackwardPlan, dspec: Sequence[
     # ---- scalars of the inputs, decay products
     w.open(f"if (tid >= 32 && tid < {32 + C})")
     w(f"const int q = tid - 32, t = {'t0 + q' if whole else 't0 + min(q, nv - 1)'}; (void)t;")
+    w("if (q == 0) bar[4] = 0;      // two flags, set by these threads after they have met, or by all after the block barrier")
     for i in s_inputs:
         w(f"{slot(nf.inputs[i])} + q] = frnn_io<{p.inputs[i].dt}>::ld(in{i}, {in_off(i, 't')});")
     for k in use_dg:
