@@ -1503,8 +1503,11 @@ def emit_vector_grads(p: Problem, nf: Normal, bp: BackwardPlan, dspec: Sequence[
     (``local_vjp``).  All products run on the tensor cores.  Where a decay of the chunk is too small to divide by, the
     chunk takes a slower path of plain loops with running products instead.
 
-    S_0 and E_C are 2 x 4 M N bytes per C timesteps, 1.1 us at HBM's rate for 128x128; the stores that bring them and their rests
-    into the tensor cores' layout and the products' reads of them keep shared memory busy for longer.  Parameters, in order: inputs, d outputs, forward row sums, kept row sums, checkpoints of S, of E,
+    S_0, E_C and the row vectors stream through in slices of 16 rows, which are what the products sum over: X and Z of a slice are
+    made beside it (all of X and Z at once took 100 KB, one CTA per SM, and the load phases of all SMs coincided: Delta Rule
+    128x128 B8 T1024 H32 640 us, in slices 493).  The bytes of a chunk, 200 KB for the Delta Rule, take 8.1 of 16.6 thousand cycles
+    at the copy rate; the stores of the slices and the products' reads of them keep shared memory busy for about as long.
+    Parameters, in order: inputs, d outputs, forward row sums, kept row sums, checkpoints of S, of E,
     gradients, error word.
     """
     v = bp.vjp
@@ -1584,7 +1587,7 @@ def emit_vector_grads(p: Problem, nf: Normal, bp: BackwardPlan, dspec: Sequence[
     n_nsum = len(nsums) + (2 if dec_sc and want_gw else 0)
     for x in ("Wp", "Ws", "gw"):
         slot(x)
-    npart = max(len(msums), n_nsum) + 1
+    npart = n_nsum + 1
     # which operands are plain 16-bit inputs, exact in tf32: they have no second term
     dt16 = (lower.DT_BF16, lower.DT_F16)
     leaf_dt = {nf.inputs[i]: p.inputs[i].dt for i in range(nin)}
@@ -1597,7 +1600,7 @@ def emit_vector_grads(p: Problem, nf: Normal, bp: BackwardPlan, dspec: Sequence[
     slow_path = bool(nf.decay) and (dec_vec or want_gw)
     few = dec_vec and want_gw and not bp.log_decay
     # padding: the eight threads of a store's phase write to different banks
-    lboX, lboZ = RX * 16 + 16, RZ * 16 + 16
+    lboX, lboZ = RX * 16 + 32, RZ * 16 + 32
     lboT, lbo1, lbo2 = 128 * 16, 2 * nA * 16, 2 * nK * 16 + 16
     LS = nK + 1
     kT_b, aT_b = nK // 4 * lboT, nA // 4 * lboT
@@ -1612,14 +1615,16 @@ def emit_vector_grads(p: Problem, nf: Normal, bp: BackwardPlan, dspec: Sequence[
             self.z0 = self.part + al(npart * 4 * C * 4)
             self.xr = self.z0 + al(128 * 4)             # what the threads of a column exchange
             self.few = self.xr + al(2 * 128 * parts * 4)   # columns with a decay too small to divide its gradient by
-            self.X = self.few + (512 if few else 0)
-            self.Z = self.X + al((M // 4 - 1) * lboX + max(2048 + 16, lboX))
-            self.sl = self.Z + al(M // 4 * lboZ)
+            # a buffer holds a slice of S_0, E_C and their rests, and of X (as first operand 128 rows of it are read) and Z
+            self.sl = self.few + (512 if few else 0)
             self.lboS = 128 * 16 + 128 // (MS // 4)
             self.sl_bytes = al(MS // 4 * self.lboS)
-            end1 = self.sl + 4 * NB * self.sl_bytes
+            self.X = 4 * self.sl_bytes
+            self.Z = self.X + al((MS // 4 - 1) * lboX + max(2048, RX * 16))
+            self.buf = self.Z + al(MS // 4 * lboZ)
+            end1 = self.sl + NB * self.buf
             # second phase, over the same memory
-            self.kT = self.X
+            self.kT = self.sl
             self.aT = self.kT + (1 if xk else 2) * kT_b
             self.L1 = self.aT + (1 if xa else 2) * aT_b
             self.L2 = self.L1 + nK // 4 * lbo1
@@ -1631,19 +1636,20 @@ def emit_vector_grads(p: Problem, nf: Normal, bp: BackwardPlan, dspec: Sequence[
             self.gw = al(self.Lr + nA * LS * 4)
             self.bytes = al(max(end1, self.gw + (C * 512 if slow_path and want_gw else 0)))
             self.ctas = 2 if self.bytes <= SMEM_BYTES // 2 - 1024 else 1
-    # two CTAs of 256 threads share an SM and hide each other's latencies; where X and Z are too large for that, one of 512 with
-    # two buffers of slices (B8 T1024 H32, us: RWKV-7 128x128 1096 against 1276 with one CTA, Mamba-2 64x128 467 against 546; Delta
-    # Rule 128x128, which two CTAs fit with slices of 8 rows only, 687 against 638)
-    lay = Layout(16, 1, 2) if M % 16 == 0 else Layout(8, 1, 2)
-    if lay.ctas == 1 and M % 16 == 0:
-        lay = Layout(16, 2, 4)
+    # two CTAs of 256 threads share an SM and hide each other's latencies, with two buffers of slices where they fit (B8 T1024 H32,
+    # us, two buffers, one, and one CTA of 512 threads with two: Delta Rule 128x128 493, 519, 508; RWKV-7 988, 1019, 1322; Mamba-2
+    # 64x128 441, 441, 457)
+    for NB in (2, 1):
+        lay = Layout(16 if M % 16 == 0 else 8, NB, 2)
+        if lay.ctas == 2:
+            break
     MS, NB, parts, ctas = lay.MS, lay.NB, lay.parts, lay.ctas
-    DP = 16 * 2 * NB // MS                   # slices that are loaded ahead
+    DP = 2                                   # slices that are loaded ahead
     nsl = M // MS
     NT = 128 * parts                         # 128 rows or columns times ``parts`` parts of the chunk's timesteps
     HC = C // parts                          # timesteps of one thread
     lboS, sl_bytes, smem_bytes = lay.lboS, lay.sl_bytes, lay.bytes
-    off_sc, off_part, off_z0, off_xr, off_X, off_Z, off_sl = lay.sc, lay.part, lay.z0, lay.xr, lay.X, lay.Z, lay.sl
+    off_sc, off_part, off_z0, off_xr, off_sl = lay.sc, lay.part, lay.z0, lay.xr, lay.sl
     off_kT, off_aT, off_L1, off_L2, off_Lr, off_slow, off_gw = lay.kT, lay.aT, lay.L1, lay.L2, lay.Lr, lay.slow, lay.gw
     cD1, cD2 = 0, RX
     cL = cD2 + RZ
@@ -1658,7 +1664,6 @@ def emit_vector_grads(p: Problem, nf: Normal, bp: BackwardPlan, dspec: Sequence[
     whole = T % C == 0
     tq = lambda q: f"t0 + {q}" if whole else f"t0 + min({q}, nv - 1)"
     live_n = " && ".join(([] if whole else ["q < nv"]) + ([] if full_n else ["ncol"])) or "true"
-    live_m = " && ".join(([] if whole else ["q < nv"]) + ([] if M == 128 else ["mrow"])) or "true"
     sel = lambda live, e, z="0.0f": e if live == "true" else f"(live ? {e} : {z})"
 
     w(lower._header(chunk_prelude()))
@@ -1766,18 +1771,16 @@ def emit_vector_grads(p: Problem, nf: Normal, bp: BackwardPlan, dspec: Sequence[
 
     # ---- what can be loaded at once: the rows' vectors, the first slices of S_0 and E_C
     w(f"const int x128 = tid & 127, hf = tid >> 7, q0 = hf * {HC};")
-    w(f"const int mc = {'x128' if M == 128 else f'min(x128, {M - 1})'}, nc = {'x128' if full_n else f'min(x128, {N - 1})'};")
-    w(f"const bool mrow = x128 < {M}, ncol = x128 < {N}; (void)mrow; (void)ncol; (void)nc;")
+    w(f"const int nc = {'x128' if full_n else f'min(x128, {N - 1})'};")
+    w(f"const bool ncol = x128 < {N}; (void)ncol; (void)nc;")
     mleaves = leaves_of(list(bp.dsig) + list(nf.ps) + [n.args[0] for n in msums], M1)
     reg = lambda a: "r_" + a.replace(".", "_")
+    QG = NT // MS                            # in a slice a thread has row mi and every QG-th timestep
+    nq = max(1, C // QG)
+    w(f"const int mi = tid % {MS}, qg = tid / {MS};")
     for a in mleaves:
-        w(f"float {reg(a)}[{HC}];")
-    w("#pragma unroll")
-    w.open(f"for (int k = 0; k < {HC}; k++)")
-    w(f"const int t = {tq('q0 + k')};")
-    for a in mleaves:
-        w(f"{reg(a)}[k] = {leaf(a, 't', 'mc')};")
-    w.close()
+        w(f"float {reg(a)}[{DP}][{nq}];")
+    at_q = lambda i: f"qg + {QG * i}" if QG <= C else f"min(qg, {C - 1})"
     q4 = MS // 4
     per = 128 // (NT // q4)        # columns per thread and slice
     w(f"const int sm4 = tid % {q4}, sn = tid / {q4};")
@@ -1793,6 +1796,8 @@ def emit_vector_grads(p: Problem, nf: Normal, bp: BackwardPlan, dspec: Sequence[
         w(f"frnn_ldv<0,4>(ckp, n * {M}L + ({sx}) * {MS} + sm4 * 4, sv[{u}][i]);")
         w(f"frnn_ldv<0,4>(ekp, n * {M}L + ({sx}) * {MS} + sm4 * 4, ev[{u}][i]);")
         w.close()
+        for i in range(nq):
+            w(f"{{ const int t = {tq(f'({at_q(i)})')}, m = ({sx}) * {MS} + mi; " + " ".join(f"{reg(a)}[{u}][{i}] = {leaf(a, 't', 'm')};" for a in mleaves) + " }")
     for u in range(min(DP, nsl)):
         load_slice(str(u), str(u))
     w("if (tid == 0) { frnn_mbar_init(&bar[0], 1); frnn_mbar_init(&bar[1], 1); frnn_mbar_init(&bar[2], 1); frnn_mbar_init(&bar[5], 1); frnn_mbar_init_fence(); }")
@@ -1827,44 +1832,30 @@ def emit_vector_grads(p: Problem, nf: Normal, bp: BackwardPlan, dspec: Sequence[
     w("frnn_block_sync();")
     w("frnn_tmem_fence_after_sync();")
     w("const u32 tm = *(volatile u32*)&bar[3];")
-    # ---- rows: X, Z and the sums over the rows
-    w.open("")
     for x in range(len(msums)):
-        w(f"float e{x}[{HC}];")
-    w("#pragma unroll")
-    w.open(f"for (int k = 0; k < {HC}; k++)")
-    w(f"const int q = q0 + k; const bool live = {live_m}; (void)live;")
-    st = Stage("x_", "q", M1, {a: f"{reg(a)}[k]" for a in mleaves})
-    vals = [(d, st.get(x), "X") for d, x in enumerate(bp.dsig)] + [(r, st.get(x), "Z") for r, x in enumerate(nf.ps)]
-    for x, n in enumerate(msums):
-        w(f"e{x}[k] = {sel(live_m, st.get(n.args[0]))};")
-    w.open(f"if (mrow)" if M < 128 else "")
-    for v_, val, which in vals:
-        lbo, off, inexact, n2 = (lboX, off_X, restX, nA) if which == "X" else (lboZ, off_Z, restZ, nK)
-        put = lambda row0, x: f"{{ const int row = {row0} + q; *(float*)(dst + (row >> 3) * 128 + (row & 7) * 16) = {x}; }}"
-        w(f"{{ const float a = {sel(live_m, val)}; unsigned char* dst = smem + {off} + (x128 >> 2) * {lbo} + (x128 & 3) * 4; {put(v_ * C, 'a')}"
-          + (" " + put(at_rest(inexact, v_, n2), "frnn_tf32_rest(a)") if v_ in inexact else "") + " }")
-    w.close()
-    w.close()
-    for x in range(len(msums)):
-        reduce_lanes(f"e{x}", HC, f"part[{x * 4 * C} + (warp & 3) * {C} + q0 + @]")
-    w.close()
-    w("frnn_async_proxy_fence();")
-    w("frnn_block_sync();")
-    w(f"const u64 dX = frnn_mma_desc(smem + {off_X}, {lboX}), dZ = frnn_mma_desc(smem + {off_Z}, {lboZ});")
-    w.open("if (warp == 0 && frnn_elect())")
-    w("#pragma unroll")
-    w(f"for (int k = 0; k < {M // 8}; k++) frnn_mma_ss_d(tm + {cL}u, frnn_mma_next(dX, {lboX}, k), frnn_mma_next(dZ, {lboZ}, k), FRNN_MMA_IDESC({RZ}), k > 0);")
-    w("frnn_mma_commit(&bar[0]);")
-    w.close()
-    # ---- second-stage scalars
-    w.open(f"if (tid >= 32 && tid < {32 + C})")
-    w("const int q = tid - 32; (void)q;")
-    for x, n in enumerate(msums):
-        w(f"{slot(n.name)} + q] = (part[{x * 4 * C} + q] + part[{x * 4 * C + C} + q]) + (part[{x * 4 * C + 2 * C} + q] + part[{x * 4 * C + 3 * C} + q]);")
-    scalar_nodes(second_s)
-    w.close()
-    # ---- S_0 and E_C, a slice of rows at a time, loaded two slices ahead
+        w(f"float rs{x}[{nq}];")
+        w("#pragma unroll")
+        w(f"for (int i = 0; i < {nq}; i++) rs{x}[i] = 0.0f;")
+    live_m = " && ".join(([] if whole else ["q < nv"]) + ([] if QG <= C else [f"qg < {C}"])) or "true"
+
+    def put_rows(u: int, buf: int):
+        """This thread's values of X and Z for a slice of rows, into buffer ``buf``, and their parts of the sums over the rows."""
+        for i in range(nq):
+            w.open("")
+            w(f"const int q = {at_q(i)}; const bool live = {live_m}; (void)live;")
+            st = Stage("x_", "q", M1, {a: f"{reg(a)}[{u}][{i}]" for a in mleaves})
+            vals = [(d, st.get(x), "X") for d, x in enumerate(bp.dsig)] + [(r, st.get(x), "Z") for r, x in enumerate(nf.ps)]
+            for x, n in enumerate(msums):
+                w(f"rs{x}[{i}] += {sel(live_m, st.get(n.args[0]))};")
+            w.open("" if QG <= C else f"if (qg < {C})")
+            for v_, val, which in vals:
+                lbo, off, inexact, n2 = (lboX, lay.X, restX, nA) if which == "X" else (lboZ, lay.Z, restZ, nK)
+                put = lambda row0, x: f"{{ const int row = {row0} + q; *(float*)(dst + (row >> 3) * 128 + (row & 7) * 16) = {x}; }}"
+                w(f"{{ const float a = {sel(live_m, val)}; unsigned char* dst = smem + {buf + off} + (mi >> 2) * {lbo} + (mi & 3) * 4; {put(v_ * C, 'a')}"
+                  + (" " + put(at_rest(inexact, v_, n2), "frnn_tf32_rest(a)") if v_ in inexact else "") + " }")
+            w.close()
+            w.close()
+    # ---- S_0, E_C, X and Z, a slice of rows at a time, loaded two slices ahead
     colv = nf.alphas + nf.kappas + ([nf.decay] if dec_vec else [])
     ngiven = [f"ga{d}" for d in range(nd)] + [f"gk{r}" for r in range(nr)] + ["gw"]
     n_outs = [o for i, o in bp.grads if p.in_cls(i) == N1]
@@ -1884,7 +1875,7 @@ def emit_vector_grads(p: Problem, nf: Normal, bp: BackwardPlan, dspec: Sequence[
         w("#pragma unroll")
         w.open(f"for (int i = 0; i < {per}; i++)")
         w(f"const int n = sn + i * {NT // q4};")
-        off_b = off_sl + (u % NB) * 4 * sl_bytes
+        off_b = off_sl + (u % NB) * lay.buf
         w(f"unsigned char* dst = smem + {off_b} + sm4 * {lboS} + (n >> 3) * 128 + (n & 7) * 16;")
         w("float r[4];")
         w("#pragma unroll")
@@ -1894,6 +1885,7 @@ def emit_vector_grads(p: Problem, nf: Normal, bp: BackwardPlan, dspec: Sequence[
         w(f"for (int k = 0; k < 4; k++) r[k] = frnn_tf32_rest(ev[{u}][i][k]);")
         w(f"frnn_stv<0,4>(dst + {2 * sl_bytes}, 0, ev[{u}][i]); frnn_stv<0,4>(dst + {3 * sl_bytes}, 0, r);")
         w.close()
+        put_rows(u, off_b)
         w(f"if (s + {DP} < {nsl}) {{")
         w.ind += 1
         load_slice(f"s + {DP}", str(u))
@@ -1902,12 +1894,15 @@ def emit_vector_grads(p: Problem, nf: Normal, bp: BackwardPlan, dspec: Sequence[
         w("frnn_async_proxy_fence();")
         w("if (!frnn_block_and(arrived)) break;")
         w.open("if (warp == 0 && frnn_elect())")
+        first = lambda k: "s > 0" if k == 0 else "true"
         for k in range(MS // 8):
-            for which, (col_, dsc, lbo, n2) in enumerate(((cD1, "dX", lboX, RX), (cD2, "dZ", lboZ, RZ))):
+            w(f"frnn_mma_ss_d(tm + {cL}u, frnn_mma_desc(smem + {off_b + lay.X + k * 2 * lboX}, {lboX}), frnn_mma_desc(smem + {off_b + lay.Z + k * 2 * lboZ}, {lboZ}), FRNN_MMA_IDESC({RZ}), {first(k)});")
+        w(f"if (s == {nsl - 1}) frnn_mma_commit(&bar[0]);")
+        for k in range(MS // 8):
+            for which, (col_, at, lbo, n2) in enumerate(((cD1, lay.X, lboX, RX), (cD2, lay.Z, lboZ, RZ))):
                 sb = off_b + 2 * which * sl_bytes + k * 2 * lboS
-                bexp = f"frnn_mma_next({dsc}, {lbo}, s * {MS // 8} + {k})"
-                w(f"frnn_mma_ss_d(tm + {col_}u, frnn_mma_desc(smem + {sb}, {lboS}), {bexp}, FRNN_MMA_IDESC({n2}), {'s > 0' if k == 0 else 'true'});")
-                w(f"frnn_mma_ss_d(tm + {col_}u, frnn_mma_desc(smem + {sb + sl_bytes}, {lboS}), {bexp}, FRNN_MMA_IDESC({n2}), true);")
+                for part_ in (sb, sb + sl_bytes):
+                    w(f"frnn_mma_ss_d(tm + {col_}u, frnn_mma_desc(smem + {part_}, {lboS}), frnn_mma_desc(smem + {off_b + at + k * 2 * lbo}, {lbo}), FRNN_MMA_IDESC({n2}), {first(k) if part_ == sb else 'true'});")
         w(f"frnn_mma_commit(&bar[{bb}]);")
         w.close()
         w.close()
@@ -1926,12 +1921,24 @@ def emit_vector_grads(p: Problem, nf: Normal, bp: BackwardPlan, dspec: Sequence[
         w(f"for (int o = {q4 // 2}; o > 0; o >>= 1) zz[i] += frnn_shfl_xor(zz[i], o);")
         w(f"if (sm4 == 0) z0[sn + i * {NT // q4}] = zz[i];")
         w.close()
+    for x, n in enumerate(msums):
+        w("#pragma unroll")
+        w.open(f"for (int i = 0; i < {nq}; i++)")
+        w("#pragma unroll")
+        w(f"for (int o = {MS // 2}; o > 0; o >>= 1) rs{x}[i] += frnn_shfl_xor(rs{x}[i], o);")
+        w(f"if (mi == 0{'' if QG <= C else f' && qg < {C}'}) {slot(n.name)} + qg + {QG} * i] = rs{x}[i];")
+        w.close()
     w(f"bool ok = frnn_mbar_wait(&bar[0], 0, err, {ERR});")
     for u in range(min(NB, nsl)):
         uses = (nsl - u + NB - 1) // NB
         w(f"ok = frnn_mbar_wait(&bar[{5 if u else 1}], {(uses - 1) & 1}, err, {ERR}) && ok;")
     w("frnn_tmem_fence_after_sync();")
     w("frnn_block_sync();       // X, Z and the slices are no longer read")
+    if second_s:
+        w.open(f"if (tid >= 32 && tid < {32 + C})")
+        w("const int q = tid - 32; (void)q;")
+        scalar_nodes(second_s)
+        w.close()
     w("const u32 lanes = tm + frnn_tmem_lane_base(warp);")
     w(f"float* Lr = (float*)(smem + {off_Lr});")
     # ---- L: rows (d, j) of hi and of rest, columns (r, i) of hi and of rest; each half of the threads takes half of the i
