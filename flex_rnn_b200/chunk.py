@@ -523,6 +523,15 @@ class ColumnCode:
         return done
 
 
+def row_closure(nodes: Sequence[Node], names: Sequence[Arg]) -> set:
+    """``names`` and everything that they are computed from."""
+    need = {a for a in names if isinstance(a, str)}
+    for n in reversed(nodes):
+        if n.name in need:
+            need.update(n.value_args())
+    return need
+
+
 def exact_vectors(names: Sequence[str], items: Sequence[Staged], decay_vec: bool) -> bool:
     """Whether the vectors are plain 16-bit inputs, which tf32 holds exactly."""
     dt = {it.key: it.spec.dt for it in items}
@@ -622,6 +631,13 @@ def emit_scan(p: Problem, s: ScanSpec, C: int, MB: int, use_tma: bool = True, st
     colS, colL, colD, colP = 0, Np, 2 * Np, 3 * Np
     colA = colP
     colG = colP + max(2 * nK, RA)
+    # the row sums that a p depends on (products 2 wait for them), and the others, which only outputs depend on
+    p_need, o_need = row_closure(s.row, s.ps), row_closure(s.row, [o[0] for o in s.outs])
+    first_sums = [d for d in range(nd) if f"sig{d}" in p_need]
+    other_sums = [d for d in range(nd) if d not in first_sums]
+    p_early = not first_sums and colP + 2 * nK + RA + RK <= TMEM_COLS      # p beside products 1, not over them
+    if p_early:
+        colA, colG = colP + 2 * nK, colP + 2 * nK + RA
     late_gram = colG + RK > TMEM_COLS and RA + RK <= 2 * nK
     if late_gram:                     # Gram over p as well: read before p is written, computed once products 2 have read p
         colG = colP + RA
@@ -678,7 +694,7 @@ def emit_scan(p: Problem, s: ScanSpec, C: int, MB: int, use_tma: bool = True, st
         chunk_head()
         for i in range(n0, len(w.lines)):
             w.lines[i] = w.lines[i].replace("{0}", const)
-    pos = (lambda q: f"(nv - 1 - ({q}))") if s.reverse else (lambda q: f"({q})")
+    pos = (lambda q: f"({C - 1 if whole else 'nv - 1'} - ({q}))") if s.reverse else (lambda q: f"({q})")
 
     # ------------------------------------------------------------------ preparing warps
     # registers: 512 threads start with 128 each; the state's rows need more, the others less (state, preparing twice, products:
@@ -752,16 +768,16 @@ def emit_scan(p: Problem, s: ScanSpec, C: int, MB: int, use_tma: bool = True, st
         hsync()
     if dec_sc:
         od = kb.wk[s.decay][1]
-        # thread q: the products of the decays before step q and after it; thread 32 + q of the next warp
-        w.open(f"if (hl < {C} || (hl >= 32 && hl < {32 + C}))")
-        w("const int j = hl & 31;")
-        w(f"float xs[{C}], W = 1.0f;")
+        # lane q: the products of the decays before step q and after it, doubling the steps that a product covers
+        w.open("if (hw == 0)")
+        w("const int j = lane;")
+        ok = " && ".join((["j < " + str(C)] if C < 32 else []) + ([] if whole else ["j < nv"]))
+        x = f"mk[max({pos('j')}, 0) * {mk_row} + {od}]"
+        w("float W = " + (f"({ok}) ? {x} : 1.0f" if ok else x) + ", before = 1.0f, after = 1.0f;")
         w("#pragma unroll")
-        w(f"for (int q = 0; q < {C}; q++) xs[q] = mk[max({pos('q')}, 0) * {mk_row} + {od}];")
-        w("#pragma unroll")
-        w(f"for (int q = 0; q < {C}; q++) if (q < nv && (hl < 32 ? q < j : q > j)) W *= xs[q];")
-        w(f"dec[{o_dec} + (hl < 32 ? 0 : {C}) + j] = W;")
-        w(f"if (hl == {C - 1}) dec[{o_dec + 2 * C}] = nv == {C} ? W * xs[{C - 1}] : W;")
+        w("for (int o = 1; o < 32; o <<= 1) { const float x = frnn_shfl_xor(W, o); if (j & o) before *= x; else after *= x; W *= x; }")
+        w((f"if (j < {C}) " if C < 32 else "") + f"{{ dec[{o_dec} + j] = before; dec[{o_dec + C} + j] = after; }}")
+        w(f"if (j == 0) dec[{o_dec + 2 * C}] = W;")
         w.close()
 
     def steps(names, n, body):
@@ -892,17 +908,23 @@ def emit_scan(p: Problem, s: ScanSpec, C: int, MB: int, use_tma: bool = True, st
             w(f"if (j < nv) frnn_st_raw<float>({s.dg_out}, {dg_off(p, k, f't0 + {pos(chr(106))}')}, z);")
         w.close()
     if dec_sc:
-        w("float W = 1.0f;")
+        # the decays between step j and step i, from the last i to the first; all of them are loaded first: loaded where the running
+        # product wants them, each waited for the one before (4700 of a chunk's 16000 cycles, Gated Delta Rule backward)
         xs = lambda q: f"mk[max({pos(q)}, 0) * {mk_row} + {od}]"
         per = min(KC, C)                 # positions of one vector that a half holds
+        live = lambda i: "" if whole else f" && {i} < nv"
+        w(f"float W = 1.0f, xv[{per}];")
         if per < C:
             w("#pragma unroll")
-            w(f"for (int i = {C - 1}; i >= {per}; i--) if (half == 0 && i < j && i < nv) W *= {xs('i')};")
+            w(f"for (int i = 0; i < {C - per}; i++) xv[i] = {xs(f'({per} + i)')};")
             w("#pragma unroll")
-            w(f"for (int i = {per - 1}; i >= 0; i--) {{ if (i0 + i < j) {{ v[i] *= W; if (i0 + i < nv) W *= {xs('i0 + i')}; }} }}")
-        else:
-            w("#pragma unroll")
-            w(f"for (int i = {C - 1}; i >= 0; i--) {{ if (i < j) {{ " + " ".join(f"v[{x * C} + i] *= W;" for x in range(KC // C)) + f" if (i < nv) W *= {xs('i')}; }} }}")
+            w(f"for (int i = {C - per - 1}; i >= 0; i--) W *= half == 0 && {per} + i < j{live(f'{per} + i')} ? xv[i] : 1.0f;")
+        w("#pragma unroll")
+        w(f"for (int i = 0; i < {per}; i++) xv[i] = {xs('(i0 + i)' if per < C else 'i')};")
+        w("#pragma unroll")
+        at = "i0 + i" if per < C else "i"
+        w(f"for (int i = {per - 1}; i >= 0; i--) {{ const bool in = {at} < j; " + " ".join(f"v[{x * C} + i] *= in ? W : 1.0f;" for x in range(max(1, KC // C)))
+          + f" W *= in{live(at)} ? xv[i] : 1.0f; }}")
     w("#pragma unroll")
     w(f"for (int i = 0; i < {KC}; i++) {{ const int ci = i0 + i; gram[((d * {nr} + ci / {C}) * {C} + ci % {C}) * {GS} + j] = v[i]; }}")
     w.close()
@@ -1132,79 +1154,139 @@ def emit_scan(p: Problem, s: ScanSpec, C: int, MB: int, use_tma: bool = True, st
     w.open(f"for (int c = 0; c < {nchunk}; c++)")
     head("const ")
     w(f"if (!frnn_mbar_wait(&bar[{B_GF} + buf], (c >> 1) & 1, err, {ERR})) return;")
-    w(f"if (!frnn_mbar_wait(&bar[{B_M1}], c & 1, err, {ERR})) return;")
-    w("frnn_tmem_fence_after_sync();")
+
+    def wait_m1():
+        w(f"if (!frnn_mbar_wait(&bar[{B_M1}], c & 1, err, {ERR})) return;")
+        w("frnn_tmem_fence_after_sync();")
+
+    def ld_sums(ds: Sequence[int]):
+        for d in ds:
+            w(f"frnn_tmem_ld<{C}>(mine + {colA + d * C}u, &g[{d * C}]);")
+            if not xa:
+                w(f"frnn_tmem_ld<{C}>(mine + {colA + nA + d * C}u, &lo[{d * C}]);")
+
+    def got_sums(ds: Sequence[int]):
+        w("frnn_tmem_wait_ld();")
+        for d in ds:
+            w("#pragma unroll")
+            v = (lambda k: f"g[{d * C} + {k}]") if xa else (lambda k: f"(g[{d * C} + {k}] + lo[{d * C} + {k}])")
+            f = (lambda k: f"{v(k)} * dec[{o_dec} + {k}]") if dec_sc else v
+            w(f"for (int k = 0; k < {C}; k += 2) g2[({d * C} + k) / 2] = frnn_pk_make({f('k')}, {f('k + 1')});")
+
+    def steps_in_turn(ds: Sequence[int], nodes: Sequence[Node], outs: Sequence[Arg], finish: Callable, midway: Optional[Callable] = None):
+        """Substitution into the row sums ``ds`` (a step's p enter the sums of the later steps) and, step by step, ``nodes``;
+        ``finish(q, value)``.  What step q reads from shared memory is loaded a step ahead."""
+        read = {x for n in nodes for x in n.value_args()} | {o for o in outs if isinstance(o, str)}
+        names = {n.name for n in nodes}
+
+        def val(a: Arg, q: int) -> str:
+            if not isinstance(a, str):
+                return lower.flit(a)
+            if a.startswith("sig") and a in special:
+                return f"g2[{(int(a[3:]) * C + q) // 2}].{'xy'[q % 2]}"
+            return f"{'v' if a in names else 'i'}{q}_" + a.replace(".", "_")
+
+        def load(q: int):
+            for nm in row_in:
+                if nm in read:
+                    cls, o = kb.wk[nm]
+                    tl = pos(str(q)) if whole or not s.reverse else f"max({pos(str(q))}, 0)"
+                    w(f"const float {val(nm, q)} = mk[{tl} * {mk_row} + {o}" + ((f" + min(tid, {MB - 1})" if MB < 128 else " + tid") if cls == M1 else "") + "];")
+            for a in sorted(read):
+                if a.startswith("dg") and a in special:
+                    w(f"const float {val(a, q)} = gram[{o_dg + int(a[2:]) * C + q}];")
+            if q + 1 < C:
+                for d in ds:
+                    for r in range(nr):
+                        j0 = (q + 1) // 4 * 4
+                        w(f"float G{q}_{d}_{r}[{C - j0}];")
+                        for j4 in range(j0, C, 4):
+                            w(f"frnn_ldv<0,4>(gram, {((d * nr + r) * C + q) * GS + j4}, &G{q}_{d}_{r}[{j4 - j0}]);")
+        w.open("")
+        load(0)
+        for q in range(C):
+            if midway and q == C // 2:
+                midway()
+            if q + 1 < C:
+                load(q + 1)
+            for n in nodes:
+                w(f"const float {val(n.name, q)} = {op_expr(n, [val(a, q) for a in n.args])};")
+            finish(q, val)
+            # the next step's sums first, alone where the pair's other one is this step's
+            j0, jp = (q + 1) // 4 * 4, (q + 2) // 2 * 2
+            for d in ds:
+                for r in range(nr):
+                    if jp > q + 1 < C:
+                        w(f"g2[{(d * C + q) // 2}].y = fmaf(ph[{r}][{q}], G{q}_{d}_{r}[{q + 1 - j0}], g2[{(d * C + q) // 2}].y);")
+            if ds and jp < C:
+                w.open("")
+                for r in range(nr):
+                    w(f"const frnn_pk pp{r} = frnn_pk_make(ph[{r}][{q}], ph[{r}][{q}]);")
+                for j in range(jp, C, 2):
+                    for d in ds:
+                        for r in range(nr):
+                            w(f"g2[{(d * C + j) // 2}] = frnn_fma2(pp{r}, frnn_pk_make(G{q}_{d}_{r}[{j - j0}], G{q}_{d}_{r}[{j + 1 - j0}]), g2[{(d * C + j) // 2}]);")
+                w.close()
+        w.close()
     w.open("")
-    w(f"float g[{nA}], ph[{nr}][{C}];")
-    for k in range(len(s.outs)):
-        w(f"float o{k}[{C}];")
-    w.open("")
-    w(f"frnn_tmem_ld<{nA}>(mine + {colA}u, g);")
+    w(f"float g[{nA}], ph[{nr}][{C}]; frnn_pk g2[{nA // 2}];")
     if not xa:
         w(f"float lo[{nA}];")
-        w(f"frnn_tmem_ld<{nA}>(mine + {colA + nA}u, lo);")
-    w("frnn_tmem_wait_ld();")
-    if not xa or dec_sc:
-        w("#pragma unroll")
-        e = "g[k] + lo[k]" if not xa else "g[k]"
-        w(f"for (int k = 0; k < {nA}; k++) g[k] = " + (f"({e}) * dec[{o_dec} + k % {C}];" if dec_sc else f"{e};"))
-    w.close()
-    w("#pragma unroll")
-    w.open(f"for (int q = 0; q < {C}; q++)")
-    w(f"const bool live = {'true' if whole else 'q < nv'}; const int tl = {pos('q')}; (void)live;")
+    if not p_early:
+        wait_m1()
+        ld_sums(first_sums or other_sums)
+        got_sums(first_sums or other_sums)
 
-    def rv(a: Arg) -> str:
-        if not isinstance(a, str):
-            return lower.flit(a)
-        if a.startswith("sig") and a in special:
-            return f"g[{int(a[3:]) * C} + q]"
-        if a.startswith("dg") and a in special:
-            return f"gram[{o_dg + int(a[2:]) * C} + q]"
-        if a in row_names:
-            return lower.vname(a)
-        return "i_" + a.replace(".", "_")
-    for nm in row_in:
-        cls, o = kb.wk[nm]
-        idx = (f"max(tl, 0)" if s.reverse and not whole else "tl") + f" * {mk_row} + {o}"
-        w(f"const float {rv(nm)} = " + (f"mk[{idx} + " + (f"min(tid, {MB - 1})" if MB < 128 else "tid") + "];" if cls == M1 else f"mk[{idx}];"))
-    for n in s.row:
-        w(f"const float {lower.vname(n.name)} = {op_expr(n, [rv(a) for a in n.args])};")
-    for r, nm in enumerate(s.ps):
-        w(f"ph[{r}][q] = " + (f"{rv(nm)};" if whole and MB == 128 else f"(live && row) ? {rv(nm)} : 0.0f;"))
-    for k, o in enumerate(s.outs):
-        w(f"o{k}[q] = {rv(o[0])};")
-    w("#pragma unroll")
-    w.open(f"for (int j4 = 0; j4 < {C}; j4 += 4)")
-    w.open("if (j4 + 3 > q)")
-    for d in range(nd):
-        for r in range(nr):
-            w(f"{{ float x[4]; frnn_ldv<0,4>(gram, ({(d * nr + r) * C} + q) * {GS} + j4, x);")
-            w("#pragma unroll")
-            w(f"for (int k = 0; k < 4; k++) if (j4 + k > q) g[{d * C} + j4 + k] = fmaf(ph[{r}][q], x[k], g[{d * C} + j4 + k]); }}")
-    w.close()
-    w.close()
-    w.close()     # q
+    def put_p(q: int, val):
+        ok = ([] if whole else [f"{q} < nv"]) + ([] if MB == 128 else ["row"])
+        for r, nm in enumerate(s.ps):
+            w(f"ph[{r}][{q}] = " + (f"{' && '.join(ok)} ? {val(nm, q)} : 0.0f;" if ok else f"{val(nm, q)};"))
+    # p first, from the sums that it depends on alone; the sums that only outputs depend on, and the outputs, while products 2 run
+    steps_in_turn(first_sums, [n for n in s.row if n.name in p_need], s.ps, put_p,
+                  (lambda: ld_sums(other_sums)) if first_sums and other_sums else None)
+    if first_sums and other_sums:
+        got_sums(other_sums)           # before p is written over them
     for r in range(nr):
-        if dec_sc:
+        for q in range(0, C, 16):
+            w.open("")
+            w("float x[16];")
             w("#pragma unroll")
-            w(f"for (int q = 0; q < {C}; q++) ph[{r}][q] *= dec[{o_dec + C} + q];")
-        w(f"frnn_tmem_st<{C}>(mine + {colP + r * C}u, ph[{r}]);")
-        w("#pragma unroll")
-        w(f"for (int q = 0; q < {C}; q++) ph[{r}][q] = frnn_tf32_rest(ph[{r}][q]);")
-        w(f"frnn_tmem_st<{C}>(mine + {colP + nK + r * C}u, ph[{r}]);")
+            w(f"for (int k = 0; k < 16; k++) x[k] = ph[{r}][{q} + k]" + (f" * dec[{o_dec + C + q} + k];" if dec_sc else ";"))
+            w(f"frnn_tmem_st<16>(mine + {colP + r * C + q}u, x);")
+            w("#pragma unroll")
+            w("for (int k = 0; k < 16; k++) x[k] = frnn_tf32_rest(x[k]);")
+            w(f"frnn_tmem_st<16>(mine + {colP + nK + r * C + q}u, x);")
+            w.close()
     w("frnn_tmem_wait_st(); frnn_tmem_fence_before_sync();")
-    w(f"frnn_mbar_arrive(&bar[{B_PB}]); frnn_mbar_arrive(&bar[{B_GE} + buf]);")
-    # the outputs leave while products 2 run
-    w.open("if (row)" if MB < 128 else "")
-    w("#pragma unroll")
-    w.open(f"for (int q = 0; q < {C}; q++)")
-    w(f"const int tl = {pos('q')};")
-    w.open("" if whole else "if (q < nv)")
-    for k, (nm, dt, ptr, at, sm) in enumerate(s.outs):
-        w(f"frnn_io<{dt}>::st({ptr}, {at('t0 + tl')} + (long)m * {sm}L, o{k}[q]);")
-    w.close()
-    w.close()
-    w.close()
+    w(f"frnn_mbar_arrive(&bar[{B_PB}]);")
+    if p_early:
+        wait_m1()
+        ld_sums(other_sums)
+        got_sums(other_sums)
+
+    def put_outs(q: int, val):
+        """The outputs of eight steps at a time, so that a chunk cut short costs one branch per eight."""
+        for k, o in enumerate(s.outs):
+            w(f"const float o{q}_{k} = {val(o[0], q)};")
+        if q % 8 < 7:
+            return
+
+        def store(x: int):
+            w(f"{{ const long t = t0 + {pos(str(x))}; " + " ".join(f"frnn_io<{dt}>::st({ptr}, {at('t')} + (long)m * {sm}L, o{x}_{k});"
+                                                                  for k, (nm, dt, ptr, at, sm) in enumerate(s.outs)) + " }")
+        row = "" if MB == 128 else "row"
+        w.open(f"if ({' && '.join(x for x in ('' if whole else f'{q} < nv', row) if x)})" if not whole or row else "")
+        for x in range(q - 7, q + 1):
+            store(x)
+        w.close()
+        if not whole:
+            w.open("else" + (f" if ({row})" if row else ""))
+            for x in range(q - 7, q):
+                w(f"if ({x} < nv)")
+                store(x)
+            w.close()
+    steps_in_turn(other_sums, [n for n in s.row if n.name in o_need], [o[0] for o in s.outs], put_outs)
+    w(f"frnn_mbar_arrive(&bar[{B_GE} + buf]);")
     w.close()
     w(f"if (!frnn_mbar_wait(&bar[{B_M2}], c & 1, err, {ERR})) return;")
     w("frnn_tmem_fence_after_sync();")
