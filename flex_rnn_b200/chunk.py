@@ -538,7 +538,7 @@ def exact_vectors(names: Sequence[str], items: Sequence[Staged], decay_vec: bool
     return not decay_vec and all(dt.get(n) in (lower.DT_BF16, lower.DT_F16) for n in names)
 
 
-def emit_scan(p: Problem, s: ScanSpec, C: int, MB: int, use_tma: bool = True, state_unroll: int = 2) -> KernelSource:
+def emit_scan(p: Problem, s: ScanSpec, C: int, MB: int, use_tma: bool = True, state_unroll: int = 0, compact: bool = False) -> KernelSource:
     """Scan over chunks of ``C`` timesteps; a CTA owns ``MB`` <= 128 rows of one (b, h).
 
     Row m of the state lives in lane m of Tensor Memory (columns: S, then what tf32 truncation leaves out of it), and
@@ -1294,9 +1294,9 @@ def emit_scan(p: Problem, s: ScanSpec, C: int, MB: int, use_tma: bool = True, st
         w(f"const float y = dec[{o_dec + 2 * C}];")
     w("float x[16], u[16];")
     w(f"frnn_tmem_ld<16>(mine + {colS}u, x); frnn_tmem_ld<16>(mine + {colD}u, u);")
-    for qi, (n0, n1) in enumerate(quarters):
-        w(f"#pragma unroll {state_unroll}")
-        w.open(f"for (int n0 = {n0}; n0 < {n1}; n0 += 16)")
+
+    def update_block():
+        """Columns n0.. of the state: decay and products 2, back into Tensor Memory, checkpoint."""
         if dec_vec:
             w("float y[16];")
             w("#pragma unroll")
@@ -1310,8 +1310,23 @@ def emit_scan(p: Problem, s: ScanSpec, C: int, MB: int, use_tma: bool = True, st
         put_state("(kc - 1)" if s.reverse else "(kc + 1)", f" && c + 1 < {nchunk}")
         w("#pragma unroll")
         w("for (int k = 0; k < 16; k++) x[k] = z[k];")
+
+    # one loop of 16 columns, or one per quarter of the state unrolled twice: see ChunkPlan.compact
+    quarter = f"frnn_tmem_wait_st(); frnn_tmem_fence_before_sync(); frnn_mbar_arrive(&bar[{B_SB} + qi]);"
+    if compact:
+        w("int qi = 0;")
+        w(f"#pragma unroll {state_unroll or 1}")
+        w.open(f"for (int n0 = 0; n0 < {Np}; n0 += 16)")
+        update_block()
+        w(f"if (n0 + 16 == {nblk} * (qi + 1) / {len(quarters)} * 16) {{ {quarter} qi++; }}")
         w.close()
-        w(f"frnn_tmem_wait_st(); frnn_tmem_fence_before_sync(); frnn_mbar_arrive(&bar[{B_SB + qi}]);")
+    else:
+        for qi, (n0, n1) in enumerate(quarters):
+            w(f"#pragma unroll {state_unroll or 2}")
+            w.open(f"for (int n0 = {n0}; n0 < {n1}; n0 += 16)")
+            update_block()
+            w.close()
+            w(quarter.replace("qi]", f"{qi}]"))
     w.close()     # chunk loop
     w("frnn_tmem_wait_st();")
     w("#pragma unroll 1")
@@ -2446,10 +2461,20 @@ class ChunkPlan:
     atomic: List[bool]
     C: int = CHUNK                            # timesteps per chunk of the training kernels
     short: bool = True                        # whether calls without gradients are chunked
+    #: The state's update in one rolled loop (10 KB less code) where more than half of the SMs have a CTA.  A scan's code, 60 to 85 KB
+    #: with all its warps' roles, does not fit an SM's instruction cache, and what lies behind that is shared: with every SM
+    #: fetching, less code is faster, with few the unrolled loops are (us, unrolled and rolled: 256 heads T1024 Delta Rule
+    #: 128x128 forward 324 and 284, backward 368 and 348, RWKV-7 650 and 581, 655 and 579, Mamba-2 64x128 295 and 260, 303 and
+    #: 264; 32 heads RWKV-7 64x64 T2048 371 and 400; 16 heads Gated Delta 128x128 T1500 222 and 214, 279 and 280; 15 heads GLA
+    #: 96x80 100 and 98, 103 and 108).
+    compact: bool = False
+
+    def scan(self, spec: ScanSpec, C: int, **kw) -> KernelSource:
+        return emit_scan(self.problem, spec, C, rows_per_cta(self.problem.M), **{"compact": self.compact, **kw})
 
     def forward(self, **kw) -> KernelSource:
         p = self.problem
-        return emit_scan(p, forward_spec(p, self.nf, self.bp.saved, True, self.C), self.C, rows_per_cta(p.M), **kw)
+        return self.scan(forward_spec(p, self.nf, self.bp.saved, True, self.C), self.C, **kw)
 
     def infer(self, **kw) -> KernelSource:
         """Without checkpoints a chunk may be longer, which pays as long as its time less than doubles.  The chain of a chunk
@@ -2461,23 +2486,24 @@ class ChunkPlan:
         p = self.problem
         if len(self.nf.alphas) * len(self.nf.kappas) <= 2 and p.T >= 4 * CHUNK:
             try:
-                ks = emit_scan(p, forward_spec(p, self.nf, [], False, 2 * CHUNK), 2 * CHUNK, rows_per_cta(p.M), **kw)
+                ks = self.scan(forward_spec(p, self.nf, [], False, 2 * CHUNK), 2 * CHUNK, **kw)
                 if ks.smem_bytes <= SMEM_BYTES:
                     return ks
             except lower.LoweringError:
                 pass
-        return emit_scan(p, forward_spec(p, self.nf, [], False, CHUNK), CHUNK, rows_per_cta(p.M), **kw)
+        return self.scan(forward_spec(p, self.nf, [], False, CHUNK), CHUNK, **kw)
 
     def backward_scan(self, **kw) -> KernelSource:
         p = self.problem
-        return emit_scan(p, backward_scan_spec(p, self.nf, self.bp, self.dspec, self.C), self.C, rows_per_cta(p.M), **kw)
+        return self.scan(backward_scan_spec(p, self.nf, self.bp, self.dspec, self.C), self.C, **kw)
 
     def vector_grads(self) -> KernelSource:
         return emit_vector_grads(self.problem, self.nf, self.bp, self.dspec, self.atomic, self.C)
 
     def variants(self) -> List[dict]:
         """Keyword arguments of the scans worth timing; member 0 is the default."""
-        return [dict(state_unroll=2), dict(state_unroll=1), dict(state_unroll=4)]
+        first = 1 if self.compact else 2
+        return [dict(state_unroll=first), dict(state_unroll=3 - first), dict(state_unroll=4)]
 
 
 def _fits(cp: ChunkPlan) -> bool:
@@ -2519,6 +2545,7 @@ def chunk_plan(plan) -> Optional[ChunkPlan]:
     if nf is None or not all(nf_inputs(nf)):
         return None
     cp = ChunkPlan(p, nf, None, [g.spec for g in plan.whole_grads], [g.atomic for g in plan.whole_grads])
+    cp.compact = 2 * p.B * p.H * (p.M // rows_per_cta(p.M)) > plan.n_sm
     try:
         cp.short = (one_wave or p.M > 64) and cp.infer().smem_bytes <= SMEM_BYTES
         if p.M <= 128 and p.M % 8 == 0:

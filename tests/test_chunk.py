@@ -261,3 +261,38 @@ def test_small_decays_gpu(T, M, N, small):
     grads = torch.autograd.grad((y, sT), leaves, (dy.cuda().to(y.dtype), dS.cuda()))
     assert f.forward_func.kernel_status("cuda:0") == 0
     check([y.detach(), sT.detach(), *grads], step, ins, s, dy, dS, torch.bfloat16)
+
+
+# the state's update in one rolled loop: five blocks of 16 columns in four quarters; one block; chunks cut short
+COMPACT = [("delta_rule", 5, 70, 15, 72, 72), ("mamba2", 3, 33, 26, 16, 16), ("rwkv7", 5, 33, 15, 64, 128)]
+
+
+def test_compact_rule_and_emulated():
+    from emu.emu import EmuLauncher
+    for B, H, M, want in [(1, 74, 64, False), (1, 75, 64, True), (1, 37, 256, False), (1, 38, 256, True)]:
+        args = [torch.empty(B, 64, H, *x, dtype=torch.bfloat16, device="meta") for x in ((1, 64), (1, 64), (M, 1), (1, 1))]
+        plan = make_plan(W.delta_rule, args, [torch.empty(B, H, M, 64, dtype=torch.bfloat16, device="meta")])[0]
+        assert chunk.chunk_plan(plan).compact == want
+    for op, T, M, N in [("gated_delta_rule", 40, 24, 72), ("rwkv7", 33, 16, 16)]:
+        step, ins, s, dy, dS = case(op, 1, T, 1, M, N, torch.bfloat16)
+        plan = make_plan(step, ins, [s])[0]
+        plan.n_sm = 1                                     # one head already fills it
+        cp = chunk.chunk_plan(plan)
+        assert cp.compact
+        yf, sf = torch.empty(1, T, 1, M), torch.empty_like(s)
+        err = torch.zeros(1, dtype=torch.int32)
+        EmuLauncher(cp.infer())([t.data_ptr() for t in (*ins, s, yf, sf, err)])
+        ry, rS, _, _ = O.fwd_bwd(step, [x.double() for x in ins], [s.double()], [dy.double()], [dS.double()], dtype=torch.float64)
+        assert int(err) == 0 and O.rel_err(yf, ry[0]) < 2e-6 and O.rel_err(sf, rS[0]) < 2e-6
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("op,B,T,H,M,N", COMPACT)
+def test_compact_gpu(op, B, T, H, M, N):
+    step, ins, s, dy, dS = case(op, B, T, H, M, N, torch.bfloat16)
+    f = flex_rnn_b200.jit(step)
+    leaves = [x.cuda().requires_grad_() for x in [*ins, s]]
+    y, sT = f(*leaves)
+    grads = torch.autograd.grad((y, sT), leaves, (dy.cuda().to(y.dtype), dS.cuda()))
+    assert f.forward_func.kernel_status("cuda:0") == 0 and [k.name for k in f.forward_func.sources] == ["frnn_cfw", "frnn_cbw"]
+    check([y.detach(), sT.detach(), *grads], step, ins, s, dy, dS, torch.bfloat16)
