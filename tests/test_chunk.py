@@ -296,3 +296,32 @@ def test_compact_gpu(op, B, T, H, M, N):
     grads = torch.autograd.grad((y, sT), leaves, (dy.cuda().to(y.dtype), dS.cuda()))
     assert f.forward_func.kernel_status("cuda:0") == 0 and [k.name for k in f.forward_func.sources] == ["frnn_cfw", "frnn_cbw"]
     check([y.detach(), sT.detach(), *grads], step, ins, s, dy, dS, torch.bfloat16)
+
+
+def test_rule_of_long_small_states():
+    for op, T, H, M, N, short, train in [("delta_rule", 255, 149, 64, 64, False, False), ("delta_rule", 256, 149, 64, 64, False, True),
+                                         ("delta_rule", 256, 149, 48, 64, False, False), ("rwkv7", 256, 149, 64, 64, False, False),
+                                         ("mamba2", 256, 149, 64, 128, True, True), ("mamba2", 255, 149, 64, 128, False, True),
+                                         ("rwkv7", 256, 149, 64, 128, False, True), ("delta_rule", 255, 148, 64, 64, True, True)]:
+        step, ins, s, _, _ = case(op, 1, 2, 2, 2, 2, torch.bfloat16)
+        at = lambda x: [1, T if x.shape[1] > 1 else 1, H, M if x.shape[3] > 1 else 1, N if x.shape[4] > 1 else 1]
+        args = [torch.empty(at(x), dtype=torch.bfloat16, device="meta") for x in ins]
+        cp = chunk.chunk_plan(make_plan(step, args, [torch.empty(1, H, M, N, dtype=torch.bfloat16, device="meta")])[0])
+        assert (cp is not None and cp.short, cp is not None and cp.bp is not None) == (short, train), (op, T, H, M, N)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("op,T,M,N,names", [("delta_rule", 257, 64, 64, ["frnn_cfw", "frnn_cbw"]), ("gated_delta_rule", 256, 48, 88, ["frnn_cfw", "frnn_cbw"]),
+                                            ("mamba2", 260, 32, 128, ["frnn_cfw", "frnn_cbw"]), ("gla", 256, 64, 128, ["frnn_cfw", "frnn_cbw"])])
+def test_long_small_states_gpu(op, T, M, N, names):
+    """Training takes the chunked kernels, calls without gradients whichever measured faster; the same results within rounding."""
+    step, ins, s, dy, dS = case(op, 3, T, 50, M, N, torch.bfloat16)
+    f = flex_rnn_b200.jit(step)
+    leaves = [x.cuda().requires_grad_() for x in [*ins, s]]
+    y, sT = f(*leaves)
+    grads = torch.autograd.grad((y, sT), leaves, (dy.cuda().to(y.dtype), dS.cuda()))
+    assert f.forward_func.kernel_status("cuda:0") == 0 and [k.name for k in f.forward_func.sources] == names
+    check([y.detach(), sT.detach(), *grads], step, ins, s, dy, dS, torch.bfloat16)
+    with torch.no_grad():
+        short = f(*leaves)
+    check(short, step, ins, s, dy, dS, torch.bfloat16)
