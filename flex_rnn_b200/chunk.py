@@ -2477,12 +2477,11 @@ class ChunkPlan:
         return self.scan(forward_spec(p, self.nf, self.bp.saved, True, self.C), self.C, **kw)
 
     def infer(self, **kw) -> KernelSource:
-        """Without checkpoints a chunk may be longer, which pays as long as its time less than doubles.  The chain of a chunk
-        takes a part that does not depend on its length (3000 to 7000 cycles, by the state's size) and a substitution of
-        2.4 to 3.8 cycles nd nr C^2.  Measured cycles a chunk with 16 and with 32 steps, one CTA per SM: Delta Rule (two pairs
-        of vectors) 128x128 6260 and 9970, 64x64 4440 and 8630, 32x32 3640 and 7550 (4 % slower); Mamba-2 (one pair) 128x128
-        7380 and 9550, 64x64 6130 and 7730; GLA (one pair) 128x128 7300 and 10510; RWKV-7 (four pairs) 64x64 7500 and
-        19200.  At 64 timesteps, two chunks, 22.0 and 20.0 us for the Delta Rule with 128x128."""
+        """Without checkpoints a chunk may be longer, which pays as long as its time less than doubles: the chain of a chunk takes
+        a part that does not depend on its length and a substitution that grows with nd nr C^2.  64 heads, T1024, us with 16 and
+        with 32 steps: Delta Rule (two pairs of vectors) 128x128 148 and 130, 64x64 111 and 113, 32x32 102 and 98; Gated Delta Rule
+        128x128 177 and 141; Mamba-2 (one pair) 128x128 164 and 116, 64x64 134 and 99; GLA (one pair) 128x128 192 and 162; RWKV-7
+        (four pairs) 64x64 229 and 391.  At 64 timesteps, two chunks, 15.9 and 15.5 us for the Delta Rule with 128x128."""
         p = self.problem
         if len(self.nf.alphas) * len(self.nf.kappas) <= 2 and p.T >= 4 * CHUNK:
             try:
