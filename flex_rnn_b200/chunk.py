@@ -1751,6 +1751,8 @@ def emit_vector_grads(p: Problem, nf: Normal, bp: BackwardPlan, dspec: Sequence[
     cD1, cD2 = 0, RX
     cL = cD2 + RZ
     tm_cols = _tmem_pow2(cL + RZ)
+    if RX > 128:              # L has them as rows: lanes of Tensor Memory
+        raise lower.LoweringError("X and its rests have more rows than a product")
     if tm_cols > 256:
         raise lower.LoweringError("the vector gradients of a chunk do not fit half of Tensor Memory")
     at_rest = lambda inexact, x, n: n + C * inexact.index(x)     # row or column where the rest of vector x begins

@@ -325,3 +325,26 @@ def test_long_small_states_gpu(op, T, M, N, names):
     with torch.no_grad():
         short = f(*leaves)
     check(short, step, ins, s, dy, dS, torch.bfloat16)
+
+
+def many_sums(nd, dt=torch.bfloat16, T=34, M=16, N=32):
+    """``nd`` row sums of the state, whose gradients are no inputs and so have a second tf32 term."""
+    def step(*a):
+        *qs, v, k, S = a
+        return sum((S * q).sum(-1, True) ** 2 for q in qs), S + v * k
+    g = torch.Generator().manual_seed(nd)
+    n = lambda *s: torch.randn(*s, generator=g)
+    rows = [(n(1, T, 1, 1, N) * N ** -0.5).to(dt) for _ in range(nd + 1)]
+    return step, [*rows[:nd], n(1, T, 1, M, 1).to(dt), rows[nd]], 0.1 * n(1, 1, M, N), n(1, T, 1, M), n(1, 1, M, N)
+
+
+# 16 steps of each sum, and as many rests: 4 sums fill the 128 rows of a product, 5 to 7 fitted Tensor Memory
+@pytest.mark.parametrize("nd,name", [(4, "frnn_cfw"), (5, "frnn_fw"), (7, "frnn_fw")])
+def test_row_sums_beyond_a_product_train(nd, name):
+    from emu.emu import EmuLauncher
+    step, ins, s, dy, dS = many_sums(nd)
+    fwd, bwd, _, _ = build_twopass(step, tuple(ins), (s,), _launcher=EmuLauncher)
+    assert fwd.sources[0].name == name
+    y, sT, ck, aux = fwd(tuple(ins), (s,))
+    dx, ds = bwd((dy.to(y.dtype),), (dS,), tuple(ins), (ck,), (aux,))
+    check([y, sT, *dx, *ds], step, ins, s, dy, dS, torch.bfloat16)
