@@ -604,6 +604,8 @@ def emit_scan(p: Problem, s: ScanSpec, C: int, MB: int, use_tma: bool = True, st
     al = lambda x: (x + 127) // 128 * 128
     nA, nK = nd * C, nr * C
     RA, RK = nA * (1 if xa else 2), nK * (1 if xk else 2)
+    if nA > 128:              # Gram has them as rows: lanes of Tensor Memory
+        raise lower.LoweringError("the row sums of a chunk have more rows than a product")
     GS = C + 4
     gram_f = nd * nr * C * GS
     dec_f = Np if dec_vec else (3 * C if dec_sc else 0)        # W_C; or, per head, W_j-1 | W_C/W_i | W_C: three of them, the

@@ -348,3 +348,13 @@ def test_row_sums_beyond_a_product_train(nd, name):
     y, sT, ck, aux = fwd(tuple(ins), (s,))
     dx, ds = bwd((dy.to(y.dtype),), (dS,), tuple(ins), (ck,), (aux,))
     check([y, sT, *dx, *ds], step, ins, s, dy, dS, torch.bfloat16)
+
+
+@pytest.mark.parametrize("nd,name", [(8, "frnn_cfw"), (9, "frnn_fw")])
+def test_row_sums_beyond_a_product_infer(nd, name):
+    """Gram has the row sums of 16 steps as rows: 8 sums fill the 128 of a product.  (Training is refused from 5 on.)"""
+    from emu.emu import EmuLauncher
+    step, ins, s, dy, dS = many_sums(nd)
+    fwd, _, _, _ = build_twopass(step, tuple(ins), (s,), _launcher=EmuLauncher)
+    check([*fwd.infer(tuple(ins), (s,))], step, ins, s, dy, dS, torch.bfloat16)
+    assert fwd.tuned["infer_src"].name == name
