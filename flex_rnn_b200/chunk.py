@@ -1698,6 +1698,9 @@ def emit_vector_grads(p: Problem, nf: Normal, bp: BackwardPlan, dspec: Sequence[
     RX, RZ = nA + C * len(restX), nK + C * len(restZ)        # rows of X and Z: the vectors, then the rests of the inexact ones
     slow_path = bool(nf.decay) and (dec_vec or want_gw)
     few = dec_vec and want_gw and not bp.log_decay
+    # which gradients of single decays are formed by running products; one expression for those who mark them and those who read the
+    # results, so that what is read has been written (a NaN is none of them: its gradient is the quotient, a NaN)
+    by_products = lambda x: f"(fabsf({x}) <= 0.0009765625f)"
     # padding: the eight threads of a store's phase write to different banks
     lboX, lboZ = RX * 16 + 32, RZ * 16 + 32
     lboT, lbo1, lbo2 = 128 * 16, 2 * nA * 16, 2 * nK * 16 + 16
@@ -1713,9 +1716,9 @@ def emit_vector_grads(p: Problem, nf: Normal, bp: BackwardPlan, dspec: Sequence[
             self.part = self.sc + al(len(sc_slots) * C * 4)
             self.z0 = self.part + al(npart * 4 * C * 4)
             self.xr = self.z0 + al(128 * 4)             # what the threads of a column exchange
-            self.few = self.xr + al(2 * 128 * parts * 4)   # columns with a decay too small to divide its gradient by
+            self.few = self.xr + al(2 * 128 * parts * 4)   # per column and part, the steps whose decays are too small to divide by
             # a buffer holds a slice of S_0, E_C and their rests, and of X (as first operand 128 rows of it are read) and Z
-            self.sl = self.few + (512 if few else 0)
+            self.sl = self.few + (al(128 * parts * 2) if few else 0)
             self.lboS = 128 * 16 + 128 // (MS // 4)
             self.sl_bytes = al(MS // 4 * self.lboS)
             self.X = 4 * self.sl_bytes
@@ -1903,8 +1906,7 @@ def emit_vector_grads(p: Problem, nf: Normal, bp: BackwardPlan, dspec: Sequence[
         load_slice(str(u), str(u))
     w("if (tid == 0) { frnn_mbar_init(&bar[0], 1); frnn_mbar_init(&bar[1], 1); frnn_mbar_init(&bar[2], 1); frnn_mbar_init(&bar[5], 1); frnn_mbar_init_fence(); }")
     if few:
-        w(f"int* fewc = (int*)(smem + {lay.few});")
-        w("if (tid < 128) fewc[tid] = 0;")
+        w(f"unsigned short* fewm = (unsigned short*)(smem + {lay.few});")
     w.open("if (warp == 0)")
     w(f"frnn_tmem_alloc((u32*)&bar[3], {tm_cols}u);")
     w("frnn_tmem_fence_before_sync();")
@@ -2127,6 +2129,16 @@ def emit_vector_grads(p: Problem, nf: Normal, bp: BackwardPlan, dspec: Sequence[
         w(f"for (int o = 0; o < {parts}; o++) {{ const float x = xr[o * 128 + x128]; if (o < hf) pre *= x; if (o > hf) post *= x; }}")
         w("rpre = frnn_rcp1(pre);")
         w("float rw = rpre, pw = pre;")
+        if few:
+            # a decay that is merely too small for its own gradient (dW/W, by a division) does not send the chunk down the slow
+            # path, 160 us for a CTA: RWKV-7's decays fall below 2^-10 about once in two million
+            w("u32 marks = 0;")
+            w.open(f"if ({by_products('wlo')})")
+            w("#pragma unroll")
+            w(f"for (int k = 0; k < {HC}; k++) if ({by_products('xw[k]')}) marks |= 1u << k;")
+            w("((volatile int*)&bar[4])[1] = 1;")
+            w.close()
+            w("fewm[tid] = (unsigned short)marks;")
     w("#pragma unroll")
     w.open(f"for (int k4 = 0; k4 < {HC}; k4 += 4)")
     names = nf.kappas + nf.alphas
@@ -2154,10 +2166,6 @@ def emit_vector_grads(p: Problem, nf: Normal, bp: BackwardPlan, dspec: Sequence[
     w.close()
     if dec_vec:
         w("if (!(wlo > 1e-25f && whi < 1e25f)) *(volatile int*)&bar[4] = 1;")
-        if few:
-            # a decay that is merely too small for its own gradient (dW/W, by a division) does not send the chunk down the slow
-            # path, 160 us for a CTA: RWKV-7's decays fall below 2^-10 about once in two million
-            w("if (!(wlo > 0.0009765625f)) { fewc[x128] = 1; ((volatile int*)&bar[4])[1] = 1; }")
     # ---- the parts of the accumulators so far, from S_0 and E_C, scaled to what those from L need
     w("float R = 0.0f; (void)R;")
 
@@ -2302,7 +2310,7 @@ def emit_vector_grads(p: Problem, nf: Normal, bp: BackwardPlan, dspec: Sequence[
         if dec_vec:
             w(f"const float wdw = R - {sel(live_n, f'({kd})')};")
             w(f"R = wdw + {sel(live_n, f'({ad})')};")
-            w(f"const float gw = slow{' || !(fabsf(xw[k]) > 0.0009765625f)' if few else ''} ? {gws} : " + ("wdw;" if bp.log_decay else "frnn_divf(wdw, xw[k]);"))
+            w(f"const float gw = slow{' || ' + by_products('xw[k]') if few else ''} ? {gws} : " + ("wdw;" if bp.log_decay else "frnn_divf(wdw, xw[k]);"))
             st.done["gw"] = "gw"
         else:
             w(f"e{n_nsum - 2}[k] = {sel(live_n, f'(slow ? {gws} : {kd})')}; e{n_nsum - 1}[k] = {sel(live_n, f'({ad})')};")
@@ -2378,7 +2386,7 @@ def emit_slow_columns(w, C, nd, nr, nA, nK, tq, live_n, sel, nf, bp, dec_vec, wa
         w(f"for (int k = 0; k < {cnt}; k++) {arr}[k] = u[k];")
         w.close()
     if few:                                  # (Tensor Memory is read by whole warps)
-        w.open("if (slow || fewc[x128])")
+        w.open("if (slow || fewm[x128] || fewm[128 + x128])")
     names = nf.alphas + nf.kappas + [nf.decay]
     lv = leaves_of(names, (0, 1))
     w("#pragma unroll 1")
@@ -2398,7 +2406,7 @@ def emit_slow_columns(w, C, nd, nr, nA, nK, tq, live_n, sel, nf, bp, dec_vec, wa
         w("#pragma unroll 1")
         w.open(f"for (int j = 0; j < {C}; j++)")
         if few:
-            w("if (!slow && fabsf(xs[j]) > 0.0009765625f) continue;")
+            w(f"if (!slow && !(fewm[j / {C // 2} * 128 + x128] >> (j % {C // 2}) & 1)) continue;")
         w("float A = 1.0f, Bj = 1.0f, g = 0.0f, s0 = 0.0f, Q = 1.0f;")
         w("for (int l = 0; l < j; l++) A *= xs[l];")
         w(f"for (int l = j + 1; l < {C}; l++) Bj *= xs[l];")

@@ -358,3 +358,63 @@ def test_row_sums_beyond_a_product_infer(nd, name):
     fwd, _, _, _ = build_twopass(step, tuple(ins), (s,), _launcher=EmuLauncher)
     check([*fwd.infer(tuple(ins), (s,))], step, ins, s, dy, dS, torch.bfloat16)
     assert fwd.tuned["infer_src"].name == name
+
+
+def output_first(q, w, k, v, S):
+    """The output reads the state before the update: no other term of a decay's gradient depends on the decay."""
+    return (S * q).sum(-1, True), S * w + v * k
+
+
+def bad_decay(op, T, M, N, bad, small):
+    """One decay of one column is ``bad``, another one of that column, in the same chunk, ``small``."""
+    g = torch.Generator().manual_seed(0)
+    n = lambda *s: torch.randn(*s, generator=g)
+    if op == "rwkv7":
+        step, ins, s, dy, dS = case(op, 1, T, 1, M, N, torch.bfloat16)
+    else:
+        step, s, dy, dS = output_first, 0.1 * n(1, 1, M, N), n(1, T, 1, M), n(1, 1, M, N)
+        ins = [(0.2 * n(1, T, 1, 1, N)).bfloat16(), torch.sigmoid(n(1, T, 1, 1, N) + 2).bfloat16(), (0.2 * n(1, T, 1, 1, N)).bfloat16(),
+               n(1, T, 1, M, 1).bfloat16()]
+    ins[1][0, T - 1, 0, 0, 5] = bad
+    if small is not None:
+        ins[1][0, T - 3, 0, 0, 5] = small
+    return step, ins, s, dy, dS
+
+
+def check_bad_decay(got, step, ins, s, dy, dS):
+    """A number only where the oracle has one, and that one; the decays of the other columns all have their gradients."""
+    ry, rS, rgx, rgs = O.fwd_bwd(step, [x.double() for x in ins], [s.double()], [dy.double()], [dS.double()], dtype=torch.float64)
+    for i, (a, b) in enumerate(zip(got, [*ry, *rS, *rgx, *rgs])):
+        a, b = a.cpu().double(), b.double()
+        fin = torch.isfinite(a)
+        assert torch.isfinite(b[fin]).all() and O.rel_err(a[fin], b[fin]) < 1e-2, i
+        if step is output_first and i == 3:
+            assert (~fin).sum() <= a.shape[1], i
+
+
+BAD_DECAYS = [("output_first", 32, 16, 32, float("nan"), None), ("output_first", 34, 16, 40, float("nan"), 2e-4), ("output_first", 37, 24, 128, float("inf"), 0.0),
+              ("output_first", 32, 16, 32, float("inf"), 1e-5), ("output_first", 32, 16, 32, float("nan"), 2.0 ** -10),
+              ("rwkv7", 33, 24, 24, float("nan"), None), ("rwkv7", 33, 24, 24, float("inf"), 2e-4)]
+
+
+@pytest.mark.parametrize("op,T,M,N,bad,small", BAD_DECAYS)
+def test_bad_decay_emulated(op, T, M, N, bad, small):
+    from emu.emu import EmuLauncher
+    step, ins, s, dy, dS = bad_decay(op, T, M, N, bad, small)
+    fwd, bwd, _, _ = build_twopass(step, tuple(ins), (s,), _launcher=EmuLauncher)
+    assert fwd.sources[0].name == "frnn_cfw"
+    y, sT, ck, aux = fwd(tuple(ins), (s,))
+    dx, ds = bwd((dy.to(y.dtype),), (dS,), tuple(ins), (ck,), (aux,))
+    check_bad_decay([y, sT, *dx, *ds], step, ins, s, dy, dS)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("op,T,M,N,bad,small", BAD_DECAYS)
+def test_bad_decay_gpu(op, T, M, N, bad, small):
+    step, ins, s, dy, dS = bad_decay(op, T, M, N, bad, small)
+    f = flex_rnn_b200.jit(step)
+    leaves = [x.cuda().requires_grad_() for x in [*ins, s]]
+    y, sT = f(*leaves)
+    grads = torch.autograd.grad((y, sT), leaves, (dy.cuda().to(y.dtype), dS.cuda()))
+    assert f.forward_func.kernel_status("cuda:0") == 0
+    check_bad_decay([y.detach(), sT.detach(), *grads], step, ins, s, dy, dS)
