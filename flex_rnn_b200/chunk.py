@@ -2517,10 +2517,6 @@ class ChunkPlan:
         return [dict(state_unroll=first), dict(state_unroll=3 - first), dict(state_unroll=4)]
 
 
-#: timesteps from which a chunked kernel's start and end no longer count, see ``chunk_plan``
-LONG = 256
-
-
 def _fits(cp: ChunkPlan) -> bool:
     """Whether the training kernels fit an SM."""
     try:
@@ -2541,13 +2537,12 @@ def chunk_plan(plan) -> Optional[ChunkPlan]:
     backward: 16 heads of 128x128 82 us against 126 us, 128 heads of 64x64 106 us against 146 us), and beyond that for
     large states (256 heads T1024 128x128: 1.65 ms against 2.57 ms; 512 heads of 64x128, T128: 434 against 436 us, Mamba-2
     412 against 485 us; but 512 heads of 64x64 376 against 321 us).  Calls without gradients beyond one CTA per SM also
-    want more than half of Tensor Memory's 128 lanes in use (512 heads of 64x128, Mamba-2: 114 against 94 us), or a long sequence
-    and at most two pairs of vectors (448 heads of 64x128, T256, chunked and recurrent: Delta Rule 143 and 219 us, Mamba-2 133 and
-    209, GLA 160 and 187).  With that, training takes states from 4096 elements on as well (64x64, T256, 160, 512 and 1024
-    heads, forward + backward: Delta Rule 191 and 259, 448 and 477, 835 and 884 us; Mamba-2 205 and 270, 492 and 500, 920 and
-    992; GLA 216 and 290, 531 and 547, 982 and 1003; 512 heads at T128 measure alike, 32x32 is 2 times slower, and RWKV-7, four
-    pairs, 360 and 455, 889 and 862, 1710 and 1553), but not calls without gradients (512 heads: 128 and 122, 119 and 104, 176
-    and 108)."""
+    want more than half of Tensor Memory's 128 lanes in use (512 heads of 64x128, Mamba-2: 114 against 94 us).
+
+    Long calls beyond these lines may be faster chunked (64x64, T256, forward + backward, chunked and recurrent: 160 heads, Delta
+    Rule, 191 and 259 us; 1024 heads 835 and 884), but not as accurate: two tf32 terms in the place of fp32 operands.  Against
+    fp64 at T128, recurrent and chunked, outputs and gradients of the initial state, in 1e-7: GLA 64x64 0.8 and 3.1, 0.5 and 1.3;
+    Delta Rule 64x64 1.7 and 2.5, 2.9 and 1.8, 64x128 1.8 and 2.8, 3.4 and 1.8.  So they stay."""
     p = plan.problem
     if plan.n_st != 1 or p.N % 8 or not 16 <= p.N <= 128 or p.T < 2 * CHUNK or 0 in (p.B, p.T, p.H):
         return None
@@ -2560,19 +2555,15 @@ def chunk_plan(plan) -> Optional[ChunkPlan]:
         if list(s.shape[:3]) != [p.B, p.T, p.H] and not (cls == S11 and s.shape[1] == 1):
             return None
     one_wave = p.B * p.H * (p.M // rows_per_cta(p.M)) <= plan.n_sm
-    if not one_wave and p.M * p.N < (4096 if p.T >= LONG else 8192):
+    if not one_wave and p.M * p.N < 8192:
         return None
     nf = normal_form(plan.g_fw, p.in_names, p.st_names[0], plan.n_out)
     if nf is None or not all(nf_inputs(nf)):
         return None
-    pairs = len(nf.alphas) * len(nf.kappas)
-    small = not one_wave and p.M * p.N < 8192            # (of 4096 elements or more, and long)
-    if small and pairs > 2:
-        return None
     cp = ChunkPlan(p, nf, None, [g.spec for g in plan.whole_grads], [g.atomic for g in plan.whole_grads])
     cp.compact = 2 * p.B * p.H * (p.M // rows_per_cta(p.M)) > plan.n_sm
     try:
-        cp.short = not small and (one_wave or p.M > 64 or (pairs <= 2 and p.T >= LONG)) and cp.infer().smem_bytes <= SMEM_BYTES
+        cp.short = (one_wave or p.M > 64) and cp.infer().smem_bytes <= SMEM_BYTES
         if p.M <= 128 and p.M % 8 == 0:
             v = local_vjp(nf, p.M, p.N)
             cp.bp = backward_plan(p, nf, *v) if v is not None else None
@@ -2580,10 +2571,10 @@ def chunk_plan(plan) -> Optional[ChunkPlan]:
         return None
     if cp.bp is not None:
         # 32 steps per chunk halve the traffic of the chunk boundaries and the chains of the scans, but not the
-        # substitution: for large states and few pairs of vectors (300 heads of 64x64, T512, Delta Rule 565 against 704 us; B8 T1024 H32 128x128, forward + backward: Delta Rule
+        # substitution: for large states and few pairs of vectors (B8 T1024 H32 128x128, forward + backward: Delta Rule
         # 1.66 ms against 1.91 ms, Mamba-2 1.30 ms against 1.67 ms; 32 heads of 64x64, T512: 199 against 224 us; 512 heads of
         # 32x32, T512: 1.18 against 1.05 ms)
-        if pairs <= 2 and p.M * p.N >= (4096 if one_wave or small else 8192) and p.T >= 4 * CHUNK:
+        if len(nf.alphas) * len(nf.kappas) <= 2 and p.M * p.N >= (4096 if one_wave else 8192) and p.T >= 4 * CHUNK:
             cp.C = 2 * CHUNK
             if not _fits(cp):
                 cp.C = CHUNK
