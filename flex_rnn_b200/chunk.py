@@ -1756,10 +1756,13 @@ def emit_vector_grads(p: Problem, nf: Normal, bp: BackwardPlan, dspec: Sequence[
     cD1, cD2 = 0, RX
     cL = cD2 + RZ
     tm_cols = _tmem_pow2(cL + RZ)
+    if 2 * nA + 4 * nK > 256:
+        # with a rest for every vector, whether it has one or not: further rank-1 terms would fit, but a backward that fits only
+        # so makes the outputs of training chunked as well, with two tf32 terms for fp32 (one row sum and four exact terms
+        # with 16x32, outputs against fp64: 1.4e-7 recurrent, 3.2e-7 chunked)
+        raise lower.LoweringError("the vector gradients of a chunk do not fit half of Tensor Memory")
     if RX > 128:              # L has them as rows: lanes of Tensor Memory
         raise lower.LoweringError("X and its rests have more rows than a product")
-    if tm_cols > 256:
-        raise lower.LoweringError("the vector gradients of a chunk do not fit half of Tensor Memory")
     at_rest = lambda inexact, x, n: n + C * inexact.index(x)     # row or column where the rest of vector x begins
     ERR = lower.ERR_STAGE_TIMEOUT
     full_n = N == 128

@@ -422,3 +422,18 @@ def test_bad_decay_gpu(op, T, M, N, bad, small):
     grads = torch.autograd.grad((y, sT), leaves, (dy.cuda().to(y.dtype), dS.cuda()))
     assert f.forward_func.kernel_status("cuda:0") == 0
     check_bad_decay([y.detach(), sT.detach(), *grads], step, ins, s, dy, dS)
+
+
+# rank-1 terms whose p are inputs need no rests, but a step that fits only without them keeps the recurrent backward
+@pytest.mark.parametrize("nd,nr,train", [(1, 3, True), (1, 4, False), (2, 3, True), (2, 4, False), (3, 3, False)])
+def test_rule_of_many_terms(nd, nr, train):
+    def step(*a):
+        qs, vs, ks, S = a[:nd], a[nd:nd + nr], a[nd + nr:-1], a[-1]
+        y = sum((S * q).sum(-1, True) ** 2 for q in qs)
+        for v, k in zip(vs, ks):
+            S = S + v * k
+        return y, S
+    for M, N, T in [(16, 32, 40), (128, 128, 64)]:
+        args = [torch.empty(1, T, 2, *x, dtype=torch.bfloat16, device="meta") for x in [(1, N)] * nd + [(M, 1)] * nr + [(1, N)] * nr]
+        cp = chunk.chunk_plan(make_plan(step, args, [torch.empty(1, 2, M, N, dtype=torch.bfloat16, device="meta")])[0])
+        assert cp.short and (cp.bp is not None) == train, (M, N)
