@@ -523,13 +523,17 @@ class ColumnCode:
         return done
 
 
-def row_closure(nodes: Sequence[Node], names: Sequence[Arg]) -> set:
-    """``names`` and everything that they are computed from."""
+def row_closure(nodes: Sequence[Node], names: Sequence[Arg], made: Sequence[str] = ()) -> set:
+    """``names`` and everything that they are computed from, except what is ``made`` and what only that is computed from."""
     need = {a for a in names if isinstance(a, str)}
     for n in reversed(nodes):
-        if n.name in need:
+        if n.name in need and n.name not in made:
             need.update(n.value_args())
-    return need
+    return need - set(made)
+
+
+#: operations of more than a few instructions
+COSTLY = ("div", "exp", "log", "sqrt", "rsqrt", "reciprocal", "sigmoid", "tanh", "log1p", "expm1", "erf", "pow")
 
 
 def exact_vectors(names: Sequence[str], items: Sequence[Staged], decay_vec: bool) -> bool:
@@ -634,7 +638,15 @@ def emit_scan(p: Problem, s: ScanSpec, C: int, MB: int, use_tma: bool = True, st
     colA = colP
     colG = colP + max(2 * nK, RA)
     # the row sums that a p depends on (products 2 wait for them), and the others, which only outputs depend on
-    p_need, o_need = row_closure(s.row, s.ps), row_closure(s.row, [o[0] for o in s.outs])
+    p_need, out_names = row_closure(s.row, s.ps), [o[0] for o in s.outs]
+    # what the outputs take over from the p instead of computing it again: the p themselves and costly values on the way to them
+    # (64x64, 64 heads, T1024, backward scan, with p computed twice and once: y = (S q)^2 368 and 212 us, two such sums 1347 and 697)
+    made = [nm for nm in s.ps if nm in {n.name for n in s.row}]
+    kept: List[str] = []
+    for n in reversed(s.row):
+        if n.op in COSTLY and n.name in p_need & row_closure(s.row, out_names, made + kept):
+            kept.append(n.name)
+    o_need = row_closure(s.row, out_names, made + kept)
     first_sums = [d for d in range(nd) if f"sig{d}" in p_need]
     other_sums = [d for d in range(nd) if d not in first_sums]
     p_early = not first_sums and colP + 2 * nK + RA + RK <= TMEM_COLS      # p beside products 1, not over them
@@ -1175,15 +1187,18 @@ def emit_scan(p: Problem, s: ScanSpec, C: int, MB: int, use_tma: bool = True, st
             f = (lambda k: f"{v(k)} * dec[{o_dec} + {k}]") if dec_sc else v
             w(f"for (int k = 0; k < {C}; k += 2) g2[({d * C} + k) / 2] = frnn_pk_make({f('k')}, {f('k + 1')});")
 
-    def steps_in_turn(ds: Sequence[int], nodes: Sequence[Node], outs: Sequence[Arg], finish: Callable, midway: Optional[Callable] = None):
+    def steps_in_turn(ds: Sequence[int], nodes: Sequence[Node], outs: Sequence[Arg], finish: Callable, midway: Optional[Callable] = None,
+                      regs: Dict[str, str] = {}):
         """Substitution into the row sums ``ds`` (a step's p enter the sums of the later steps) and, step by step, ``nodes``;
-        ``finish(q, value)``.  What step q reads from shared memory is loaded a step ahead."""
-        read = {x for n in nodes for x in n.value_args()} | {o for o in outs if isinstance(o, str)}
+        ``finish(q, value)``.  What step q reads from shared memory is loaded a step ahead.  ``regs``: values that are in registers."""
+        read = ({x for n in nodes for x in n.value_args()} | {o for o in outs if isinstance(o, str)}) - set(regs)
         names = {n.name for n in nodes}
 
         def val(a: Arg, q: int) -> str:
             if not isinstance(a, str):
                 return lower.flit(a)
+            if a in regs:
+                return f"{regs[a]}[{q}]"
             if a.startswith("sig") and a in special:
                 return f"g2[{(int(a[3:]) * C + q) // 2}].{'xy'[q % 2]}"
             return f"{'v' if a in names else 'i'}{q}_" + a.replace(".", "_")
@@ -1232,6 +1247,8 @@ def emit_scan(p: Problem, s: ScanSpec, C: int, MB: int, use_tma: bool = True, st
         w.close()
     w.open("")
     w(f"float g[{nA}], ph[{nr}][{C}]; frnn_pk g2[{nA // 2}];")
+    for x in range(len(kept)):
+        w(f"float kept{x}[{C}];")
     if not xa:
         w(f"float lo[{nA}];")
     if not p_early:
@@ -1243,6 +1260,8 @@ def emit_scan(p: Problem, s: ScanSpec, C: int, MB: int, use_tma: bool = True, st
         ok = ([] if whole else [f"{q} < nv"]) + ([] if MB == 128 else ["row"])
         for r, nm in enumerate(s.ps):
             w(f"ph[{r}][{q}] = " + (f"{' && '.join(ok)} ? {val(nm, q)} : 0.0f;" if ok else f"{val(nm, q)};"))
+        for x, nm in enumerate(kept):
+            w(f"kept{x}[{q}] = {val(nm, q)};")
     # p first, from the sums that it depends on alone; the sums that only outputs depend on, and the outputs, while products 2 run
     steps_in_turn(first_sums, [n for n in s.row if n.name in p_need], s.ps, put_p,
                   (lambda: ld_sums(other_sums)) if first_sums and other_sums else None)
@@ -1287,7 +1306,9 @@ def emit_scan(p: Problem, s: ScanSpec, C: int, MB: int, use_tma: bool = True, st
                 w(f"if ({x} < nv)")
                 store(x)
             w.close()
-    steps_in_turn(other_sums, [n for n in s.row if n.name in o_need], [o[0] for o in s.outs], put_outs)
+    # (a step or row whose p is 0 instead of its value stores no outputs)
+    regs = {**{nm: f"ph[{r}]" for r, nm in enumerate(s.ps) if nm in made}, **{nm: f"kept{x}" for x, nm in enumerate(kept)}}
+    steps_in_turn(other_sums, [n for n in s.row if n.name in o_need], out_names, put_outs, regs=regs)
     w(f"frnn_mbar_arrive(&bar[{B_GE} + buf]);")
     w.close()
     w(f"if (!frnn_mbar_wait(&bar[{B_M2}], c & 1, err, {ERR})) return;")

@@ -437,3 +437,67 @@ def test_rule_of_many_terms(nd, nr, train):
         args = [torch.empty(1, T, 2, *x, dtype=torch.bfloat16, device="meta") for x in [(1, N)] * nd + [(M, 1)] * nr + [(1, N)] * nr]
         cp = chunk.chunk_plan(make_plan(step, args, [torch.empty(1, 2, M, N, dtype=torch.bfloat16, device="meta")])[0])
         assert cp.short and (cp.bp is not None) == train, (M, N)
+
+
+def tanh_out(q, v, k, S):
+    """The backward's p are made of the forward's tanh, and so are its outputs."""
+    S = S + (v - (S * k).sum(-1, True)) * k
+    return torch.tanh((S * q).sum(-1, True)), S
+
+
+def tanh_p(q, v, k, S):
+    """p is no output, but the output takes the tanh that p is made of."""
+    e = torch.tanh(v - (S * k).sum(-1, True))
+    S = S + (e * v) * k
+    return (S * q).sum(-1, True) + e, S
+
+
+def square_out(q, v, k, S):
+    """p of the backward from the forward's sums, before its own: powf in each step."""
+    S = S + v * k
+    return (S * q).sum(-1, True) ** 2, S
+
+
+def costly_case(step, T, M, N):
+    g = torch.Generator().manual_seed(3)
+    n = lambda *s: torch.randn(*s, generator=g)
+    row = lambda: (n(1, T, 2, 1, N) * N ** -0.5).bfloat16()
+    return [row(), n(1, T, 2, M, 1).bfloat16(), row()], 0.1 * n(1, 2, M, N), n(1, T, 2, M), n(1, 2, M, N)
+
+
+COSTLY = [(tanh_out, "frnn_expf(", 32), (tanh_p, "frnn_expf(", 32), (square_out, "powf(", 32)]
+
+
+@pytest.mark.parametrize("step,call,C", COSTLY)
+def test_costly_values_are_computed_once(step, call, C):
+    """The state warps' code for a chunk holds each step of it: a value that both the p and the outputs are made of is there once."""
+    shapes = [(1, 64), (64, 1), (1, 64)]
+    args = [torch.empty(1, 64, 2, *x, dtype=torch.bfloat16, device="meta") for x in shapes]
+    cp = chunk.chunk_plan(make_plan(step, args, [torch.empty(1, 2, 64, 64, dtype=torch.bfloat16, device="meta")])[0])
+    assert cp.C == C
+    for ks in (cp.forward(), cp.infer(), cp.backward_scan()):
+        assert ks.source[ks.source.index('extern "C"'):].count(call) <= C, ks.name
+
+
+@pytest.mark.parametrize("step,T,M,N", [(tanh_out, 34, 16, 32), (tanh_p, 70, 24, 16), (square_out, 64, 16, 24)])
+def test_costly_values_emulated(step, T, M, N):
+    from emu.emu import EmuLauncher
+    ins, s, dy, dS = costly_case(step, T, M, N)
+    fwd, bwd, _, _ = build_twopass(step, tuple(ins), (s,), _launcher=EmuLauncher)
+    assert fwd.sources[0].name == "frnn_cfw"
+    y, sT, ck, aux = fwd(tuple(ins), (s,))
+    dx, ds = bwd((dy.to(y.dtype),), (dS,), tuple(ins), (ck,), (aux,))
+    check([y, sT, *dx, *ds], step, ins, s, dy, dS, torch.bfloat16)
+    check([*fwd.infer(tuple(ins), (s,))], step, ins, s, dy, dS, torch.bfloat16)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("step,T,M,N", [(tanh_out, 100, 128, 128), (tanh_p, 70, 72, 80), (square_out, 64, 64, 64)])
+def test_costly_values_gpu(step, T, M, N):
+    ins, s, dy, dS = costly_case(step, T, M, N)
+    f = flex_rnn_b200.jit(step)
+    leaves = [x.cuda().requires_grad_() for x in [*ins, s]]
+    y, sT = f(*leaves)
+    grads = torch.autograd.grad((y, sT), leaves, (dy.cuda().to(y.dtype), dS.cuda()))
+    assert f.forward_func.kernel_status("cuda:0") == 0 and f.forward_func.sources[0].name == "frnn_cfw"
+    check([y.detach(), sT.detach(), *grads], step, ins, s, dy, dS, torch.bfloat16)
