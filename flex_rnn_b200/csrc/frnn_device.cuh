@@ -202,11 +202,18 @@ template <int N> FRNN_DEV void frnn_tmem_ld(u32 taddr, float* v) {
 FRNN_DEV bool frnn_mbar_wait(u64* bar, u32 parity, int* err, int code) {
     if (frnn_mbar_try(bar, parity)) return true;
     u64 t0 = frnn_now_ns();
-    // not unrolled: 64 copies were 2 KB of code at every wait, half of a chunked kernel's, and what is beyond the 32 KB of the
-    // instruction cache slows every warp of the SM
+    // Not unrolled: 64 copies were 2 KB of code at every wait, half of a chunked kernel's, and what is beyond the 32 KB of the
+    // instruction cache slows every warp of the SM.  The recurrent backward kernels (up to 13 waits, by warps of several roles) do
+    // define FRNN_UNROLLED_WAITS: rolled and unrolled, us, Mamba 128x16 of 320 heads T360 839 and 699 (in some processes, 700 in others), RWKV-7
+    // 128x48 of 416 heads T237 601 and 583, Delta Rule 256x128 of 16 heads T400 178 and 183, geometric mean over 29 calls 1.004.
+    // Forward kernels have one wait: 0.989 over 49 calls (Delta Rule 64x64 of 256 heads T300 81 and 96, HGRN 7 x 1728 T567 32.4 and 31.8).
+#ifndef FRNN_UNROLLED_WAITS
 #pragma unroll 1
+#endif
     for (;;) {
+#ifndef FRNN_UNROLLED_WAITS
 #pragma unroll 1
+#endif
         for (int i = 0; i < 64; i++)
             if (frnn_mbar_try(bar, parity)) return true;
         if (frnn_now_ns() - t0 > FRNN_WAIT_LIMIT_NS) {

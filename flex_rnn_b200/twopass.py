@@ -703,7 +703,8 @@ def generate_backward(plan: Plan, tile: Optional[lower.Tile] = None,
             k //= 2
     for kf, nb in cands:
         bw = emit_backward(p, plan.g_re, plan.g_bw, plan.aux, plan.n_out, plan.grads, plan.dy_names,   # type: ignore[attr-defined]
-                           plan.dnext_names, tile or plan.bw_tile, sg, tu.nslots, tu.use_tma, prelude(),  # type: ignore[attr-defined]
+                           plan.dnext_names, tile or plan.bw_tile, sg, tu.nslots, tu.use_tma,  # type: ignore[attr-defined]
+                           "#define FRNN_UNROLLED_WAITS\n" + prelude(),           # see frnn_mbar_wait
                            kflush=kf, ring_bufs=nb, reverse=plan.reverse, step_unroll=tu.bw_unroll,
                            min_blocks=max(1, tu.bw_min_blocks), pack2=pack2, col_major=bool(tu.col_major),
                            helper_warps=tu.bw_helper, max_acc=tu.bw_acc, tmem_slots=tu.bw_tmem_slots,

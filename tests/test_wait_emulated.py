@@ -57,3 +57,14 @@ def test_some_threads_time_out(name, bar, nth):
         p.join()
     assert not stranded, f"threads are stranded after a wait on barrier {bar} ran out in others"
     assert p.exitcode == 0 and out.get() == ERR_STAGE_TIMEOUT
+
+
+def test_which_kernels_unroll_their_waits():
+    """The recurrent backward only (its kernels measured slower with rolled waits, the others faster)."""
+    from flex_rnn_b200 import chunk
+    from flex_rnn_b200.twopass import generate, make_plan
+    *ins, s = W.synthetic("delta_rule", 1, 64, 1, 64, 32, torch.bfloat16)[0]
+    plan = make_plan(W.delta_rule, ins, (s,))[0]
+    cp = chunk.chunk_plan(plan)
+    for ks in (*generate(plan), cp.forward(), cp.infer(), cp.backward_scan(), cp.vector_grads()):
+        assert ("#define FRNN_UNROLLED_WAITS" in ks.source) == (ks.name == "frnn_bw"), ks.name
