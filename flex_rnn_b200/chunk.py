@@ -1728,18 +1728,21 @@ def emit_vector_grads(p: Problem, nf: Normal, bp: BackwardPlan, dspec: Sequence[
     LS = nK + 1
     kT_b, aT_b = nK // 4 * lboT, nA // 4 * lboT
 
-    class Layout:
-        """Shared memory with slices of ``MS`` rows in ``NB`` buffers and ``parts`` x 128 threads."""
+    NT = 256                                 # 128 rows or columns times two halves of the chunk's timesteps
+    HC = C // 2                              # timesteps of one thread
 
-        def __init__(self, MS: int, NB: int, parts: int):
-            self.MS, self.NB, self.parts = MS, NB, parts
+    class Layout:
+        """Shared memory with slices of ``MS`` rows in ``NB`` buffers."""
+
+        def __init__(self, MS: int, NB: int):
+            self.MS, self.NB = MS, NB
             self.sc = 256
             self.part = self.sc + al(len(sc_slots) * C * 4)
             self.z0 = self.part + al(npart * 4 * C * 4)
             self.xr = self.z0 + al(128 * 4)             # what the threads of a column exchange
-            self.few = self.xr + al(2 * 128 * parts * 4)   # per column and part, the steps whose decays are too small to divide by
+            self.few = self.xr + al(2 * NT * 4)         # per column and half, the steps whose decays are too small to divide by
             # a buffer holds a slice of S_0, E_C and their rests, and of X (as first operand 128 rows of it are read) and Z
-            self.sl = self.few + (al(128 * parts * 2) if few else 0)
+            self.sl = self.few + (al(NT * 2) if few else 0)
             self.lboS = 128 * 16 + 128 // (MS // 4)
             self.sl_bytes = al(MS // 4 * self.lboS)
             self.X = 4 * self.sl_bytes
@@ -1763,14 +1766,12 @@ def emit_vector_grads(p: Problem, nf: Normal, bp: BackwardPlan, dspec: Sequence[
     # us, two buffers, one, and one CTA of 512 threads with two: Delta Rule 128x128 493, 519, 508; RWKV-7 988, 1019, 1322; Mamba-2
     # 64x128 441, 441, 457)
     for NB in (2, 1):
-        lay = Layout(16 if M % 16 == 0 else 8, NB, 2)
+        lay = Layout(16 if M % 16 == 0 else 8, NB)
         if lay.ctas == 2:
             break
-    MS, NB, parts, ctas = lay.MS, lay.NB, lay.parts, lay.ctas
+    MS, NB, ctas = lay.MS, lay.NB, lay.ctas
     DP = 2                                   # slices that are loaded ahead
     nsl = M // MS
-    NT = 128 * parts                         # 128 rows or columns times ``parts`` parts of the chunk's timesteps
-    HC = C // parts                          # timesteps of one thread
     lboS, sl_bytes, smem_bytes = lay.lboS, lay.sl_bytes, lay.bytes
     off_sc, off_part, off_z0, off_xr, off_sl = lay.sc, lay.part, lay.z0, lay.xr, lay.sl
     off_kT, off_aT, off_L1, off_L2, off_Lr, off_slow, off_gw = lay.kT, lay.aT, lay.L1, lay.L2, lay.Lr, lay.slow, lay.gw
@@ -2146,11 +2147,11 @@ def emit_vector_grads(p: Problem, nf: Normal, bp: BackwardPlan, dspec: Sequence[
         w.close()
         w("prod *= xw[k];")
         w.close()
-        # the products of the other parts' decays come through shared memory
+        # the product of the other half's decays comes through shared memory
         w("xr[tid] = prod;")
         w("frnn_block_sync();")
         w("#pragma unroll")
-        w(f"for (int o = 0; o < {parts}; o++) {{ const float x = xr[o * 128 + x128]; if (o < hf) pre *= x; if (o > hf) post *= x; }}")
+        w("for (int o = 0; o < 2; o++) { const float x = xr[o * 128 + x128]; if (o < hf) pre *= x; if (o > hf) post *= x; }")
         w("rpre = frnn_rcp1(pre);")
         w("float rw = rpre, pw = pre;")
         if few:
@@ -2303,7 +2304,7 @@ def emit_vector_grads(p: Problem, nf: Normal, bp: BackwardPlan, dspec: Sequence[
         w.close()
         w.close()
     if dec_vec and want_gw:
-        # the later parts' share of the sums that lead from R_C to the earlier ones
+        # the later half's share of the sums that lead from R_C to the earlier one
         w("float P = 0.0f;")
         w("#pragma unroll")
         w.open(f"for (int k = 0; k < {HC}; k++)")
@@ -2317,7 +2318,7 @@ def emit_vector_grads(p: Problem, nf: Normal, bp: BackwardPlan, dspec: Sequence[
         w("frnn_block_sync();")
         w("R = 0.0f;")
         w("#pragma unroll")
-        w(f"for (int o = 0; o < {parts}; o++) R += xr[o * 128 + x128] + (o > hf ? xr[{NT} + o * 128 + x128] : 0.0f);")
+        w(f"for (int o = 0; o < 2; o++) R += xr[o * 128 + x128] + (o > hf ? xr[{NT} + o * 128 + x128] : 0.0f);")
     for x in range(n_nsum):
         w(f"float e{x}[{HC}];")
     w("#pragma unroll")
