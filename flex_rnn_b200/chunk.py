@@ -1769,6 +1769,11 @@ def emit_vector_grads(p: Problem, nf: Normal, bp: BackwardPlan, dspec: Sequence[
         lay = Layout(16 if M % 16 == 0 else 8, NB)
         if lay.ctas == 2:
             break
+    else:
+        # one CTA per SM, which then has two buffers as well (steps with a decay per column and several sums; 64x64, 64 heads, T1024, us, one
+        # buffer and two: two sums 197 and 190, four 344 and 331, four and two terms 383 and 368)
+        two = Layout(lay.MS, 2)
+        lay = two if two.bytes <= SMEM_BYTES else lay
     MS, NB, ctas = lay.MS, lay.NB, lay.ctas
     DP = 2                                   # slices that are loaded ahead
     nsl = M // MS

@@ -501,3 +501,42 @@ def test_costly_values_gpu(step, T, M, N):
     grads = torch.autograd.grad((y, sT), leaves, (dy.cuda().to(y.dtype), dS.cuda()))
     assert f.forward_func.kernel_status("cuda:0") == 0 and f.forward_func.sources[0].name == "frnn_cfw"
     check([y.detach(), sT.detach(), *grads], step, ins, s, dy, dS, torch.bfloat16)
+
+
+def sums_and_decay(q0, q1, q2, q3, v, k, w, S):
+    """Four row sums beside a decay per column: the second phase of the vector gradients leaves room for one CTA per SM."""
+    S = S * w + v * k
+    return sum((S * q).sum(-1, True) ** 2 for q in (q0, q1, q2, q3)), S
+
+
+def sums_and_decay_case(T, M, N):
+    g = torch.Generator().manual_seed(4)
+    n = lambda *s: torch.randn(*s, generator=g)
+    row = lambda: (n(1, T, 2, 1, N) * N ** -0.5).bfloat16()
+    ins = [row(), row(), row(), row(), n(1, T, 2, M, 1).bfloat16(), row(), torch.sigmoid(n(1, T, 2, 1, N) + 2).bfloat16()]
+    return ins, 0.1 * n(1, 2, M, N), n(1, T, 2, M), n(1, 2, M, N)
+
+
+# two slices of 16 rows in two buffers; three slices of 8 rows and a chunk cut short
+@pytest.mark.parametrize("T,M,N", [(32, 32, 16), (37, 24, 32)])
+def test_vector_gradients_with_one_cta_per_sm_emulated(T, M, N):
+    from emu.emu import EmuLauncher
+    ins, s, dy, dS = sums_and_decay_case(T, M, N)
+    ks = chunk.chunk_plan(make_plan(sums_and_decay, ins, [s])[0]).vector_grads()
+    assert "__launch_bounds__(256, 1)" in ks.source and "s < 2 || frnn_mbar_wait" in ks.source and ks.smem_bytes <= chunk.SMEM_BYTES
+    fwd, bwd, _, _ = build_twopass(sums_and_decay, tuple(ins), (s,), _launcher=EmuLauncher)
+    y, sT, ck, aux = fwd(tuple(ins), (s,))
+    dx, ds = bwd((dy.to(y.dtype),), (dS,), tuple(ins), (ck,), (aux,))
+    check([y, sT, *dx, *ds], sums_and_decay, ins, s, dy, dS, torch.bfloat16)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("T,M,N", [(100, 64, 64), (37, 24, 32)])
+def test_vector_gradients_with_one_cta_per_sm_gpu(T, M, N):
+    ins, s, dy, dS = sums_and_decay_case(T, M, N)
+    f = flex_rnn_b200.jit(sums_and_decay)
+    leaves = [x.cuda().requires_grad_() for x in [*ins, s]]
+    y, sT = f(*leaves)
+    grads = torch.autograd.grad((y, sT), leaves, (dy.cuda().to(y.dtype), dS.cuda()))
+    assert f.forward_func.kernel_status("cuda:0") == 0 and f.forward_func.sources[0].name == "frnn_cfw"
+    check([y.detach(), sT.detach(), *grads], sums_and_decay, ins, s, dy, dS, torch.bfloat16)
