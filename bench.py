@@ -659,8 +659,9 @@ def run_ours(args, rank, world, local):
                                            "gradients and dS0 written)",
                          "algorithmic_bytes": extra["bytes_bw_alg"],
                          "peak_source": (f"measured in this run by the FMA probe kernel ({bench.sms} SMs); " if extra["bound"] == "fp32" else
-                                         "busy cycles of the tensor cores: 46 per product of 128x8 with up to 64 columns, 65 with 128 "
-                                         "(measured); " if extra["bound"] == "tensor" else "") + f"HBM copy peak {bench.hbm} GB/s "
+                                         "busy cycles of the tensor cores, per product of 128x8 with n columns: max(10, n / 2), with its first "
+                                         "operand in shared memory max(39.5, n / 2, 32 + n / 4) (measured); "
+                                         if extra["bound"] == "tensor" else "") + f"HBM copy peak {bench.hbm} GB/s "
                                         + ("of measured" if bench.peaks else "of fallback"),
                          "flops_per_launch": extra["flops_bw"], "k_joint": rec["k_joint"], "k_fwd": rec["k_fwd"],
                          "hbm_bound_ms": rec["hbm_bound_ms"], "fp32_bound_ms": rec["fp32_bound_ms"],

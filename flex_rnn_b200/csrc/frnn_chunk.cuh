@@ -32,9 +32,8 @@ FRNN_DEV void frnn_mma_ss_d(u32 d, u64 a, u64 b, u32 idesc, bool accumulate) {
 FRNN_DEV void frnn_mma_commit(u64* bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(frnn_smem_addr(bar)) : "memory");
 }
-// One thread of a whole warp, the same in every call.  The products are issued inside `if (frnn_elect())`: the compiler knows
-// from elect.sync that one thread runs there and keeps descriptors and addresses in uniform registers; inside `if (lane == 0)`
-// it moves them there for every product, one lane at a time, which takes 45 cycles whatever the product's width.
+// One thread of a whole warp, the same in every call.  The products are issued inside `if (frnn_elect())`: measured, a product
+// takes the cycles given at the top there, and 45, whatever its width, inside `if (lane == 0)` (why was not established).
 FRNN_DEV bool frnn_elect() {
     u32 r;
     asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(r));
