@@ -2563,11 +2563,12 @@ def chunk_plan(plan) -> Optional[ChunkPlan]:
     CTA.  The inputs have 16 bits; for fp32 inputs the recurrent kernels stay, whose sums are fp32 throughout.
 
     A chunk costs a CTA the same chain whatever the state's size, and only one CTA fits an SM; the recurrent kernels' time
-    grows with the state and they share an SM.  So: where every SM has at most one CTA (T128 Delta Rule, forward +
-    backward: 16 heads of 128x128 82 us against 126 us, 128 heads of 64x64 106 us against 146 us), and beyond that for
-    large states (256 heads T1024 128x128: 1.65 ms against 2.57 ms; 512 heads of 64x128, T128: 434 against 436 us, Mamba-2
-    412 against 485 us; but 512 heads of 64x64 376 against 321 us).  Calls without gradients beyond one CTA per SM also
-    want more than half of Tensor Memory's 128 lanes in use (512 heads of 64x128, Mamba-2: 114 against 94 us).
+    grows with the state and they share an SM.  So, in kernel time, forward + backward: where every SM has at most one CTA (T128
+    Delta Rule: 16 heads of 128x128 62 us against 100 us, 128 heads of 64x64 67 us against 91 us), and beyond that for
+    large states (256 heads T1024 128x128: 1.12 ms against 2.56 ms; 512 heads of 64x128, T128: 288 against 353 us, Mamba-2
+    293 against 432 us; but with the kernels before their last rework 512 heads of 64x64 376 against 321 us).  Calls without
+    gradients beyond one CTA per SM also want more than half of Tensor Memory's 128 lanes in use (512 heads of 64x128, Mamba-2,
+    before that rework: 114 against 94 us).
 
     Long calls beyond these lines may be faster chunked (64x64, T256, forward + backward, chunked and recurrent: 160 heads, Delta
     Rule, 191 and 259 us; 1024 heads 835 and 884), but not as accurate: two tf32 terms in the place of fp32 operands.  Against
@@ -2601,9 +2602,9 @@ def chunk_plan(plan) -> Optional[ChunkPlan]:
         return None
     if cp.bp is not None:
         # 32 steps per chunk halve the traffic of the chunk boundaries and the chains of the scans, but not the
-        # substitution: for large states and few pairs of vectors (B8 T1024 H32 128x128, forward + backward: Delta Rule
-        # 1.66 ms against 1.91 ms, Mamba-2 1.30 ms against 1.67 ms; 32 heads of 64x64, T512: 199 against 224 us; 512 heads of
-        # 32x32, T512: 1.18 against 1.05 ms)
+        # substitution: for large states and few pairs of vectors (kernels, forward + backward: B8 T1024 H32 128x128 Delta Rule
+        # 1.12 ms against 1.54 ms, Mamba-2 1.16 ms against 1.73 ms, 64x128 0.96 against 1.32; 64x64, T512, 32 heads 147 against 166
+        # us, 140 heads 251 against 277; 140 heads of 32x32 202 both)
         if len(nf.alphas) * len(nf.kappas) <= 2 and p.M * p.N >= (4096 if one_wave else 8192) and p.T >= 4 * CHUNK:
             cp.C = 2 * CHUNK
             if not _fits(cp):
